@@ -45,9 +45,11 @@ void moe_router_topk(const float* logits, const int* replay_ids, int* topk_ids, 
 // to a multiple of `align`; outputs: dest_row[T*K], row_src[max_rows] (-1 for padding), expert_offsets[E+1]
 // (padded), tile_group[max_tiles][4] = {expert, row0, rows, 0}, num_m_tiles[2] = {tiles, live rows},
 // expert_counts[E].
+// ints of scratch that moe_build_permutation needs for these sizes
+long long moe_permutation_scratch(int T, int K, int max_rows, int E);
 void moe_build_permutation(const int* topk_ids, int T, int K, int E, int max_rows, int max_tiles, int align,
                            int* expert_counts, int* expert_offsets, int* dest_row, int* row_src, int* tile_group,
-                           int* num_m_tiles, cudaStream_t s);
+                           int* num_m_tiles, int* scratch, cudaStream_t s);
 void moe_permute(const void* x, const int* row_src, const int* num_m_tiles, void* x_perm, int max_rows, int H, int K,
                  cudaStream_t s);
 // out[t] = (residual[t] +) sum_k w[t,k] * y_perm[dest_row[t,k]]

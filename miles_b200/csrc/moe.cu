@@ -178,219 +178,277 @@ __global__ void router_bwd_kernel(const float* __restrict__ probs, const int* __
 }
 
 // ---------------------------------------------------------------- permutation
-// Pass 1: one CTA per expert counts its entries.
-__global__ void count_kernel(const int* __restrict__ ids, int n, int* __restrict__ counts) {
-  __shared__ int red[32];
-  const int e = blockIdx.x;
-  int c = 0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) c += (ids[i] == e);
+// A stable counting sort of the n = T * K entries by expert. The entries are dealt to warps in contiguous runs; a warp
+// walks over its run 32 entries at a time, and the lanes that hold the same expert find one another with a match
+// instruction, so an entry's rank among the warp's earlier entries of its expert costs one shared-memory read. The
+// ranks become rows once every warp's counts are summed over the warps (and blocks) before it. What bounds it is latency:
+// 131072 ids are half a megabyte. (One block per expert that reads every id, which this replaced, read them 2 E times:
+// 131072 entries over 128 experts took 282 us in three kernels, these take 20 us; 128 entries 10.7 us, now 3.2 us.)
+constexpr int SORT_ROUNDS = 16;  // entries per lane and warp at most
+constexpr int SORT_WARPS = 4;    // warps per block of the many-block variant: their counts fit shared memory up to 14000 experts
+
+// One warp: `rank[r]` of entry first + 32 r + lane among the warp's entries of the same expert, the warp's counts in
+// `hist` (shared memory, zeroed by the caller). Ids outside [0, E) get no rank. The last entry is `last` - 1.
+template <int ROUNDS>
+__device__ __forceinline__ void warp_ranks(const int* __restrict__ ids, int first, int last, int E, int* hist, int (&id)[ROUNDS],
+                                           int (&rank)[ROUNDS]) {
+  const int lane = threadIdx.x & 31;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = c;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    int v = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0;
+  for (int r = 0; r < ROUNDS; ++r) {
+    const int i = first + 32 * r + lane;
+    const int e = i < last ? ids[i] : -1;
+    id[r] = (e >= 0 && e < E) ? e : -1;
+  }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (threadIdx.x == 0) counts[e] = v;
+  for (int r = 0; r < ROUNDS; ++r) {
+    rank[r] = 0;
+    if (first + 32 * r >= last) continue;  // warp-uniform
+    const unsigned same = __match_any_sync(0xffffffffu, id[r]);
+    const unsigned below = same & ((1u << lane) - 1u);
+    const int before = id[r] >= 0 ? hist[id[r]] : 0;
+    rank[r] = before + __popc(below);
+    __syncwarp();
+    if (id[r] >= 0 && below == 0) hist[id[r]] = before + __popc(same);
+    __syncwarp();
   }
 }
 
-// Pass 2: single CTA: exclusive scan of the per-expert row counts padded to `align`, the list of GEMM row
-// tiles (expert, first row, rows to compute; a tile never straddles experts and is at most 128 rows), the
-// number of tiles and the number of live rows. tiles[t] = {expert, row0, rows, 0}; totals = {num tiles, live rows}.
-__global__ void scan_kernel(const int* __restrict__ counts, int E, int max_rows, int max_tiles, int align,
-                            int* __restrict__ offsets, int* __restrict__ tiles, int* __restrict__ totals) {
-  extern __shared__ int tile_start[];  // [E+1]
-  if (threadIdx.x == 0) {
-    int off = 0, t = 0;
-    for (int e = 0; e < E; ++e) {
-      offsets[e] = off;
-      tile_start[e] = t;
-      int padded = ((counts[e] + align - 1) / align) * align;
-      if (off + padded > max_rows) padded = max_rows - off > 0 ? ((max_rows - off) / align) * align : 0;
-      off += padded;
-      t += (padded + 127) / 128;
-    }
-    offsets[E] = off;
-    tile_start[E] = t < max_tiles ? t : max_tiles;
-    totals[0] = tile_start[E];
-    totals[1] = off;
+// One warp: exclusive scans over the experts. First the row offsets, every expert's rows padded to `align` and clamped to
+// the capacity (offsets are multiples of `align`, so clamping both ends of an expert's range equals shrinking the expert
+// that overflows and giving the later ones nothing), then the starts of the 128-row tiles of the clamped ranges; lane l
+// owns experts [l*per, (l+1)*per). off[0..E], tstart[0..E]; totals = {number of tiles, live rows}.
+__device__ __forceinline__ void scan_experts(const int* cnt, int E, int max_rows, int max_tiles, int align, int* off, int* tstart,
+                                             int* __restrict__ totals) {
+  const int lane = threadIdx.x & 31;
+  const int per = (E + 31) / 32;
+  const int e0 = min(E, lane * per), e1 = min(E, e0 + per);
+  const int cap = (max_rows / align) * align;
+  int local = 0;
+  for (int e = e0; e < e1; ++e) local += ((cnt[e] + align - 1) / align) * align;
+  int incl = local;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
   }
-  __syncthreads();
-  for (int e = 0; e < E; ++e) {
-    const int rows_e = offsets[e + 1] - offsets[e];
-    for (int j = threadIdx.x; tile_start[e] + j < tile_start[e + 1] && tile_start[e] + j < max_tiles; j += blockDim.x) {
-      int* t = tiles + 4 * (tile_start[e] + j);
-      t[0] = e;
-      t[1] = offsets[e] + 128 * j;
-      t[2] = min(128, rows_e - 128 * j);
-      t[3] = 0;
-    }
+  int run = incl - local;
+  int tl = 0;
+  for (int e = e0; e < e1; ++e) {
+    const int s0 = min(run, cap);
+    run += ((cnt[e] + align - 1) / align) * align;
+    const int s1 = min(run, cap);
+    off[e] = s0;
+    tl += (s1 - s0 + 127) / 128;
+    tstart[e] = s1 - s0;  // rows of the expert for now; turned into a tile start below
   }
-}
-
-// Pass 3: one CTA per expert assigns stable ranks (ascending entry index) to its entries.
-__global__ void assign_kernel(const int* __restrict__ ids, int n, const int* __restrict__ offsets,
-                              int* __restrict__ dest_row, int* __restrict__ row_src) {
-  __shared__ int warp_tot[32];
-  __shared__ int base_s;
-  const int e = blockIdx.x;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  if (threadIdx.x == 0) base_s = 0;
-  __syncthreads();
-  const int cap = offsets[e + 1] - offsets[e];
-  for (int start = 0; start < n; start += blockDim.x) {
-    const int i = start + threadIdx.x;
-    const bool hit = i < n && ids[i] == e;
-    const unsigned m = __ballot_sync(0xffffffffu, hit);
-    const int in_warp = __popc(m & ((1u << lane) - 1u));
-    if (lane == 0) warp_tot[w] = __popc(m);
-    __syncthreads();
-    int before = 0;
-    for (int j = 0; j < w; ++j) before += warp_tot[j];
-    const int rank = base_s + before + in_warp;
-    if (hit) {
-      if (rank < cap) {
-        dest_row[i] = offsets[e] + rank;
-        row_src[offsets[e] + rank] = i;
-      } else {
-        dest_row[i] = -1;  // capacity overflow: dropped (only if max_rows was under-provisioned)
-      }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int tot = 0;
-      for (int j = 0; j < nw; ++j) tot += warp_tot[j];
-      base_s += tot;
-    }
-    __syncthreads();
+  const int total_rows = min(__shfl_sync(0xffffffffu, incl, 31), cap);
+  int tincl = tl;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, tincl, o);
+    if (lane >= o) tincl += v;
+  }
+  int trun = tincl - tl;
+  for (int e = e0; e < e1; ++e) {
+    const int rows = tstart[e];
+    tstart[e] = trun;
+    trun += (rows + 127) / 128;
+  }
+  const int total_tiles = __shfl_sync(0xffffffffu, tincl, 31);
+  if (lane == 0) {
+    off[E] = total_rows;
+    tstart[E] = total_tiles < max_tiles ? total_tiles : max_tiles;
+    totals[0] = tstart[E];
+    totals[1] = total_rows;
   }
 }
 
-// Single-CTA variant for small problems (decode steps): counts, scan, tile list and the stable assignment
-// in one launch. Also initialises row_src / dest_row, so the caller needs no memset or fill kernels.
-__global__ void __launch_bounds__(1024)
+// The tile list: tile t of an expert covers its rows 128 j .. 128 j + 127; tiles[t] = {expert, first row, rows, 0}.
+__device__ __forceinline__ void write_tiles(const int* off, const int* tstart, int E, int max_tiles, int* __restrict__ tiles) {
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+    const int rows_e = off[e + 1] - off[e];
+    for (int j = 0; tstart[e] + j < tstart[e + 1] && tstart[e] + j < max_tiles; ++j)
+      reinterpret_cast<int4*>(tiles)[tstart[e] + j] = make_int4(e, off[e] + 128 * j, min(128, rows_e - 128 * j), 0);
+  }
+}
+
+// Small problems (decode steps) in one block: ranks, scans, tile list and rows, with nothing to initialise beforehand.
+template <int ROUNDS>
+__global__ void __launch_bounds__(512)
 build_small_kernel(const int* __restrict__ ids, int n, int E, int max_rows, int max_tiles, int align,
                    int* __restrict__ counts_out, int* __restrict__ offsets, int* __restrict__ dest_row,
                    int* __restrict__ row_src, int* __restrict__ tiles, int* __restrict__ totals) {
-  extern __shared__ int sm[];  // counts[E], off[E+1], tile_start[E+1], ids[n]
+  extern __shared__ int sm[];  // cnt[E], off[E+1], tstart[E+1], hist[warps][E]
   int* cnt = sm;
-  int* off = sm + E;
+  int* off = cnt + E;
   int* tstart = off + E + 1;
-  int* sid = tstart + E + 1;
+  int* hist = tstart + E + 1;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  for (int i = threadIdx.x; i < E; i += blockDim.x) cnt[i] = 0;
+  for (int i = threadIdx.x; i < nwarps * E; i += blockDim.x) hist[i] = 0;
   for (int i = threadIdx.x; i < max_rows; i += blockDim.x) row_src[i] = -1;
   __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {  // the only global read of the ids
-    const int e = ids[i];
-    sid[i] = e;
-    if (e >= 0 && e < E) atomicAdd(&cnt[e], 1);
-    else dest_row[i] = -1;
+  const int first = warp * ROUNDS * 32;
+  int id[ROUNDS], rank[ROUNDS];
+  warp_ranks<ROUNDS>(ids, first, min(n, first + ROUNDS * 32), E, hist + warp * E, id, rank);
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+    int run = 0;
+    for (int w = 0; w < nwarps; ++w) {
+      const int v = hist[w * E + e];
+      hist[w * E + e] = run;
+      run += v;
+    }
+    cnt[e] = run;
+    counts_out[e] = run;
   }
   __syncthreads();
-  if (warp == 0) {
-    // Exclusive scans by one warp: lane l owns experts [l*per, (l+1)*per). First the padded row offsets, clamped to
-    // the capacity (offsets are multiples of `align`, so clamping both ends of an expert's range equals shrinking the
-    // expert that overflows and giving the later ones nothing), then the 128-row tile starts of the clamped ranges.
-    const int per = (E + 31) / 32;
-    const int e0 = lane * per, e1 = min(E, e0 + per);
-    const int cap = (max_rows / align) * align;
-    int local = 0;
-    for (int e = e0; e < e1; ++e) local += ((cnt[e] + align - 1) / align) * align;
-    int incl = local;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += v;
-    }
-    int run = incl - local;
-    int tl = 0;
-    for (int e = e0; e < e1; ++e) {
-      const int s0 = min(run, cap);
-      run += ((cnt[e] + align - 1) / align) * align;
-      const int s1 = min(run, cap);
-      off[e] = s0;
-      tl += (s1 - s0 + 127) / 128;
-      tstart[e] = s1 - s0;  // rows of the expert for now; turned into a tile start below
-    }
-    const int total_rows = min(__shfl_sync(0xffffffffu, incl, 31), cap);
-    int tincl = tl;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, tincl, o);
-      if (lane >= o) tincl += v;
-    }
-    int trun = tincl - tl;
-    for (int e = e0; e < e1; ++e) {
-      const int rows = tstart[e];
-      tstart[e] = trun;
-      trun += (rows + 127) / 128;
-    }
-    const int total_tiles = __shfl_sync(0xffffffffu, tincl, 31);
-    if (lane == 0) {
-      off[E] = total_rows;
-      tstart[E] = total_tiles < max_tiles ? total_tiles : max_tiles;
-      totals[0] = tstart[E];
-      totals[1] = total_rows;
-    }
-  }
+  if (warp == 0) scan_experts(cnt, E, max_rows, max_tiles, align, off, tstart, totals);
   __syncthreads();
-  for (int e = threadIdx.x; e <= E; e += blockDim.x) {
-    offsets[e] = off[e];
-    if (e < E) counts_out[e] = cnt[e];
-  }
-  // tiles and stable ranks: one warp per expert, ids read from shared memory
-  for (int e = warp; e < E; e += nwarps) {
-    const int rows_e = off[e + 1] - off[e];
-    for (int j = lane; tstart[e] + j < tstart[e + 1] && tstart[e] + j < max_tiles; j += 32) {
-      int* t = tiles + 4 * (tstart[e] + j);
-      t[0] = e;
-      t[1] = off[e] + 128 * j;
-      t[2] = min(128, rows_e - 128 * j);
-      t[3] = 0;
-    }
-    if (cnt[e] == 0) continue;
-    int base = 0;
-    for (int start = 0; start < n; start += 32) {
-      const int i = start + lane;
-      const bool hit = i < n && sid[i] == e;
-      const unsigned m = __ballot_sync(0xffffffffu, hit);
-      if (hit) {
-        const int rank = base + __popc(m & ((1u << lane) - 1u));
-        if (rank < rows_e) {
-          dest_row[i] = off[e] + rank;
-          row_src[off[e] + rank] = i;
-        } else {
-          dest_row[i] = -1;
-        }
+  for (int e = threadIdx.x; e <= E; e += blockDim.x) offsets[e] = off[e];
+  write_tiles(off, tstart, E, max_tiles, tiles);
+#pragma unroll
+  for (int r = 0; r < ROUNDS; ++r) {
+    const int i = first + 32 * r + lane;
+    if (i >= n) continue;
+    const int e = id[r];
+    int row = -1;  // an id outside the experts, or no room for it
+    if (e >= 0) {
+      const int k = hist[warp * E + e] + rank[r];
+      if (k < off[e + 1] - off[e]) {
+        row = off[e] + k;
+        row_src[row] = i;
       }
-      base += __popc(m);
-      if (base >= cnt[e]) break;  // all entries of this expert placed (warp-uniform)
     }
+    dest_row[i] = row;
   }
 }
 
-struct alignas(16) V8 {
-  uint4 v;
-};
+// Larger problems, pass 1: every block counts its SORT_WARPS * SORT_ROUNDS * 32 entries by expert.
+__global__ void __launch_bounds__(SORT_WARPS * 32)
+count_kernel(const int* __restrict__ ids, int n, int E, int* __restrict__ block_hist) {
+  extern __shared__ int hist[];  // [E]
+  for (int e = threadIdx.x; e < E; e += blockDim.x) hist[e] = 0;
+  __syncthreads();
+  const int first = blockIdx.x * SORT_WARPS * SORT_ROUNDS * 32;
+  const int last = min(n, first + SORT_WARPS * SORT_ROUNDS * 32);
+#pragma unroll 4
+  for (int i = first + threadIdx.x; i < last; i += SORT_WARPS * 32) {
+    const int e = ids[i];
+    if (e >= 0 && e < E) atomicAdd(&hist[e], 1);
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += blockDim.x) block_hist[static_cast<long long>(blockIdx.x) * E + e] = hist[e];
+}
 
-// x_perm[row] = x[row_src[row] / K] or zeros for padding rows. One warp per row chunk.
+// Pass 2, one block: block_hist becomes the number of an expert's entries in the blocks before each; scans and tile list.
+__global__ void __launch_bounds__(1024)
+scan_kernel(int* __restrict__ block_hist, int blocks, int parts, int E, int max_rows, int max_tiles, int align, int* __restrict__ counts,
+            int* __restrict__ offsets, int* __restrict__ tiles, int* __restrict__ totals) {
+  extern __shared__ int sm[];  // cnt[E], off[E+1], tstart[E+1], part[parts][E]
+  int* cnt = sm;
+  int* off = cnt + E;
+  int* tstart = off + E + 1;
+  int* part = tstart + E + 1;
+  const int run_len = (blocks + parts - 1) / parts;  // the blocks in several runs: as many chains of loads per expert are in flight
+  for (int i = threadIdx.x; i < parts * E; i += blockDim.x) {
+    const int p = i / E, e = i - p * E;
+    const int b1 = min(blocks, (p + 1) * run_len);
+    int sum = 0;
+#pragma unroll 8
+    for (int b = p * run_len; b < b1; ++b) sum += block_hist[static_cast<long long>(b) * E + e];
+    part[i] = sum;
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+    int run = 0;
+    for (int p = 0; p < parts; ++p) {
+      const int v = part[p * E + e];
+      part[p * E + e] = run;
+      run += v;
+    }
+    cnt[e] = run;
+    counts[e] = run;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < parts * E; i += blockDim.x) {
+    const int p = i / E, e = i - p * E;
+    const int b1 = min(blocks, (p + 1) * run_len);
+    int run = part[i];
+#pragma unroll 8
+    for (int b = p * run_len; b < b1; ++b) {
+      int* h = block_hist + static_cast<long long>(b) * E + e;
+      const int v = *h;
+      *h = run;
+      run += v;
+    }
+  }
+  if (threadIdx.x < 32) scan_experts(cnt, E, max_rows, max_tiles, align, off, tstart, totals);
+  __syncthreads();
+  for (int e = threadIdx.x; e <= E; e += blockDim.x) offsets[e] = off[e];
+  write_tiles(off, tstart, E, max_tiles, tiles);
+}
+
+// Pass 3: the rows of a block's entries.
+__global__ void __launch_bounds__(SORT_WARPS * 32)
+assign_kernel(const int* __restrict__ ids, int n, int E, const int* __restrict__ block_hist, const int* __restrict__ offsets,
+              int* __restrict__ dest_row, int* __restrict__ row_src) {
+  extern __shared__ int hist[];  // [SORT_WARPS][E]
+  for (int i = threadIdx.x; i < SORT_WARPS * E; i += blockDim.x) hist[i] = 0;
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int first = (blockIdx.x * SORT_WARPS + warp) * SORT_ROUNDS * 32;
+  int id[SORT_ROUNDS], rank[SORT_ROUNDS];
+  warp_ranks<SORT_ROUNDS>(ids, first, min(n, first + SORT_ROUNDS * 32), E, hist + warp * E, id, rank);
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+    int run = block_hist[static_cast<long long>(blockIdx.x) * E + e];
+#pragma unroll
+    for (int w = 0; w < SORT_WARPS; ++w) {
+      const int v = hist[w * E + e];
+      hist[w * E + e] = run;
+      run += v;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < SORT_ROUNDS; ++r) {
+    const int i = first + 32 * r + lane;
+    if (i >= n) continue;
+    const int e = id[r];
+    int row = -1;  // an id outside the experts, or no room for it (only if max_rows was under-provisioned)
+    if (e >= 0) {
+      const int k = hist[warp * E + e] + rank[r];
+      const int o = offsets[e];
+      if (k < offsets[e + 1] - o) {
+        row = o + k;
+        row_src[row] = i;
+      }
+    }
+    dest_row[i] = row;
+  }
+}
+
+// x_perm[row] = x[row_src[row] / K] or zeros for padding rows. One warp per row, four 16-byte loads of it in flight per lane
+// (131072 rows of 2048: 158 us when every thread placed its own 16 bytes after a 64-bit division, 148 us now; the copy alone
+// is 604 MB).
 __global__ void permute_kernel(const bf16* __restrict__ x, const int* __restrict__ row_src,
                                const int* __restrict__ num_m_tiles, bf16* __restrict__ x_perm, int max_rows, int H,
                                int K) {
   const int live_rows = min(num_m_tiles[1], max_rows);
   const int vec_per_row = H / 8;
-  const long long total = static_cast<long long>(live_rows) * vec_per_row;
-  for (long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; idx < total;
-       idx += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int row = idx / vec_per_row;
-    const int c = idx - static_cast<long long>(row) * vec_per_row;
+  const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
+  for (int row = blockIdx.x * wpb + (threadIdx.x >> 5); row < live_rows; row += gridDim.x * wpb) {
     const int src = row_src[row];
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (src >= 0) v = reinterpret_cast<const uint4*>(x + static_cast<long long>(src / K) * H)[c];
-    reinterpret_cast<uint4*>(x_perm + static_cast<long long>(row) * H)[c] = v;
+    const uint4* from = reinterpret_cast<const uint4*>(x + static_cast<long long>(src < 0 ? 0 : src / K) * H);
+    uint4* to = reinterpret_cast<uint4*>(x_perm + static_cast<long long>(row) * H);
+    for (int c0 = lane; c0 < vec_per_row; c0 += 128) {
+      uint4 v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = (src >= 0 && c0 + 32 * u < vec_per_row) ? from[c0 + 32 * u] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (c0 + 32 * u < vec_per_row) to[c0 + 32 * u] = v[u];
+    }
   }
 }
 
@@ -413,23 +471,36 @@ __device__ __forceinline__ uint4 pack8(const float (&a)[8]) {
   return r;
 }
 
-// out[t] = sum_k w[t,k] * y_perm[dest_row[t,k]]; with w == nullptr the weights are 1 (permute backward).
-__global__ void combine_kernel(const bf16* __restrict__ y_perm, const int* __restrict__ dest_row,
-                               const float* __restrict__ topk_w, const bf16* __restrict__ residual,
-                               bf16* __restrict__ out, int T, int K, int H) {
+// out[t] = sum_k w[t,k] * y_perm[dest_row[t,k]]; with w == nullptr the weights are 1 (permute backward). A block takes 128
+// 16-byte columns of one token after another; the rows of up to eight choices are asked for together and added in order
+// (16384 tokens, 8 choices, 2048 columns: 185 us with one load in flight per thread, 128 us with eight; 671 MB move).
+constexpr int COMBINE_THREADS = 128;
+__global__ void __launch_bounds__(COMBINE_THREADS)
+combine_kernel(const bf16* __restrict__ y_perm, const int* __restrict__ dest_row, const float* __restrict__ topk_w,
+               const bf16* __restrict__ residual, bf16* __restrict__ out, int T, int K, int H) {
   const int vec_per_row = H / 8;
-  const long long total = static_cast<long long>(T) * vec_per_row;
-  for (long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; idx < total;
-       idx += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int t = idx / vec_per_row;
-    const int c = idx - static_cast<long long>(t) * vec_per_row;
+  const int c = blockIdx.y * COMBINE_THREADS + threadIdx.x;
+  if (c >= vec_per_row) return;
+  for (int t = blockIdx.x; t < T; t += gridDim.x) {
     float a[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (residual) acc8(reinterpret_cast<const uint4*>(residual + static_cast<long long>(t) * H)[c], 1.f, a);
-    for (int k = 0; k < K; ++k) {
-      const int row = dest_row[static_cast<long long>(t) * K + k];
-      if (row < 0) continue;
-      const float w = topk_w ? topk_w[static_cast<long long>(t) * K + k] : 1.f;
-      acc8(reinterpret_cast<const uint4*>(y_perm + static_cast<long long>(row) * H)[c], w, a);
+    for (int k0 = 0; k0 < K; k0 += 8) {
+      const long long at = static_cast<long long>(t) * K + k0;
+      int row[8];
+      float w[8];
+      uint4 v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const bool has = k0 + k < K;
+        row[k] = has ? dest_row[at + k] : -1;
+        w[k] = (has && topk_w) ? topk_w[at + k] : 1.f;
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (row[k] >= 0) v[k] = reinterpret_cast<const uint4*>(y_perm + static_cast<long long>(row[k]) * H)[c];
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (row[k] >= 0) acc8(v[k], w[k], a);
     }
     reinterpret_cast<uint4*>(out + static_cast<long long>(t) * H)[c] = pack8(a);
   }
@@ -454,19 +525,31 @@ __global__ void combine_bwd_kernel(const bf16* __restrict__ dout, const bf16* __
     const uint4* g = reinterpret_cast<const uint4*>(dout + static_cast<long long>(src / K) * H);
     const uint4* y = reinterpret_cast<const uint4*>(y_perm + static_cast<long long>(row) * H);
     float dot = 0.f;
-    for (int c = lane; c < H / 8; c += 32) {
-      const uint4 gr = g[c];
-      float a[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-      acc8(gr, w, a);
-      dst[c] = pack8(a);
-      if (dtopk_w) {
-        const uint4 yr = y[c];
-        const __nv_bfloat162* gb = reinterpret_cast<const __nv_bfloat162*>(&gr);
-        const __nv_bfloat162* yb = reinterpret_cast<const __nv_bfloat162*>(&yr);
+    const int vec_per_row = H / 8;
+    for (int c0 = lane; c0 < vec_per_row; c0 += 128) {  // four columns of both rows in flight
+      uint4 gr[4], yr[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float2 gf = __bfloat1622float2(gb[i]), yf = __bfloat1622float2(yb[i]);
-          dot += gf.x * yf.x + gf.y * yf.y;
+      for (int u = 0; u < 4; ++u) {
+        gr[u] = yr[u] = make_uint4(0, 0, 0, 0);
+        if (c0 + 32 * u < vec_per_row) {
+          gr[u] = g[c0 + 32 * u];
+          if (dtopk_w) yr[u] = y[c0 + 32 * u];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (c0 + 32 * u >= vec_per_row) break;
+        float a[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        acc8(gr[u], w, a);
+        dst[c0 + 32 * u] = pack8(a);
+        if (dtopk_w) {
+          const __nv_bfloat162* gb = reinterpret_cast<const __nv_bfloat162*>(&gr[u]);
+          const __nv_bfloat162* yb = reinterpret_cast<const __nv_bfloat162*>(&yr[u]);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float2 gf = __bfloat1622float2(gb[i]), yf = __bfloat1622float2(yb[i]);
+            dot += gf.x * yf.x + gf.y * yf.y;
+          }
         }
       }
     }
@@ -501,35 +584,57 @@ void moe_router_bwd(const float* probs, const int* topk_ids, const float* topk_w
                                                              renorm ? 1 : 0);
 }
 
+// Blocks of the many-block variant; their counts are its scratch, ints [blocks][E].
+static int sort_blocks(int n) { return n > 0 ? (n + SORT_WARPS * SORT_ROUNDS * 32 - 1) / (SORT_WARPS * SORT_ROUNDS * 32) : 1; }
+// One block up to 4096 entries (16 warps of 8 rounds; its counts per warp need 4 (16 + 3) E bytes of shared memory).
+static bool sort_in_one_block(int n, int max_rows, int E) { return n <= 4096 && max_rows <= 16384 && E <= 512; }
+
+long long moe_permutation_scratch(int T, int K, int max_rows, int E) {
+  return sort_in_one_block(T * K, max_rows, E) ? 0 : static_cast<long long>(sort_blocks(T * K)) * E;
+}
+
 void moe_build_permutation(const int* topk_ids, int T, int K, int E, int max_rows, int max_tiles, int align,
                            int* expert_counts, int* expert_offsets, int* dest_row, int* row_src, int* tile_group,
-                           int* num_m_tiles, cudaStream_t s) {
+                           int* num_m_tiles, int* scratch, cudaStream_t s) {
   const int n = T * K;
-  if (n <= 4096 && max_rows <= 16384 && E <= 512) {
-    build_small_kernel<<<1, n <= 128 ? 256 : 1024, (3 * E + 2 + n) * sizeof(int), s>>>(topk_ids, n, E, max_rows, max_tiles, align, expert_counts,
-                                                                   expert_offsets, dest_row, row_src, tile_group, num_m_tiles);
+  if (sort_in_one_block(n, max_rows, E)) {
+    const auto smem = [&](int warps) { return static_cast<size_t>((warps + 3) * E + 2) * sizeof(int); };
+    if (n <= 512) {
+      const int warps = n <= 128 ? 4 : 16;  // (four also fill row_src and the tile list quickly enough)
+      build_small_kernel<1><<<1, 32 * warps, smem(warps), s>>>(topk_ids, n, E, max_rows, max_tiles, align, expert_counts,
+                                                               expert_offsets, dest_row, row_src, tile_group, num_m_tiles);
+    } else {
+      build_small_kernel<8><<<1, 512, smem(16), s>>>(topk_ids, n, E, max_rows, max_tiles, align, expert_counts, expert_offsets,
+                                                     dest_row, row_src, tile_group, num_m_tiles);
+    }
     return;
   }
-  cudaMemsetAsync(dest_row, 0xff, sizeof(int) * static_cast<size_t>(n), s);
+  const int blocks = sort_blocks(n);
+  const int parts = E <= 1024 ? 8 : 1;  // (more experts: enough threads have one to follow, and shared memory holds their counts once)
+  const size_t scan_smem = static_cast<size_t>((3 + parts) * E + 2) * sizeof(int), assign_smem = static_cast<size_t>(SORT_WARPS) * E * sizeof(int);
+  if (scan_smem > 48 * 1024) cudaFuncSetAttribute(scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(scan_smem));
+  if (assign_smem > 48 * 1024)
+    cudaFuncSetAttribute(assign_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(assign_smem));
   cudaMemsetAsync(row_src, 0xff, sizeof(int) * static_cast<size_t>(max_rows), s);
-  count_kernel<<<E, 512, 0, s>>>(topk_ids, n, expert_counts);
-  scan_kernel<<<1, 256, (E + 1) * sizeof(int), s>>>(expert_counts, E, max_rows, max_tiles, align, expert_offsets, tile_group,
-                                                     num_m_tiles);
-  assign_kernel<<<E, 512, 0, s>>>(topk_ids, n, expert_offsets, dest_row, row_src);
+  count_kernel<<<blocks, SORT_WARPS * 32, E * sizeof(int), s>>>(topk_ids, n, E, scratch);
+  scan_kernel<<<1, 1024, scan_smem, s>>>(scratch, blocks, parts, E, max_rows, max_tiles, align, expert_counts, expert_offsets, tile_group,
+                                         num_m_tiles);
+  assign_kernel<<<blocks, SORT_WARPS * 32, assign_smem, s>>>(topk_ids, n, E, scratch, expert_offsets, dest_row, row_src);
 }
 
 void moe_permute(const void* x, const int* row_src, const int* num_m_tiles, void* x_perm, int max_rows, int H, int K,
                  cudaStream_t s) {
   if (max_rows <= 0) return;
-  permute_kernel<<<grid_for(static_cast<long long>(max_rows) * (H / 8), 256), 256, 0, s>>>(
-      static_cast<const bf16*>(x), row_src, num_m_tiles, static_cast<bf16*>(x_perm), max_rows, H, K);
+  permute_kernel<<<grid_for(max_rows, 8), 256, 0, s>>>(static_cast<const bf16*>(x), row_src, num_m_tiles,
+                                                       static_cast<bf16*>(x_perm), max_rows, H, K);
 }
 
 void moe_combine(const void* y_perm, const int* dest_row, const float* topk_w, const void* residual, void* out, int T,
                  int K, int H, cudaStream_t s) {
   if (T <= 0) return;
-  combine_kernel<<<grid_for(static_cast<long long>(T) * (H / 8), 256), 256, 0, s>>>(
-      static_cast<const bf16*>(y_perm), dest_row, topk_w, static_cast<const bf16*>(residual), static_cast<bf16*>(out), T, K, H);
+  const dim3 grid(T, (H / 8 + COMBINE_THREADS - 1) / COMBINE_THREADS);
+  combine_kernel<<<grid, COMBINE_THREADS, 0, s>>>(static_cast<const bf16*>(y_perm), dest_row, topk_w,
+                                                  static_cast<const bf16*>(residual), static_cast<bf16*>(out), T, K, H);
 }
 
 void moe_unpermute_sum(const void* dx_perm, const int* dest_row, void* dx, int T, int K, int H, cudaStream_t s) {
