@@ -242,35 +242,51 @@ __global__ void __launch_bounds__(256) small_gemv_multi_kernel(const bf16* __res
 // Outputs: topk_ids[T,K], topk_w[T,K], and for the MoE kernels the compact list of active experts with, per
 // expert, the (token, slot) pairs routed to it: active[0] = count, active[1..] = expert ids, pair_count[E],
 // pair_list[E][TOK] (pair = t*K + k; a token picks an expert at most once).
+// A token's warp keeps its logits in registers (VALS per lane) and takes one maximum after another; the lists come from one
+// mask of token bits per expert and a ballot over each 32 experts. One row over 128 experts: 4.0 us, 11.4 us when the logits
+// and the experts already taken were read again for every choice and one thread collected the active experts.
+template <int VALS>
 __global__ void __launch_bounds__(256) router_small_kernel(const float* __restrict__ logits, int T, int E, int K,
                                                            int renorm, int* __restrict__ topk_ids,
                                                            float* __restrict__ topk_w, int* __restrict__ active,
                                                            int* __restrict__ pair_count, int* __restrict__ pair_list) {
-  __shared__ int ids_s[TOK][32];
-  __shared__ int cnt_s[1024];
+  __shared__ unsigned mask_s[32 * VALS];  // tokens that chose the expert
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp < T) {
-    const float* lg = logits + static_cast<long long>(warp) * E;
-    float m = -FLT_MAX;
-    for (int e = lane; e < E; e += 32) m = fmaxf(m, lg[e]);
+  for (int e = threadIdx.x; e < E; e += blockDim.x) mask_s[e] = 0u;
+  float v[VALS];
+  float m = -FLT_MAX;
+  const bool has = warp < T;
+  if (has) {
+#pragma unroll
+    for (int i = 0; i < VALS; ++i) {
+      const int e = lane + 32 * i;
+      v[i] = e < E ? logits[static_cast<long long>(warp) * E + e] : -FLT_MAX;
+      m = fmaxf(m, v[i]);
+    }
+  }
+  __syncthreads();
+  float my_w = 0.f;
+  int my_id = 0;
+  if (has) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     float s = 0.f;
-    for (int e = lane; e < E; e += 32) s += __expf(lg[e] - m);
+#pragma unroll
+    for (int i = 0; i < VALS; ++i)
+      if (lane + 32 * i < E) s += __expf(v[i] - m);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     const float inv = 1.f / s;
-    float wsum = 0.f, my_w = 0.f;
-    int my_id = 0;
+    float wsum = 0.f;
+    unsigned taken = 0u;  // this lane's experts among the choices so far
     for (int k = 0; k < K; ++k) {
       float best = -FLT_MAX;
       int bi = 0x7fffffff;
-      for (int e = lane; e < E; e += 32) {
-        bool taken = false;
-        for (int j = 0; j < k; ++j) taken |= (ids_s[warp][j] == e);
-        const float v = lg[e];
-        if (!taken && (v > best || (v == best && e < bi))) {
-          best = v;
+#pragma unroll
+      for (int i = 0; i < VALS; ++i) {
+        const int e = lane + 32 * i;
+        if (e < E && !((taken >> i) & 1u) && (v[i] > best || (v[i] == best && e < bi))) {
+          best = v[i];
           bi = e;
         }
       }
@@ -283,8 +299,7 @@ __global__ void __launch_bounds__(256) router_small_kernel(const float* __restri
           bi = oi;
         }
       }
-      if (lane == 0) ids_s[warp][k] = bi;
-      __syncwarp();
+      if ((bi & 31) == lane) taken |= 1u << (bi >> 5 & 31);
       const float pw = __expf(best - m) * inv;
       wsum += pw;
       if (lane == k) {
@@ -295,23 +310,23 @@ __global__ void __launch_bounds__(256) router_small_kernel(const float* __restri
     if (lane < K) {
       topk_ids[warp * K + lane] = my_id;
       topk_w[warp * K + lane] = renorm ? my_w / wsum : my_w;
+      if (my_id < E) atomicOr(&mask_s[my_id], 1u << warp);
     }
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+  // a token picks an expert at most once, so its place in the expert's list is the number of earlier tokens in the mask
+  if (has && lane < K && my_id < E)
+    pair_list[my_id * TOK + __popc(mask_s[my_id] & ((1u << warp) - 1u))] = warp * K + lane;
+  for (int e = threadIdx.x; e < E; e += blockDim.x) pair_count[e] = __popc(mask_s[e]);
+  if (warp == 7) {  // the experts in use, in order
     int n = 0;
-    for (int t = 0; t < T; ++t)
-      for (int k = 0; k < K; ++k)
-        if (ids_s[t][k] == e) pair_list[e * TOK + n++] = t * K + k;
-    pair_count[e] = n;
-    cnt_s[e] = n;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int n = 0;
-    for (int e = 0; e < E; ++e)
-      if (cnt_s[e] > 0) active[1 + n++] = e;
-    active[0] = n;
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      const bool on = e0 + lane < E && mask_s[e0 + lane] != 0u;
+      const unsigned b = __ballot_sync(0xffffffffu, on);
+      if (on) active[1 + n + __popc(b & ((1u << lane) - 1u))] = e0 + lane;
+      n += __popc(b);
+    }
+    if (lane == 0) active[0] = n;
   }
 }
 
@@ -344,7 +359,10 @@ void small_gemv_direct(const void* x, int T, const void* norm_w, float eps, cons
 
 void router_small(const float* logits, int T, int E, int K, bool renorm, int* topk_ids, float* topk_w, int* active,
                   int* pair_count, int* pair_list, cudaStream_t s) {
-  router_small_kernel<<<1, 256, 0, s>>>(logits, T, E, K, renorm ? 1 : 0, topk_ids, topk_w, active, pair_count, pair_list);
+  if (E <= 128)
+    router_small_kernel<4><<<1, 256, 0, s>>>(logits, T, E, K, renorm ? 1 : 0, topk_ids, topk_w, active, pair_count, pair_list);
+  else  // up to 1024 experts (checked by the caller)
+    router_small_kernel<32><<<1, 256, 0, s>>>(logits, T, E, K, renorm ? 1 : 0, topk_ids, topk_w, active, pair_count, pair_list);
 }
 
 }  // namespace mb
