@@ -23,7 +23,7 @@ TARGET = PKG / "_C.so"
 HYBRID_TARGET = PKG / "_hybrid.so"
 HYBRID_ONLY = {"hybrid_ops.cu", "mamba2.cu", "latent_attention.cu", "cached_attention.cu", "cached_prefill.cu", "linear_attention.cu",
                "sequential_ops.cu", "hybrid_bindings.cpp"}
-HYBRID_SHARED = {"gemm.cu", "decode_small.cu", "decode_stream.cu", "sampling.cu", "serve_bindings.cpp"}
+HYBRID_SHARED = {"gemm.cu", "gemm_skinny.cu", "decode_small.cu", "decode_stream.cu", "sampling.cu", "serve_bindings.cpp"}
 TARGETS = {"_C": TARGET, "_hybrid": HYBRID_TARGET}
 
 NVCC_FLAGS = [

@@ -26,6 +26,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "gemm.h"
 #include "launchers.h"
 #include "ptx.cuh"
 
@@ -364,8 +365,30 @@ int launch_stream(StreamArgs a, int max_groups, cudaStream_t s) {
 void small_gemv_direct(const void* x, int T, const void* norm_w, float eps, const void* W, int N, int K,
                        const void* residual, void* out, bool out_fp32, cudaStream_t s);  // decode_small.cu
 
-void small_gemv(const void* x, int T, const void* norm_w, float eps, const void* W, int N, int K, const void* residual,
-                void* out, bool out_fp32, int* status, cudaStream_t s) {
+int small_gemv(const void* x, int T, const void* norm_w, float eps, const void* W, int N, int K, const void* residual,
+               void* out, bool out_fp32, int* status, cudaStream_t s) {
+  // 9..64 rows, and large matrices without a norm to fold in: the split tensor-core kernel (8 rows of 2560 x 9728: 13.1 us,
+  // 17.3 with the blocks of decode_small.cu, which start faster and win for small matrices: 2048 x 4096 6.0 us, 8.2 there;
+  // the two meet at 6144 x 2560)
+  const long long bytes = static_cast<long long>(N) * K * 2;
+  if (T > TOK || (!norm_w && bytes >= (24ll << 20))) {
+    GemmProblem p = {};
+    p.mode = GEMM_DENSE;
+    p.M = T;
+    p.N = N;
+    p.K = K;
+    p.a = {x, T, K, K, false};
+    p.b = {W, N, K, K, false};
+    p.c = out;
+    p.ldc = N;
+    p.out_fp32 = out_fp32;
+    p.status = status;
+    return gemm_skinny_launch(p, residual, s);
+  }
+  if (bytes < (48ll << 20)) {  // small matrix: the direct kernel
+    small_gemv_direct(x, T, norm_w, eps, W, N, K, residual, out, out_fp32, s);
+    return 0;
+  }
   StreamArgs a = {};
   a.W = static_cast<const bf16*>(W);
   a.rows = N;
@@ -380,11 +403,8 @@ void small_gemv(const void* x, int T, const void* norm_w, float eps, const void*
   a.out_fp32 = out_fp32 ? 1 : 0;
   a.residual = static_cast<const bf16*>(residual);
   a.status = status;
-  if (T > TOK || static_cast<long long>(N) * K * 2 < (48ll << 20)) {  // small matrix or 9..64 rows: the direct kernels
-    small_gemv_direct(x, T, norm_w, eps, W, N, K, residual, out, out_fp32, s);
-    return;
-  }
   launch_stream(a, 1, s);
+  return 0;
 }
 
 void moe_small_up(const void* x, const void* norm_w, float eps, const void* W1, const int* active, const int* pair_count,

@@ -538,8 +538,12 @@ int fail(const std::string& m) {
   return -1;
 }
 
+}  // namespace
+
+int gemm_fail(const std::string& m) { return fail(m); }
+
 // 2-D bf16 tensor map over a row-major [rows, cols] matrix with a [box_rows, 64] box.
-int make_map(CUtensorMap* map, const GemmOperand& op, int box_rows) {
+int gemm_make_map(CUtensorMap* map, const GemmOperand& op, int box_rows) {
   EncodeTiledFn enc = get_encode();
   if (!enc) return fail("cuTensorMapEncodeTiled is not available");
   if ((reinterpret_cast<uintptr_t>(op.ptr) & 15) != 0) return fail("operand base must be 16-byte aligned");
@@ -555,6 +559,8 @@ int make_map(CUtensorMap* map, const GemmOperand& op, int box_rows) {
   return 0;
 }
 
+namespace {
+
 template <int BLOCK_N, bool A_MN, bool B_MN>
 int launch(const GemmProblem& p, const KArgs& ka, cudaStream_t stream) {
   // the 128-wide variant gives one pipeline stage to a 32 KB staging buffer for scattered (peer) output rows
@@ -563,8 +569,8 @@ int launch(const GemmProblem& p, const KArgs& ka, cudaStream_t stream) {
   constexpr int SMEM = STAGES * (A_STAGE_BYTES + B_STAGE_BYTES) + 8 * (2 * STAGES + 5) + 1024 +
                        (BLOCK_N == 128 ? 4 * 32 * 256 + 16 : 0);
   CUtensorMap ma, mb_;
-  if (make_map(&ma, p.a, A_MN ? BLOCK_K : BLOCK_M)) return -1;
-  if (make_map(&mb_, p.b, B_MN ? BLOCK_K : BLOCK_N)) return -1;
+  if (gemm_make_map(&ma, p.a, A_MN ? BLOCK_K : BLOCK_M)) return -1;
+  if (gemm_make_map(&mb_, p.b, B_MN ? BLOCK_K : BLOCK_N)) return -1;
   auto kern = gemm_bf16_kernel<BLOCK_N, A_MN, B_MN, STAGES>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)  // per (function, device)
     return fail("cudaFuncSetAttribute(MaxDynamicSharedMemorySize) failed");
@@ -628,6 +634,7 @@ int gemm_bf16_launch(const GemmProblem& p, cudaStream_t stream) {
 
   int bn = p.block_n;
   const bool amn = p.a.mn_major, bmn = p.b.mn_major;
+  if (bn == 0 && gemm_is_skinny(p)) return gemm_skinny_launch(p, nullptr, stream);
   if (bn == 0) {
     const int sms = 148;
     const long long m_tiles = p.mode == GEMM_GROUPED_ROWS ? p.max_tiles : (p.M + BLOCK_M - 1) / BLOCK_M;

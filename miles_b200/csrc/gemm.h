@@ -1,7 +1,10 @@
 // Host API of the tcgen05 bf16 GEMM family (dense, grouped-by-rows, grouped-by-contraction).
 #pragma once
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <string>
 
 namespace mb {
 
@@ -88,5 +91,12 @@ void sf_swizzle(const uint8_t* in, uint8_t* out, long long rows, int S, cudaStre
 // Launches on `stream`. Returns 0 or a negative host-side error code (bad argument / driver error).
 int gemm_bf16_launch(const GemmProblem& p, cudaStream_t stream);
 const char* gemm_last_error();
+
+// At most 128 rows of A against a weight matrix (gemm_skinny.cu): C = A . B^T (+ residual, bf16 in C's layout, may be null).
+bool gemm_is_skinny(const GemmProblem& p);
+int gemm_skinny_launch(const GemmProblem& p, const void* residual, cudaStream_t stream);
+// Shared by the two: the tensor map of an operand with a [box_rows, 64] box, and the error message of a failed call.
+int gemm_make_map(CUtensorMap* map, const GemmOperand& op, int box_rows);
+int gemm_fail(const std::string& m);
 
 }  // namespace mb

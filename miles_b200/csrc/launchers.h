@@ -112,7 +112,8 @@ const char* flash_attn_bwd_last_error();
 
 // ---- decode_stream.cu / decode_small.cu (at most 8 tokens: persistent weight-streaming mma.sync kernel fed by
 // bulk asynchronous copies, RMSNorm folded in; `status` receives a code if a bounded wait gives up)
-void small_gemv(const void* x, int T, const void* norm_w, float eps, const void* W, int N, int K, const void* residual,
+// Returns 0, or -1 with gemm_last_error() set.
+int small_gemv(const void* x, int T, const void* norm_w, float eps, const void* W, int N, int K, const void* residual,
                 void* out, bool out_fp32, int* status, cudaStream_t s);
 void router_small(const float* logits, int T, int E, int K, bool renorm, int* topk_ids, float* topk_w, int* active,
                   int* pair_count, int* pair_list, cudaStream_t s);

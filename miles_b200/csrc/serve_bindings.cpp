@@ -72,9 +72,10 @@ void small_gemv(const at::Tensor& x, const c10::optional<at::Tensor>& norm_w, do
   if (norm_w.has_value()) CHECK_BF16((*norm_w));
   if (residual.has_value()) { CHECK_BF16((*residual)); TORCH_CHECK(residual->numel() == out.numel(), "small_gemv: residual shape"); }
   const c10::cuda::CUDAGuard guard(x.device());
-  mb::small_gemv(x.data_ptr(), T, norm_w.has_value() ? norm_w->data_ptr() : nullptr, eps, W.data_ptr(), N, K,
-                 residual.has_value() ? residual->data_ptr() : nullptr, out.data_ptr(), f32,
-                 status.has_value() ? status->data_ptr<int>() : nullptr, cur_stream());
+  const int rc = mb::small_gemv(x.data_ptr(), T, norm_w.has_value() ? norm_w->data_ptr() : nullptr, eps, W.data_ptr(), N, K,
+                                residual.has_value() ? residual->data_ptr() : nullptr, out.data_ptr(), f32,
+                                status.has_value() ? status->data_ptr<int>() : nullptr, cur_stream());
+  TORCH_CHECK(rc == 0, "small_gemv: ", mb::gemm_last_error());
 }
 
 }  // namespace

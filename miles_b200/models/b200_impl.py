@@ -166,9 +166,8 @@ class B200Qwen3:
         if mx and T > 32 and out_dtype == torch.bfloat16 and w.data_ptr() in mx:
             return self._mx_linear(x.contiguous(), mx[w.data_ptr()])
         out = torch.empty(x.shape[0], w.shape[0], dtype=out_dtype, device=x.device)
-        if T <= 32 and self.small_decode and N % 16 == 0 and K % 32 == 0 and N * K * 2 < (48 << 20) and x.is_contiguous():
-            # a few rows against a small weight matrix (decode projections): the weight-streaming mma.sync kernel
-            # (measured: faster than the narrow tcgen05 tiles up to 32 rows, slower at 64)
+        if T <= 8 and self.small_decode and N % 16 == 0 and K % 32 == 0 and N * K * 2 < (48 << 20) and x.is_contiguous():
+            # a few rows against a small weight matrix (decode projections): the blocks that start fastest
             self.C.small_gemv(x, None, 0.0, w, None, out, self.status)
             self.launches += 1
             return out
@@ -463,6 +462,12 @@ class B200Qwen3:
     def _o_proj_ln2(self, i, att2, x):
         """Attention output projection, residual add and the second RMSNorm: returns (h2, rstd2, x2)."""
         cfg, P, C = self.cfg, self.store.params, self.C
+        if (residual is not None and self.SMALL_T < a.shape[0] <= 64 and self.small_decode and not getattr(self, "mx", None)
+                and a.is_contiguous() and w.shape[0] % 16 == 0 and w.shape[1] % 32 == 0):
+            y = torch.empty_like(residual)  # the residual joins the sums before they are rounded
+            self.C.small_gemv(a, None, 0.0, w, residual, y, self.status)
+            self.launches += 1
+            return y
         p = f"layers.{i}."
         self.launches += 1
         if self.tp is not None:
@@ -554,7 +559,12 @@ class B200Qwen3:
             return y
         wgu = P[p + "mlp.gate_up.weight"]
         gu = torch.empty(T, wgu.shape[0], dtype=torch.bfloat16, device=dev)
-        C.small_gemv(x2, ln2, cfg.rms_eps, wgu, None, gu, self.status)
+        if wgu.numel() >= 24 << 20:  # (the split kernel reads 100 MB in 20 us, the one that folds the norm in takes 32)
+            h2, _ = C.rmsnorm_fwd(x2, None, ln2, cfg.rms_eps)
+            C.small_gemv(h2, None, 0.0, wgu, None, gu, self.status)
+            self.launches += 1
+        else:
+            C.small_gemv(x2, ln2, cfg.rms_eps, wgu, None, gu, self.status)
         y = torch.empty_like(x)
         C.small_gemv(C.swiglu_fwd(gu), None, cfg.rms_eps, P[p + "mlp.down.weight"], x2, y, self.status)
         self.launches += 3

@@ -1,0 +1,54 @@
+"""The split product of few rows where its tiles, splits and rings change: one row, the edges of every token tile, an output
+narrower than a tile, contractions shorter than the ring or not a multiple of a block, strided rows, fp32 and residual."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.fixture(scope="module")
+def ext():
+    from miles_b200.ops import _ext
+
+    return _ext.load(required=True)
+
+
+def _check(got, x, w, res=None):
+    want = x.double() @ w.double().t()
+    size = x.double().abs() @ w.double().abs().t()
+    if res is not None:
+        want = want + res.double()
+    # products summed in fp32 in any order, then one rounding to the output's type
+    bound = size * x.shape[1] ** 0.5 * 2 ** -24 * 4 + (want.abs() * 2 ** -8 if got.dtype == torch.bfloat16 else want.abs() * 2 ** -23)
+    assert ((got.double() - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("T", [1, 9, 16, 17, 32, 33, 64, 65, 93, 128])
+@pytest.mark.parametrize("N,K", [(8, 64), (128, 2048), (130, 72), (2048, 4096), (5120, 2048), (2560, 1000), (12296, 520), (57000, 64)])
+def test_product_of_few_rows(ext, T, N, K):
+    g = torch.Generator(DEV).manual_seed(T * N + K)
+    st = torch.zeros(1, dtype=torch.int32, device=DEV)
+    x = torch.randn(T, K + 8, generator=g, device=DEV).bfloat16()[:, :K]  # rows longer than the contraction
+    w = torch.randn(N, K, generator=g, device=DEV).bfloat16()
+    for dtype in (torch.bfloat16, torch.float32):
+        out = torch.full((T, N + 5), 7.0, device=DEV, dtype=dtype)
+        ext.gemm(x, w, out[:, :N], False, False, False, 0, st)
+        _check(out[:, :N], x, w)
+        assert (out[:, N:] == 7).all()
+    if T <= 64 and K % 32 == 0 and N % 16 == 0:
+        res = torch.randn(T, N, generator=g, device=DEV).bfloat16()
+        out = torch.empty(T, N, device=DEV, dtype=torch.bfloat16)
+        ext.small_gemv(x.contiguous(), None, 0.0, w, res, out, st)
+        _check(out, x, w, res)
+    assert st.item() == 0
+
+
+def test_repeated_products_are_bitwise_equal(ext):
+    g = torch.Generator(DEV).manual_seed(0)
+    st = torch.zeros(1, dtype=torch.int32, device=DEV)
+    x, w = torch.randn(23, 9728, generator=g, device=DEV).bfloat16(), torch.randn(2560, 9728, generator=g, device=DEV).bfloat16()
+    outs = [torch.empty(23, 2560, device=DEV, dtype=torch.bfloat16) for _ in range(4)]
+    for o in outs:
+        ext.gemm(x, w, o, False, False, False, 0, st)
+    assert all(torch.equal(o, outs[0]) for o in outs)
