@@ -45,6 +45,16 @@ void moe_router_topk(const float* logits, const int* replay_ids, int* topk_ids, 
 // to a multiple of `align`; outputs: dest_row[T*K], row_src[max_rows] (-1 for padding), expert_offsets[E+1]
 // (padded), tile_group[max_tiles][4] = {expert, row0, rows, 0}, num_m_tiles[2] = {tiles, live rows},
 // expert_counts[E].
+// kv_gather.cu: rows of `vecs` 16-byte vectors; pitches of the new rows in vectors
+struct PrefixGather {
+  const void *k_new, *v_new, *k_cache, *v_cache;
+  void *k_out, *v_out;
+  const long long *pre_slots, *pre_dst, *new_dst;
+  long long n_pre, n_new, num_slots, total, k_pitch, v_pitch;
+  int vecs;
+  int* status;
+};
+void gather_prefix_kv(const PrefixGather& a, cudaStream_t s);
 // ints of scratch that moe_build_permutation needs for these sizes
 long long moe_permutation_scratch(int T, int K, int max_rows, int E);
 void moe_build_permutation(const int* topk_ids, int T, int K, int E, int max_rows, int max_tiles, int align,

@@ -32,6 +32,48 @@ void paged_decode_attention(const at::Tensor& q, const at::Tensor& k_cache, cons
   TORCH_CHECK(e == 0, "paged_decode_attention launch failed: ", cudaGetErrorString(static_cast<cudaError_t>(e)));
 }
 
+// k_new / v_new [n, Hk, 128] (heads packed in a row, any row pitch of whole 16-byte vectors), caches [slots, Hk, 128]:
+// row new_dst[i] of the outputs is new row i, row pre_dst[j] is cache row pre_slots[j].
+std::vector<at::Tensor> gather_prefix_kv(const at::Tensor& k_new, const at::Tensor& v_new, const at::Tensor& k_cache, const at::Tensor& v_cache,
+                                         const at::Tensor& pre_slots, const at::Tensor& pre_dst, const at::Tensor& new_dst, int64_t total,
+                                         const c10::optional<at::Tensor>& status) {
+  CHECK_BF16(k_cache); CHECK_BF16(v_cache);
+  for (const at::Tensor* t : {&k_new, &v_new}) {
+    TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kBFloat16 && t->dim() == 3 && t->stride(2) == 1 && t->stride(1) == t->size(2) &&
+                    t->stride(0) % 8 == 0 && reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 == 0,
+                "gather_prefix_kv: new rows must be bf16, packed along each row and 16-byte aligned");
+    TORCH_CHECK(t->size(0) == new_dst.numel() && t->size(1) == k_cache.size(1) && t->size(2) == k_cache.size(2), "gather_prefix_kv: shapes differ");
+  }
+  TORCH_CHECK(k_cache.dim() == 3 && v_cache.sizes() == k_cache.sizes(), "gather_prefix_kv: caches must be [slots, heads, head_dim] alike");
+  for (const at::Tensor* t : {&pre_slots, &pre_dst, &new_dst})
+    TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kLong && t->is_contiguous(), "gather_prefix_kv: indices must be contiguous int64");
+  TORCH_CHECK(pre_slots.numel() == pre_dst.numel() && total >= 0, "gather_prefix_kv: bad index sizes");
+  const int64_t row = k_cache.size(1) * k_cache.size(2);
+  TORCH_CHECK(row % 8 == 0, "gather_prefix_kv: a row must be whole 16-byte vectors");
+  const c10::cuda::CUDAGuard guard(k_new.device());
+  at::Tensor kf = at::empty({total, k_cache.size(1), k_cache.size(2)}, k_new.options()), vf = at::empty_like(kf);
+  mb::PrefixGather a{};
+  a.k_new = k_new.data_ptr();
+  a.v_new = v_new.data_ptr();
+  a.k_cache = k_cache.data_ptr();
+  a.v_cache = v_cache.data_ptr();
+  a.k_out = kf.data_ptr();
+  a.v_out = vf.data_ptr();
+  a.pre_slots = reinterpret_cast<const long long*>(pre_slots.data_ptr<int64_t>());
+  a.pre_dst = reinterpret_cast<const long long*>(pre_dst.data_ptr<int64_t>());
+  a.new_dst = reinterpret_cast<const long long*>(new_dst.data_ptr<int64_t>());
+  a.n_pre = pre_slots.numel();
+  a.n_new = new_dst.numel();
+  a.num_slots = k_cache.size(0);
+  a.total = total;
+  a.k_pitch = k_new.stride(0) / 8;
+  a.v_pitch = v_new.stride(0) / 8;
+  a.vecs = static_cast<int>(row / 8);
+  if (status.has_value()) { CHECK_I32((*status)); a.status = status->data_ptr<int>(); }
+  mb::gather_prefix_kv(a, cur_stream());
+  return {kf, vf};
+}
+
 // q [Tq, Hq, 128], k/v [Tkv, Hk, 128] (last dim contiguous, arbitrary row pitch); tiles int32 [n, 4].
 std::vector<at::Tensor> flash_attn_fwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& tiles,
                                        double scale, const c10::optional<at::Tensor>& status) {
@@ -213,6 +255,7 @@ void register_more(pybind11::module_& m) {
   m.def("flash_attn_fwd", &flash_attn_fwd);
   m.def("flash_attn_bwd", &flash_attn_bwd);
   m.def("router_small", &router_small);
+  m.def("gather_prefix_kv", &gather_prefix_kv);
   m.def("moe_small_up", &moe_small_up);
   m.def("moe_small_down", &moe_small_down);
   m.def("gae", &gae);

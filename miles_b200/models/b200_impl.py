@@ -429,7 +429,7 @@ class B200Qwen3:
         elif meta is not None and getattr(meta, "prefix", None) is not None:
             # prefill behind a cached prefix: the keys / values of the cached tokens come from their pages, the tile
             # table gives every query tile its sequence's key range and the position of its first query
-            kf, vf = meta.prefix.full_kv(k, self._v_view(qkv), *kv_cache[i])
+            kf, vf = self._full_kv(meta.prefix, k, self._v_view(qkv), *kv_cache[i])
             att, _ = self.C.flash_attn_fwd(q, kf, vf, meta.prefix.tiles, scale, self.status)
             self.launches += 5
         else:
@@ -450,24 +450,30 @@ class B200Qwen3:
             return yn.add_(x2)
         return self._row_parallel(C.swiglu_fwd(gu), P[p + "mlp.down.weight"], x2)
 
+    def _full_kv(self, prefix, k, v, kc, vc):
+        """``PrefixInfo.full_kv`` in one launch for caches of the activations' type."""
+        if kc.dtype != torch.bfloat16 or vc.dtype != torch.bfloat16:
+            return prefix.full_kv(k, v, kc, vc)
+        return self.C.gather_prefix_kv(k, v, kc, vc, prefix.pre_slots, prefix.pre_dst, prefix.new_dst, prefix.total, self.status)
+
     def _row_parallel(self, a, w, residual):
         """``residual + a @ w^T`` for a row-parallel weight: under tensor parallelism the GEMM epilogue pushes the
         partial sums to the peers and the slots are added in rank order (one fused GEMM + all-reduce)."""
         if self.tp is not None:
             self.launches += 3
             return self.tp.linear_allreduce(a, w, residual=residual, gemm_status=self.status)
-        y = self.linear(a, w)
-        return y.add_(residual) if residual is not None else y
-
-    def _o_proj_ln2(self, i, att2, x):
-        """Attention output projection, residual add and the second RMSNorm: returns (h2, rstd2, x2)."""
-        cfg, P, C = self.cfg, self.store.params, self.C
         if (residual is not None and self.SMALL_T < a.shape[0] <= 64 and self.small_decode and not getattr(self, "mx", None)
                 and a.is_contiguous() and w.shape[0] % 16 == 0 and w.shape[1] % 32 == 0):
             y = torch.empty_like(residual)  # the residual joins the sums before they are rounded
             self.C.small_gemv(a, None, 0.0, w, residual, y, self.status)
             self.launches += 1
             return y
+        y = self.linear(a, w)
+        return y.add_(residual) if residual is not None else y
+
+    def _o_proj_ln2(self, i, att2, x):
+        """Attention output projection, residual add and the second RMSNorm: returns (h2, rstd2, x2)."""
+        cfg, P, C = self.cfg, self.store.params, self.C
         p = f"layers.{i}."
         self.launches += 1
         if self.tp is not None:
