@@ -3,7 +3,8 @@
 // Cache layout: k_cache / v_cache are [num_slots, Hk, 128] bf16 where slot = page * page_size + offset
 // and block_table[b, i] is the i-th page of sequence b. Grid = (B, Hk, splits); every CTA serves all
 // G = Hq/Hk query heads of one KV head over its slice of the context so that each K/V row is read from
-// HBM exactly once. Partial (max, sum, out) triples are merged by a second kernel.
+// HBM exactly once. Up to 16 splits of one (sequence, KV head) form a cluster and merge their partial (max, sum, out)
+// triples through distributed shared memory; more splits go through scratch and a second kernel.
 //
 // Reference counterpart: flashinfer's trtllm_mha decode backend selected by the B200 recipe
 // (scripts/run_qwen3_30b_a3b.py:311-324).
@@ -45,14 +46,19 @@ __global__ void decode_merge_kernel(const float* __restrict__ part_o, const floa
 
 
 // ---------------------------------------------------------------------------------------------------
-// Tensor-core variant: K/V pages are staged through shared memory with cp.async (double buffered, 64
-// tokens per stage) and the G query heads of one KV head form the (zero padded) 16-row A operand of
+// K/V pages are staged through shared memory with cp.async (three stages of 64 tokens, so that two are in flight while
+// one is used: what bounds the kernel is how much of the cache each SM has asked for) and the G query heads of one KV head form the (zero padded) 16-row A operand of
 // mma.sync m16n8k16, so the work per K/V byte is a handful of instructions and the kernel runs at the
 // speed of the cache stream. Each of the 4 warps owns 16 tokens of a stage and keeps its own running
 // (max, sum, out); warps are merged through shared memory at the end.
 constexpr int TOK = 64;          // tokens per stage
 constexpr int LDS = D + 8;       // padded row (272 B) -> conflict-free ldmatrix
 constexpr int STAGE_ELEMS = TOK * LDS;
+constexpr int DSTAGES = 3;       // 104 KB: two CTAs per SM
+constexpr int MAX_CLUSTER_SPLITS = 16;
+// Measured (us a launch, pages of 64, caches larger than L2; before: two stages behind a CTA barrier and one page lookup per
+// row, merged by a second kernel; the keys' and values' bytes alone): 64 sequences of 1500 tokens, 4 KV heads 63 -> 37 (27);
+// 23 of 2300, 8 heads 58 -> 43 (30); 4 of 7900, 4 heads 28 -> 19.5 (9); 1 of 3000, 4 heads 13.8 -> 9.1 (0.8).
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int src_bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
@@ -73,15 +79,27 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&t);
 }
 
-template <int G>
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float ld_cluster_f32(uint32_t local_addr, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local_addr), "r"(rank));
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+
+// CLUSTER: the splits of one (b, h) are the CTAs of one cluster (rank = split) and merge here; `part_*` is not used.
+template <int G, bool CLUSTER>
 __global__ void __launch_bounds__(WARPS * 32)
 decode_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_cache, const bf16* __restrict__ v_cache,
                   const int* __restrict__ block_table, const int* __restrict__ seq_lens, float* __restrict__ part_o,
                   float* __restrict__ part_ml, bf16* __restrict__ out, int Hq, int Hk, int page_size, int max_pages,
                   int num_splits, float scale, long long num_slots, int* __restrict__ status) {
   extern __shared__ __align__(16) unsigned char dsm[];
-  bf16* Ks = reinterpret_cast<bf16*>(dsm);            // [2][TOK][LDS]
-  bf16* Vs = Ks + 2 * STAGE_ELEMS;                    // [2][TOK][LDS]
+  bf16* Ks = reinterpret_cast<bf16*>(dsm);            // [DSTAGES][TOK][LDS]
+  bf16* Vs = Ks + DSTAGES * STAGE_ELEMS;              // [DSTAGES][TOK][LDS]
   const int b = blockIdx.x, h = blockIdx.y, split = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // The length and the page ids come from device memory the caller filled: a length beyond the block-table row is
@@ -117,43 +135,74 @@ decode_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_cache, 
 #pragma unroll
   for (int j = 0; j < 16; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
 
-  auto issue = [&](int chunk, int stage) {
-    const int base = t_lo + chunk * TOK;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int piece = threadIdx.x + i * (WARPS * 32);
-      const int r = piece >> 4, c16 = piece & 15;
-      const int t = base + r;
-      bool ok = t < t_hi;
-      long long slot = 0;
-      if (ok) {
-        const long long page = table[t / page_size];
-        if (page < 0 || (num_slots > 0 && (page + 1) * page_size > num_slots)) {
-          ok = false;
-          if (c16 == 0 && status) atomicCAS(status, 0, 9);
-        } else {
-          slot = page * page_size + (t % page_size);
-        }
-      }
-      const long long off = (slot * Hk + h) * D + c16 * 8;
-      const uint32_t dk = static_cast<uint32_t>(__cvta_generic_to_shared(Ks + stage * STAGE_ELEMS + r * LDS + c16 * 8));
-      const uint32_t dv = static_cast<uint32_t>(__cvta_generic_to_shared(Vs + stage * STAGE_ELEMS + r * LDS + c16 * 8));
-      cp_async16(dk, k_cache + off, ok ? 16 : 0);
-      cp_async16(dv, v_cache + off, ok ? 16 : 0);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
+  // Every warp fetches the 16 tokens of a chunk that it multiplies itself, so warps wait for their own copies only and a
+  // stall of one is covered by the others. A chunk starts on a multiple of 64 tokens, so with pages of whole chunks it lies
+  // in one page; the page of the chunk after the next is looked up while this one is copied, since the lookup is a dependent
+  // access that would otherwise stand before every copy.
+  const bool whole = page_size % TOK == 0;
+  const int lrow = lane >> 4, c16 = lane & 15;
+  const uint32_t dk0 = static_cast<uint32_t>(__cvta_generic_to_shared(Ks + (warp * 16 + lrow) * LDS + c16 * 8));
+  const uint32_t dv0 = static_cast<uint32_t>(__cvta_generic_to_shared(Vs + (warp * 16 + lrow) * LDS + c16 * 8));
+  const long long row_elems = static_cast<long long>(Hk) * D;
+  int next_page = (whole && n_chunks > 0) ? table[t_lo / page_size] : 0;
+  int in_page = whole ? t_lo % page_size : 0, page_at = whole ? t_lo / page_size : 0;
+  auto valid = [&](long long page) {
+    const bool ok = !(page < 0 || (num_slots > 0 && (page + 1) * page_size > num_slots));
+    if (!ok && c16 == 0 && status) atomicCAS(status, 0, 9);
+    return ok;
   };
-
-  if (n_chunks > 0) issue(0, 0);
-  for (int ch = 0; ch < n_chunks; ++ch) {
-    const int stage = ch & 1;
-    if (ch + 1 < n_chunks) {
-      issue(ch + 1, stage ^ 1);
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
+  auto issue = [&](int chunk) {  // called for chunks 0, 1, 2, .. in order
+    const int stage = chunk % DSTAGES;
+    const int t0 = t_lo + chunk * TOK + warp * 16 + lrow;
+    const uint32_t dk = dk0 + stage * (STAGE_ELEMS * 2), dv = dv0 + stage * (STAGE_ELEMS * 2);
+    if (whole) {
+      const long long page = next_page;
+      const bool ok = valid(page);
+      const long long off = ((ok ? page * page_size + in_page : 0) + warp * 16 + lrow) * row_elems + h * D + c16 * 8;
+      const bf16 *ks = k_cache + off, *vs = v_cache + off;
+      in_page += TOK;
+      if (in_page == page_size) {
+        in_page = 0;
+        ++page_at;
+      }
+      if (chunk + 1 < n_chunks) next_page = table[page_at];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const bool live = ok && t0 + 2 * i < t_hi;  // (nothing is read where the size is 0; the address stays in the cache all the same)
+        const long long step = live ? 2 * i * row_elems : 0;
+        cp_async16(dk + i * (2 * LDS * 2), live ? ks + step : k_cache, live ? 16 : 0);
+        cp_async16(dv + i * (2 * LDS * 2), live ? vs + step : v_cache, live ? 16 : 0);
+      }
     } else {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int t = t0 + 2 * i;
+        bool ok = t < t_hi;
+        long long slot = 0;
+        if (ok) {
+          const long long page = table[t / page_size];
+          ok = valid(page);
+          if (ok) slot = page * page_size + t % page_size;
+        }
+        const long long off = slot * row_elems + h * D + c16 * 8;
+        cp_async16(dk + i * (2 * LDS * 2), k_cache + off, ok ? 16 : 0);
+        cp_async16(dv + i * (2 * LDS * 2), v_cache + off, ok ? 16 : 0);
+      }
     }
-    __syncthreads();
+  };
+  auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
+
+#pragma unroll
+  for (int ch = 0; ch < DSTAGES - 1; ++ch) {
+    if (ch < n_chunks) issue(ch);
+    commit();
+  }
+  for (int ch = 0; ch < n_chunks; ++ch) {
+    const int stage = ch % DSTAGES;
+    asm volatile("cp.async.wait_group %0;" ::"n"(DSTAGES - 2) : "memory");
+    __syncwarp();  // the chunk has landed for every lane, and every lane is done with the previous one, whose stage is refilled
+    if (ch + DSTAGES - 1 < n_chunks) issue(ch + DSTAGES - 1);
+    commit();  // (empty at the end, so that the group count stays)
     const bf16* Kst = Ks + stage * STAGE_ELEMS + (warp * 16) * LDS;
     const bf16* Vst = Vs + stage * STAGE_ELEMS + (warp * 16) * LDS;
     // ---- S = Q K^T for this warp's 16 tokens (two 8-token n-tiles)
@@ -206,8 +255,8 @@ decode_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_cache, 
       mma16816(o[2 * jp], pa, b0, b1);
       mma16816(o[2 * jp + 1], pa, b2, b3);
     }
-    __syncthreads();  // everyone is done with this stage before it is refilled
   }
+  __syncthreads();  // everyone is done with the stages, which the merge overlays
   // ---- merge the four warps (rows < G only) and write this split's partial
   float lsum = l_run;
   lsum += __shfl_xor_sync(0xffffffffu, lsum, 1);
@@ -215,6 +264,8 @@ decode_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_cache, 
   float* sm_o = reinterpret_cast<float*>(dsm);              // [WARPS][8][D]
   float* sm_m = sm_o + WARPS * 8 * D;                        // [WARPS][8]
   float* sm_l = sm_m + WARPS * 8;
+  float* cl_o = sm_l + WARPS * 8;                            // [8][D] this CTA's sums, for the cluster
+  float* cl_m = cl_o + 8 * D;                                // [8] maximum, [8] sum
   const int r0 = lane >> 2;
   if (r0 < G) {
 #pragma unroll
@@ -241,6 +292,14 @@ decode_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_cache, 
       gl += sm_l[w * 8 + g] * c;
       go += sm_o[(w * 8 + g) * D + d] * c;
     }
+    if constexpr (CLUSTER) {
+      cl_o[idx] = go;
+      if (d == 0) {
+        cl_m[g] = gm;
+        cl_m[8 + g] = gl;
+      }
+      continue;
+    }
     if (num_splits == 1) {  // nothing to merge: write the normalised output directly
       out[(static_cast<long long>(b) * Hq + h * G + g) * D + d] = __float2bfloat16(gl > 0.f ? go / gl : 0.f);
       continue;
@@ -251,6 +310,37 @@ decode_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_cache, 
       part_ml[base * 2] = gm;
       part_ml[base * 2 + 1] = gl;
     }
+  }
+  if constexpr (CLUSTER) {
+    // every CTA arrives, also one whose slice is empty; each then merges a share of the outputs in split order
+    cluster_sync_all();
+    const uint32_t o_addr = static_cast<uint32_t>(__cvta_generic_to_shared(cl_o));
+    const uint32_t m_addr = static_cast<uint32_t>(__cvta_generic_to_shared(cl_m));
+    for (int idx = split * (WARPS * 32) + threadIdx.x; idx < G * D; idx += num_splits * WARPS * 32) {
+      const int g = idx / D;
+      float m[MAX_CLUSTER_SPLITS], l[MAX_CLUSTER_SPLITS], v[MAX_CLUSTER_SPLITS];
+      float gm = -FLT_MAX;
+#pragma unroll
+      for (int sp = 0; sp < MAX_CLUSTER_SPLITS; ++sp)
+        if (sp < num_splits) {
+          m[sp] = ld_cluster_f32(m_addr + g * 4, sp);
+          l[sp] = ld_cluster_f32(m_addr + (8 + g) * 4, sp);
+          v[sp] = ld_cluster_f32(o_addr + idx * 4, sp);
+        }
+#pragma unroll
+      for (int sp = 0; sp < MAX_CLUSTER_SPLITS; ++sp)
+        if (sp < num_splits) gm = fmaxf(gm, m[sp]);
+      float gl = 0.f, go = 0.f;
+#pragma unroll
+      for (int sp = 0; sp < MAX_CLUSTER_SPLITS; ++sp)
+        if (sp < num_splits) {
+          const float c = m[sp] == -FLT_MAX ? 0.f : __expf(m[sp] - gm);
+          gl += l[sp] * c;
+          go += v[sp] * c;
+        }
+      out[(static_cast<long long>(b) * Hq + h * G) * D + idx] = __float2bfloat16(gl > 0.f ? go / gl : 0.f);
+    }
+    cluster_sync_all();  // no CTA leaves while another still reads its shared memory
   }
 }
 
@@ -267,26 +357,48 @@ int paged_decode_attention(const void* q, const void* k_cache, const void* v_cac
   float* part_ml = scratch + static_cast<long long>(B) * Hq * num_splits * D;
   const dim3 grid(B, Hk, num_splits);
   const int G = Hq / Hk;
-  constexpr int SMEM = 4 * STAGE_ELEMS * 2;  // K and V, two stages each
+  constexpr int SMEM = DSTAGES * 2 * STAGE_ELEMS * 2;
+  static_assert(SMEM >= ((WARPS + 1) * 8 * (D + 2)) * 4, "the merge overlays the stages");
   const bf16 *qp = static_cast<const bf16*>(q), *kp = static_cast<const bf16*>(k_cache), *vp = static_cast<const bf16*>(v_cache);
   bf16* op = static_cast<bf16*>(out);
   void* args[] = {&qp, &kp, &vp, &block_table, &seq_lens, &part_o, &part_ml, &op, &Hq, &Hk, &page_size, &max_pages,
                   &num_splits, &scale, &num_slots, &status};
+  const bool cluster = num_splits > 1 && num_splits <= MAX_CLUSTER_SPLITS;
   const void* fn = nullptr;
+#define MB_DECODE(G) fn = cluster ? reinterpret_cast<const void*>(&decode_mma_kernel<G, true>) : reinterpret_cast<const void*>(&decode_mma_kernel<G, false>)
   switch (G) {
-    case 1: fn = reinterpret_cast<const void*>(&decode_mma_kernel<1>); break;
-    case 2: fn = reinterpret_cast<const void*>(&decode_mma_kernel<2>); break;
-    case 4: fn = reinterpret_cast<const void*>(&decode_mma_kernel<4>); break;
-    case 8: fn = reinterpret_cast<const void*>(&decode_mma_kernel<8>); break;
+    case 1: MB_DECODE(1); break;
+    case 2: MB_DECODE(2); break;
+    case 4: MB_DECODE(4); break;
+    case 8: MB_DECODE(8); break;
     default: return static_cast<int>(cudaErrorInvalidValue);
   }
+#undef MB_DECODE
   // The attribute belongs to the (function, device) pair; setting it costs a table lookup, so it is set on every
   // call rather than remembered per process (a second device would otherwise launch with the 48 KB default).
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
   if (e != cudaSuccess) return static_cast<int>(e);
-  e = cudaLaunchKernel(fn, grid, dim3(WARPS * 32), args, SMEM, s);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(WARPS * 32);
+  cfg.dynamicSmemBytes = SMEM;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  if (cluster) {
+    if (num_splits > 8) {  // beyond the portable cluster size
+      e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      if (e != cudaSuccess) return static_cast<int>(e);
+    }
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = num_splits;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+  }
+  e = cudaLaunchKernelExC(&cfg, fn, args);
   if (e != cudaSuccess) return static_cast<int>(e);
-  if (num_splits > 1) {
+  if (num_splits > 1 && !cluster) {
     const float *po = part_o, *pm = part_ml;
     void* margs[] = {&po, &pm, &op, &num_splits};
     e = cudaLaunchKernel(reinterpret_cast<const void*>(&decode_merge_kernel), dim3(B * Hq), dim3(D), margs, 0, s);

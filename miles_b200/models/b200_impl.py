@@ -577,8 +577,11 @@ class B200Qwen3:
         return y
 
     def _decode_splits(self, B: int, meta: InferMeta) -> int:
-        ctas = B * self.cfg.num_kv_heads
-        return max(1, min(16, (148 * 3) // max(ctas, 1)))
+        # Two CTAs per SM at most: the splits of a sequence are a cluster that has to be placed as a whole. Clusters beyond the
+        # portable size of 8 fit only while they fill about two thirds of that (4 rows, 4 heads, us: 12 splits 19.5, 16 29.0).
+        ctas = max(B * self.cfg.num_kv_heads, 1)
+        splits = max(1, 296 // ctas)
+        return splits if splits <= 8 else min(16, max(8, 192 // ctas))
 
     def layer_backward(self, i, x, dy, positions, cu, max_seqlen, replay_ids=None):
         """Recompute layer i from its input ``x`` and back-propagate ``dy``; returns dx."""
