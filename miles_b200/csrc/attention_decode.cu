@@ -14,6 +14,7 @@
 #include <stdint.h>
 
 #include "launchers.h"
+#include "pdl.cuh"
 
 namespace mb {
 namespace {
@@ -32,6 +33,7 @@ __global__ void decode_merge_kernel(const float* __restrict__ part_o, const floa
                                     bf16* __restrict__ out, int num_splits) {
   const long long bh = blockIdx.x;  // b * Hq + head
   const int d = threadIdx.x;
+  pdl_enter();
   float gm = -FLT_MAX;
   for (int s = 0; s < num_splits; ++s) gm = fmaxf(gm, part_ml[(bh * num_splits + s) * 2]);
   float gl = 0.f, go = 0.f;
@@ -102,6 +104,7 @@ decode_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_cache, 
   bf16* Vs = Ks + DSTAGES * STAGE_ELEMS;              // [DSTAGES][TOK][LDS]
   const int b = blockIdx.x, h = blockIdx.y, split = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  pdl_enter();
   // The length and the page ids come from device memory the caller filled: a length beyond the block-table row is
   // clamped, and a page outside the cache is read as zeros (status 9) instead of being dereferenced.
   int len = seq_lens[b];
@@ -383,25 +386,26 @@ int paged_decode_attention(const void* q, const void* k_cache, const void* v_cac
   cfg.blockDim = dim3(WARPS * 32);
   cfg.dynamicSmemBytes = SMEM;
   cfg.stream = s;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
   if (cluster) {
     if (num_splits > 8) {  // beyond the portable cluster size
       e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
       if (e != cudaSuccess) return static_cast<int>(e);
     }
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = num_splits;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 1;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = num_splits;
+    cfg.numAttrs = 2;
   }
   e = cudaLaunchKernelExC(&cfg, fn, args);
   if (e != cudaSuccess) return static_cast<int>(e);
   if (num_splits > 1 && !cluster) {
-    const float *po = part_o, *pm = part_ml;
-    void* margs[] = {&po, &pm, &op, &num_splits};
-    e = cudaLaunchKernel(reinterpret_cast<const void*>(&decode_merge_kernel), dim3(B * Hq), dim3(D), margs, 0, s);
+    e = pdl_launch(decode_merge_kernel, dim3(B * Hq), dim3(D), 0, s, part_o, part_ml, op, num_splits);
   }
   return static_cast<int>(e);
 }

@@ -25,6 +25,7 @@
 #include <string>
 
 #include "launchers.h"
+#include "pdl.cuh"
 #include "ptx.cuh"
 
 namespace mb {
@@ -63,6 +64,7 @@ __device__ __forceinline__ float ex2(float x) {
 __global__ void __launch_bounds__(FA_THREADS, 1)
 fa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
               const __grid_constant__ CUtensorMap map_v, const FaArgs p) {
+  pdl_enter();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t q_s = base;
@@ -414,8 +416,7 @@ int flash_attn_fwd(const void* q, long long q_ld, const void* k, long long k_ld,
   a.T = Tq;
   a.scale_log2 = scale * 1.4426950408889634f;
   a.status = status;
-  fa_fwd_kernel<<<dim3(num_tiles, Hq), FA_THREADS, FA_SMEM, stream>>>(mq, mk, mv, a);
-  if (cudaGetLastError() != cudaSuccess) return fa_fail("attention forward launch failed");
+  if (pdl_launch(fa_fwd_kernel, dim3(num_tiles, Hq), FA_THREADS, FA_SMEM, stream, mq, mk, mv, a) != cudaSuccess) return fa_fail("attention forward launch failed");
   return 0;
 }
 

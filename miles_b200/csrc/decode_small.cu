@@ -17,6 +17,7 @@
 #include <stdint.h>
 
 #include "launchers.h"
+#include "pdl.cuh"
 
 namespace mb {
 namespace {
@@ -130,6 +131,10 @@ __global__ void __launch_bounds__(1024) small_gemv_kernel(const bf16* __restrict
   int k_begin, k_end;
   k_range(K, warp, nwarps, k_begin, k_end);
   const bool live = r < T;
+  // this warp's weights on their way into L2 while the predecessor finishes: 16 rows, a 128-byte line per lane and step
+  for (int k = k_begin + (lane & 1) * 64; k < k_end; k += 128)
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(W + static_cast<long long>(n0 + (lane >> 1)) * K + k));
+  pdl_enter();
   float acc[4] = {0.f, 0.f, 0.f, 0.f};
   float ss = 0.f;
   warp_dot<NORM, 4>(acc, W + static_cast<long long>(n0 + r) * K, W + static_cast<long long>(n0 + r + 8) * K,
@@ -176,6 +181,7 @@ __global__ void __launch_bounds__(256) router_small_kernel(const float* __restri
                                                            int renorm, int* __restrict__ topk_ids,
                                                            float* __restrict__ topk_w, int* __restrict__ active,
                                                            int* __restrict__ pair_count, int* __restrict__ pair_list) {
+  pdl_enter();
   __shared__ unsigned mask_s[32 * VALS];  // tokens that chose the expert
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int e = threadIdx.x; e < E; e += blockDim.x) mask_s[e] = 0u;
@@ -262,11 +268,11 @@ void small_gemv_direct(const void* x, int T, const void* norm_w, float eps, cons
                        const void* residual, void* out, bool out_fp32, cudaStream_t s) {
   const int threads = 32 * (warps_for(K) < 4 ? 4 : warps_for(K));  // the epilogue needs 128 threads
   if (norm_w)
-    small_gemv_kernel<true><<<N / 16, threads, 0, s>>>(static_cast<const bf16*>(x), T, static_cast<const bf16*>(norm_w),
+    pdl_launch(small_gemv_kernel<true>, N / 16, threads, 0, s, static_cast<const bf16*>(x), T, static_cast<const bf16*>(norm_w),
                                                        eps, static_cast<const bf16*>(W), N, K,
                                                        static_cast<const bf16*>(residual), out, out_fp32 ? 1 : 0);
   else
-    small_gemv_kernel<false><<<N / 16, threads, 0, s>>>(static_cast<const bf16*>(x), T, nullptr, eps,
+    pdl_launch(small_gemv_kernel<false>, N / 16, threads, 0, s, static_cast<const bf16*>(x), T, nullptr, eps,
                                                         static_cast<const bf16*>(W), N, K,
                                                         static_cast<const bf16*>(residual), out, out_fp32 ? 1 : 0);
 }
@@ -274,9 +280,9 @@ void small_gemv_direct(const void* x, int T, const void* norm_w, float eps, cons
 void router_small(const float* logits, int T, int E, int K, bool renorm, int* topk_ids, float* topk_w, int* active,
                   int* pair_count, int* pair_list, cudaStream_t s) {
   if (E <= 128)
-    router_small_kernel<4><<<1, 256, 0, s>>>(logits, T, E, K, renorm ? 1 : 0, topk_ids, topk_w, active, pair_count, pair_list);
+    pdl_launch(router_small_kernel<4>, 1, 256, 0, s, logits, T, E, K, renorm ? 1 : 0, topk_ids, topk_w, active, pair_count, pair_list);
   else  // up to 1024 experts (checked by the caller)
-    router_small_kernel<32><<<1, 256, 0, s>>>(logits, T, E, K, renorm ? 1 : 0, topk_ids, topk_w, active, pair_count, pair_list);
+    pdl_launch(router_small_kernel<32>, 1, 256, 0, s, logits, T, E, K, renorm ? 1 : 0, topk_ids, topk_w, active, pair_count, pair_list);
 }
 
 }  // namespace mb

@@ -28,6 +28,7 @@
 
 #include "gemm.h"
 #include "launchers.h"
+#include "pdl.cuh"
 #include "ptx.cuh"
 
 namespace mb {
@@ -127,6 +128,7 @@ __global__ void __launch_bounds__(THREADS, 1) stream_kernel(const StreamArgs a) 
     fence_barrier_init();
   }
   __syncthreads();
+  pdl_enter();
   const int n_groups = a.active ? a.active[0] : 1;
   const int tiles = a.rows / (ROWS * RT);
   const int total = n_groups * tiles;
@@ -313,8 +315,7 @@ int launch_variant(const StreamArgs& a, int grid, int smem, cudaStream_t s) {
   auto kern = stream_kernel<CPW, RT, EXACT>;
   // the attribute belongs to the (function, device) pair: set on every launch rather than once per process
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, RING_BYTES + 1024) != cudaSuccess) return -1;
-  kern<<<grid, THREADS, smem, s>>>(a);
-  return cudaGetLastError() == cudaSuccess ? 0 : -1;
+  return pdl_launch(kern, grid, THREADS, smem, s, a) == cudaSuccess ? 0 : -1;
 }
 
 int g_sms = 0;

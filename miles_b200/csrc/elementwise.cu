@@ -9,6 +9,7 @@
 #include <stdint.h>
 
 #include "launchers.h"
+#include "pdl.cuh"
 
 namespace mb {
 namespace {
@@ -69,6 +70,7 @@ template <int THREADS>
 __global__ void rmsnorm_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ res,
                                    const bf16* __restrict__ w, bf16* __restrict__ y, bf16* __restrict__ res_out,
                                    float* __restrict__ rstd, int H, float eps) {
+  pdl_enter();
   __shared__ float red[32];
   const long long row = blockIdx.x;
   const bf16* xr = x + row * H;
@@ -231,6 +233,7 @@ qk_norm_rope_fwd_kernel(const bf16* __restrict__ qkv, const bf16* __restrict__ q
                         float* __restrict__ q_rstd, float* __restrict__ k_rstd, bf16* __restrict__ k_cache,
                         bf16* __restrict__ v_cache, const int* __restrict__ slot_mapping, int T, int Hq, int Hk, float theta,
                         float eps, int use_norm, const float* __restrict__ inv_freq_tab, int rot_half, int chunks, int per) {
+  pdl_enter();
   constexpr int D = ROPE_D;
   const int lane = threadIdx.x & 31, half = lane >> 4, l = lane & 15;
   const int heads = Hq + 2 * Hk;
@@ -414,6 +417,7 @@ qk_norm_rope_bwd_kernel(const bf16* __restrict__ dq, const bf16* __restrict__ dk
 // blocks per SM, whose threads wait for one item's loads before they ask for the next.
 template <typename Index>
 __global__ void swiglu_fwd_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, Index n8, Index per_row) {
+  pdl_enter();
   for (Index idx = static_cast<Index>(blockIdx.x) * blockDim.x + threadIdx.x; idx < n8;
        idx += static_cast<Index>(gridDim.x) * blockDim.x) {
     const Index row = idx / per_row;
@@ -691,7 +695,7 @@ int grid_for(long long work_items, int threads, int cap = 148 * 8) {
 void rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void* res_out, float* rstd, int T, int H,
                  float eps, cudaStream_t s) {
   if (T <= 0) return;
-  rmsnorm_fwd_kernel<256><<<T, 256, 0, s>>>(static_cast<const bf16*>(x), static_cast<const bf16*>(res),
+  pdl_launch(rmsnorm_fwd_kernel<256>, T, 256, 0, s, static_cast<const bf16*>(x), static_cast<const bf16*>(res),
                                             static_cast<const bf16*>(w), static_cast<bf16*>(y),
                                             static_cast<bf16*>(res_out), rstd, H, eps);
 }
@@ -731,7 +735,7 @@ void qk_norm_rope_fwd(const void* qkv, const void* qw, const void* kw, const int
                       int rotary_dim) {
   if (T <= 0) return;
   const RopeSplit sp = rope_split(T, Hq + 2 * Hk, 148 * 8);
-  qk_norm_rope_fwd_kernel<<<sp.blocks, 256, 0, s>>>(
+  pdl_launch(qk_norm_rope_fwd_kernel, sp.blocks, 256, 0, s, 
       static_cast<const bf16*>(qkv), static_cast<const bf16*>(qw), static_cast<const bf16*>(kw), pos,
       static_cast<bf16*>(q_out), static_cast<bf16*>(k_out), q_rstd, k_rstd, static_cast<bf16*>(k_cache),
       static_cast<bf16*>(v_cache), slot_mapping, T, Hq, Hk, theta, eps, use_norm ? 1 : 0, inv_freq, rotary_dim / 2, sp.chunks, sp.per);
@@ -755,8 +759,8 @@ void swiglu_fwd(const void* in, void* out, long long T, int I, cudaStream_t s) {
   const int grid = grid_for(n8, 256, 1 << 24);
   const bf16* src = static_cast<const bf16*>(in);
   bf16* dst = static_cast<bf16*>(out);
-  if (n8 < (1ll << 31)) swiglu_fwd_kernel<unsigned><<<grid, 256, 0, s>>>(src, dst, static_cast<unsigned>(n8), static_cast<unsigned>(I / 8));
-  else swiglu_fwd_kernel<long long><<<grid, 256, 0, s>>>(src, dst, n8, I / 8);
+  if (n8 < (1ll << 31)) pdl_launch(swiglu_fwd_kernel<unsigned>, grid, 256, 0, s, src, dst, static_cast<unsigned>(n8), static_cast<unsigned>(I / 8));
+  else pdl_launch(swiglu_fwd_kernel<long long>, grid, 256, 0, s, src, dst, n8, I / 8);
 }
 
 void swiglu_bwd(const void* dout, const void* in, void* din, long long T, int I, cudaStream_t s) {

@@ -21,6 +21,7 @@
 #include <mutex>
 #include <string>
 
+#include "pdl.cuh"
 #include "ptx.cuh"
 
 namespace mb {
@@ -283,6 +284,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   }
   __syncthreads();
   const uint32_t tmem_base = tmem_base_s;
+  pdl_enter();
 
   const int total_tiles = num_tiles_of<BLOCK_N, B_MN>(p);
 
@@ -584,8 +586,7 @@ int launch(const GemmProblem& p, const KArgs& ka, cudaStream_t stream) {
   int grid = static_cast<int>(tiles < sms ? tiles : sms);
   if (p.max_ctas > 0 && grid > p.max_ctas) grid = p.max_ctas;
   if (grid <= 0) return 0;
-  kern<<<grid, kThreads, SMEM, stream>>>(ma, mb_, ka);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = pdl_launch(kern, grid, kThreads, SMEM, stream, ma, mb_, ka);
   if (e != cudaSuccess) return fail(std::string("gemm launch failed: ") + cudaGetErrorString(e));
   return 0;
 }

@@ -24,6 +24,7 @@
 #include <string>
 
 #include "gemm.h"
+#include "pdl.cuh"
 #include "ptx.cuh"
 
 namespace mb {
@@ -116,6 +117,11 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&tmem_slot_s);
+
+  // the first ring of weights on its way into L2 while the predecessor finishes
+  if (warp == 0 && lane == 0)
+    for (int kb = 0; kb < min(k_iters, p.stages); ++kb) tma_prefetch_2d(&map_w, (kb0 + kb) * BK, n0);
+  pdl_enter();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -293,13 +299,15 @@ int launch_skinny(const GemmProblem& g, const __nv_bfloat16* residual, cudaStrea
   cfg.blockDim = dim3(SK_THREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = split;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, mw, mx, p);
   if (e != cudaSuccess) return gemm_fail(std::string("skinny gemm launch failed: ") + cudaGetErrorString(e));
   return 0;

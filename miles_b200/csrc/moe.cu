@@ -20,6 +20,7 @@
 #include <stdint.h>
 
 #include "launchers.h"
+#include "pdl.cuh"
 
 namespace mb {
 namespace {
@@ -42,6 +43,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 __global__ void router_topk_kernel(const float* __restrict__ logits, const int* __restrict__ replay_ids,
                                    int* __restrict__ topk_ids, float* __restrict__ topk_w,
                                    float* __restrict__ probs_out, int T, int E, int K, int renorm) {
+  pdl_enter();
   const int wpb = blockDim.x >> 5;
   const int t = blockIdx.x * wpb + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -278,6 +280,7 @@ __global__ void __launch_bounds__(512)
 build_small_kernel(const int* __restrict__ ids, int n, int E, int max_rows, int max_tiles, int align,
                    int* __restrict__ counts_out, int* __restrict__ offsets, int* __restrict__ dest_row,
                    int* __restrict__ row_src, int* __restrict__ tiles, int* __restrict__ totals) {
+  pdl_enter();
   extern __shared__ int sm[];  // cnt[E], off[E+1], tstart[E+1], hist[warps][E]
   int* cnt = sm;
   int* off = cnt + E;
@@ -434,6 +437,7 @@ assign_kernel(const int* __restrict__ ids, int n, int E, const int* __restrict__
 __global__ void permute_kernel(const bf16* __restrict__ x, const int* __restrict__ row_src,
                                const int* __restrict__ num_m_tiles, bf16* __restrict__ x_perm, int max_rows, int H,
                                int K) {
+  pdl_enter();
   const int live_rows = min(num_m_tiles[1], max_rows);
   const int vec_per_row = H / 8;
   const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
@@ -478,6 +482,7 @@ constexpr int COMBINE_THREADS = 128;
 __global__ void __launch_bounds__(COMBINE_THREADS)
 combine_kernel(const bf16* __restrict__ y_perm, const int* __restrict__ dest_row, const float* __restrict__ topk_w,
                const bf16* __restrict__ residual, bf16* __restrict__ out, int T, int K, int H) {
+  pdl_enter();
   const int vec_per_row = H / 8;
   const int c = blockIdx.y * COMBINE_THREADS + threadIdx.x;
   if (c >= vec_per_row) return;
@@ -572,7 +577,7 @@ void moe_router_topk(const float* logits, const int* replay_ids, int* topk_ids, 
                      int T, int E, int K, bool renorm, cudaStream_t s) {
   if (T <= 0) return;
   const int wpb = 4;
-  router_topk_kernel<<<(T + wpb - 1) / wpb, wpb * 32, 0, s>>>(logits, replay_ids, topk_ids, topk_w, probs_out, T, E, K,
+  pdl_launch(router_topk_kernel, (T + wpb - 1) / wpb, wpb * 32, 0, s, logits, replay_ids, topk_ids, topk_w, probs_out, T, E, K,
                                                               renorm ? 1 : 0);
 }
 
@@ -601,10 +606,10 @@ void moe_build_permutation(const int* topk_ids, int T, int K, int E, int max_row
     const auto smem = [&](int warps) { return static_cast<size_t>((warps + 3) * E + 2) * sizeof(int); };
     if (n <= 512) {
       const int warps = n <= 128 ? 4 : 16;  // (four also fill row_src and the tile list quickly enough)
-      build_small_kernel<1><<<1, 32 * warps, smem(warps), s>>>(topk_ids, n, E, max_rows, max_tiles, align, expert_counts,
+      pdl_launch(build_small_kernel<1>, 1, 32 * warps, smem(warps), s, topk_ids, n, E, max_rows, max_tiles, align, expert_counts,
                                                                expert_offsets, dest_row, row_src, tile_group, num_m_tiles);
     } else {
-      build_small_kernel<8><<<1, 512, smem(16), s>>>(topk_ids, n, E, max_rows, max_tiles, align, expert_counts, expert_offsets,
+      pdl_launch(build_small_kernel<8>, 1, 512, smem(16), s, topk_ids, n, E, max_rows, max_tiles, align, expert_counts, expert_offsets,
                                                      dest_row, row_src, tile_group, num_m_tiles);
     }
     return;
@@ -625,7 +630,7 @@ void moe_build_permutation(const int* topk_ids, int T, int K, int E, int max_row
 void moe_permute(const void* x, const int* row_src, const int* num_m_tiles, void* x_perm, int max_rows, int H, int K,
                  cudaStream_t s) {
   if (max_rows <= 0) return;
-  permute_kernel<<<grid_for(max_rows, 8), 256, 0, s>>>(static_cast<const bf16*>(x), row_src, num_m_tiles,
+  pdl_launch(permute_kernel, grid_for(max_rows, 8), 256, 0, s, static_cast<const bf16*>(x), row_src, num_m_tiles,
                                                        static_cast<bf16*>(x_perm), max_rows, H, K);
 }
 
@@ -633,7 +638,7 @@ void moe_combine(const void* y_perm, const int* dest_row, const float* topk_w, c
                  int K, int H, cudaStream_t s) {
   if (T <= 0) return;
   const dim3 grid(T, (H / 8 + COMBINE_THREADS - 1) / COMBINE_THREADS);
-  combine_kernel<<<grid, COMBINE_THREADS, 0, s>>>(static_cast<const bf16*>(y_perm), dest_row, topk_w,
+  pdl_launch(combine_kernel, grid, COMBINE_THREADS, 0, s, static_cast<const bf16*>(y_perm), dest_row, topk_w,
                                                   static_cast<const bf16*>(residual), static_cast<bf16*>(out), T, K, H);
 }
 

@@ -1,0 +1,43 @@
+// Programmatic dependent launch: a kernel launched with `pdl_launch` may become resident while its predecessor in the stream
+// still runs, and waits for it on the device. What a decode step of a few rows pays for most is not bytes but the start of a
+// hundred and more short kernels a step: launch latency, CTA start, barrier and TMEM set-up, tensor-map and instruction
+// fetches now overlap with the kernel before.
+//
+// Measured on whole calls (before -> after): a 93-token prompt of a dense model 1.58 -> 1.37 ms, 24 decode steps of 16 rows of
+// the mixture 91 -> 85 ms, of 64 rows 142 -> 139, of one row 32.3 -> 31.3.
+//
+// Rules that keep it safe:
+//   * every kernel launched this way calls `pdl_enter` (or `pdl_wait`) in every thread before it touches global memory other
+//     than to prefetch into L2, the point of coherence: the wait returns when the predecessor has completed and its writes
+//     are visible; since that one did the same, all earlier kernels of the stream have completed too;
+//   * dependents are let in only after the wait, by CTAs that are resident, so no CTA of a kernel waits for a place that a
+//     later kernel holds;
+//   * a kernel launched in the ordinary way before or after depends, and is depended on, as always.
+#pragma once
+#include <cuda_runtime.h>
+
+namespace mb {
+
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_let_dependents_in() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_enter() {
+  pdl_wait();
+  pdl_let_dependents_in();
+}
+
+template <typename... P, typename... A>
+cudaError_t pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+}  // namespace mb
