@@ -21,8 +21,15 @@
 //   warps 2..9  : P^T / dS^T math, two threads per key row (32 query columns each); dK / dV epilogue
 //   warps 10..13: dQ^T read-out and global accumulation (one thread per d)
 //
-// TMEM columns: S^T 0..63, dP^T 64..127, dV 128..255, dK 256..383, dQ^T 384..447. Every mbarrier wait is bounded
-// (ptx.cuh): on expiry the CTA records a status code, leaves its loops, frees TMEM and returns.
+// Two tiles are in flight: S^T / dP^T have two buffers in TMEM and P^T / dS^T two in shared memory, so the tensor core runs
+// dV, dK, dQ^T of one tile and S^T, dP^T of the tile after the next while the threads work on the tile between. dQ^T of a
+// tile goes where its S^T was (read by then), and the S^T after the next waits for the dQ^T to be read out.
+//
+// TMEM columns: S^T / dQ^T 0..63 and 64..127, dP^T 128..191 and 192..255, dV 256..383, dK 384..511. Every mbarrier wait is
+// bounded (ptx.cuh): on expiry the CTA records a status code, leaves its loops, frees TMEM and returns.
+//
+// Measured: 9216 tokens in one sequence, 32 heads over 8: 4.43 ms with one tile in flight, 3.74 ms with two; 16384 tokens in 6
+// equal sequences, 32 heads over 4: 1.95 ms (470 TFLOP/s). What bounds it now is not known; the dQ sums in L2 are the first suspect.
 //
 // Reference counterpart: the flash-attention backward behind `--attention-backend flash`
 // (scripts/run_qwen3_30b_a3b.py:203).
@@ -48,7 +55,7 @@ constexpr int QTILE = 2 * ATOM_Q;    // Q or dO tile
 constexpr int PTILE = ATOM_K;        // P^T or dS^T: 128 keys x 64 q
 constexpr int STAGES = 3;
 constexpr int BWD_THREADS = 14 * 32;
-constexpr int BWD_SMEM = 2 * KTILE + 2 * PTILE + STAGES * 2 * QTILE + STAGES * 2 * BQ * 4 + 256 + 1024;
+constexpr int BWD_SMEM = 2 * KTILE + 4 * PTILE + STAGES * 2 * QTILE + STAGES * 2 * BQ * 4 + 256 + 1024;
 
 struct FaBwdArgs {
   const int4* blocks;  // {kv_row0 (global token index of the block's first key), kv_rows, kv_pos0 (its position in the
@@ -85,12 +92,12 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
   const uint32_t v_s = k_s + KTILE;
   const uint32_t pt_s = v_s + KTILE;
   const uint32_t ds_s = pt_s + PTILE;
-  const uint32_t ring = ds_s + PTILE;                      // per stage: Q tile, dO tile
+  const uint32_t ring = pt_s + 4 * PTILE;                  // (P^T, dS^T) twice; per stage: Q tile, dO tile
   const uint32_t stats = ring + STAGES * 2 * QTILE;        // per stage: lse2[64], dsum[64]
   const uint32_t bars = stats + STAGES * 2 * BQ * 4;
   auto BAR = [&](int i) { return bars + 8u * i; };
-  constexpr int B_KVF = 0, B_QF = 1, B_QE = 4, B_SF = 7, B_PF = 8, B_DQF = 9, B_DQE = 10, B_FIN = 11;
-  const uint32_t tmem_slot = bars + 8u * 12;
+  constexpr int B_KVF = 0, B_QF = 1, B_QE = 4, B_SF = 7, B_PF = 9, B_DQF = 11, B_DQE = 12, B_FIN = 13;
+  const uint32_t tmem_slot = bars + 8u * 14;
   __shared__ int abort_s;
   __shared__ uint32_t tmem_base_s;
   volatile int* abort_flag = &abort_s;
@@ -114,8 +121,10 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
       mbar_init(BAR(B_QF + s), 1);
       mbar_init(BAR(B_QE + s), 1);
     }
-    mbar_init(BAR(B_SF), 1);
-    mbar_init(BAR(B_PF), 8);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(BAR(B_SF + b), 1);
+      mbar_init(BAR(B_PF + b), 8);
+    }
     mbar_init(BAR(B_DQF), 1);
     mbar_init(BAR(B_DQE), 4);
     mbar_init(BAR(B_FIN), 1);
@@ -139,7 +148,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
   }
   __syncthreads();
   const uint32_t tmem = tmem_base_s;
-  const uint32_t t_S = tmem, t_dP = tmem + 64, t_dV = tmem + 128, t_dK = tmem + 256, t_dQ = tmem + 384;
+  const uint32_t t_S = tmem, t_dP = tmem + 128, t_dV = tmem + 256, t_dK = tmem + 384;  // t_S, t_dP: + 64 for odd tiles
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -194,64 +203,63 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
       if (!mbar_wait(BAR(B_QF + st), (it / STAGES) & 1, abort_flag, p.status, ERR_WAIT_FULL)) return false;
       tc_fence_after();
       if (lane == 0) {
-        const uint32_t qd = ring + st * 2 * QTILE, dd = qd + QTILE;
+        const uint32_t qd = ring + st * 2 * QTILE, dd = qd + QTILE, buf = (it & 1) * 64;
 #pragma unroll
         for (int k = 0; k < HD / 16; ++k) {
           const uint32_t ka = (k >> 2) * ATOM_K + (k & 3) * 32, qa = (k >> 2) * ATOM_Q + (k & 3) * 32;
-          umma_f16(t_S, make_smem_desc(k_s + ka, 16, 1024), make_smem_desc(qd + qa, 16, 1024), id_s, k > 0 ? 1u : 0u);
+          umma_f16(t_S + buf, make_smem_desc(k_s + ka, 16, 1024), make_smem_desc(qd + qa, 16, 1024), id_s, k > 0 ? 1u : 0u);
         }
 #pragma unroll
         for (int k = 0; k < HD / 16; ++k) {
           const uint32_t ka = (k >> 2) * ATOM_K + (k & 3) * 32, qa = (k >> 2) * ATOM_Q + (k & 3) * 32;
-          umma_f16(t_dP, make_smem_desc(v_s + ka, 16, 1024), make_smem_desc(dd + qa, 16, 1024), id_s, k > 0 ? 1u : 0u);
+          umma_f16(t_dP + buf, make_smem_desc(v_s + ka, 16, 1024), make_smem_desc(dd + qa, 16, 1024), id_s, k > 0 ? 1u : 0u);
         }
-        umma_commit(BAR(B_SF));
+        umma_commit(BAR(B_SF + (it & 1)));
       }
       __syncwarp();
       return true;
     };
     if (ok && n_it > 0) ok = issue_s(0);
+    if (ok && n_it > 1) ok = issue_s(1);
     for (int it = 0; ok && it < n_it; ++it) {
       const int st = it % STAGES;
-      if (!mbar_wait(BAR(B_PF), it & 1, abort_flag, p.status, ERR_WAIT_TMEM_EMPTY)) {
+      if (!mbar_wait(BAR(B_PF + (it & 1)), (it >> 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_EMPTY)) {
         ok = false;
         break;
       }
       tc_fence_after();
       if (lane == 0) {
         const uint32_t qd = ring + st * 2 * QTILE, dd = qd + QTILE;
+        const uint32_t pt = pt_s + (it & 1) * 2 * PTILE, ds = ds_s + (it & 1) * 2 * PTILE;
+        // dQ^T first, since its read-out is the longest way to the next S^T; it overwrites this tile's S^T, which has been read
+#pragma unroll
+        for (int k = 0; k < BK / 16; ++k) {  // contraction over the 128 keys
+          umma_f16(t_S + (it & 1) * 64, make_smem_desc(k_s + k * 2048, ATOM_K, 1024), make_smem_desc(ds + k * 2048, ATOM_K, 1024), id_dq,
+                   k > 0 ? 1u : 0u);
+        }
+        umma_commit(BAR(B_DQF));
 #pragma unroll
         for (int k = 0; k < BQ / 16; ++k) {  // contraction over the 64 queries of the tile
-          umma_f16(t_dV, make_smem_desc(pt_s + k * 32, 16, 1024), make_smem_desc(dd + k * 2048, ATOM_Q, 1024), id_acc,
+          umma_f16(t_dV, make_smem_desc(pt + k * 32, 16, 1024), make_smem_desc(dd + k * 2048, ATOM_Q, 1024), id_acc,
                    (it > 0 || k > 0) ? 1u : 0u);
         }
 #pragma unroll
         for (int k = 0; k < BQ / 16; ++k) {
-          umma_f16(t_dK, make_smem_desc(ds_s + k * 32, 16, 1024), make_smem_desc(qd + k * 2048, ATOM_Q, 1024), id_acc,
+          umma_f16(t_dK, make_smem_desc(ds + k * 32, 16, 1024), make_smem_desc(qd + k * 2048, ATOM_Q, 1024), id_acc,
                    (it > 0 || k > 0) ? 1u : 0u);
         }
         umma_commit(BAR(B_QE + st));  // the (Q, dO) stage is free once these have run
       }
       __syncwarp();
-      if (it + 1 < n_it && !issue_s(it + 1)) {
+      // dQ^T of this tile is out before the next one's is announced, and before an S^T takes its place
+      if (it + 1 < n_it && !mbar_wait(BAR(B_DQE), it & 1, abort_flag, p.status, ERR_WAIT_TMEM_EMPTY)) {
         ok = false;
         break;
       }
-      // dQ^T of this tile overwrites the read-out buffer of the previous one
-      if (it > 0 && !mbar_wait(BAR(B_DQE), (it - 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_EMPTY)) {
+      if (it + 2 < n_it && !issue_s(it + 2)) {
         ok = false;
         break;
       }
-      tc_fence_after();
-      if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < BK / 16; ++k) {  // contraction over the 128 keys
-          umma_f16(t_dQ, make_smem_desc(k_s + k * 2048, ATOM_K, 1024), make_smem_desc(ds_s + k * 2048, ATOM_K, 1024), id_dq,
-                   k > 0 ? 1u : 0u);
-        }
-        umma_commit(BAR(B_DQF));
-      }
-      __syncwarp();
     }
     if (ok && lane == 0) umma_commit(BAR(B_FIN));
     __syncwarp();
@@ -266,14 +274,15 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     for (int it = 0; it < n_it; ++it) {
       const int st = it % STAGES;
       const int g = it / n_qt, qt = it - g * n_qt;
-      if (!mbar_wait(BAR(B_SF), it & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) {
+      if (!mbar_wait(BAR(B_SF + (it & 1)), (it >> 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) {
         ok = false;
         break;
       }
       tc_fence_after();
       uint32_t s[32], d[32];
-      tmem_ld_32x32(t_S + lane_addr + half * 32, s);
-      tmem_ld_32x32(t_dP + lane_addr + half * 32, d);
+      const uint32_t buf = (it & 1) * 64;
+      tmem_ld_32x32(t_S + buf + lane_addr + half * 32, s);
+      tmem_ld_32x32(t_dP + buf + lane_addr + half * 32, d);
       tmem_ld_wait();
       const float* sp = stats_g + st * 2 * BQ + half * 32;
       // query j of this thread sits at sequence offset qt*64 + half*32 + j from the block's first key
@@ -294,25 +303,22 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
         pp[j] = pack_bf16(pv[0], pv[1]);
         dd[j] = pack_bf16(dv[0], dv[1]);
       }
-      // the P^T / dS^T tiles are still read by the MMAs of the previous tile until its dQ^T has run
-      if (it > 0 && !mbar_wait(BAR(B_DQF), (it - 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) {
-        ok = false;
-        break;
-      }
+      // (this buffer of P^T / dS^T was read by the MMAs of the tile before the last, which ran before this tile's S^T did)
+      const uint32_t pt = pt_s + (it & 1) * 2 * PTILE, ds = ds_s + (it & 1) * 2 * PTILE;
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         const uint32_t o = swz_off(row, half * 4 + c);
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(pt_s + o), "r"(pp[4 * c]), "r"(pp[4 * c + 1]),
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(pt + o), "r"(pp[4 * c]), "r"(pp[4 * c + 1]),
                      "r"(pp[4 * c + 2]), "r"(pp[4 * c + 3])
                      : "memory");
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(ds_s + o), "r"(dd[4 * c]), "r"(dd[4 * c + 1]),
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(ds + o), "r"(dd[4 * c]), "r"(dd[4 * c + 1]),
                      "r"(dd[4 * c + 2]), "r"(dd[4 * c + 3])
                      : "memory");
       }
       fence_proxy_async();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(BAR(B_PF));
+      if (lane == 0) mbar_arrive(BAR(B_PF + (it & 1)));
     }
     // ---- epilogue: dV, dK (scaled) -> bf16
     if (ok) ok = mbar_wait(BAR(B_FIN), 0, abort_flag, p.status, ERR_WAIT_TMEM_FULL);
@@ -354,8 +360,8 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
       if (!mbar_wait(BAR(B_DQF), it & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL)) break;
       tc_fence_after();
       uint32_t a[32], b[32];
-      tmem_ld_32x32(t_dQ + lane_addr, a);
-      tmem_ld_32x32(t_dQ + lane_addr + 32, b);
+      tmem_ld_32x32(t_S + (it & 1) * 64 + lane_addr, a);
+      tmem_ld_32x32(t_S + (it & 1) * 64 + lane_addr + 32, b);
       tmem_ld_wait();
       tc_fence_before();
       __syncwarp();
