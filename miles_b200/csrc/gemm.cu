@@ -820,9 +820,18 @@ int gemm_bf16_launch(const GemmProblem& p, cudaStream_t stream) {
     const long long m_tiles = p.mode == GEMM_GROUPED_ROWS ? p.max_tiles : (p.M + BLOCK_M - 1) / BLOCK_M;
     const long long groups = p.mode == GEMM_GROUPED_CONTR ? p.num_groups : 1;
     auto tiles = [&](int b) { return m_tiles * ((p.N + b - 1) / b) * groups; };
-    // Prefer the 128x256 tile unless it leaves most SMs idle or wastes a large share of the tile.
-    const bool waste256 = (p.N % 256) != 0 && (p.N % 256) <= 128;
-    bn = (tiles(256) >= sms && !waste256) || (p.N >= 256 && tiles(256) >= 2 * sms) ? 256 : 128;
+    if (p.mode == GEMM_GROUPED_ROWS) {
+      // (how many row tiles are live is known on the device only: prefer the 128x256 tile unless even the capacity leaves most
+      // SMs idle or it wastes a large share of the tile)
+      const bool waste256 = (p.N % 256) != 0 && (p.N % 256) <= 128;
+      bn = (tiles(256) >= sms && !waste256) || (p.N >= 256 && tiles(256) >= 2 * sms) ? 256 : 128;
+    } else {
+      // A wave of 128x256 tiles takes as long as one of 128x128 tiles, which are bound by what they read from shared memory
+      // (777 x 2048, K = 9728, one wave of either: 59 and 62 us), so the wider tile whenever it needs fewer waves (2048 x 2048,
+      // K = 151936, 128 or 256 tiles: 905 us against 1402).
+      const auto waves = [&](int b) { return (tiles(b) + sms - 1) / sms; };
+      bn = waves(256) < waves(128) ? 256 : 128;
+    }
     if (p.N <= 128) bn = 128;
     // Skinny problems (decode projections): narrower tiles spread the weight stream over more SMs.
     if (!amn && !bmn && tiles(bn) < sms) {
