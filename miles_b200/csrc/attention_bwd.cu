@@ -28,8 +28,9 @@
 // TMEM columns: S^T / dQ^T 0..63 and 64..127, dP^T 128..191 and 192..255, dV 256..383, dK 384..511. Every mbarrier wait is
 // bounded (ptx.cuh): on expiry the CTA records a status code, leaves its loops, frees TMEM and returns.
 //
-// Measured: 9216 tokens in one sequence, 32 heads over 8: 4.43 ms with one tile in flight, 3.74 ms with two; 16384 tokens in 6
-// equal sequences, 32 heads over 4: 1.95 ms (470 TFLOP/s). What bounds it now is not known; the dQ sums in L2 are the first suspect.
+// Measured, 32 heads: 9216 tokens in one sequence, 8 KV heads, 4.02 ms with one tile in flight and one head's blocks after
+// another, 3.74 with two tiles, 3.07 (567 TFLOP/s) with heads fastest; 16384 in six sequences, 4 KV heads, 2.07 -> 1.89 ms. The
+// sums into dQ keep L2's atomic units 12 % busy: the chain from S^T to dQ^T of a tile is what bounds it.
 //
 // Reference counterpart: the flash-attention backward behind `--attention-backend flash`
 // (scripts/run_qwen3_30b_a3b.py:203).
@@ -105,8 +106,10 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
   float* stats_g = reinterpret_cast<float*>(gen + (stats - base));
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int4 blk = p.blocks[blockIdx.x];
-  const int hk = blockIdx.y;
+  // Heads vary fastest: the list starts with the blocks that have the most queries after them, and all heads' long blocks have
+  // to start before anyone's short ones (one head after another left SMs with 1.4 times the average work at the end).
+  const int4 blk = p.blocks[blockIdx.x / p.Hk];
+  const int hk = blockIdx.x % p.Hk;
   const int G = p.Hq / p.Hk;
   const int kv_row0 = blk.x, kv_rows = blk.y, kv_pos0 = blk.z, seq_end = blk.w;
   // query rows at or after the block's first key (positions kv_pos0 ..): global rows kv_row0 .. seq_end - 1
@@ -504,7 +507,7 @@ int flash_attn_bwd(const void* q, long long q_ld, const void* k, long long k_ld,
   a.scale = scale;
   a.scale_log2 = scale * 1.4426950408889634f;
   a.status = status;
-  fa_bwd_kernel<<<dim3(num_blocks, Hk), BWD_THREADS, BWD_SMEM, stream>>>(mq, mdo, mk, mv, a);
+  fa_bwd_kernel<<<num_blocks * Hk, BWD_THREADS, BWD_SMEM, stream>>>(mq, mdo, mk, mv, a);
   if (cudaPeekAtLastError() != cudaSuccess) return fail("attention backward launch failed");
   const long long n4 = T * Hq * HD / 4;
   long long cb = (n4 + 255) / 256;

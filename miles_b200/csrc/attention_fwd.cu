@@ -82,8 +82,10 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
   volatile int* abort_flag = &abort_s;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int4 tile = p.tiles[blockIdx.x];
-  const int hq = blockIdx.y;
+  // Heads vary fastest: the list starts with the tiles of the longest key ranges, and all heads' long tiles have to start
+  // before anyone's short ones; heads that share keys and values also run side by side.
+  const int4 tile = p.tiles[blockIdx.x / p.Hq];
+  const int hq = blockIdx.x % p.Hq;
   const int hk = hq / (p.Hq / p.Hk);
   const int q_row0 = tile.x, q_rows = tile.y, kv_row0 = tile.z, q_pos0 = tile.w;
   const int kv_len = q_pos0 + q_rows;               // causal: keys up to the last query of the tile
@@ -416,7 +418,7 @@ int flash_attn_fwd(const void* q, long long q_ld, const void* k, long long k_ld,
   a.T = Tq;
   a.scale_log2 = scale * 1.4426950408889634f;
   a.status = status;
-  if (pdl_launch(fa_fwd_kernel, dim3(num_tiles, Hq), FA_THREADS, FA_SMEM, stream, mq, mk, mv, a) != cudaSuccess) return fa_fail("attention forward launch failed");
+  if (pdl_launch(fa_fwd_kernel, num_tiles * Hq, FA_THREADS, FA_SMEM, stream, mq, mk, mv, a) != cudaSuccess) return fa_fail("attention forward launch failed");
   return 0;
 }
 
