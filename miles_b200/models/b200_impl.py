@@ -211,7 +211,7 @@ class B200Qwen3:
         T, K = ids.shape
         max_rows = max(T * K + E_local * (align - 1), 1)
         counts, offsets, dest, src, tg, nt = self.C.moe_build_permutation(ids, E_local, max_rows, align)
-        self.launches += 3
+        self.launches += 1 if T * K <= 4096 and max_rows <= 16384 and E_local <= 512 else 3
         ctx = MoeCtx(ids, None, None, offsets, dest, src, tg, nt, max_rows)
         ctx.align = align
         return ctx
@@ -425,13 +425,13 @@ class B200Qwen3:
             kc, vc = kv_cache[i]
             C.paged_decode_attention(q, kc, vc, meta.block_table, meta.seq_lens, att, self._decode_scratch, meta.page_size,
                                      splits, scale)
-            self.launches += 2
+            self.launches += 1
         elif meta is not None and getattr(meta, "prefix", None) is not None:
             # prefill behind a cached prefix: the keys / values of the cached tokens come from their pages, the tile
             # table gives every query tile its sequence's key range and the position of its first query
             kf, vf = self._full_kv(meta.prefix, k, self._v_view(qkv), *kv_cache[i])
             att, _ = self.C.flash_attn_fwd(q, kf, vf, meta.prefix.tiles, scale, self.status)
-            self.launches += 5
+            self.launches += 2
         else:
             att, _ = self.attention(q, k, self._v_view(qkv), cu)
         h2, _, x2 = self._o_proj_ln2(i, att.view(att.shape[0], -1), x)
@@ -530,7 +530,7 @@ class B200Qwen3:
                                  splits, cfg.head_dim ** -0.5)
         x2 = torch.empty_like(x)
         C.small_gemv(att.view(T, -1), None, cfg.rms_eps, P[p + "attn.o.weight"], x, x2, self.status)
-        self.launches += 6
+        self.launches += 4
         return x2
 
     def _layer_forward_small(self, i, x, positions, meta: InferMeta, kv_cache, record=None):
