@@ -172,7 +172,7 @@ __global__ void colsum_kernel(const float* __restrict__ part, float* __restrict_
 // the four they pair with, so a rotation needs no exchange; the four angles of a lane are shared with the other half-warp,
 // each takes two. A token's heads are dealt to `chunks` warps: few tokens (decoding) need the parallelism, many do not.
 // 16384 tokens, 32 query + 4 key heads: forward 363 -> 125 us, backward 416 -> 172 us (302 and 453 MB moved);
-// one token (in a captured graph): 2.9 -> 2.6 us..
+// one token (in a captured graph): 2.9 -> 2.6 us.
 constexpr int ROPE_D = 128;
 
 struct Four {
@@ -186,10 +186,22 @@ __device__ __forceinline__ Four unpack4(const uint2& r) {
 __device__ __forceinline__ uint2 pack4(const Four& f) { return make_uint2(pack2(f.v[0], f.v[1]), pack2(f.v[2], f.v[3])); }
 __device__ __forceinline__ uint2 ld8b(const bf16* p) { return *reinterpret_cast<const uint2*>(p); }
 __device__ __forceinline__ void st8b(bf16* p, const uint2& v) { *reinterpret_cast<uint2*>(p) = v; }
-__device__ __forceinline__ float half_warp_sum(float v) {
+// Sum over a head from a lane's two sums of four. The order is fixed, whatever rot_half and the lanes' share of a head: sums of
+// four consecutive dimensions, to which the ones 64, 32, 16, 8 and 4 dimensions further are added in turn. (Another order, or
+// another place of the fused multiply-add in the rotation, rounds one value in 10^5 differently; through the layers that became
+// 1 % of a short pack's gradients, and single values of sparse ones by more than their root mean square.)
+__device__ __forceinline__ float head_sum(float a, float b, int rot_half) {
+  if (rot_half == 64) {  // (b lies 64 dimensions after a, the lane 8 further 32)
+    a += b;
+    a += __shfl_xor_sync(0xffffffffu, a, 8);
+  } else {  // (the other way round)
+    a += __shfl_xor_sync(0xffffffffu, a, 8);
+    b += __shfl_xor_sync(0xffffffffu, b, 8);
+    a += b;
+  }
 #pragma unroll
-  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
+  for (int o = 4; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+  return a;
 }
 
 // Where lane l of a half-warp finds its values in a head, and the angles it rotates them by. rot_half = 64: dimension d pairs with
@@ -257,10 +269,13 @@ qk_norm_rope_fwd_kernel(const bf16* __restrict__ qkv, const bf16* __restrict__ q
       if (act) ra = ld8b(row + h * D + rl.a), rb = ld8b(row + h * D + rl.b);
       Four x = unpack4(ra), y = unpack4(rb);
       if (use_norm) {
-        float ss = 0.f;
+        float sx = 0.f, sy = 0.f;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) ss += x.v[i] * x.v[i] + y.v[i] * y.v[i];
-        ss = half_warp_sum(ss);
+        for (int i = 0; i < 4; ++i) {
+          sx += x.v[i] * x.v[i];
+          sy += y.v[i] * y.v[i];
+        }
+        const float ss = head_sum(sx, sy, rot_half);
         const float r = rsqrtf(ss / D + eps);
         const Four wa = unpack4(is_q ? wqa : wka), wb = unpack4(is_q ? wqb : wkb);
         // match the unfused path: the normalised value is rounded to bf16 before the rotation
@@ -283,12 +298,13 @@ qk_norm_rope_fwd_kernel(const bf16* __restrict__ qkv, const bf16* __restrict__ q
         }
         continue;
       }
-      // rotate-half RoPE: out[d] = x[d]*cos - x[d+64]*sin (d<64); out[d+64] = x[d+64]*cos + x[d]*sin
+      // rotate-half RoPE: out[d] = x[d]*cos - x[d+64]*sin (d<64); out[d+64] = x[d+64]*cos + x[d]*sin, each with the first
+      // dimension's product fused and the other one rounded, whatever the compiler would choose
       Four u, w;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        u.v[i] = x.v[i] * cs.v[i] - y.v[i] * sn.v[i];
-        w.v[i] = y.v[i] * cs.v[i] + x.v[i] * sn.v[i];
+        u.v[i] = __fmaf_rn(x.v[i], cs.v[i], -__fmul_rn(y.v[i], sn.v[i]));
+        w.v[i] = __fmaf_rn(x.v[i], sn.v[i], __fmul_rn(y.v[i], cs.v[i]));
       }
       if (!rl.rotated) u = x, w = y;
       const uint2 oa = pack4(u), ob = pack4(w);
@@ -360,21 +376,24 @@ qk_norm_rope_bwd_kernel(const bf16* __restrict__ dq, const bf16* __restrict__ dk
         }
       }
       const Four g = unpack4(ga), e = unpack4(gb);
-      // inverse rotation: dx[d] = g[d]*cos + g[d+64]*sin ; dx[d+64] = g[d+64]*cos - g[d]*sin
+      // inverse rotation: dx[d] = g[d]*cos + g[d+64]*sin ; dx[d+64] = g[d+64]*cos - g[d]*sin (the second one's product fused)
       Four u, w;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        u.v[i] = g.v[i] * cs.v[i] + e.v[i] * sn.v[i];
-        w.v[i] = e.v[i] * cs.v[i] - g.v[i] * sn.v[i];
+        u.v[i] = __fmaf_rn(e.v[i], sn.v[i], __fmul_rn(g.v[i], cs.v[i]));
+        w.v[i] = __fmaf_rn(e.v[i], cs.v[i], -__fmul_rn(g.v[i], sn.v[i]));
       }
       if (!rl.rotated) u = g, w = e;
       if (use_norm) {
         const Four x = unpack4(xa), y = unpack4(xb);
         const Four wa = unpack4(is_q ? wqa : wka), wb = unpack4(is_q ? wqb : wkb);
-        float dot = 0.f;
+        float dx = 0.f, dy = 0.f;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) dot += u.v[i] * wa.v[i] * x.v[i] * r + w.v[i] * wb.v[i] * y.v[i] * r;
-        dot = half_warp_sum(dot) / D;
+        for (int i = 0; i < 4; ++i) {
+          dx = __fmaf_rn(__fmul_rn(__fmul_rn(u.v[i], wa.v[i]), x.v[i]), r, dx);
+          dy = __fmaf_rn(__fmul_rn(__fmul_rn(w.v[i], wb.v[i]), y.v[i]), r, dy);
+        }
+        const float dot = head_sum(dx, dy, rot_half) / D;
         const bool to_k = !is_q && !is_v;  // (a V head's lanes hold nothing that a sum may see)
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -383,8 +402,8 @@ qk_norm_rope_bwd_kernel(const bf16* __restrict__ dq, const bf16* __restrict__ dk
           aqb.v[i] += is_q ? db : 0.f;
           aka.v[i] += to_k ? da : 0.f;
           akb.v[i] += to_k ? db : 0.f;
-          u.v[i] = r * (u.v[i] * wa.v[i] - xh * dot);
-          w.v[i] = r * (w.v[i] * wb.v[i] - yh * dot);
+          u.v[i] = __fmul_rn(r, __fmaf_rn(-xh, dot, __fmul_rn(u.v[i], wa.v[i])));
+          w.v[i] = __fmul_rn(r, __fmaf_rn(-yh, dot, __fmul_rn(w.v[i], wb.v[i])));
         }
       }
       if (act) {
