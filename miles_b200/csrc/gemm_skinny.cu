@@ -319,7 +319,7 @@ int launch_skinny(const GemmProblem& g, const __nv_bfloat16* residual, cudaStrea
 // 100 us, 95 at 6.5 TB/s).
 bool gemm_is_skinny(const GemmProblem& p) {
   return p.mode == GEMM_DENSE && p.M <= 128 && !p.a.mn_major && !p.b.mn_major && !p.accumulate && !p.row_ptrs && p.n_dest == 0 &&
-         p.max_ctas == 0 && p.N <= 148 * 3 * BM;
+         p.max_ctas == 0 && !p.whole_k && p.N <= 148 * 3 * BM;
 }
 
 int gemm_skinny_launch(const GemmProblem& g, const void* residual, cudaStream_t stream) {

@@ -160,7 +160,10 @@ class B200Qwen3:
         self.launches += 3
         return mx_linear(xq, wq, self.status, tile_group, num_tiles, n)
 
-    def linear(self, x, w, out_dtype=torch.bfloat16):
+    def linear(self, x, w, out_dtype=torch.bfloat16, serving=False):
+        """``x @ w^T``. In passes that train or score, every sum over K of 33 rows and more runs in one order, so that a sample's
+        log-probs and gradients do not depend on how much else is in its pack. Passes of the engine (``serving``) may split
+        the contraction of up to 128 rows over a cluster (csrc/gemm_skinny.cu)."""
         T, (N, K) = x.shape[0], w.shape
         mx = getattr(self, "mx", None)
         if mx and T > 32 and out_dtype == torch.bfloat16 and w.data_ptr() in mx:
@@ -171,7 +174,10 @@ class B200Qwen3:
             self.C.small_gemv(x, None, 0.0, w, None, out, self.status)
             self.launches += 1
             return out
-        return self._gemm(x, w, out)
+        split = self.small_decode and (serving or T <= 32)
+        self.C.gemm(x, w, out, False, False, False, 0, self.status, whole_k=not split)
+        self.launches += 1
+        return out
 
     def linear_dgrad(self, dy, w):
         dx = torch.empty(dy.shape[0], w.shape[1], dtype=torch.bfloat16, device=dy.device)
@@ -188,9 +194,9 @@ class B200Qwen3:
             raise RuntimeError(f"a miles_b200 kernel reported error status {code} (bounded wait expired)")
 
     # ------------------------------------------------------------------ MoE block
-    def _route(self, h2, router_w, replay_ids, bias=None):
+    def _route(self, h2, router_w, replay_ids, bias=None, serving=False):
         cfg, C = self.cfg, self.C
-        logits = self.linear(h2, router_w, torch.float32)
+        logits = self.linear(h2, router_w, torch.float32, serving)
         if cfg.router_score == "sigmoid":
             # GLM-4.5 / DeepSeek-V3 routing: a [T, E] problem, done with framework ops (ops/reference.py); what the
             # backward needs is the logits, kept in the place of the softmax probabilities
@@ -241,16 +247,16 @@ class B200Qwen3:
         self.launches += 3
         return (gu, act, yp) if keep else (None, None, yp)
 
-    def moe_forward(self, i, h2, replay_ids=None, record=None, keep=False, residual=None):
+    def moe_forward(self, i, h2, replay_ids=None, record=None, keep=False, residual=None, serving=False):
         cfg, P, C = self.cfg, self.store.params, self.C
         p = f"layers.{i}.moe."
-        ids, w, probs = self._route(h2, P[p + "router.weight"], replay_ids, P.get(p + "router.bias"))
+        ids, w, probs = self._route(h2, P[p + "router.weight"], replay_ids, P.get(p + "router.bias"), serving)
         if record is not None:
             record.append(ids)
         if cfg.shared_expert_ffn and not (keep and residual is None):  # (the backward's recompute does not need the output)
             # the shared expert sees every token: its output joins the residual that the combine adds
-            sh_gu = self.linear(h2, P[p + "shared.gate_up.weight"])
-            sh_y = self.linear(C.swiglu_fwd(sh_gu), P[p + "shared.down.weight"])
+            sh_gu = self.linear(h2, P[p + "shared.gate_up.weight"], serving=serving)
+            sh_y = self.linear(C.swiglu_fwd(sh_gu), P[p + "shared.down.weight"], serving=serving)
             if cfg.shared_expert_gate:  # one sigmoid gate value per token (a [T, H] x [H] product: framework ops)
                 g = torch.sigmoid(h2.float() @ P[p + "shared.gate.weight"].float().t())
                 sh_y = (sh_y.float() * g).to(sh_y.dtype)
@@ -358,7 +364,7 @@ class B200Qwen3:
         cfg, P, C = self.cfg, self.store.params, self.C
         p = f"layers.{i}."
         h1, rstd1 = C.rmsnorm_fwd(x, None, P[p + "ln1.weight"], cfg.rms_eps)
-        qkv = self.linear(h1, P[p + "attn.qkv.weight"])
+        qkv = self.linear(h1, P[p + "attn.qkv.weight"], serving=meta is not None)
         if cfg.qkv_bias:
             qkv += P[p + "attn.qkv.bias"]
         kc = vc = slots = None
@@ -411,8 +417,9 @@ class B200Qwen3:
                 return self.ep.moe_decode(self, i, x2, None, record)
             h2, _ = C.rmsnorm_fwd(x2, None, P[p + "ln2.weight"], cfg.rms_eps)
             self.launches += 1
-            y, _ = self.moe_forward(i, h2, replay_ids, record, keep=False, residual=x2)
+            y, _ = self.moe_forward(i, h2, replay_ids, record, keep=False, residual=x2, serving=True)
             return y
+        serving = meta is not None
         h1, rstd1, qkv, q, k, _, _ = self._attn_qkv(i, x, positions, meta, kv_cache)
         scale = cfg.head_dim ** -0.5
         if meta is not None and not meta.is_prefill:
@@ -434,21 +441,21 @@ class B200Qwen3:
             self.launches += 2
         else:
             att, _ = self.attention(q, k, self._v_view(qkv), cu)
-        h2, _, x2 = self._o_proj_ln2(i, att.view(att.shape[0], -1), x)
+        h2, _, x2 = self._o_proj_ln2(i, att.view(att.shape[0], -1), x, serving)
         if cfg.layer_is_moe(i):
             if (meta is not None and not meta.is_prefill and replay_ids is None and getattr(self.ep, "low_latency", False)
                     and x.shape[0] <= self.ep.rows and cfg.router_score == "softmax" and not cfg.shared_expert_ffn):
                 return self.ep.moe_decode(self, i, x2, h2, record)
-            y, _ = self.moe_forward(i, h2, replay_ids, record, keep=False, residual=x2)
+            y, _ = self.moe_forward(i, h2, replay_ids, record, keep=False, residual=x2, serving=serving)
             return y
-        gu = self.linear(h2, P[p + "mlp.gate_up.weight"])
+        gu = self.linear(h2, P[p + "mlp.gate_up.weight"], serving=serving)
         self.launches += 1
         if cfg.post_norms:
-            y = self.linear(C.swiglu_fwd(gu), P[p + "mlp.down.weight"])
+            y = self.linear(C.swiglu_fwd(gu), P[p + "mlp.down.weight"], serving=serving)
             yn, _ = C.rmsnorm_fwd(y, None, P[p + "post_mlp_ln.weight"], cfg.rms_eps)
             self.launches += 2
             return yn.add_(x2)
-        return self._row_parallel(C.swiglu_fwd(gu), P[p + "mlp.down.weight"], x2)
+        return self._row_parallel(C.swiglu_fwd(gu), P[p + "mlp.down.weight"], x2, serving)
 
     def _full_kv(self, prefix, k, v, kc, vc):
         """``PrefixInfo.full_kv`` in one launch for caches of the activations' type."""
@@ -456,32 +463,32 @@ class B200Qwen3:
             return prefix.full_kv(k, v, kc, vc)
         return self.C.gather_prefix_kv(k, v, kc, vc, prefix.pre_slots, prefix.pre_dst, prefix.new_dst, prefix.total, self.status)
 
-    def _row_parallel(self, a, w, residual):
+    def _row_parallel(self, a, w, residual, serving=False):
         """``residual + a @ w^T`` for a row-parallel weight: under tensor parallelism the GEMM epilogue pushes the
         partial sums to the peers and the slots are added in rank order (one fused GEMM + all-reduce)."""
         if self.tp is not None:
             self.launches += 3
             return self.tp.linear_allreduce(a, w, residual=residual, gemm_status=self.status)
-        if (residual is not None and self.SMALL_T < a.shape[0] <= 64 and self.small_decode and not getattr(self, "mx", None)
+        if (serving and residual is not None and self.SMALL_T < a.shape[0] <= 64 and self.small_decode and not getattr(self, "mx", None)
                 and a.is_contiguous() and w.shape[0] % 16 == 0 and w.shape[1] % 32 == 0):
             y = torch.empty_like(residual)  # the residual joins the sums before they are rounded
             self.C.small_gemv(a, None, 0.0, w, residual, y, self.status)
             self.launches += 1
             return y
-        y = self.linear(a, w)
+        y = self.linear(a, w, serving=serving)
         return y.add_(residual) if residual is not None else y
 
-    def _o_proj_ln2(self, i, att2, x):
+    def _o_proj_ln2(self, i, att2, x, serving=False):
         """Attention output projection, residual add and the second RMSNorm: returns (h2, rstd2, x2)."""
         cfg, P, C = self.cfg, self.store.params, self.C
         p = f"layers.{i}."
         self.launches += 1
         if self.tp is not None:
             assert not cfg.post_norms, "models with sandwich norms run without tensor parallelism"
-            x2 = self._row_parallel(att2, P[p + "attn.o.weight"], x)
+            x2 = self._row_parallel(att2, P[p + "attn.o.weight"], x, serving)
             h2, rstd2 = C.rmsnorm_fwd(x2, None, P[p + "ln2.weight"], cfg.rms_eps)
             return h2, rstd2, x2
-        o = self.linear(att2, P[p + "attn.o.weight"])
+        o = self.linear(att2, P[p + "attn.o.weight"], serving=serving)
         if cfg.post_norms:
             # sandwich norm (GLM-4 dense): the attention output is normalised before it joins the residual stream; the
             # backward's recompute picks the un-normalised output and its statistics up from here
@@ -733,8 +740,8 @@ class B200Qwen3:
         return loss.detach(), metrics
 
     @torch.no_grad()
-    def logits(self, hidden_rows, out_dtype=torch.float32):
-        return self.linear(hidden_rows.contiguous(), self.store.lm_head(), out_dtype)
+    def logits(self, hidden_rows, out_dtype=torch.float32, serving=True):
+        return self.linear(hidden_rows.contiguous(), self.store.lm_head(), out_dtype, serving)
 
     @torch.no_grad()
     def logprobs_entropy(self, hidden_rows, targets, inv_temp: float, chunk: int = 0, keep_stats: bool = False):
@@ -748,7 +755,7 @@ class B200Qwen3:
         tg = targets.to(torch.int32).contiguous()
         for a in range(0, n, chunk):
             b = min(a + chunk, n)
-            lg = self.logits(hidden_rows[a:b])
+            lg = self.logits(hidden_rows[a:b], serving=False)
             l1, e1, s1, p1 = C.logprob_entropy_fwd(lg, tg[a:b], inv_temp)
             self.launches += 1
             lp[a:b], ent[a:b] = l1, e1
@@ -793,7 +800,7 @@ class B200Qwen3:
             dhr = torch.empty_like(hr)
             for a in range(0, hr.shape[0], chunk):
                 b = min(a + chunk, hr.shape[0])
-                lg = self.logits(hr[a:b])
+                lg = self.logits(hr[a:b], serving=False)
                 dl = C.logprob_entropy_bwd(lg, tg[a:b], lse[a:b].contiguous(), px[a:b].contiguous(), dlp[a:b].contiguous(),
                                            dent[a:b].contiguous() if dent is not None else None, inv_temp)
                 del lg

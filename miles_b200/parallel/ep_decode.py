@@ -86,7 +86,7 @@ class EpDecodeLL:
             C.small_gemv(x2, ln2, cfg.rms_eps, P[p + "moe.router.weight"], None, logits, model.status)
             rows_in, ln = x2, ln2
         else:
-            logits = model.linear(h2, P[p + "moe.router.weight"], torch.float32)
+            logits = model.linear(h2, P[p + "moe.router.weight"], torch.float32, serving=True)
             rows_in, ln = h2, None
         ids = torch.empty(T, self.K, dtype=torch.int32, device=x2.device)
         w = torch.empty(T, self.K, dtype=torch.float32, device=x2.device)

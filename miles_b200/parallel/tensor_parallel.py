@@ -68,10 +68,10 @@ class TensorParallel:
         assert N == self.H and T <= self.max_tokens, (N, self.H, T, self.max_tokens)
         out = torch.empty(T, N, dtype=torch.bfloat16, device=a.device)
         if self.n == 1:
-            self.C.gemm(a, w, out, False, b_mn, False, 0, gemm_status)
+            self.C.gemm(a, w, out, False, b_mn, False, 0, gemm_status, whole_k=True)  # (as the fused form sums)
             return out if residual is None else out.add_(residual)
         if not self.fused:
-            self.C.gemm(a, w, out, False, b_mn, False, 0, gemm_status)
+            self.C.gemm(a, w, out, False, b_mn, False, 0, gemm_status, whole_k=True)  # (as the fused form sums)
             dist.all_reduce(out, group=self.group)
             return out if residual is None else out.add_(residual)
         g = self._parity

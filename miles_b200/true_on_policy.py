@@ -25,8 +25,8 @@ CONTRACT_V1 = (
     Clause("routing", "MoE expert choice of the engine is replayed in the trainer (rollout routing replay)"),
     Clause("attention", "prefill / training attention and paged decode attention agree to bf16 rounding; bit equality "
            "needs the same KV block order, which split-KV decode does not give"),
-    Clause("batch_invariance", "reductions do not depend on the batch composition (tile shapes are fixed per problem size, "
-           "the small-batch decode path changes kernels below 9 rows)"),
+    Clause("batch_invariance", "reductions do not depend on the batch composition (the trainer's products sum in one order from 33 "
+           "rows on; the engine's change kernels above 8 and above 128 rows, and between them split a contraction by the number of rows)"),
     Clause("sampling_temperature", "log-probs are taken at the rollout temperature on the full distribution "
            "(top-k / top-p truncation does not enter the reported log-prob)", True),
     Clause("lm_head", "LM head and log-softmax run in the same precision (bf16 GEMM, fp32 soft-max statistics)", True),

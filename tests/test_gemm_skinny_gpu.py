@@ -52,3 +52,38 @@ def test_repeated_products_are_bitwise_equal(ext):
     for o in outs:
         ext.gemm(x, w, o, False, False, False, 0, st)
     assert all(torch.equal(o, outs[0]) for o in outs)
+
+
+@pytest.mark.parametrize("T", [33, 64, 65, 128])
+@pytest.mark.parametrize("N,K", [(130, 2632), (2048, 2048), (2560, 9728)])
+def test_whole_contractions_do_not_depend_on_the_rows(ext, T, N, K):
+    g = torch.Generator(DEV).manual_seed(T + N)
+    st = torch.zeros(1, dtype=torch.int32, device=DEV)
+    x, w = torch.randn(300, K, generator=g, device=DEV).bfloat16(), torch.randn(N, K, generator=g, device=DEV).bfloat16()
+    for dtype in (torch.bfloat16, torch.float32):
+        few, many = (torch.empty(n, N, device=DEV, dtype=dtype) for n in (T, 300))
+        ext.gemm(x[:T], w, few, False, False, False, 0, st, whole_k=True)
+        ext.gemm(x, w, many, False, False, False, 0, st)
+        assert torch.equal(few, many[:T])
+        _check(few, x[:T], w)
+    assert st.item() == 0
+
+
+@pytest.mark.parametrize("name", ["qwen3-smoke", "qwen3-smoke-moe", "glm4-smoke"])
+@pytest.mark.parametrize("tokens", [49, 70, 128])
+def test_logprobs_of_a_sample_do_not_depend_on_its_pack(name, tokens):
+    from miles_b200.models import ParamStore, build_model, get_config
+
+    cfg = get_config(name)
+    model = build_model(cfg, ParamStore(cfg, torch.device(DEV), torch.bfloat16, init_std=0.05, seed=3), "b200")
+    g = torch.Generator().manual_seed(tokens)
+    lens = [tokens, 200]
+    ids = torch.randint(0, cfg.vocab_size, (sum(lens),), generator=g).to(DEV, torch.int32)
+    pos = torch.cat([torch.arange(n) for n in lens]).to(DEV, torch.int32)
+    rows = torch.arange(tokens - 1, device=DEV)
+    cu = torch.tensor([0, tokens, sum(lens)], dtype=torch.int32, device=DEV)
+    alone = model.forward_logprobs(ids[:tokens], pos[:tokens], cu[:2], rows, ids[1:tokens], 1.0)
+    packed = model.forward_logprobs(ids, pos, cu, torch.cat([rows, torch.arange(tokens, tokens + 199, device=DEV)]),
+                                    torch.cat([ids[1:tokens], ids[tokens + 1:]]), 1.0)
+    model.check_status()
+    assert all(torch.equal(a, b[:tokens - 1]) for a, b in zip(alone, packed))
