@@ -19,7 +19,7 @@ __global__ void gather_prefix_kv_kernel(const PrefixGather a) {
     const long long r = val ? w - rows : w;
     const uint4* src;
     long long dst;
-    bool ok = true;
+    bool ok = true;  // a slot outside the cache is reported and reads as zeros, as a bad page does in paged decoding
     if (r < a.n_pre) {
       const long long slot = a.pre_slots[r];
       dst = a.pre_dst[r];
@@ -29,17 +29,15 @@ __global__ void gather_prefix_kv_kernel(const PrefixGather a) {
       dst = a.new_dst[r - a.n_pre];
       src = static_cast<const uint4*>(val ? a.v_new : a.k_new) + (r - a.n_pre) * (val ? a.v_pitch : a.k_pitch);
     }
-    if (dst < 0 || dst >= a.total) ok = false;
-    if (!ok) {  // a row outside the cache or the output: reported, not followed
-      if (lane == 0 && a.status) atomicCAS(a.status, 0, 9);
-      continue;
-    }
+    const bool place = dst >= 0 && dst < a.total;
+    if (!(ok && place) && lane == 0 && a.status) atomicCAS(a.status, 0, 9);
+    if (!place) continue;
     uint4* to = static_cast<uint4*>(val ? a.v_out : a.k_out) + dst * a.vecs;
     for (int c0 = lane; c0 < a.vecs; c0 += 128) {
       uint4 v[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-        if (c0 + 32 * u < a.vecs) v[u] = src[c0 + 32 * u];
+        if (c0 + 32 * u < a.vecs) v[u] = ok ? src[c0 + 32 * u] : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
       for (int u = 0; u < 4; ++u)
         if (c0 + 32 * u < a.vecs) to[c0 + 32 * u] = v[u];

@@ -1,5 +1,5 @@
 """Packed keys / values behind a cached prefix: against indexing, for rows of odd numbers of vectors, strided new rows,
-sequences without a prefix, and a slot outside the cache, which is reported."""
+sequences without a prefix, and slots outside the cache, which are reported and read as zeros."""
 import pytest
 import torch
 
@@ -25,6 +25,11 @@ def test_gather_equals_indexing(heads, prefix, new):
     got = ext.gather_prefix_kv(k, v, kc, vc, info.pre_slots, info.pre_dst, info.new_dst, info.total, st)
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]) and st.item() == 0
     bad = info.pre_slots.clone()
-    bad[0] = kc.shape[0]
-    ext.gather_prefix_kv(k, v, kc, vc, bad, info.pre_dst, info.new_dst, info.total, st)
+    bad[0], bad[-1] = kc.shape[0], -1
+    torch.full((4 * info.total * heads * 128,), float("nan"), dtype=torch.bfloat16, device=DEV)  # what freed memory may hold
+    got = ext.gather_prefix_kv(k, v, kc, vc, bad, info.pre_dst, info.new_dst, info.total, st)
+    for t, w in zip(got, want):
+        w = w.clone()
+        w[info.pre_dst[[0, -1]]] = 0
+        assert torch.equal(t, w)
     assert st.item() == 9
