@@ -234,6 +234,7 @@ class Engine:
         # two generations of result buffers: one decode step may be in flight while the previous one is read
         self.h_out = torch.zeros(2, B, dtype=torch.int32, pin_memory=pin)
         self.h_lp = torch.zeros(2, B, dtype=torch.float32, pin_memory=pin)
+        self.h_status = torch.zeros(2, dtype=torch.int32, pin_memory=pin)  # the model's status word after each step
         self._h_routes: list = [None, None]
         self._parity = 0
         self._pending: Optional[dict] = None
@@ -667,6 +668,7 @@ class Engine:
             tok, lp = self._sample(logits, [batch[i] for i in ends])
             for i, t, l in zip(ends, tok.tolist(), lp.tolist()):
                 tok_l[i], lp_l[i] = t, l
+            self._check_model()
         routes = torch.stack(record, 1).cpu() if want_routes else None  # [T, L, K]
         self.d2h_bytes += 8 * len(batch) + (routes.numel() * 4 if routes is not None else 0)
         self.stats["prefill_tokens"] += len(toks)
@@ -798,6 +800,19 @@ class Engine:
         self._rows = list(reqs)
         self._rows_B = B
 
+    # ------------------------------------------------------------------ what kernels report
+    def _status_word(self) -> Optional[torch.Tensor]:
+        """The word in which the model's kernels leave what they could not raise: a wait that ran out, a page or a slot
+        outside the cache. None for models without one."""
+        word = getattr(self.model, "status", None)
+        return word if torch.is_tensor(word) and hasattr(self.model, "check_status") else None
+
+    def _check_model(self) -> None:
+        """Raise if a kernel has reported an error. Called where the results of a pass are read on the host anyway, so that
+        no token of such a pass is handed out."""
+        if self._status_word() is not None:
+            self.model.check_status()
+
     # ------------------------------------------------------------------ decode: launch / process, one step in flight
     def _grow_pages_ahead(self, lookahead: int) -> bool:
         """Pages for ``lookahead`` more positions of every running request, without retracting anybody.
@@ -853,6 +868,9 @@ class Engine:
         par = self._parity
         self._parity ^= 1
         pend = {"reqs": reqs, "n": n, "parity": par, "event": None, "routes": None, "bucket": B}
+        word = self._status_word()
+        if word is not None:
+            self.h_status[par:par + 1].copy_(word, non_blocking=self.on_gpu)
         if self.on_gpu:
             self.h_out[par, :n].copy_(self.d_out_tokens[:n], non_blocking=True)
             self.h_lp[par, :n].copy_(self.d_out_logprobs[:n], non_blocking=True)
@@ -877,6 +895,8 @@ class Engine:
         retracted or aborted after the step was launched ignores its row)."""
         if pend["event"] is not None:
             pend["event"].synchronize()
+        if int(self.h_status[pend["parity"]]):
+            self._check_model()
         now = time.perf_counter()
         if self._t_last_decode is not None and pend.get("bucket"):
             bt = self.bucket_time.setdefault(pend["bucket"], [0.0, 0])
@@ -1131,7 +1151,9 @@ class Engine:
         else:
             lp, _ = self.model.forward_logprobs(tok, pos, cu, rows, tok[1:], inv_t, **kw)
         self.stats["scored_tokens"] = self.stats.get("scored_tokens", 0) + n
-        return {"logprobs": [None] + [float(x) for x in lp.tolist()], "top": top}
+        lp = lp.tolist()
+        self._check_model()
+        return {"logprobs": [None] + [float(x) for x in lp], "top": top}
 
     # ------------------------------------------------------------------ convenience
     def generate(self, prompts: Sequence[Sequence[int]], params: SamplingParams | Sequence[SamplingParams] | dict | None = None,

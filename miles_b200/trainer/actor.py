@@ -807,6 +807,8 @@ class TrainActor:
                         self.events.log(ev_weight_checksum(self.global_step, self.store.version, f"{ck.get('dense', 0.0):.6e}"))
         if self.on_gpu:
             torch.cuda.synchronize()
+        if hasattr(self.model, "check_status"):
+            self.model.check_status()  # what a kernel reported (a wait that ran out): the weights of this step are not to be used
         elapsed = time.perf_counter() - t_start
         T.flush_cuda()
         out = self._finalize_metrics(metrics_acc, grad_norm, n_tokens_local, elapsed, len(mbs))

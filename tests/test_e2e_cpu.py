@@ -239,3 +239,19 @@ def test_model_provider_plugin_builds_the_trainer_and_engine_model():
     assert isinstance(loop.actor.model, SoftCappedQwen3) and loop.engine.model is loop.actor.model
     m = loop.run()[0]
     assert m["train/train_rollout_logprob_abs_diff"] < 1e-5 and m["train/grad_norm"] > 0
+
+
+def test_a_training_step_raises_what_a_kernel_reported():
+    from miles_b200.loop import RLLoop
+
+    loop = RLLoop(parse_args(BASE + ["--actor-num-gpus-per-node", "1", "--num-rollout", "1"]))
+    called = []
+
+    def check_status():
+        called.append(1)
+        raise RuntimeError("status 3")
+
+    loop.actor.model.check_status = check_status
+    with pytest.raises(RuntimeError, match="status 3"):
+        loop.run()
+    assert called == [1]

@@ -290,3 +290,49 @@ def test_default_sampling_seeds_follow_the_salt_not_the_process():
     ra, rb, rc = (e.generate(prompts, sp) for e in (a, b, c))
     assert [r["output_ids"] for r in ra] == [r["output_ids"] for r in rb]
     assert [r["output_ids"] for r in ra] != [r["output_ids"] for r in rc]
+
+
+class _Reports:
+    """A model whose kernels report an error in the pass ``at`` (counted from 0), as the GPU models do: a word on the device."""
+
+    def __init__(self, model, at):
+        self.model, self.at, self.passes = model, at, 0
+        self.status = torch.zeros(1, dtype=torch.int32)
+
+    def __getattr__(self, name):
+        return getattr(self.model, name)
+
+    def forward_hidden(self, *a, **kw):
+        if self.passes == self.at:
+            self.status.fill_(9)
+        self.passes += 1
+        return self.model.forward_hidden(*a, **kw)
+
+    def forward_logprobs(self, *a, **kw):
+        self.status.fill_(9)
+        return self.model.forward_logprobs(*a, **kw)
+
+    def check_status(self):
+        code = int(self.status.item())
+        self.status.zero_()
+        if code:
+            raise RuntimeError(f"status {code}")
+
+
+@pytest.mark.parametrize("at", [0, 1, 3])  # the prompts' pass, the first decode step, a later one
+def test_an_error_that_a_kernel_reports_is_raised(at):
+    cfg, m, eng = _engine()
+    eng.model = _Reports(m, at)
+    with pytest.raises(RuntimeError, match="status 9"):
+        eng.generate(_prompts(cfg, [5, 9]), SamplingParams(max_new_tokens=6, sampling_seed=1))
+    with pytest.raises(RuntimeError, match="status 9"):
+        eng.score([1, 2, 3, 4])
+
+
+def test_a_model_that_reports_nothing_generates():
+    cfg, m, eng = _engine()
+    p, sp = _prompts(cfg, [5, 9]), SamplingParams(max_new_tokens=6, sampling_seed=1)
+    want = [r["output_ids"] for r in eng.generate(p, sp)]
+    _, m2, eng2 = _engine()
+    eng2.model = _Reports(m2, -1)
+    assert [r["output_ids"] for r in eng2.generate(p, sp)] == want
