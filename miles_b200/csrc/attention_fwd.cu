@@ -64,7 +64,6 @@ __device__ __forceinline__ float ex2(float x) {
 __global__ void __launch_bounds__(FA_THREADS, 1)
 fa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
               const __grid_constant__ CUtensorMap map_v, const FaArgs p) {
-  pdl_enter();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t q_s = base;
@@ -82,15 +81,6 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
   volatile int* abort_flag = &abort_s;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // Heads vary fastest: the list starts with the tiles of the longest key ranges, and all heads' long tiles have to start
-  // before anyone's short ones; heads that share keys and values also run side by side.
-  const int4 tile = p.tiles[blockIdx.x / p.Hq];
-  const int hq = blockIdx.x % p.Hq;
-  const int hk = hq / (p.Hq / p.Hk);
-  const int q_row0 = tile.x, q_rows = tile.y, kv_row0 = tile.z, q_pos0 = tile.w;
-  const int kv_len = q_pos0 + q_rows;               // causal: keys up to the last query of the tile
-  const int n_blocks = (kv_len + BN - 1) / BN;
-
   if (threadIdx.x == 0) {
     abort_s = 0;
     mbar_init(BAR(B_QF), 1);
@@ -123,6 +113,16 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
   }
   __syncthreads();
   const uint32_t tmem = tmem_base_s;
+  pdl_enter();  // (behind the allocation: see the rules in pdl.cuh)
+
+  // Heads vary fastest: the list starts with the tiles of the longest key ranges, and all heads' long tiles have to start
+  // before anyone's short ones; heads that share keys and values also run side by side.
+  const int4 tile = p.tiles[blockIdx.x / p.Hq];
+  const int hq = blockIdx.x % p.Hq;
+  const int hk = hq / (p.Hq / p.Hk);
+  const int q_row0 = tile.x, q_rows = tile.y, kv_row0 = tile.z, q_pos0 = tile.w;
+  const int kv_len = q_pos0 + q_rows;               // causal: keys up to the last query of the tile
+  const int n_blocks = (kv_len + BN - 1) / BN;
   auto T_S = [&](int b) { return tmem + static_cast<uint32_t>(b) * 128u; };  // two score buffers
   const uint32_t t_O = tmem + 256;                                             // output accumulator
   if (warp == 0) {

@@ -12,6 +12,9 @@
 //     are visible; since that one did the same, all earlier kernels of the stream have completed too;
 //   * dependents are let in only after the wait, by CTAs that are resident, so no CTA of a kernel waits for a place that a
 //     later kernel holds;
+//   * the same for TMEM: a kernel that uses it allocates before it lets dependents in. A dependent allocates before its own
+//     wait and holds on until this kernel has completed; had it come first, each would wait for the other, and
+//     `tcgen05.alloc` has no limit (tests/test_dependent_launch.py looks for it in the sources);
 //   * a kernel launched in the ordinary way before or after depends, and is depended on, as always.
 #pragma once
 #include <cuda_runtime.h>
