@@ -264,17 +264,12 @@ __global__ void __launch_bounds__(256) router_small_kernel(const float* __restri
 
 }  // namespace
 
-void small_gemv_direct(const void* x, int T, const void* norm_w, float eps, const void* W, int N, int K,
-                       const void* residual, void* out, bool out_fp32, cudaStream_t s) {
+cudaError_t small_gemv_direct(const void* x, int T, const void* norm_w, float eps, const void* W, int N, int K,
+                              const void* residual, void* out, bool out_fp32, cudaStream_t s) {
   const int threads = 32 * (warps_for(K) < 4 ? 4 : warps_for(K));  // the epilogue needs 128 threads
-  if (norm_w)
-    pdl_launch(small_gemv_kernel<true>, N / 16, threads, 0, s, static_cast<const bf16*>(x), T, static_cast<const bf16*>(norm_w),
-                                                       eps, static_cast<const bf16*>(W), N, K,
-                                                       static_cast<const bf16*>(residual), out, out_fp32 ? 1 : 0);
-  else
-    pdl_launch(small_gemv_kernel<false>, N / 16, threads, 0, s, static_cast<const bf16*>(x), T, nullptr, eps,
-                                                        static_cast<const bf16*>(W), N, K,
-                                                        static_cast<const bf16*>(residual), out, out_fp32 ? 1 : 0);
+  return pdl_launch(norm_w ? small_gemv_kernel<true> : small_gemv_kernel<false>, N / 16, threads, 0, s, static_cast<const bf16*>(x), T,
+                    static_cast<const bf16*>(norm_w), eps, static_cast<const bf16*>(W), N, K, static_cast<const bf16*>(residual), out,
+                    out_fp32 ? 1 : 0);
 }
 
 void router_small(const float* logits, int T, int E, int K, bool renorm, int* topk_ids, float* topk_w, int* active,

@@ -26,6 +26,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <string>
+
 #include "gemm.h"
 #include "launchers.h"
 #include "pdl.cuh"
@@ -311,16 +313,16 @@ __global__ void __launch_bounds__(THREADS, 1) stream_kernel(const StreamArgs a) 
 }
 
 template <int CPW, int RT, bool EXACT>
-int launch_variant(const StreamArgs& a, int grid, int smem, cudaStream_t s) {
+cudaError_t launch_variant(const StreamArgs& a, int grid, int smem, cudaStream_t s) {
   auto kern = stream_kernel<CPW, RT, EXACT>;
   // the attribute belongs to the (function, device) pair: set on every launch rather than once per process
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, RING_BYTES + 1024) != cudaSuccess) return -1;
-  return pdl_launch(kern, grid, THREADS, smem, s, a) == cudaSuccess ? 0 : -1;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, RING_BYTES + 1024);
+  return e == cudaSuccess ? pdl_launch(kern, grid, THREADS, smem, s, a) : e;
 }
 
 int g_sms = 0;
 
-int launch_stream(StreamArgs a, int max_groups, cudaStream_t s) {
+cudaError_t launch_stream(StreamArgs a, int max_groups, cudaStream_t s) {
   a.kc = a.K < MAX_KC ? a.K : MAX_KC;
   a.n_kc = (a.K + a.kc - 1) / a.kc;
   const int chunks = a.kc / 32;
@@ -361,10 +363,17 @@ int launch_stream(StreamArgs a, int max_groups, cudaStream_t s) {
   return launch_variant<8, 1, false>(a, grid, smem, s);
 }
 
+// 0, or -1 with gemm_last_error() set. The error is reported here, so it is not left for whoever asks the runtime next.
+int launched(cudaError_t e, const char* what) {
+  if (e == cudaSuccess) return 0;
+  cudaGetLastError();
+  return gemm_fail(std::string(what) + " launch failed: " + cudaGetErrorString(e));
+}
+
 }  // namespace
 
-void small_gemv_direct(const void* x, int T, const void* norm_w, float eps, const void* W, int N, int K,
-                       const void* residual, void* out, bool out_fp32, cudaStream_t s);  // decode_small.cu
+cudaError_t small_gemv_direct(const void* x, int T, const void* norm_w, float eps, const void* W, int N, int K,
+                              const void* residual, void* out, bool out_fp32, cudaStream_t s);  // decode_small.cu
 
 int small_gemv(const void* x, int T, const void* norm_w, float eps, const void* W, int N, int K, const void* residual,
                void* out, bool out_fp32, int* status, cudaStream_t s) {
@@ -386,10 +395,8 @@ int small_gemv(const void* x, int T, const void* norm_w, float eps, const void* 
     p.status = status;
     return gemm_skinny_launch(p, residual, s);
   }
-  if (bytes < (48ll << 20)) {  // small matrix: the direct kernel
-    small_gemv_direct(x, T, norm_w, eps, W, N, K, residual, out, out_fp32, s);
-    return 0;
-  }
+  if (bytes < (48ll << 20))  // small matrix: the direct kernel
+    return launched(small_gemv_direct(x, T, norm_w, eps, W, N, K, residual, out, out_fp32, s), "small_gemv");
   StreamArgs a = {};
   a.W = static_cast<const bf16*>(W);
   a.rows = N;
@@ -404,11 +411,10 @@ int small_gemv(const void* x, int T, const void* norm_w, float eps, const void* 
   a.out_fp32 = out_fp32 ? 1 : 0;
   a.residual = static_cast<const bf16*>(residual);
   a.status = status;
-  launch_stream(a, 1, s);
-  return 0;
+  return launched(launch_stream(a, 1, s), "small_gemv");
 }
 
-void moe_small_up(const void* x, const void* norm_w, float eps, const void* W1, const int* active, const int* pair_count,
+int moe_small_up(const void* x, const void* norm_w, float eps, const void* W1, const int* active, const int* pair_count,
                   const int* pair_list, int max_active, int H, int I, int K, void* gu, int* status, cudaStream_t s) {
   StreamArgs a = {};
   a.W = static_cast<const bf16*>(W1);
@@ -426,10 +432,10 @@ void moe_small_up(const void* x, const void* norm_w, float eps, const void* W1, 
   a.out = gu;
   a.out_ld = 2 * I;
   a.status = status;
-  launch_stream(a, max_active, s);
+  return launched(launch_stream(a, max_active, s), "moe_small_up");
 }
 
-void moe_small_down(const void* gu, const void* W2, const int* active, const int* pair_count, const int* pair_list,
+int moe_small_down(const void* gu, const void* W2, const int* active, const int* pair_count, const int* pair_list,
                     int max_active, int H, int I, void* y, int* status, cudaStream_t s) {
   StreamArgs a = {};
   a.W = static_cast<const bf16*>(W2);
@@ -445,7 +451,7 @@ void moe_small_down(const void* gu, const void* W2, const int* active, const int
   a.out = y;
   a.out_ld = H;
   a.status = status;
-  launch_stream(a, max_active, s);
+  return launched(launch_stream(a, max_active, s), "moe_small_down");
 }
 
 }  // namespace mb

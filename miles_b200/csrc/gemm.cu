@@ -766,7 +766,10 @@ int launch(const GemmProblem& p, const KArgs& ka, cudaStream_t stream) {
   if (p.max_ctas > 0 && grid > p.max_ctas) grid = p.max_ctas;
   if (grid <= 0) return 0;
   const cudaError_t e = pdl_launch(kern, grid, kThreads, SMEM, stream, ma, mb_, ka);
-  if (e != cudaSuccess) return fail(std::string("gemm launch failed: ") + cudaGetErrorString(e));
+  if (e != cudaSuccess) {
+    cudaGetLastError();  // (reported here)
+    return fail(std::string("gemm launch failed: ") + cudaGetErrorString(e));
+  }
   return 0;
 }
 

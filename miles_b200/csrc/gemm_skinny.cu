@@ -309,7 +309,10 @@ int launch_skinny(const GemmProblem& g, const __nv_bfloat16* residual, cudaStrea
   cfg.attrs = attr;
   cfg.numAttrs = 2;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, mw, mx, p);
-  if (e != cudaSuccess) return gemm_fail(std::string("skinny gemm launch failed: ") + cudaGetErrorString(e));
+  if (e != cudaSuccess) {
+    cudaGetLastError();  // (reported here)
+    return gemm_fail(std::string("skinny gemm launch failed: ") + cudaGetErrorString(e));
+  }
   return 0;
 }
 

@@ -146,9 +146,10 @@ void moe_small_up(const at::Tensor& x, const at::Tensor& norm_w, double eps, con
   TORCH_CHECK(W1.dim() == 3 && W1.size(2) == H && H % 32 == 0 && I % 8 == 0 && act.size(1) == 2 * I, "moe_small_up: unsupported shape");
   TORCH_CHECK((2 * I) % 16 == 0, "moe_small_up: 2I must be a multiple of 16");
   const c10::cuda::CUDAGuard guard(x.device());
-  mb::moe_small_up(x.data_ptr(), norm_w.data_ptr(), eps, W1.data_ptr(), active.data_ptr<int>(), pair_count.data_ptr<int>(),
-                   pair_list.data_ptr<int>(), max_active, H, I, K, act.data_ptr(),
-                   status.has_value() ? status->data_ptr<int>() : nullptr, cur_stream());
+  const int rc = mb::moe_small_up(x.data_ptr(), norm_w.data_ptr(), eps, W1.data_ptr(), active.data_ptr<int>(),
+                                  pair_count.data_ptr<int>(), pair_list.data_ptr<int>(), max_active, H, I, K, act.data_ptr(),
+                                  status.has_value() ? status->data_ptr<int>() : nullptr, cur_stream());
+  TORCH_CHECK(rc == 0, mb::gemm_last_error());
 }
 
 void moe_small_down(const at::Tensor& act, const at::Tensor& W2, const at::Tensor& active, const at::Tensor& pair_count,
@@ -157,8 +158,10 @@ void moe_small_down(const at::Tensor& act, const at::Tensor& W2, const at::Tenso
   const int I = act.size(1) / 2, H = W2.size(1);
   TORCH_CHECK(W2.dim() == 3 && W2.size(2) == I && H % 16 == 0 && I % 32 == 0 && y.size(1) == H, "moe_small_down: unsupported shape");
   const c10::cuda::CUDAGuard guard(act.device());
-  mb::moe_small_down(act.data_ptr(), W2.data_ptr(), active.data_ptr<int>(), pair_count.data_ptr<int>(), pair_list.data_ptr<int>(),
-                     max_active, H, I, y.data_ptr(), status.has_value() ? status->data_ptr<int>() : nullptr, cur_stream());
+  const int rc = mb::moe_small_down(act.data_ptr(), W2.data_ptr(), active.data_ptr<int>(), pair_count.data_ptr<int>(),
+                                    pair_list.data_ptr<int>(), max_active, H, I, y.data_ptr(),
+                                    status.has_value() ? status->data_ptr<int>() : nullptr, cur_stream());
+  TORCH_CHECK(rc == 0, mb::gemm_last_error());
 }
 
 std::vector<at::Tensor> gae(const at::Tensor& rewards, const at::Tensor& values, const at::Tensor& cu, double gamma, double lam) {

@@ -87,3 +87,17 @@ def test_logprobs_of_a_sample_do_not_depend_on_its_pack(name, tokens):
                                     torch.cat([ids[1:tokens], ids[tokens + 1:]]), 1.0)
     model.check_status()
     assert all(torch.equal(a, b[:tokens - 1]) for a, b in zip(alone, packed))
+
+
+def test_a_launch_that_the_runtime_refuses_is_raised(ext):
+    st = torch.zeros(1, dtype=torch.int32, device=DEV)
+    x, none = torch.zeros(2, 64, dtype=torch.bfloat16, device=DEV), torch.zeros(0, 64, dtype=torch.bfloat16, device=DEV)
+    with pytest.raises(RuntimeError, match="small_gemv"):  # no rows of weights: an empty grid
+        ext.small_gemv(x, None, 0.0, none, None, torch.zeros(2, 0, dtype=torch.bfloat16, device=DEV), st)
+    w = torch.zeros(4, 128, 64, dtype=torch.bfloat16, device=DEV)
+    i32 = torch.zeros(64, dtype=torch.int32, device=DEV)
+    with pytest.raises(RuntimeError, match="moe_small_up"):  # no expert: the same
+        ext.moe_small_up(x, x[0].clone(), 1e-6, w, i32, i32, i32, 0, 2, torch.zeros(4, 128, dtype=torch.bfloat16, device=DEV), st)
+    with pytest.raises(RuntimeError, match="moe_small_down"):
+        ext.moe_small_down(torch.zeros(4, 128, dtype=torch.bfloat16, device=DEV), w, i32, i32, i32, 0, torch.zeros(4, 128, dtype=torch.bfloat16, device=DEV), st)
+    assert torch.ones(3, device=DEV).sum().item() == 3  # and is not found again by the next call
