@@ -44,22 +44,11 @@ void moe_router_topk(const float* logits, const int* replay_ids, int* topk_ids, 
 // Deterministic counting sort of the T*K (token, slot) pairs by expert. Rows of each expert are padded
 // to a multiple of `align`; outputs: dest_row[T*K], row_src[max_rows] (-1 for padding), expert_offsets[E+1]
 // (padded), tile_group[max_tiles][4] = {expert, row0, rows, 0}, num_m_tiles[2] = {tiles, live rows},
-// expert_counts[E].
-// kv_gather.cu: rows of `vecs` 16-byte vectors; pitches of the new rows in vectors
-struct PrefixGather {
-  const void *k_new, *v_new, *k_cache, *v_cache;
-  void *k_out, *v_out;
-  const long long *pre_slots, *pre_dst, *new_dst;
-  long long n_pre, n_new, num_slots, total, k_pitch, v_pitch;
-  int vecs;
-  int* status;
-};
-void gather_prefix_kv(const PrefixGather& a, cudaStream_t s);
-// ints of scratch that moe_build_permutation needs for these sizes
+// expert_counts[E]. Scratch: as many ints as moe_permutation_scratch says for these sizes.
 long long moe_permutation_scratch(int T, int K, int max_rows, int E);
-void moe_build_permutation(const int* topk_ids, int T, int K, int E, int max_rows, int max_tiles, int align,
-                           int* expert_counts, int* expert_offsets, int* dest_row, int* row_src, int* tile_group,
-                           int* num_m_tiles, int* scratch, cudaStream_t s);
+cudaError_t moe_build_permutation(const int* topk_ids, int T, int K, int E, int max_rows, int max_tiles, int align,
+                                  int* expert_counts, int* expert_offsets, int* dest_row, int* row_src, int* tile_group,
+                                  int* num_m_tiles, int* scratch, cudaStream_t s);
 void moe_permute(const void* x, const int* row_src, const int* num_m_tiles, void* x_perm, int max_rows, int H, int K,
                  cudaStream_t s);
 // out[t] = (residual[t] +) sum_k w[t,k] * y_perm[dest_row[t,k]]
@@ -91,6 +80,17 @@ void logprob_entropy_bwd(const void* logits, bool fp32, const int* targets, cons
 void sample_rows(const void* logits, bool fp32, int T, int V, long long ld, const float* temperature, const int* top_k,
                  const float* top_p, const unsigned long long* seeds, const int* step, int* out_token, float* out_logprob,
                  cudaStream_t s);
+
+// ---- kv_gather.cu: packed keys / values behind a cached prefix; rows of `vecs` 16-byte vectors, pitches of the new rows in vectors
+struct PrefixGather {
+  const void *k_new, *v_new, *k_cache, *v_cache;
+  void *k_out, *v_out;
+  const long long *pre_slots, *pre_dst, *new_dst;
+  long long n_pre, n_new, num_slots, total, k_pitch, v_pitch;
+  int vecs;
+  int* status;
+};
+void gather_prefix_kv(const PrefixGather& a, cudaStream_t s);
 
 // ---- attention.cu
 // Returns the CUDA error code of its own launches (0 = ok). `num_slots` = rows of the cache (0: unchecked page ids),

@@ -187,7 +187,7 @@ __global__ void router_bwd_kernel(const float* __restrict__ probs, const int* __
 // 131072 ids are half a megabyte. (One block per expert that reads every id, which this replaced, read them 2 E times:
 // 131072 entries over 128 experts took 282 us in three kernels, these take 20 us; 128 entries 10.7 us, now 3.2 us.)
 constexpr int SORT_ROUNDS = 16;  // entries per lane and warp at most
-constexpr int SORT_WARPS = 4;    // warps per block of the many-block variant: their counts fit shared memory up to 14000 experts
+constexpr int SORT_WARPS = 4;    // warps per block of the many-block variant: counts and scans fit shared memory up to 14500 experts
 
 // One warp: `rank[r]` of entry first + 32 r + lane among the warp's entries of the same expert, the warp's counts in
 // `hist` (shared memory, zeroed by the caller). Ids outside [0, E) get no rank. The last entry is `last` - 1.
@@ -598,33 +598,37 @@ long long moe_permutation_scratch(int T, int K, int max_rows, int E) {
   return sort_in_one_block(T * K, max_rows, E) ? 0 : static_cast<long long>(sort_blocks(T * K)) * E;
 }
 
-void moe_build_permutation(const int* topk_ids, int T, int K, int E, int max_rows, int max_tiles, int align,
-                           int* expert_counts, int* expert_offsets, int* dest_row, int* row_src, int* tile_group,
-                           int* num_m_tiles, int* scratch, cudaStream_t s) {
+cudaError_t moe_build_permutation(const int* topk_ids, int T, int K, int E, int max_rows, int max_tiles, int align,
+                                  int* expert_counts, int* expert_offsets, int* dest_row, int* row_src, int* tile_group,
+                                  int* num_m_tiles, int* scratch, cudaStream_t s) {
   const int n = T * K;
   if (sort_in_one_block(n, max_rows, E)) {
     const auto smem = [&](int warps) { return static_cast<size_t>((warps + 3) * E + 2) * sizeof(int); };
-    if (n <= 512) {
-      const int warps = n <= 128 ? 4 : 16;  // (four also fill row_src and the tile list quickly enough)
-      pdl_launch(build_small_kernel<1>, 1, 32 * warps, smem(warps), s, topk_ids, n, E, max_rows, max_tiles, align, expert_counts,
-                                                               expert_offsets, dest_row, row_src, tile_group, num_m_tiles);
-    } else {
-      pdl_launch(build_small_kernel<8>, 1, 512, smem(16), s, topk_ids, n, E, max_rows, max_tiles, align, expert_counts, expert_offsets,
-                                                     dest_row, row_src, tile_group, num_m_tiles);
-    }
-    return;
+    const int warps = n <= 128 ? 4 : 16;  // (four also fill row_src and the tile list quickly enough)
+    return pdl_launch(n <= 512 ? build_small_kernel<1> : build_small_kernel<8>, 1, 32 * warps, smem(warps), s, topk_ids, n, E, max_rows,
+                      max_tiles, align, expert_counts, expert_offsets, dest_row, row_src, tile_group, num_m_tiles);
   }
   const int blocks = sort_blocks(n);
   const int parts = E <= 1024 ? 8 : 1;  // (more experts: enough threads have one to follow, and shared memory holds their counts once)
-  const size_t scan_smem = static_cast<size_t>((3 + parts) * E + 2) * sizeof(int), assign_smem = static_cast<size_t>(SORT_WARPS) * E * sizeof(int);
-  if (scan_smem > 48 * 1024) cudaFuncSetAttribute(scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(scan_smem));
-  if (assign_smem > 48 * 1024)
-    cudaFuncSetAttribute(assign_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(assign_smem));
-  cudaMemsetAsync(row_src, 0xff, sizeof(int) * static_cast<size_t>(max_rows), s);
-  count_kernel<<<blocks, SORT_WARPS * 32, E * sizeof(int), s>>>(topk_ids, n, E, scratch);
+  const size_t count_smem = static_cast<size_t>(E) * sizeof(int), assign_smem = SORT_WARPS * count_smem;
+  const size_t scan_smem = static_cast<size_t>((3 + parts) * E + 2) * sizeof(int);
+  // All three get their shared memory before the first is launched: a pass without the one before it would follow counts
+  // that nobody wrote. Too many experts for it are refused here.
+  const auto allow = [](auto kernel, size_t bytes) {
+    return bytes <= 48 * 1024 ? cudaSuccess : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+  };
+  cudaError_t e = allow(count_kernel, count_smem);
+  if (e == cudaSuccess) e = allow(scan_kernel, scan_smem);
+  if (e == cudaSuccess) e = allow(assign_kernel, assign_smem);
+  if (e == cudaSuccess) e = cudaMemsetAsync(row_src, 0xff, sizeof(int) * static_cast<size_t>(max_rows), s);
+  if (e != cudaSuccess) return e;
+  count_kernel<<<blocks, SORT_WARPS * 32, count_smem, s>>>(topk_ids, n, E, scratch);
+  if ((e = cudaPeekAtLastError()) != cudaSuccess) return e;
   scan_kernel<<<1, 1024, scan_smem, s>>>(scratch, blocks, parts, E, max_rows, max_tiles, align, expert_counts, expert_offsets, tile_group,
                                          num_m_tiles);
+  if ((e = cudaPeekAtLastError()) != cudaSuccess) return e;
   assign_kernel<<<blocks, SORT_WARPS * 32, assign_smem, s>>>(topk_ids, n, E, scratch, expert_offsets, dest_row, row_src);
+  return cudaPeekAtLastError();
 }
 
 void moe_permute(const void* x, const int* row_src, const int* num_m_tiles, void* x_perm, int max_rows, int H, int K,

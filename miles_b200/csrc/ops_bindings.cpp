@@ -234,9 +234,11 @@ std::vector<at::Tensor> moe_build_permutation(const at::Tensor& ids, int64_t E, 
   at::Tensor counts = at::empty({E}, o), offsets = at::empty({E + 1}, o), dest = at::empty({T * K}, o);
   at::Tensor src = at::empty({max_rows}, o), tg = at::empty({max_tiles, 4}, o), nt = at::empty({2}, o);
   at::Tensor scratch = at::empty({mb::moe_permutation_scratch(T, K, max_rows, E)}, o);
-  mb::moe_build_permutation(ids.data_ptr<int>(), T, K, E, max_rows, max_tiles, align, counts.data_ptr<int>(),
-                            offsets.data_ptr<int>(), dest.data_ptr<int>(), src.data_ptr<int>(), tg.data_ptr<int>(),
-                            nt.data_ptr<int>(), scratch.data_ptr<int>(), cur_stream());
+  const cudaError_t e = mb::moe_build_permutation(ids.data_ptr<int>(), T, K, E, max_rows, max_tiles, align, counts.data_ptr<int>(),
+                                                  offsets.data_ptr<int>(), dest.data_ptr<int>(), src.data_ptr<int>(), tg.data_ptr<int>(),
+                                                  nt.data_ptr<int>(), scratch.data_ptr<int>(), cur_stream());
+  if (e != cudaSuccess) cudaGetLastError();  // (reported here)
+  TORCH_CHECK(e == cudaSuccess, "moe_build_permutation of ", T * K, " entries over ", E, " experts: ", cudaGetErrorString(e));
   return {counts, offsets, dest, src, tg, nt};
 }
 

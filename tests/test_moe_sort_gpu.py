@@ -40,7 +40,7 @@ def _expected(ids, E, max_rows, align):
 
 
 @pytest.mark.parametrize("T,K,E", [(1, 1, 1), (1, 8, 128), (16, 8, 128), (43, 3, 5), (64, 8, 128), (65, 8, 128), (512, 8, 512), (513, 8, 128),
-                                   (2049, 8, 1500), (9001, 8, 160)])
+                                   (2049, 8, 1500), (9001, 8, 160), (700, 8, 12288), (700, 8, 12289), (700, 8, 14500)])
 @pytest.mark.parametrize("align", [1, 64])
 @pytest.mark.parametrize("short", [False, True])
 def test_expert_sort_equals_a_sequential_one(ext, T, K, E, align, short):
@@ -55,6 +55,13 @@ def test_expert_sort_equals_a_sequential_one(ext, T, K, E, align, short):
     got = ext.moe_build_permutation(ids.to(DEV), E, max_rows, align)
     assert got[0].tolist() == counts and got[1].tolist() == off and got[2].tolist() == dest and got[3].tolist() == src
     assert got[5].tolist() == [len(tiles), off[-1]] and got[4][:len(tiles)].tolist() == tiles
+
+
+def test_more_experts_than_shared_memory_holds_are_refused(ext):
+    ids = torch.zeros(700, 8, dtype=torch.int32, device=DEV)
+    with pytest.raises(RuntimeError, match="20000 experts"):
+        ext.moe_build_permutation(ids, 20000, 5600, 1)
+    assert ext.moe_build_permutation(ids, 16, 5600, 1)[0].tolist() == [5600] + [0] * 15  # the refusal leaves no error behind
 
 
 @pytest.mark.parametrize("T,E,K", [(1, 16, 1), (1, 128, 8), (8, 128, 8), (5, 160, 6), (8, 1024, 32)])
