@@ -164,3 +164,36 @@ def test_logprob_entropy_forward_and_backward(ext, T, V, dtype):
     lf2 = logits.detach().clone().float().requires_grad_(True)
     (R.logprob_entropy(lf2, tg, inv_t)[0] * dlp).sum().backward()
     _close(ext.logprob_entropy_bwd(logits.clone(), tg, lse, px, dlp, None, inv_t), lf2.grad, 1e-2, 1e-6, frac=2e-3)
+
+
+@pytest.mark.parametrize("V,pitch", [(1, 1), (1003, 1003), (1000, 1003), (1004, 1004), (1000, 1000), (4104, 4112)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_logprob_backward_for_rows_of_any_width_and_alignment(V, pitch, dtype, shift):
+    """Whole vectors, single values, and rows or a first element off the vectors' boundaries; bf16 logits in place."""
+    from miles_b200.ops import _ext
+
+    ext, T, inv_t = _ext.load(required=True), 7, 1.25
+    g = torch.Generator().manual_seed(V + pitch)
+    buf = torch.full((T * pitch + shift,), 7.0, dtype=dtype, device="cuda")
+    logits = buf[shift:].view(T, pitch)[:, :V]
+    logits.copy_((3 * torch.randn(T, V, generator=g)).to(dtype))
+    tg = torch.randint(0, V, (T,), generator=g).to("cuda", torch.int32)
+    dlp, dent = (torch.randn(T, generator=g).cuda() for _ in range(2))
+    x = logits.double() * inv_t
+    lse = torch.logsumexp(x, -1)
+    p = torch.exp(x - lse[:, None])
+    px = (p * x).sum(-1)
+    want = -dlp[:, None] * p - dent[:, None] * p * (x - px[:, None])
+    want[torch.arange(T), tg.long()] += dlp
+    want = want * inv_t
+    out = ext.logprob_entropy_bwd(logits, tg, lse.float(), px.float(), dlp, dent, inv_t)
+    # one rounding to bf16; probabilities from fp32 differences of logits and sums of about 10 (2^-24 each, and the fast exponential)
+    size = (dlp.abs()[:, None] * p + dent.abs()[:, None] * p * ((x - px[:, None]).abs() + 1)) * inv_t
+    size[torch.arange(T), tg.long()] += dlp.abs() * inv_t
+    assert ((out.double() - want).abs() <= want.abs() * 2 ** -8 + size * 2e-5).all()
+    if dtype == torch.bfloat16:
+        assert out.data_ptr() == logits.data_ptr()
+        rest = torch.ones(T * pitch + shift, dtype=torch.bool, device="cuda")
+        rest[shift:].view(T, pitch)[:, :V] = False
+        assert (buf[rest] == 7).all()
