@@ -13,7 +13,7 @@
 // from the stage and from the activations with the same addressing.
 //
 // One kernel serves every small-batch product:
-//   dense    y[T, N]      = (norm?)(x) W^T (+ residual)           qkv / o / router logits / dense MLP
+//   dense    y[T, N]      = (norm?)(x) W^T (+ residual)           matrices of 48 MB and more with a norm to fold in
 //   MoE up   gu[pair, 2I] = W1[e] norm(x[token of pair])          for the active experts only
 //   MoE down y[pair, H]   = W2[e] (silu(gate) * up)[pair]         SwiGLU applied while gu is loaded
 // RMSNorm is folded in: y = rstd[t] * sum_k W[n,k] (g[k] x[t,k]); sum_k x^2 comes from the activation chunks the

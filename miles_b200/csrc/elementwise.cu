@@ -431,7 +431,7 @@ qk_norm_rope_bwd_kernel(const bf16* __restrict__ dq, const bf16* __restrict__ dk
 
 // ------------------------------------------------------------------ SwiGLU
 // in: [T, 2I] = [gate | up]; out: [T, I] = silu(gate) * up.
-// Eight values per thread and iteration. `Index` is 32 bits wide wherever the item count allows: a 64-bit division per item
+// Eight values per thread and iteration. `Index` is 32 bits wide wherever the item count allows (up to 64 GB of input): a 64-bit division per item
 // had bound these kernels (131072 rows of 2 x 768: forward 150 -> 132 us, backward of 139264 rows 211 -> 187 us), as had a grid of a few
 // blocks per SM, whose threads wait for one item's loads before they ask for the next.
 template <typename Index>

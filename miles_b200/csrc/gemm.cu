@@ -838,7 +838,6 @@ int gemm_bf16_launch(const GemmProblem& p, cudaStream_t stream) {
     if (p.N <= 128) bn = 128;
     // Skinny problems (decode projections): narrower tiles spread the weight stream over more SMs.
     if (!amn && !bmn && tiles(bn) < sms) {
-      if (bn == 256 && tiles(128) <= sms) bn = 128;
       if (bn == 128 && tiles(128) < sms / 2 && p.N >= 64) bn = 64;
       if (bn == 64 && tiles(64) < sms / 2 && p.N >= 32) bn = 32;
     }

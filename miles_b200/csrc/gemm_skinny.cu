@@ -1,4 +1,4 @@
-// y[T, N] = x[T, K] W[N, K]^T (+ residual) for at most 128 rows of x: decode steps and short prompts.
+// y[T, N] = x[T, K] W[N, K]^T (+ residual) for at most 128 rows of x: decode steps and short prompts of the engine.
 //
 // Such a product is bound by the bytes of W, and what decides its speed is how many of them are in flight, from how many
 // SMs, how soon after the launch. The weights are therefore the 128-row operand of the tensor-core tile and the tokens its

@@ -46,6 +46,7 @@ void moe_router_topk(const float* logits, const int* replay_ids, int* topk_ids, 
 // (padded), tile_group[max_tiles][4] = {expert, row0, rows, 0}, num_m_tiles[2] = {tiles, live rows},
 // expert_counts[E]. Scratch: as many ints as moe_permutation_scratch says for these sizes.
 long long moe_permutation_scratch(int T, int K, int max_rows, int E);
+int moe_permutation_launches(int T, int K, int max_rows, int E);  // kernels of one call
 cudaError_t moe_build_permutation(const int* topk_ids, int T, int K, int E, int max_rows, int max_tiles, int align,
                                   int* expert_counts, int* expert_offsets, int* dest_row, int* row_src, int* tile_group,
                                   int* num_m_tiles, int* scratch, cudaStream_t s);
@@ -92,7 +93,7 @@ struct PrefixGather {
 };
 void gather_prefix_kv(const PrefixGather& a, cudaStream_t s);
 
-// ---- attention.cu
+// ---- attention_decode.cu
 // Returns the CUDA error code of its own launches (0 = ok). `num_slots` = rows of the cache (0: unchecked page ids),
 // `status` (device int or null) receives 8 / 9 for a length / page id outside the tables.
 int paged_decode_attention(const void* q, const void* k_cache, const void* v_cache, const int* block_table,
@@ -121,7 +122,8 @@ int flash_attn_bwd(const void* q, long long q_ld, const void* k, long long k_ld,
 const char* flash_attn_bwd_last_error();
 
 // ---- decode_stream.cu / decode_small.cu (at most 8 tokens: persistent weight-streaming mma.sync kernel fed by
-// bulk asynchronous copies, RMSNorm folded in; `status` receives a code if a bounded wait gives up)
+// bulk asynchronous copies, RMSNorm folded in; `status` receives a code if a bounded wait gives up). small_gemv takes up to
+// 64 rows; above 8, and for large matrices without a norm, it is the split product of gemm_skinny.cu.
 // These return 0, or -1 with gemm_last_error() set.
 int small_gemv(const void* x, int T, const void* norm_w, float eps, const void* W, int N, int K, const void* residual,
                 void* out, bool out_fp32, int* status, cudaStream_t s);

@@ -594,6 +594,8 @@ static int sort_blocks(int n) { return n > 0 ? (n + SORT_WARPS * SORT_ROUNDS * 3
 // One block up to 4096 entries (16 warps of 8 rounds; its counts per warp need 4 (16 + 3) E bytes of shared memory).
 static bool sort_in_one_block(int n, int max_rows, int E) { return n <= 4096 && max_rows <= 16384 && E <= 512; }
 
+int moe_permutation_launches(int T, int K, int max_rows, int E) { return sort_in_one_block(T * K, max_rows, E) ? 1 : 3; }
+
 long long moe_permutation_scratch(int T, int K, int max_rows, int E) {
   return sort_in_one_block(T * K, max_rows, E) ? 0 : static_cast<long long>(sort_blocks(T * K)) * E;
 }

@@ -325,6 +325,7 @@ void register_elementwise(pybind11::module_& m) {
   m.def("moe_router_topk", &moe_router_topk);
   m.def("moe_router_bwd", &moe_router_bwd);
   m.def("moe_build_permutation", &moe_build_permutation);
+  m.def("moe_permutation_launches", &mb::moe_permutation_launches);
   m.def("moe_permute", &moe_permute);
   m.def("moe_combine", &moe_combine, pybind11::arg("y_perm"), pybind11::arg("dest_row"), pybind11::arg("w"), pybind11::arg("T"),
         pybind11::arg("K"), pybind11::arg("residual") = c10::optional<at::Tensor>());

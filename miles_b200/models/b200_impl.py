@@ -8,7 +8,8 @@ weight gradients are accumulated by the GEMM epilogue directly into the persiste
 (the role of Megatron's ``main_grad`` + gradient-accumulation fusion).
 
 The same object serves the rollout engine (prefill and paged-KV decode), so trainer and engine share
-kernels and reduction orders — the basis for trainer/rollout log-prob parity.
+weights, kernels and rounding points — the basis for trainer/rollout log-prob parity. Reduction orders are the same in
+passes of more than 128 rows; for fewer the engine has kernels that cut a sum over K into parts (``linear``).
 """
 from __future__ import annotations
 
@@ -217,7 +218,7 @@ class B200Qwen3:
         T, K = ids.shape
         max_rows = max(T * K + E_local * (align - 1), 1)
         counts, offsets, dest, src, tg, nt = self.C.moe_build_permutation(ids, E_local, max_rows, align)
-        self.launches += 1 if T * K <= 4096 and max_rows <= 16384 and E_local <= 512 else 3
+        self.launches += self.C.moe_permutation_launches(T, K, max_rows, E_local)
         ctx = MoeCtx(ids, None, None, offsets, dest, src, tg, nt, max_rows)
         ctx.align = align
         return ctx
