@@ -624,13 +624,21 @@ cudaError_t moe_build_permutation(const int* topk_ids, int T, int K, int E, int 
   if (e == cudaSuccess) e = allow(assign_kernel, assign_smem);
   if (e == cudaSuccess) e = cudaMemsetAsync(row_src, 0xff, sizeof(int) * static_cast<size_t>(max_rows), s);
   if (e != cudaSuccess) return e;
-  count_kernel<<<blocks, SORT_WARPS * 32, count_smem, s>>>(topk_ids, n, E, scratch);
-  if ((e = cudaPeekAtLastError()) != cudaSuccess) return e;
-  scan_kernel<<<1, 1024, scan_smem, s>>>(scratch, blocks, parts, E, max_rows, max_tiles, align, expert_counts, expert_offsets, tile_group,
-                                         num_m_tiles);
-  if ((e = cudaPeekAtLastError()) != cudaSuccess) return e;
-  assign_kernel<<<blocks, SORT_WARPS * 32, assign_smem, s>>>(topk_ids, n, E, scratch, expert_offsets, dest_row, row_src);
-  return cudaPeekAtLastError();
+  const auto launch = [s](auto kernel, int grid, int threads, size_t smem, auto... args) {  // its own result, not what others left
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = threads;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+  };
+  e = launch(count_kernel, blocks, SORT_WARPS * 32, count_smem, topk_ids, n, E, scratch);
+  if (e == cudaSuccess)
+    e = launch(scan_kernel, 1, 1024, scan_smem, scratch, blocks, parts, E, max_rows, max_tiles, align, expert_counts, expert_offsets,
+               tile_group, num_m_tiles);
+  if (e == cudaSuccess)
+    e = launch(assign_kernel, blocks, SORT_WARPS * 32, assign_smem, topk_ids, n, E, scratch, expert_offsets, dest_row, row_src);
+  return e;
 }
 
 void moe_permute(const void* x, const int* row_src, const int* num_m_tiles, void* x_perm, int max_rows, int H, int K,
