@@ -2,10 +2,11 @@
 
 There is no autograd graph and no tracing compiler on this path: forward and backward of a decoder
 layer are explicit sequences of kernel launches (tcgen05 GEMMs, fused norm / rope / swiglu / routing
-kernels), activations are recomputed layer by layer in the backward pass (only each layer's input is
-kept, the "full recompute" policy of the reference recipe scripts/run_qwen3_30b_a3b.py:168-175), and
-weight gradients are accumulated by the GEMM epilogue directly into the persistent flat gradient buffer
-(the role of Megatron's ``main_grad`` + gradient-accumulation fusion).
+kernels). The backward takes the activations of the last layers, and the logits, from where the forward
+left them as far as the device has room, and recomputes the other layers from their inputs (the "full
+recompute" policy of the reference recipe scripts/run_qwen3_30b_a3b.py:168-175, which runs where nothing
+fits). Weight gradients are accumulated by the GEMM epilogue directly into the persistent flat gradient
+buffer (the role of Megatron's ``main_grad`` + gradient-accumulation fusion).
 
 The same object serves the rollout engine (prefill and paged-KV decode), so trainer and engine share
 weights, kernels and rounding points — the basis for trainer/rollout log-prob parity. Reduction orders are the same in
@@ -14,7 +15,7 @@ passes of more than 128 rows; for fewer the engine has kernels that cut a sum ov
 from __future__ import annotations
 
 from dataclasses import dataclass
-from typing import Optional
+from typing import NamedTuple, Optional
 
 import torch
 
@@ -39,6 +40,34 @@ class MoeCtx:
     align: int = 1
 
 
+class LayerActs(NamedTuple):
+    """What the backward of a layer needs of its forward."""
+    qkv: tuple                    # h1, rstd1, qkv, q, k, q_rstd, k_rstd
+    att: torch.Tensor
+    lse: object
+    ln2: tuple                    # h2, rstd2, x2
+    post_attn: Optional[tuple]
+    moe: Optional[tuple]
+    mlp: Optional[tuple]          # gate | up, SwiGLU
+
+
+def plan_kept(room: int, head_bytes: int, layer_bytes: list, first: int) -> tuple[bool, int]:
+    """What fits into ``room`` bytes: (the logits, the first of the last layers whose activations are kept). The last ones,
+    since they are the first to be given back. A mixture's layer of 16384 tokens is 2.4 GB and 3.2 ms of recomputation, 12288
+    rows of 151936 logits are 7.5 GB and 6 ms, so the logits come first. Whole passes, all recomputed -> all kept: four layers
+    and 16384 tokens of the mixture with its head 91.7 -> 70.5 ms, 777 tokens 12.3 -> 10.5, three layers of 4096 x 12288 with
+    9216 tokens 89.8 -> 71.6."""
+    head = 0 < head_bytes <= room
+    room -= head_bytes if head else 0
+    keep = first + len(layer_bytes)
+    for b in reversed(layer_bytes):
+        if b > room:
+            break
+        room -= b
+        keep -= 1
+    return head, keep
+
+
 class B200Qwen3:
     def __init__(self, cfg: ModelConfig, store: ParamStore, ep=None, tp=None):
         assert cfg.head_dim == 128, "the sm_100a attention/rope kernels are specialised for head_dim 128"
@@ -56,6 +85,7 @@ class B200Qwen3:
         self.cp_ctx = None  # (sample lengths, cp size, cp rank, group, comm, layout) while a context-parallel micro-batch runs
         self._ident: Optional[torch.Tensor] = None
         self.small_decode = True  # weight-streaming kernels for decode steps of at most SMALL_T rows
+        self.act_room: Optional[int] = None  # bytes of activations a training pass may keep (None: by what is free, see _room_for_acts)
         self.lm_chunk = 2048      # rows of the LM head per pass (--log-probs-chunk-size)
 
     def attention(self, q, k, v, cu):
@@ -591,27 +621,79 @@ class B200Qwen3:
         splits = max(1, 296 // ctas)
         return splits if splits <= 8 else min(16, max(8, 192 // ctas))
 
-    def layer_backward(self, i, x, dy, positions, cu, max_seqlen, replay_ids=None):
-        """Recompute layer i from its input ``x`` and back-propagate ``dy``; returns dx."""
-        cfg, P, G, C = self.cfg, self.store.params, self.store.grads, self.C
+    def _layer_acts(self, i, x, positions, cu, replay_ids=None, output: bool = False):
+        """Forward of layer i that keeps what its backward needs: (activations, layer output or None). The values are those
+        of ``layer_forward``, bit for bit: the same kernels, with the experts' rows padded for the weight gradients."""
+        cfg, P, C = self.cfg, self.store.params, self.C
         p = f"layers.{i}."
-        scale = cfg.head_dim ** -0.5
-        # ---- recompute forward, keeping what the backward needs
-        h1, rstd1, qkv, q, k, qr, kr = self._attn_qkv(i, x, positions, None, None)
-        v = self._v_view(qkv)
-        att, lse = self.attention(q, k, v, cu)
-        att2 = att.view(att.shape[0], -1)
-        h2, rstd2, x2 = self._o_proj_ln2(i, att2, x)
+        qkv = self._attn_qkv(i, x, positions, None, None)
+        att, lse = self.attention(qkv[3], qkv[4], self._v_view(qkv[2]), cu)
+        ln2 = h2, _, x2 = self._o_proj_ln2(i, att.view(att.shape[0], -1), x)
         post_attn = getattr(self, "_post_attn_saved", None) if cfg.post_norms else None
         self._post_attn_saved = None
         is_moe = cfg.layer_is_moe(i)
         assert not (is_moe and cfg.post_norms), "sandwich norms are wired for dense MLP layers"
         if is_moe:
-            _, saved = self.moe_forward(i, h2, replay_ids, None, keep=True)
-        else:
-            gu = self.linear(h2, P[p + "mlp.gate_up.weight"])
-            act = C.swiglu_fwd(gu)
+            y, saved = self.moe_forward(i, h2, replay_ids, None, keep=True, residual=x2 if output else None)
+            return LayerActs(qkv, att, lse, ln2, post_attn, saved, None), y
+        gu = self.linear(h2, P[p + "mlp.gate_up.weight"])
+        act = C.swiglu_fwd(gu)
+        self.launches += 1
+        y = None
+        if output and cfg.post_norms:
+            y, _ = C.rmsnorm_fwd(self.linear(act, P[p + "mlp.down.weight"]), None, P[p + "post_mlp_ln.weight"], cfg.rms_eps)
+            y = y.add_(x2)
             self.launches += 1
+        elif output:
+            y = self._row_parallel(act, P[p + "mlp.down.weight"], x2)
+        return LayerActs(qkv, att, lse, ln2, post_attn, None, (gu, act)), y
+
+    # ------------------------------------------------------------------ activations kept between the two directions
+    def _layer_act_bytes(self, i: int, T: int) -> int:
+        """Bytes of one layer's ``LayerActs`` over T tokens (matrices; the per-row statistics are a hundredth of them)."""
+        cfg = self.cfg
+        H, D = cfg.hidden_size, cfg.head_dim
+        cols = 3 * H + (3 * cfg.num_q_heads + 3 * cfg.num_kv_heads) * D  # h1, h2, x2; qkv and q, k; att
+        if not cfg.layer_is_moe(i):
+            return 2 * T * (cols + 3 * cfg.ffn_hidden_size)
+        rows = T * cfg.moe_top_k + cfg.num_experts * 63
+        return 2 * T * cols + 2 * rows * (2 * H + 3 * cfg.moe_ffn_hidden_size) + 4 * T * cfg.num_experts
+
+    def _room_for_acts(self) -> int:
+        """Bytes a training pass may hold on to: what the device and the allocator's cache have free beyond a seventh of the
+        device, the share that every part of this package that sizes itself by free memory leaves to activations."""
+        if self.act_room is not None:
+            return self.act_room
+        free, total = torch.cuda.mem_get_info(self.dev)
+        return free + torch.cuda.memory_reserved(self.dev) - torch.cuda.memory_allocated(self.dev) - total // 7
+
+    def _plan_acts(self, T: int, head_rows: int) -> tuple[bool, int]:
+        """(whether the logits are kept, first layer whose activations are). Where a pass exchanges data with other ranks
+        everything is recomputed: they have to take the same steps, and how much is free is each rank's own. So it is for a
+        subclass with layers of its own."""
+        lo, hi = self.store.layer_range
+        cls = type(self)
+        if (self.ep is not None or self.tp is not None or self.cp_ctx is not None or getattr(self.store, "begin_pass", None) is not None
+                or any(getattr(cls, f) is not getattr(B200Qwen3, f) for f in ("layer_forward", "layer_backward", "forward_hidden", "layers_backward"))):
+            return False, hi
+        return plan_kept(self._room_for_acts(), 4 * head_rows * self.store.lm_head().shape[0] if head_rows else 0,
+                         [self._layer_act_bytes(i, T) for i in range(lo, hi)], lo)
+
+    def layer_backward(self, i, x, dy, positions, cu, max_seqlen, replay_ids=None, acts: Optional[LayerActs] = None):
+        """Back-propagate ``dy`` through layer i, from the activations its forward kept or else recomputed from its input
+        ``x``; returns dx."""
+        cfg, P, G, C = self.cfg, self.store.params, self.store.grads, self.C
+        p = f"layers.{i}."
+        if acts is None:
+            acts, _ = self._layer_acts(i, x, positions, cu, replay_ids)
+        h1, rstd1, qkv, q, k, qr, kr = acts.qkv
+        v, att, lse = self._v_view(qkv), acts.att, acts.lse
+        att2 = att.view(att.shape[0], -1)
+        h2, rstd2, x2 = acts.ln2
+        post_attn, saved = acts.post_attn, acts.moe
+        is_moe = cfg.layer_is_moe(i)
+        if not is_moe:
+            gu, act = acts.mlp
         # ---- backward: MLP / MoE
         if is_moe:
             dh2 = self.moe_backward(i, h2, dy, saved)
@@ -663,10 +745,12 @@ class B200Qwen3:
     @torch.no_grad()
     def forward_hidden(self, tokens, positions, cu_seqlens, meta: Optional[InferMeta] = None, kv_cache=None,
                        replay: Optional[torch.Tensor] = None, record: Optional[list] = None, max_seqlen: int = 0,
-                       save_inputs: Optional[list] = None, x_in: Optional[torch.Tensor] = None):
+                       save_inputs: Optional[list] = None, x_in: Optional[torch.Tensor] = None, save_acts: Optional[dict] = None,
+                       keep_from: int = 0):
         """Runs this pipeline stage's layers (all of them without pipeline parallelism). The first stage embeds
         ``tokens``, later stages continue from ``x_in``; every stage but the last returns the raw hidden states that
-        the next stage consumes, the last one applies the final norm."""
+        the next stage consumes, the last one applies the final norm. ``save_acts`` receives the activations of the layers
+        from ``keep_from`` on, for ``layer_backward``."""
         cfg, P, C = self.cfg, self.store.params, self.C
         begin = getattr(self.store, "begin_pass", None)
         if begin is not None:
@@ -684,6 +768,9 @@ class B200Qwen3:
                 if replay is not None:
                     rid = replay[:, moe_idx]
                 moe_idx += 1
+            if save_acts is not None and i >= keep_from:
+                save_acts[i], x = self._layer_acts(i, x, positions, cu_seqlens, rid, output=True)
+                continue
             x = self.layer_forward(i, x, positions, cu_seqlens, max_seqlen, meta, kv_cache, rid, record)
         if save_inputs is not None:
             save_inputs.append(x)
@@ -694,7 +781,7 @@ class B200Qwen3:
         return h
 
     @torch.no_grad()
-    def _trunk_backward(self, inputs, x_last, h, rows, dhr, tokens, positions, cu_seqlens, max_seqlen, replay):
+    def _trunk_backward(self, inputs, x_last, h, rows, dhr, tokens, positions, cu_seqlens, max_seqlen, replay, acts=None):
         """Back-propagate ``dhr`` (gradient wrt the final-normed hidden rows) through the norm, layers and embedding."""
         cfg, P, G, C = self.cfg, self.store.params, self.store.grads, self.C
         dh = torch.zeros_like(h)
@@ -703,19 +790,21 @@ class B200Qwen3:
         dx = C.rmsnorm_bwd(dh, x_last, P["final_norm.weight"], rstd, None, G["final_norm.weight"], True)
         self.launches += 3
         del dh
-        return self.layers_backward(inputs, dx, tokens, positions, cu_seqlens, max_seqlen, replay)
+        return self.layers_backward(inputs, dx, tokens, positions, cu_seqlens, max_seqlen, replay, **(dict(acts=acts) if acts else {}))
 
     @torch.no_grad()
-    def layers_backward(self, inputs, dx, tokens, positions, cu_seqlens, max_seqlen, replay):
-        """Backward through this stage's layers: ``inputs[j]`` is the saved input of local layer ``j``, ``dx`` the
-        gradient of the stage's output. Returns the gradient of the stage's input (on the first stage it has been
+    def layers_backward(self, inputs, dx, tokens, positions, cu_seqlens, max_seqlen, replay, acts: Optional[dict] = None):
+        """Backward through this stage's layers: ``inputs[j]`` is the saved input of local layer ``j``, ``acts`` the activations
+        of the layers that kept them (given back as they are used), ``dx`` the gradient of the stage's output. Returns the gradient of the stage's input (on the first stage it has been
         added into the embedding gradient) and keeps it in ``self.last_dx_in``."""
         cfg, G = self.cfg, self.store.grads
         lo, hi = self.store.layer_range
         moe_layers = [i for i in range(cfg.num_layers) if cfg.layer_is_moe(i)]
         for i in reversed(range(lo, hi)):
             rid = replay[:, moe_layers.index(i)] if (replay is not None and cfg.layer_is_moe(i)) else None
-            dx = self.layer_backward(i, inputs[i - lo], dx, positions, cu_seqlens, max_seqlen, rid)
+            kw = dict(acts=acts.pop(i)) if acts and i in acts else {}
+            dx = self.layer_backward(i, inputs[i - lo], dx, positions, cu_seqlens, max_seqlen, rid, **kw)
+            del kw
             inputs[i - lo] = None
         if self.store.is_first_stage:
             G["embed.weight"].index_add_(0, tokens.long(), dx.to(G["embed.weight"].dtype))
@@ -730,14 +819,17 @@ class B200Qwen3:
         if not max_seqlen:
             max_seqlen = int((cu_seqlens[1:] - cu_seqlens[:-1]).max().item())
         inputs: list = []
-        h = self.forward_hidden(tokens, positions, cu_seqlens, replay=replay, max_seqlen=max_seqlen, save_inputs=inputs, x_in=x_in)
+        acts: dict = {}
+        keep_from = self._plan_acts(positions.shape[0], 0)[1]
+        keep = dict(save_acts=acts, keep_from=keep_from) if keep_from < self.store.layer_range[1] else {}
+        h = self.forward_hidden(tokens, positions, cu_seqlens, replay=replay, max_seqlen=max_seqlen, save_inputs=inputs, x_in=x_in, **keep)
         x_last = inputs.pop()
         rows = row_index.long()
         leaf = h[rows].float().detach().requires_grad_(True)
         with torch.enable_grad():
             loss, metrics = head_fn(leaf)
             loss.backward()
-        self._trunk_backward(inputs, x_last, h, rows, leaf.grad, tokens, positions, cu_seqlens, max_seqlen, replay)
+        self._trunk_backward(inputs, x_last, h, rows, leaf.grad, tokens, positions, cu_seqlens, max_seqlen, replay, acts)
         return loss.detach(), metrics
 
     @torch.no_grad()
@@ -745,7 +837,7 @@ class B200Qwen3:
         return self.linear(hidden_rows.contiguous(), self.store.lm_head(), out_dtype, serving)
 
     @torch.no_grad()
-    def logprobs_entropy(self, hidden_rows, targets, inv_temp: float, chunk: int = 0, keep_stats: bool = False):
+    def logprobs_entropy(self, hidden_rows, targets, inv_temp: float, chunk: int = 0, keep_stats: bool = False, keep_logits: Optional[list] = None):
         C = self.C
         chunk = chunk or self.lm_chunk
         n = hidden_rows.shape[0]
@@ -760,6 +852,8 @@ class B200Qwen3:
             l1, e1, s1, p1 = C.logprob_entropy_fwd(lg, tg[a:b], inv_temp)
             self.launches += 1
             lp[a:b], ent[a:b] = l1, e1
+            if keep_logits is not None:
+                keep_logits.append(lg)
             if keep_stats:
                 lse[a:b], px[a:b] = s1, p1
         return (lp, ent, lse, px) if keep_stats else (lp, ent)
@@ -781,13 +875,17 @@ class B200Qwen3:
         if not max_seqlen:
             max_seqlen = int((cu_seqlens[1:] - cu_seqlens[:-1]).max().item())
         inputs: list[torch.Tensor] = []
-        h = self.forward_hidden(tokens, positions, cu_seqlens, replay=replay, max_seqlen=max_seqlen, save_inputs=inputs, x_in=x_in)
+        acts: dict = {}
+        keep_head, keep_from = self._plan_acts(positions.shape[0], row_index.shape[0])
+        keep = dict(save_acts=acts, keep_from=keep_from) if keep_from < self.store.layer_range[1] else {}
+        h = self.forward_hidden(tokens, positions, cu_seqlens, replay=replay, max_seqlen=max_seqlen, save_inputs=inputs, x_in=x_in, **keep)
         x_last = inputs.pop()  # input of the final norm
         rows = row_index.long()
         hr = h[rows].contiguous()
         tg = targets.to(torch.int32).contiguous()
+        kept: Optional[list] = [] if keep_head else None
         with torch.no_grad():
-            lp, ent, lse, px = self.logprobs_entropy(hr, tg, inv_temp, chunk, keep_stats=True)
+            lp, ent, lse, px = self.logprobs_entropy(hr, tg, inv_temp, chunk, keep_stats=True, keep_logits=kept)
         lp_leaf, ent_leaf = lp.detach().requires_grad_(True), ent.detach().requires_grad_(True)
         with torch.enable_grad():
             loss, metrics = loss_fn(lp_leaf, ent_leaf)
@@ -795,18 +893,20 @@ class B200Qwen3:
         dlp = grads[0].float().contiguous() if grads[0] is not None else torch.zeros_like(lp)
         dent = grads[1].float().contiguous() if grads[1] is not None else None
         with torch.no_grad():
-            # ---- LM head backward, chunked: recompute logits, turn them into dlogits in place
+            # ---- LM head backward, chunked: the logits, kept or recomputed, become dlogits
             W = self.store.lm_head()
             gW = G["embed.weight"] if cfg.tie_embeddings else G["lm_head.weight"]
             dhr = torch.empty_like(hr)
-            for a in range(0, hr.shape[0], chunk):
+            for j, a in enumerate(range(0, hr.shape[0], chunk)):
                 b = min(a + chunk, hr.shape[0])
-                lg = self.logits(hr[a:b], serving=False)
+                lg = kept[j] if kept is not None else self.logits(hr[a:b], serving=False)
                 dl = C.logprob_entropy_bwd(lg, tg[a:b], lse[a:b].contiguous(), px[a:b].contiguous(), dlp[a:b].contiguous(),
                                            dent[a:b].contiguous() if dent is not None else None, inv_temp)
                 del lg
+                if kept is not None:
+                    kept[j] = None
                 self._gemm(dl, W, dhr[a:b], False, True)
                 self.linear_wgrad(dl, hr[a:b], gW)
                 self.launches += 1
-            self._trunk_backward(inputs, x_last, h, rows, dhr, tokens, positions, cu_seqlens, max_seqlen, replay)
+            self._trunk_backward(inputs, x_last, h, rows, dhr, tokens, positions, cu_seqlens, max_seqlen, replay, acts)
         return loss.detach(), metrics, lp.detach(), ent.detach()
