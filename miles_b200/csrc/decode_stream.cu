@@ -136,8 +136,8 @@ __global__ void __launch_bounds__(THREADS, 1) stream_kernel(const StreamArgs a) 
   const int total = n_groups * tiles;
   // contiguous ranges: a CTA stays inside one expert for most of its items, so the activation fragments and the
   // index chain behind them are reloaded once or twice per launch, not once per tile
-  const int per_cta = (total + gridDim.x - 1) / gridDim.x;
-  const int L_begin = min(total, static_cast<int>(blockIdx.x) * per_cta), L_end = min(total, L_begin + per_cta);
+  const int L_begin = static_cast<int>(static_cast<long long>(total) * blockIdx.x / gridDim.x);
+  const int L_end = static_cast<int>(static_cast<long long>(total) * (blockIdx.x + 1) / gridDim.x);
   int g = L_begin / tiles, t = L_begin - g * tiles;
   int stage = 0;
   uint32_t phase = 0;

@@ -136,6 +136,16 @@ int moe_small_up(const void* x, const void* norm_w, float eps, const void* W1, c
 int moe_small_down(const void* gu, const void* W2, const int* active, const int* pair_count, const int* pair_list,
                     int max_active, int H, int I, void* y, int* status, cudaStream_t s);
 
+// ---- decode_moe.cu (at most 8 tokens; the plan has moe_decode_plan_size ints)
+int moe_decode_plan_size(int E);
+bool moe_decode_fits(int E, int K, int H, int I);
+int router_decode(const void* x, int T, const void* norm_w, float eps, const void* W, int E, int H, int K, bool renorm, int* topk_ids,
+                  float* topk_w, int* plan, cudaStream_t s);
+int moe_decode_up(const void* x, int T, const void* norm_w, float eps, const void* W1, const int* plan, int max_active, int E, int H, int I,
+                  void* act, int* status, cudaStream_t s);
+int moe_decode_down(const void* act, const void* W2, const int* plan, const void* residual, int T, int E, int H, int I, void* y, int* status,
+                    cudaStream_t s);
+
 // ---- rl.cu
 void gae_reverse_scan(const float* rewards, const float* values, const int* cu_seqlens, float* adv, float* ret,
                       int num_seqs, float gamma, float lam, cudaStream_t s);

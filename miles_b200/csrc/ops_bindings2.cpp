@@ -164,6 +164,46 @@ void moe_small_down(const at::Tensor& act, const at::Tensor& W2, const at::Tenso
   TORCH_CHECK(rc == 0, mb::gemm_last_error());
 }
 
+bool moe_decode_fits(int64_t E, int64_t K, int64_t H, int64_t I) { return mb::moe_decode_fits(E, K, H, I); }
+int64_t moe_decode_plan_size(int64_t E) { return mb::moe_decode_plan_size(E); }
+
+// Routing of at most 8 rows: expert ids and weights [T, K], and the plan that the next two take.
+void router_decode(const at::Tensor& x, const at::Tensor& norm_w, double eps, const at::Tensor& W, bool renorm, at::Tensor& ids, at::Tensor& w,
+                   at::Tensor& plan) {
+  CHECK_BF16(x); CHECK_BF16(norm_w); CHECK_BF16(W); CHECK_I32(ids); CHECK_F32(w); CHECK_I32(plan);
+  const int T = x.size(0), H = x.size(1), E = W.size(0), K = ids.size(1);
+  TORCH_CHECK(T >= 1 && T <= 8 && W.size(1) == H && norm_w.numel() == H && ids.size(0) == T && w.sizes() == ids.sizes() &&
+                  plan.numel() >= mb::moe_decode_plan_size(E) && mb::moe_decode_fits(E, K, H, 32), "router_decode: unsupported shape");
+  const c10::cuda::CUDAGuard guard(x.device());
+  const int rc = mb::router_decode(x.data_ptr(), T, norm_w.data_ptr(), eps, W.data_ptr(), E, H, K, renorm, ids.data_ptr<int>(), w.data_ptr<float>(),
+                                   plan.data_ptr<int>(), cur_stream());
+  TORCH_CHECK(rc == 0, mb::gemm_last_error());
+}
+
+void moe_decode_up(const at::Tensor& x, const at::Tensor& norm_w, double eps, const at::Tensor& W1, const at::Tensor& plan, at::Tensor& act,
+                   const c10::optional<at::Tensor>& status) {
+  CHECK_BF16(x); CHECK_BF16(norm_w); CHECK_BF16(W1); CHECK_I32(plan); CHECK_BF16(act);
+  const int T = x.size(0), H = x.size(1), I = act.size(1), E = W1.size(0), pairs = act.size(0);
+  TORCH_CHECK(W1.dim() == 3 && T >= 1 && T <= 8 && pairs % T == 0 && W1.size(1) == 2 * I && W1.size(2) == H && norm_w.numel() == H &&
+                  plan.numel() >= mb::moe_decode_plan_size(E) && mb::moe_decode_fits(E, pairs / T, H, I), "moe_decode_up: unsupported shape");
+  const c10::cuda::CUDAGuard guard(x.device());
+  const int rc = mb::moe_decode_up(x.data_ptr(), T, norm_w.data_ptr(), eps, W1.data_ptr(), plan.data_ptr<int>(), std::min(E, pairs), E, H, I,
+                                   act.data_ptr(), status.has_value() ? status->data_ptr<int>() : nullptr, cur_stream());
+  TORCH_CHECK(rc == 0, mb::gemm_last_error());
+}
+
+void moe_decode_down(const at::Tensor& act, const at::Tensor& W2, const at::Tensor& plan, const at::Tensor& residual, at::Tensor& y,
+                     const c10::optional<at::Tensor>& status) {
+  CHECK_BF16(act); CHECK_BF16(W2); CHECK_BF16(residual); CHECK_BF16(y); CHECK_I32(plan);
+  const int T = y.size(0), I = act.size(1), H = W2.size(1), E = W2.size(0), pairs = act.size(0);
+  TORCH_CHECK(W2.dim() == 3 && T >= 1 && T <= 8 && pairs % T == 0 && W2.size(2) == I && y.size(1) == H && residual.numel() == y.numel() &&
+                  plan.numel() >= mb::moe_decode_plan_size(E) && mb::moe_decode_fits(E, pairs / T, H, I), "moe_decode_down: unsupported shape");
+  const c10::cuda::CUDAGuard guard(act.device());
+  const int rc = mb::moe_decode_down(act.data_ptr(), W2.data_ptr(), plan.data_ptr<int>(), residual.data_ptr(), T, E, H, I, y.data_ptr(),
+                                     status.has_value() ? status->data_ptr<int>() : nullptr, cur_stream());
+  TORCH_CHECK(rc == 0, mb::gemm_last_error());
+}
+
 std::vector<at::Tensor> gae(const at::Tensor& rewards, const at::Tensor& values, const at::Tensor& cu, double gamma, double lam) {
   CHECK_F32(rewards); CHECK_F32(values); CHECK_I32(cu);
   const c10::cuda::CUDAGuard guard(rewards.device());
@@ -256,6 +296,11 @@ void register_more(pybind11::module_& m) {
         pybind11::arg("block_table"), pybind11::arg("seq_lens"), pybind11::arg("out"), pybind11::arg("scratch"),
         pybind11::arg("page_size"), pybind11::arg("num_splits"), pybind11::arg("scale"), pybind11::arg("status") = pybind11::none());
   m.def("flash_attn_fwd", &flash_attn_fwd);
+  m.def("router_decode", &router_decode);
+  m.def("moe_decode_down", &moe_decode_down);
+  m.def("moe_decode_up", &moe_decode_up);
+  m.def("moe_decode_fits", &moe_decode_fits);
+  m.def("moe_decode_plan_size", &moe_decode_plan_size);
   m.def("flash_attn_bwd", &flash_attn_bwd);
   m.def("router_small", &router_small);
   m.def("gather_prefix_kv", &gather_prefix_kv);

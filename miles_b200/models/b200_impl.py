@@ -572,8 +572,8 @@ class B200Qwen3:
         return x2
 
     def _layer_forward_small(self, i, x, positions, meta: InferMeta, kv_cache, record=None):
-        """Decode forward of one layer for at most 8 rows: 8-9 light launches instead of 14-15, the two RMSNorms
-        folded into the projections that consume them, no expert permutation (per-expert pair lists)."""
+        """Decode forward of one layer for at most 8 rows: few light launches instead of 14-15, the two RMSNorms folded into the
+        projections that consume them, SwiGLU and the combination into the experts', no expert permutation (per-expert pair lists)."""
         cfg, P, C = self.cfg, self.store.params, self.C
         p = f"layers.{i}."
         T, dev = x.shape[0], x.device
@@ -582,8 +582,20 @@ class B200Qwen3:
         if cfg.layer_is_moe(i):
             E, K = cfg.num_experts, cfg.moe_top_k
             w1, w2 = P[p + "moe.w1"], P[p + "moe.w2"]
+            I = w2.shape[2]
             ids = torch.empty(T, K, dtype=torch.int32, device=dev)
             w = torch.empty(T, K, dtype=torch.float32, device=dev)
+            if C.moe_decode_fits(E, K, x.shape[1], I):
+                plan = torch.empty(C.moe_decode_plan_size(E), dtype=torch.int32, device=dev)
+                C.router_decode(x2, ln2, cfg.rms_eps, P[p + "moe.router.weight"], cfg.norm_topk_prob, ids, w, plan)
+                if record is not None:
+                    record.append(ids)
+                act = torch.empty(T * K, I, dtype=torch.bfloat16, device=dev)
+                C.moe_decode_up(x2, ln2, cfg.rms_eps, w1, plan, act, self.status)
+                y = torch.empty_like(x2)
+                C.moe_decode_down(act, w2, plan, x2, y, self.status)
+                self.launches += 3
+                return y
             lists = torch.empty(1 + E + E + 8 * E, dtype=torch.int32, device=dev)
             active, pc, pl = lists[:1 + E], lists[1 + E:1 + 2 * E], lists[1 + 2 * E:]
             logits = torch.empty(T, E, dtype=torch.float32, device=dev)
