@@ -66,24 +66,28 @@ struct Tile {
   long long c_base;
 };
 
-template <int BLOCK_N, bool B_MN>
+// CG: CTAs that share a tile (BLOCK_M rows each).
+template <int BLOCK_N, bool B_MN, int CG>
 __device__ __forceinline__ int num_tiles_of(const KArgs& p) {
   const int n_tiles = (p.N + BLOCK_N - 1) / BLOCK_N;
-  if (p.mode == GEMM_DENSE) return ((p.M + BLOCK_M - 1) / BLOCK_M) * n_tiles;
+  constexpr int TILE_M = BLOCK_M * CG;
+  if (p.mode == GEMM_DENSE) return ((p.M + TILE_M - 1) / TILE_M) * n_tiles;
   if (p.mode == GEMM_GROUPED_ROWS) {
     int live = *p.num_m_tiles;
     const int cap = p.max_tiles;
     live = live < 0 ? 0 : (live > cap ? cap : live);
     return live * n_tiles;
   }
-  return p.num_groups * ((p.M + BLOCK_M - 1) / BLOCK_M) * n_tiles;
+  return p.num_groups * ((p.M + TILE_M - 1) / TILE_M) * n_tiles;
 }
 
-template <int BLOCK_N, bool B_MN>
-__device__ __forceinline__ Tile decode_tile(const KArgs& p, int t) {
+// `rank`: of the CTA among those that share the tile; rows are its own, columns the whole tile's.
+template <int BLOCK_N, bool B_MN, int CG>
+__device__ __forceinline__ Tile decode_tile(const KArgs& p, int t, int rank) {
   Tile r;
+  constexpr int TILE_M = BLOCK_M * CG;
   const int n_tiles = (p.N + BLOCK_N - 1) / BLOCK_N;
-  const int m_tiles = (p.M + BLOCK_M - 1) / BLOCK_M;
+  const int m_tiles = (p.M + TILE_M - 1) / TILE_M;
   if (p.mode == GEMM_DENSE) {
     // Rasterise in bands of 8 row tiles so that concurrently running CTAs share B tiles in L2.
     constexpr int BAND = 8;
@@ -94,7 +98,7 @@ __device__ __forceinline__ Tile decode_tile(const KArgs& p, int t) {
     const int in_band = t - band * per_band;
     const int mt = first_m + in_band % band_rows;
     const int nt = in_band / band_rows;
-    r.a_mn0 = mt * BLOCK_M;
+    r.a_mn0 = mt * TILE_M + rank * BLOCK_M;
     r.b_mn0 = nt * BLOCK_N;
     r.a_k0 = 0;
     r.b_k0 = 0;
@@ -131,7 +135,7 @@ __device__ __forceinline__ Tile decode_tile(const KArgs& p, int t) {
     const int nt = rem - mt * n_tiles;
     const int k_lo = p.group_offsets[g];
     const int k_hi = p.group_offsets[g + 1];
-    r.a_mn0 = mt * BLOCK_M;
+    r.a_mn0 = mt * TILE_M + rank * BLOCK_M;
     r.b_mn0 = nt * BLOCK_N;
     r.a_k0 = k_lo;
     r.b_k0 = k_lo;
@@ -372,11 +376,20 @@ struct StagedEpilogue {
   }
 };
 
-template <int BLOCK_N, bool A_MN, bool B_MN, int STAGES>
+// CG = 2: a pair of CTAs (a cluster) multiplies 256 x 256 tiles with `cta_group::2`: each holds its 128 rows of A and half of B's,
+// so that a tile's operands are read from shared memory, and from L2, two thirds as often for the same work. That is what bounds the
+// one-CTA tile: per 16 of K it reads 12 KB of shared memory and receives another 12 KB in the 128 clocks of its product (at 128 bytes
+// a clock), and under the power cap those reads cost clock. The CTA of rank 0 issues; its `full` barrier counts both CTAs' copies, its
+// `tempty` both epilogues; `empty` and `tfull` are raised in both by its commits. Sums are those of one CTA bit for bit.
+// Measured over seconds, at the power cap, TFLOP/s one CTA -> pair: 8192^3 1181 -> 1283 (cuBLAS 1372), 16384 x 5120 x 2048 1170 ->
+// 1233, 9216 x 24576 x 4096 1202 -> 1288, its weight gradient 1116 -> 1209, 2048 x 151936 x 2048 to fp32 1044 -> 1159. Grouped
+// contractions gain nothing (131072 rows over 128 experts 872 and 893, 65536 rows 668 and 656) and stay with one CTA.
+template <int BLOCK_N, bool A_MN, bool B_MN, int STAGES, int CG>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                  const KArgs p) {
-  constexpr int B_STAGE_BYTES = BLOCK_N * BLOCK_K * 2;
+  constexpr int B_ROWS = BLOCK_N / CG;  // of this CTA
+  constexpr int B_STAGE_BYTES = B_ROWS * BLOCK_K * 2;
   constexpr uint32_t TMEM_COLS = 2 * BLOCK_N;  // 256 or 512: a power of two >= 32
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -395,6 +408,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
+  const int rank = CG == 2 ? static_cast<int>(cluster_ctarank()) : 0;
+  const int first_tile = blockIdx.x / CG, tile_step = gridDim.x / CG;
 
   if (threadIdx.x == 0) {
     abort_flag_s = 0;
@@ -404,15 +419,19 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(tfull_bar(a), 1);
-      mbar_init(tempty_bar(a), 8);  // one arrive per epilogue warp
+      mbar_init(tempty_bar(a), 8 * CG);  // one arrive per epilogue warp
     }
     fence_barrier_init();
     prefetch_tensormap(&tma_a);
     prefetch_tensormap(&tma_b);
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, TMEM_COLS);
-    tmem_relinquish();
+    if constexpr (CG == 2) {
+      tmem_alloc_pair(tmem_slot, TMEM_COLS);
+    } else {
+      tmem_alloc(tmem_slot, TMEM_COLS);
+      tmem_relinquish();
+    }
   }
   tc_fence_before();
   __syncthreads();
@@ -424,9 +443,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   }
   __syncthreads();
   const uint32_t tmem_base = tmem_base_s;
+  if constexpr (CG == 2) cluster_sync_all();  // both CTAs' barriers and TMEM are there before either uses the other's
   pdl_enter();
 
-  const int total_tiles = num_tiles_of<BLOCK_N, B_MN>(p);
+  const int total_tiles = num_tiles_of<BLOCK_N, B_MN, CG>(p);
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -434,32 +454,45 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int t = blockIdx.x; ok && t < total_tiles; t += gridDim.x) {
-        const Tile tl = decode_tile<BLOCK_N, B_MN>(p, t);
+      const auto load = [](uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
+        if constexpr (CG == 2) tma_load_2d_pair(dst, map, bar, c0, c1);
+        else tma_load_2d(dst, map, bar, c0, c1);
+      };
+      for (int t = first_tile; ok && t < total_tiles; t += tile_step) {
+        const Tile tl = decode_tile<BLOCK_N, B_MN, CG>(p, t, rank);
+        const int b_mn0 = tl.b_mn0 + rank * B_ROWS;
         for (int kb = 0; kb < tl.k_iters; ++kb) {
           if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, p.status, ERR_WAIT_EMPTY)) {
             ok = false;
             break;
           }
-          mbar_expect_tx(full_bar(stage), A_STAGE_BYTES + B_STAGE_BYTES);
+          if (rank == 0) mbar_expect_tx(full_bar(stage), CG * (A_STAGE_BYTES + B_STAGE_BYTES));
+          const uint32_t full = CG == 2 ? map_to_rank(full_bar(stage), 0) : full_bar(stage);
           const uint32_t a_dst = a_smem + stage * A_STAGE_BYTES;
           const uint32_t b_dst = b_smem + stage * B_STAGE_BYTES;
           const int ka = tl.a_k0 + kb * BLOCK_K;
           const int kbb = tl.b_k0 + kb * BLOCK_K;
           if (A_MN) {
 #pragma unroll
-            for (int i = 0; i < BLOCK_M / 64; ++i)
-              tma_load_2d(a_dst + i * (BLOCK_K * 128), &tma_a, full_bar(stage), tl.a_mn0 + 64 * i, ka);
+            for (int i = 0; i < BLOCK_M / 64; ++i) load(a_dst + i * (BLOCK_K * 128), &tma_a, full, tl.a_mn0 + 64 * i, ka);
           } else {
-            tma_load_2d(a_dst, &tma_a, full_bar(stage), ka, tl.a_mn0);
+            load(a_dst, &tma_a, full, ka, tl.a_mn0);
           }
           if (B_MN) {
 #pragma unroll
-            for (int i = 0; i < BLOCK_N / 64; ++i)
-              tma_load_2d(b_dst + i * (BLOCK_K * 128), &tma_b, full_bar(stage), tl.b_mn0 + 64 * i, kbb);
+            for (int i = 0; i < B_ROWS / 64; ++i) load(b_dst + i * (BLOCK_K * 128), &tma_b, full, b_mn0 + 64 * i, kbb);
           } else {
-            tma_load_2d(b_dst, &tma_b, full_bar(stage), kbb, tl.b_mn0);
+            load(b_dst, &tma_b, full, kbb, b_mn0);
           }
+          if (++stage == STAGES) {
+            stage = 0;
+            phase ^= 1u;
+          }
+        }
+      }
+      if constexpr (CG == 2) {  // the other CTA's commits have arrived before this one leaves
+        for (int s = 0; ok && s < STAGES; ++s) {
+          ok = mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, p.status, ERR_WAIT_EMPTY);
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1u;
@@ -475,13 +508,17 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    constexpr uint32_t idesc = make_idesc_bf16(BLOCK_M, BLOCK_N, A_MN, B_MN);
+    constexpr uint32_t idesc = make_idesc_bf16(BLOCK_M * CG, BLOCK_N, A_MN, B_MN);
+    const auto commit = [](uint32_t bar) {
+      if constexpr (CG == 2) umma_commit_pair(bar);
+      else umma_commit(bar);
+    };
     int stage = 0;
     uint32_t phase = 0;
     int iter = 0;  // counts only tiles that use an accumulator, so both roles stay in phase
     bool ok = true;
-    for (int t = blockIdx.x; ok && t < total_tiles; t += gridDim.x) {
-      const Tile tl = decode_tile<BLOCK_N, B_MN>(p, t);
+    for (int t = first_tile; ok && rank == 0 && t < total_tiles; t += tile_step) {
+      const Tile tl = decode_tile<BLOCK_N, B_MN, CG>(p, t, rank);
       if (tl.k_iters == 0) continue;  // epilogue writes zeros without touching TMEM
       const int acc = iter & 1;
       const uint32_t acc_phase = (iter >> 1) & 1u;
@@ -506,9 +543,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                                         : make_smem_desc(a_addr + k * UMMA_K * 2, 16, 1024);
             const uint64_t bdesc = B_MN ? make_smem_desc(b_addr + k * UMMA_K * 128, BLOCK_K * 128, 1024)
                                         : make_smem_desc(b_addr + k * UMMA_K * 2, 16, 1024);
-            umma_f16(d_tmem, adesc, bdesc, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            if constexpr (CG == 2) umma_f16_pair(d_tmem, adesc, bdesc, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            else umma_f16(d_tmem, adesc, bdesc, idesc, (kb > 0 || k > 0) ? 1u : 0u);
           }
-          umma_commit(empty_bar(stage));
+          commit(empty_bar(stage));
         }
         __syncwarp();
         if (++stage == STAGES) {
@@ -516,7 +554,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
           phase ^= 1u;
         }
       }
-      if (ok && lane == 0) umma_commit(tfull_bar(acc));
+      if (ok && lane == 0) commit(tfull_bar(acc));
       __syncwarp();
       ++iter;
     }
@@ -527,23 +565,29 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     const bool staged = BLOCK_N >= 64 && p.vec_ok && !p.row_ptrs && p.n_dest == 0;
     int iter = 0;
     bool ok = true;
+    const auto release = [&](int acc) {  // this warp's share of the accumulator has been read
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        if (CG == 2 && rank != 0) mbar_arrive_remote(map_to_rank(tempty_bar(acc), 0));
+        else mbar_arrive(tempty_bar(acc));
+      }
+    };
     auto add_tiles = [&](auto e) {
       const uint32_t stg = stage_buf + static_cast<uint32_t>(warp - 2) * 4096;
       int ready = -1;  // the tile whose first old values are on their way
-      for (int t = blockIdx.x; t < total_tiles; t += gridDim.x) {
-        const Tile tl = decode_tile<BLOCK_N, B_MN>(p, t);
+      for (int t = first_tile; t < total_tiles; t += tile_step) {
+        const Tile tl = decode_tile<BLOCK_N, B_MN, CG>(p, t, rank);
         if (tl.k_iters == 0) continue;
-        const int row0 = tl.c_row0 + quad * 32, acc = iter & 1, tn = t + gridDim.x;
+        const int row0 = tl.c_row0 + quad * 32, acc = iter & 1, tn = t + tile_step;
         if (ready != t) e.begin(p, tl, row0, lane, half);
-        const Tile next = decode_tile<BLOCK_N, B_MN>(p, tn < total_tiles ? tn : t);
+        const Tile next = decode_tile<BLOCK_N, B_MN, CG>(p, tn < total_tiles ? tn : t, rank);
         const bool more = tn < total_tiles && next.k_iters > 0;
         if (!__all_sync(0xffffffffu, mbar_wait(tfull_bar(acc), (iter >> 1) & 1u, abort_flag, p.status, ERR_WAIT_TMEM_FULL))) break;
         tc_fence_after();
         const uint32_t t_addr = tmem_base + acc * BLOCK_N + (static_cast<uint32_t>(quad * 32) << 16);
         ready = e.run(p, tl, next, more, row0, next.c_row0 + quad * 32, lane, half, t_addr, stg) ? tn : -1;
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(tempty_bar(acc));
+        release(acc);
         ++iter;
       }
     };
@@ -552,8 +596,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       if (adds && p.out_fp32) add_tiles(StagedEpilogue<BLOCK_N, true, true>());
       else if (adds) add_tiles(StagedEpilogue<BLOCK_N, false, true>());
     }
-    for (int t = blockIdx.x; ok && !adds && t < total_tiles; t += gridDim.x) {
-      const Tile tl = decode_tile<BLOCK_N, B_MN>(p, t);
+    for (int t = first_tile; ok && !adds && t < total_tiles; t += tile_step) {
+      const Tile tl = decode_tile<BLOCK_N, B_MN, CG>(p, t, rank);
       const int row = tl.c_row0 + quad * 32 + lane;
       uint32_t acc_regs[32];
       if (tl.k_iters == 0) {
@@ -665,9 +709,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
           e.run(p, tl, tl, false, row0, row0, lane, half, t_addr, stg);
         }
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(tempty_bar(acc));
+      release(acc);
       ++iter;
     }
     if (p.row_ptrs || p.n_dest > 0) __threadfence_system();  // peer stores are visible before the CTA reports in
@@ -675,9 +717,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 
   tc_fence_before();
   __syncthreads();
+  if constexpr (CG == 2) cluster_sync_all();  // neither CTA leaves while the other's products, copies or arrivals may reach it
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, TMEM_COLS);
+    if constexpr (CG == 2) tmem_dealloc_pair(tmem_base, TMEM_COLS);
+    else tmem_dealloc(tmem_base, TMEM_COLS);
   }
   if (p.sig_ctrl && threadIdx.x == 0) {
     __threadfence_system();
@@ -742,30 +786,44 @@ int gemm_make_map(CUtensorMap* map, const GemmOperand& op, int box_rows) {
 
 namespace {
 
-template <int BLOCK_N, bool A_MN, bool B_MN>
+template <int BLOCK_N, bool A_MN, bool B_MN, int CG = 1>
 int launch(const GemmProblem& p, const KArgs& ka, cudaStream_t stream) {
   // (the 32 KB staging buffer takes a pipeline stage from the 128-wide variant)
-  constexpr int STAGES = BLOCK_N == 256 ? 4 : (BLOCK_N == 128 ? 5 : 8);
-  constexpr int B_STAGE_BYTES = BLOCK_N * BLOCK_K * 2;
+  constexpr int STAGES = CG == 2 ? 6 : (BLOCK_N == 256 ? 4 : (BLOCK_N == 128 ? 5 : 8));
+  constexpr int B_STAGE_BYTES = BLOCK_N / CG * BLOCK_K * 2;
   constexpr int SMEM = STAGES * (A_STAGE_BYTES + B_STAGE_BYTES) + 8 * (2 * STAGES + 5) + 1024 +
                        8 * 4096 + 128;
   CUtensorMap ma, mb_;
   if (gemm_make_map(&ma, p.a, A_MN ? BLOCK_K : BLOCK_M)) return -1;
-  if (gemm_make_map(&mb_, p.b, B_MN ? BLOCK_K : BLOCK_N)) return -1;
-  auto kern = gemm_bf16_kernel<BLOCK_N, A_MN, B_MN, STAGES>;
+  if (gemm_make_map(&mb_, p.b, B_MN ? BLOCK_K : BLOCK_N / CG)) return -1;
+  auto kern = gemm_bf16_kernel<BLOCK_N, A_MN, B_MN, STAGES, CG>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)  // per (function, device)
     return fail("cudaFuncSetAttribute(MaxDynamicSharedMemorySize) failed");
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long long m_tiles = (p.M + BLOCK_M - 1) / BLOCK_M;
+  const long long m_tiles = (p.M + CG * BLOCK_M - 1) / (CG * BLOCK_M);
   const long long n_tiles = (p.N + BLOCK_N - 1) / BLOCK_N;
   long long tiles = (p.mode == GEMM_GROUPED_ROWS ? static_cast<long long>(p.max_tiles) : m_tiles) * n_tiles *
                     (p.mode == GEMM_GROUPED_CONTR ? p.num_groups : 1);
-  int grid = static_cast<int>(tiles < sms ? tiles : sms);
-  if (p.max_ctas > 0 && grid > p.max_ctas) grid = p.max_ctas;
+  int grid = static_cast<int>(tiles < sms / CG ? tiles : sms / CG);
+  if (p.max_ctas > 0 && grid > p.max_ctas / CG) grid = p.max_ctas / CG;
   if (grid <= 0) return 0;
-  const cudaError_t e = pdl_launch(kern, grid, kThreads, SMEM, stream, ma, mb_, ka);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid * CG;
+  cfg.blockDim = kThreads;
+  cfg.dynamicSmemBytes = SMEM;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = CG;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = CG == 2 ? 2 : 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ma, mb_, ka);
   if (e != cudaSuccess) {
     cudaGetLastError();  // (reported here)
     return fail(std::string("gemm launch failed: ") + cudaGetErrorString(e));
@@ -842,11 +900,27 @@ int gemm_bf16_launch(const GemmProblem& p, cudaStream_t stream) {
       if (bn == 64 && tiles(64) < sms / 2 && p.N >= 32) bn = 32;
     }
   }
+  // Tiles of two CTAs where they need no more waves than the one-CTA tiles (rows that a pair pads cost as much as others: 777 x 5120,
+  // K = 2048, two waves instead of one, 906 -> 575 TFLOP/s) and a wave is long enough to carry the pair's start: K of 1024 at least
+  // (5120 x 2048, two tiles per CTA, K = 2000 817 -> 843, K = 777 582 -> 573), or many waves (151936 x 2048, K = 583: 544 -> 557).
+  // More than one wave, because a single one gains nothing (2000 x 2048, K = 4096: 1114 and 1088).
+  bool pair = bn == 256 && p.mode == GEMM_DENSE && !p.row_ptrs && p.n_dest == 0 && (p.max_ctas == 0 || p.max_ctas >= 2) && p.pair != 1;
+  if (pair && p.pair == 0) {
+    const long long n_tiles = (p.N + 255) / 256, sms = 148;
+    const long long single = ((p.M + 127) / 128 * n_tiles + sms - 1) / sms, paired = ((p.M + 255) / 256 * n_tiles + sms / 2 - 1) / (sms / 2);
+    pair = p.block_n == 0 && paired <= single && single > 1 && (p.K >= 1024 || single >= 16);
+  }
   if (p.row_ptrs || p.n_dest > 0) bn = 128;  // the staged scatter epilogue lives in the 128-wide variant
   if (bn != 32 && bn != 64 && bn != 128 && bn != 256) return fail("block_n must be 32, 64, 128 or 256");
   if ((bn == 32 || bn == 64) && (amn || bmn)) return fail("narrow tiles support K-major operands only");
   if (bn == 32) return launch<32, false, false>(p, ka, stream);
   if (bn == 64) return launch<64, false, false>(p, ka, stream);
+  if (pair) {
+    if (!amn && !bmn) return launch<256, false, false, 2>(p, ka, stream);
+    if (!amn && bmn) return launch<256, false, true, 2>(p, ka, stream);
+    if (amn && !bmn) return launch<256, true, false, 2>(p, ka, stream);
+    return launch<256, true, true, 2>(p, ka, stream);
+  }
 #define MB_DISPATCH(BN)                                                     \
   if (!amn && !bmn) return launch<BN, false, false>(p, ka, stream);         \
   if (!amn && bmn) return launch<BN, false, true>(p, ka, stream);           \

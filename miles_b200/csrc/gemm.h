@@ -40,6 +40,7 @@ struct GemmProblem {
   const int* group_offsets;  // mode 2: [num_groups+1] row offsets, multiples of 64
   int* status;               // device status word (0 = ok); may be null
   int block_n;               // 0 = choose, else 128 or 256
+  int pair;                  // tiles of two CTAs: 0 = choose, 1 = never, 2 = wherever they can be (dense, block_n 256)
   bool whole_k;              // block_n 0: every sum runs over K in one order, however few the rows
   int max_ctas;              // 0 = all SMs
   // Scattered output (bf16, no accumulate): row r of C is stored at byte address row_ptrs[r] (0 = drop the row)

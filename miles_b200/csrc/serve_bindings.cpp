@@ -8,7 +8,8 @@ using namespace mb_bind;
 
 void gemm(const at::Tensor& a, const at::Tensor& b, at::Tensor& c, bool a_mn, bool b_mn, bool accumulate,
           int64_t block_n, const c10::optional<at::Tensor>& status, const std::vector<int64_t>& dest,
-          const c10::optional<at::Tensor>& sig_ctrl, const std::vector<int64_t>& sig_flags, int64_t sig_me, bool whole_k) {
+          const c10::optional<at::Tensor>& sig_ctrl, const std::vector<int64_t>& sig_flags, int64_t sig_me, bool whole_k,
+          int64_t pair) {
   check_bf16_2d(a, "a");
   check_bf16_2d(b, "b");
   TORCH_CHECK(c.dim() == 2, "c must be 2-D");
@@ -29,6 +30,7 @@ void gemm(const at::Tensor& a, const at::Tensor& b, at::Tensor& c, bool a_mn, bo
   p.status = status_ptr(status);
   p.block_n = static_cast<int>(block_n);
   p.whole_k = whole_k;
+  p.pair = static_cast<int>(pair);
   if (!dest.empty()) {  // replicated output: each destination receives the tile at the offset it has in c
     TORCH_CHECK(dest.size() <= 8, "at most 8 destinations");
     p.n_dest = static_cast<int>(dest.size());
@@ -86,7 +88,7 @@ void register_serving(pybind11::module_& m) {
   m.def("gemm", &gemm, "bf16 tcgen05 GEMM: c (+)= a . b^T with selectable operand majors", py::arg("a"), py::arg("b"),
         py::arg("c"), py::arg("a_mn"), py::arg("b_mn"), py::arg("accumulate"), py::arg("block_n"), py::arg("status"),
         py::arg("dest") = std::vector<int64_t>(), py::arg("sig_ctrl") = py::none(),
-        py::arg("sig_flags") = std::vector<int64_t>(), py::arg("sig_me") = 0, py::arg("whole_k") = false);
+        py::arg("sig_flags") = std::vector<int64_t>(), py::arg("sig_me") = 0, py::arg("whole_k") = false, py::arg("pair") = 0);
   m.def("sample_rows", &sample_rows);
   m.def("small_gemv", &small_gemv);
 }
