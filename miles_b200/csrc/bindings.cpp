@@ -56,6 +56,47 @@ void grouped_gemm_rows(const at::Tensor& a, const at::Tensor& b, at::Tensor& c, 
   TORCH_CHECK(mb::gemm_bf16_launch(p, cur_stream()) == 0, "grouped_gemm_rows: ", mb::gemm_last_error());
 }
 
+// act [rows, I] = silu(gate) * up for gate | up = a . b[g]^T, b [G, 2I, K] (or [2I, K] without tiles: one product over all rows);
+// gu [rows, 2I] or none: gate | up too.
+void gated_gemm(const at::Tensor& a, const at::Tensor& b, at::Tensor& act, const c10::optional<at::Tensor>& gu,
+                const c10::optional<at::Tensor>& tile_group, const c10::optional<at::Tensor>& num_m_tiles, const c10::optional<at::Tensor>& status,
+                int64_t pair) {
+  check_bf16_2d(a, "a");
+  check_bf16_2d(act, "act");
+  TORCH_CHECK(b.is_cuda() && b.scalar_type() == at::kBFloat16 && b.is_contiguous() && b.dim() == (tile_group.has_value() ? 3 : 2),
+              "b must be contiguous bf16, [G, 2I, K] with tiles and [2I, K] without");
+  TORCH_CHECK(tile_group.has_value() == num_m_tiles.has_value(), "tiles and their number go together");
+  const c10::cuda::CUDAGuard guard(a.device());
+  mb::GemmProblem p{};
+  p.mode = tile_group.has_value() ? mb::GEMM_GROUPED_ROWS : mb::GEMM_DENSE;
+  p.num_groups = tile_group.has_value() ? b.size(0) : 1;
+  p.M = a.size(0);
+  p.K = a.size(1);
+  p.N = b.size(-2);
+  TORCH_CHECK(b.size(-1) == p.K && act.size(0) == p.M && act.size(1) * 2 == p.N, "shapes differ");
+  p.a = operand(a, false);
+  p.b = operand(b.view({-1, p.K}), false);
+  fill_out(p, act);
+  p.ldc = act.stride(0);
+  p.glu = true;
+  if (gu.has_value()) {
+    check_bf16_2d(*gu, "gu");
+    TORCH_CHECK(gu->size(0) == p.M && gu->size(1) == p.N, "gu must be [rows, 2I]");
+    p.gu = gu->data_ptr();
+    p.gu_ld = gu->stride(0);
+  }
+  if (tile_group.has_value()) {
+    TORCH_CHECK(tile_group->scalar_type() == at::kInt && num_m_tiles->scalar_type() == at::kInt && tile_group->dim() == 2 &&
+                    tile_group->size(1) == 4 && num_m_tiles->numel() >= 1, "tile maps must be int32 [tiles, 4] and [2]");
+    p.max_tiles = tile_group->size(0);
+    p.tile_group = tile_group->data_ptr<int>();
+    p.num_m_tiles = num_m_tiles->data_ptr<int>();
+  }
+  p.status = status_ptr(status);
+  p.pair = static_cast<int>(pair);
+  TORCH_CHECK(mb::gemm_bf16_launch(p, cur_stream()) == 0, "gated_gemm: ", mb::gemm_last_error());
+}
+
 // c[g] (+)= a[rows of g]^T . b[rows of g];  a: [R, M], b: [R, N], c: [G, M, N].
 void grouped_gemm_contr(const at::Tensor& a, const at::Tensor& b, at::Tensor& c, const at::Tensor& group_offsets,
                         bool accumulate, int64_t block_n, const c10::optional<at::Tensor>& status) {
@@ -97,6 +138,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("b"), py::arg("c"), py::arg("tile_group"), py::arg("num_m_tiles"), py::arg("b_mn"), py::arg("accumulate"),
         py::arg("block_n"), py::arg("status"), py::arg("row_ptrs") = py::none(), py::arg("sig_ctrl") = py::none(),
         py::arg("sig_flags") = std::vector<int64_t>(), py::arg("sig_me") = 0);
+  m.def("gated_gemm", &gated_gemm, py::arg("a"), py::arg("b"), py::arg("act"), py::arg("gu"), py::arg("tile_group"), py::arg("num_m_tiles"),
+        py::arg("status"), py::arg("pair") = 0);
   m.def("grouped_gemm_contr", &grouped_gemm_contr, "MoE weight-gradient GEMM (contraction over each group's rows)");
   register_elementwise(m);
   register_vmm(m);

@@ -55,6 +55,8 @@ struct KArgs {
   int sig_nranks, sig_me;
   void* dest[8];
   int n_dest;
+  void* gu;
+  long long gu_ld;
 };
 
 struct Tile {
@@ -66,10 +68,10 @@ struct Tile {
   long long c_base;
 };
 
-// CG: CTAs that share a tile (BLOCK_M rows each).
-template <int BLOCK_N, bool B_MN, int CG>
+// CG: CTAs that share a tile (BLOCK_M rows each). GLU: a tile is BLOCK_N / 2 gate columns and the up columns that go with them.
+template <int BLOCK_N, bool B_MN, int CG, bool GLU>
 __device__ __forceinline__ int num_tiles_of(const KArgs& p) {
-  const int n_tiles = (p.N + BLOCK_N - 1) / BLOCK_N;
+  const int n_tiles = (p.N + BLOCK_N - 1) / BLOCK_N;  // (of N / 2 by BLOCK_N / 2 as many)
   constexpr int TILE_M = BLOCK_M * CG;
   if (p.mode == GEMM_DENSE) return ((p.M + TILE_M - 1) / TILE_M) * n_tiles;
   if (p.mode == GEMM_GROUPED_ROWS) {
@@ -82,10 +84,11 @@ __device__ __forceinline__ int num_tiles_of(const KArgs& p) {
 }
 
 // `rank`: of the CTA among those that share the tile; rows are its own, columns the whole tile's.
-template <int BLOCK_N, bool B_MN, int CG>
+template <int BLOCK_N, bool B_MN, int CG, bool GLU>
 __device__ __forceinline__ Tile decode_tile(const KArgs& p, int t, int rank) {
   Tile r;
   constexpr int TILE_M = BLOCK_M * CG;
+  constexpr int TILE_N = GLU ? BLOCK_N / 2 : BLOCK_N;  // columns of the output
   const int n_tiles = (p.N + BLOCK_N - 1) / BLOCK_N;
   const int m_tiles = (p.M + TILE_M - 1) / TILE_M;
   if (p.mode == GEMM_DENSE) {
@@ -99,7 +102,7 @@ __device__ __forceinline__ Tile decode_tile(const KArgs& p, int t, int rank) {
     const int mt = first_m + in_band % band_rows;
     const int nt = in_band / band_rows;
     r.a_mn0 = mt * TILE_M + rank * BLOCK_M;
-    r.b_mn0 = nt * BLOCK_N;
+    r.b_mn0 = nt * TILE_N;
     r.a_k0 = 0;
     r.b_k0 = 0;
     r.k_iters = (p.K + BLOCK_K - 1) / BLOCK_K;
@@ -120,12 +123,12 @@ __device__ __forceinline__ Tile decode_tile(const KArgs& p, int t, int rank) {
       r.b_mn0 = nt * BLOCK_N;
       r.b_k0 = g * p.K;
     } else {
-      r.b_mn0 = g * p.N + nt * BLOCK_N;
+      r.b_mn0 = g * p.N + nt * TILE_N;
       r.b_k0 = 0;
     }
     r.k_iters = (p.K + BLOCK_K - 1) / BLOCK_K;
     r.c_row0 = r.a_mn0;
-    r.c_col0 = nt * BLOCK_N;
+    r.c_col0 = nt * TILE_N;
     r.c_base = 0;
   } else {
     const int per_group = m_tiles * n_tiles;
@@ -273,6 +276,21 @@ __device__ __forceinline__ void load_old(const KArgs& p, const Tile& t, int row0
     if (it * (32 / C::LANES) < rows) old[it] = *reinterpret_cast<const uint4*>(at);
 }
 
+// Sixty-four bf16 columns of a warp's 32 rows, staged by its lanes, to global memory.
+__device__ __forceinline__ void store_rows64(void* c, long long ld, int row0, int row_end, int col, int col_end, int lane, uint32_t stg) {
+  __syncwarp();
+  const int rows = row_end - row0 - lane / 8;
+  uint8_t* at = static_cast<uint8_t*>(c) + ((row0 + lane / 8) * ld + col) * 2 + (lane & 7) * 16;
+  const bool in = col + (lane & 7) * 8 + 8 <= col_end;
+#pragma unroll
+  for (int it = 0; it < 8; ++it, at += 8 * ld) {
+    const int r = it * 4 + lane / 8;
+    const uint4 v = lds16(stg + r * 128 + (((lane & 7) ^ (r & 7)) << 4));
+    if (in && it * 4 < rows) *reinterpret_cast<uint4*>(at) = v;
+  }
+  __syncwarp();
+}
+
 template <int BLOCK_N, bool FP32, bool ACC>
 struct StagedEpilogue {
   using C = Chunk<FP32, ACC>;
@@ -384,7 +402,12 @@ struct StagedEpilogue {
 // Measured over seconds, at the power cap, TFLOP/s one CTA -> pair: 8192^3 1181 -> 1283 (cuBLAS 1372), 16384 x 5120 x 2048 1170 ->
 // 1233, 9216 x 24576 x 4096 1202 -> 1288, its weight gradient 1116 -> 1209, 2048 x 151936 x 2048 to fp32 1044 -> 1159. Grouped
 // contractions gain nothing (131072 rows over 128 experts 872 and 893, 65536 rows 668 and 656) and stay with one CTA.
-template <int BLOCK_N, bool A_MN, bool B_MN, int STAGES, int CG>
+//
+// GLU: the accumulator of a tile holds 128 gate columns and their 128 up columns, and silu(gate) * up leaves instead of them (or
+// beside them, for a backward): rounded to bf16 before the activation, as the separate kernel reads them, so the same bits. What it
+// saves is the activation's launch and its pass over gate and up. 131072 rows over 128 experts
+// of 768 x 2048: 931 -> 741 us (924 with gate and up kept), 65536 rows 492 -> 386 (429), 8000 rows 162 -> 144.
+template <int BLOCK_N, bool A_MN, bool B_MN, int STAGES, int CG, bool GLU>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                  const KArgs p) {
@@ -446,7 +469,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   if constexpr (CG == 2) cluster_sync_all();  // both CTAs' barriers and TMEM are there before either uses the other's
   pdl_enter();
 
-  const int total_tiles = num_tiles_of<BLOCK_N, B_MN, CG>(p);
+  const int total_tiles = num_tiles_of<BLOCK_N, B_MN, CG, GLU>(p);
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -459,8 +482,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         else tma_load_2d(dst, map, bar, c0, c1);
       };
       for (int t = first_tile; ok && t < total_tiles; t += tile_step) {
-        const Tile tl = decode_tile<BLOCK_N, B_MN, CG>(p, t, rank);
-        const int b_mn0 = tl.b_mn0 + rank * B_ROWS;
+        const Tile tl = decode_tile<BLOCK_N, B_MN, CG, GLU>(p, t, rank);
+        const int b_mn0 = tl.b_mn0 + rank * (GLU ? p.N / 2 : B_ROWS);  // (GLU, a pair: gate rows in the first CTA, up rows in the other)
         for (int kb = 0; kb < tl.k_iters; ++kb) {
           if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, p.status, ERR_WAIT_EMPTY)) {
             ok = false;
@@ -483,6 +506,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             for (int i = 0; i < B_ROWS / 64; ++i) load(b_dst + i * (BLOCK_K * 128), &tma_b, full, b_mn0 + 64 * i, kbb);
           } else {
             load(b_dst, &tma_b, full, kbb, b_mn0);
+            if (GLU && CG == 1) load(b_dst + BLOCK_N / 2 * (BLOCK_K * 2), &tma_b, full, kbb, b_mn0 + p.N / 2);
           }
           if (++stage == STAGES) {
             stage = 0;
@@ -518,7 +542,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     int iter = 0;  // counts only tiles that use an accumulator, so both roles stay in phase
     bool ok = true;
     for (int t = first_tile; ok && rank == 0 && t < total_tiles; t += tile_step) {
-      const Tile tl = decode_tile<BLOCK_N, B_MN, CG>(p, t, rank);
+      const Tile tl = decode_tile<BLOCK_N, B_MN, CG, GLU>(p, t, rank);
       if (tl.k_iters == 0) continue;  // epilogue writes zeros without touching TMEM
       const int acc = iter & 1;
       const uint32_t acc_phase = (iter >> 1) & 1u;
@@ -577,11 +601,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       const uint32_t stg = stage_buf + static_cast<uint32_t>(warp - 2) * 4096;
       int ready = -1;  // the tile whose first old values are on their way
       for (int t = first_tile; t < total_tiles; t += tile_step) {
-        const Tile tl = decode_tile<BLOCK_N, B_MN, CG>(p, t, rank);
+        const Tile tl = decode_tile<BLOCK_N, B_MN, CG, GLU>(p, t, rank);
         if (tl.k_iters == 0) continue;
         const int row0 = tl.c_row0 + quad * 32, acc = iter & 1, tn = t + tile_step;
         if (ready != t) e.begin(p, tl, row0, lane, half);
-        const Tile next = decode_tile<BLOCK_N, B_MN, CG>(p, tn < total_tiles ? tn : t, rank);
+        const Tile next = decode_tile<BLOCK_N, B_MN, CG, GLU>(p, tn < total_tiles ? tn : t, rank);
         const bool more = tn < total_tiles && next.k_iters > 0;
         if (!__all_sync(0xffffffffu, mbar_wait(tfull_bar(acc), (iter >> 1) & 1u, abort_flag, p.status, ERR_WAIT_TMEM_FULL))) break;
         tc_fence_after();
@@ -591,13 +615,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         ++iter;
       }
     };
-    const bool adds = staged && p.accumulate;
-    if constexpr (BLOCK_N >= 64) {
+    const bool adds = !GLU && staged && p.accumulate;
+    if constexpr (BLOCK_N >= 64 && !GLU) {
       if (adds && p.out_fp32) add_tiles(StagedEpilogue<BLOCK_N, true, true>());
       else if (adds) add_tiles(StagedEpilogue<BLOCK_N, false, true>());
     }
     for (int t = first_tile; ok && !adds && t < total_tiles; t += tile_step) {
-      const Tile tl = decode_tile<BLOCK_N, B_MN, CG>(p, t, rank);
+      const Tile tl = decode_tile<BLOCK_N, B_MN, CG, GLU>(p, t, rank);
       const int row = tl.c_row0 + quad * 32 + lane;
       uint32_t acc_regs[32];
       if (tl.k_iters == 0) {
@@ -616,7 +640,48 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         break;
       }
       tc_fence_after();
-      if (BLOCK_N == 128 && (p.n_dest > 0 || p.row_ptrs) && half == 1) {
+      if constexpr (GLU) {
+        const uint32_t stg = stage_buf + static_cast<uint32_t>(warp - 2) * 4096;
+        const int row0 = tl.c_row0 + quad * 32, col = tl.c_col0 + half * 64, width = p.N / 2;
+        if (row0 >= tl.row_end) {  // (warp-uniform; the tiles of a few rows that decode steps have leave three of four quadrants empty)
+          release(acc);
+          ++iter;
+          continue;
+        }
+        // Sixteen columns at a time in a rolled loop: unrolled, the activation is thousands of instructions, which a launch of a few
+        // tiles per CTA fetches cold (4000 rows of 8 choices over 128 experts 242 -> 232 us).
+        const uint32_t mine = stg + lane * 128, x = lane & 7;
+        const auto pass = [&](void* c, long long ld, bool gate, bool up) {  // gate columns, up columns, or silu(gate) * up of both
+#pragma unroll 1
+          for (int i = 0; i < 4; ++i) {
+            uint32_t g[16], u[16];
+            if (gate) tmem_ld_32x16(t_addr + half * 64 + i * 16, g);
+            if (up) tmem_ld_32x16(t_addr + BLOCK_N / 2 + half * 64 + i * 16, u);
+            tmem_ld_wait();
+            uint32_t w[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const uint32_t gw = gate ? pack_bf16(__uint_as_float(g[2 * j]), __uint_as_float(g[2 * j + 1])) : 0u;
+              const uint32_t uw = up ? pack_bf16(__uint_as_float(u[2 * j]), __uint_as_float(u[2 * j + 1])) : 0u;
+              if (gate && up) {
+                const float2 gf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&gw));
+                const float2 uf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&uw));
+                w[j] = pack_bf16(gf.x / (1.f + __expf(-gf.x)) * uf.x, gf.y / (1.f + __expf(-gf.y)) * uf.y);
+              } else {
+                w[j] = gate ? gw : uw;
+              }
+            }
+            sts16(mine + (((2 * i) ^ x) << 4), w[0], w[1], w[2], w[3]);
+            sts16(mine + (((2 * i + 1) ^ x) << 4), w[4], w[5], w[6], w[7]);
+          }
+          store_rows64(c, ld, row0, tl.row_end, col, width, lane, stg);
+        };
+        if (p.gu) {
+          pass(p.gu, p.gu_ld, true, false);
+          pass(static_cast<__nv_bfloat16*>(p.gu) + width, p.gu_ld, false, true);
+        }
+        pass(p.c, p.ldc, true, true);
+      } else if (BLOCK_N == 128 && (p.n_dest > 0 || p.row_ptrs) && half == 1) {
         // (one warp per quadrant stages whole rows below)
       } else if (BLOCK_N == 128 && p.n_dest > 0) {
         // Replicated tile (tensor-parallel partial sums): same staging, every row segment goes to each destination.
@@ -786,7 +851,7 @@ int gemm_make_map(CUtensorMap* map, const GemmOperand& op, int box_rows) {
 
 namespace {
 
-template <int BLOCK_N, bool A_MN, bool B_MN, int CG = 1>
+template <int BLOCK_N, bool A_MN, bool B_MN, int CG = 1, bool GLU = false>
 int launch(const GemmProblem& p, const KArgs& ka, cudaStream_t stream) {
   // (the 32 KB staging buffer takes a pipeline stage from the 128-wide variant)
   constexpr int STAGES = CG == 2 ? 6 : (BLOCK_N == 256 ? 4 : (BLOCK_N == 128 ? 5 : 8));
@@ -795,8 +860,8 @@ int launch(const GemmProblem& p, const KArgs& ka, cudaStream_t stream) {
                        8 * 4096 + 128;
   CUtensorMap ma, mb_;
   if (gemm_make_map(&ma, p.a, A_MN ? BLOCK_K : BLOCK_M)) return -1;
-  if (gemm_make_map(&mb_, p.b, B_MN ? BLOCK_K : BLOCK_N / CG)) return -1;
-  auto kern = gemm_bf16_kernel<BLOCK_N, A_MN, B_MN, STAGES, CG>;
+  if (gemm_make_map(&mb_, p.b, B_MN ? BLOCK_K : GLU ? BLOCK_N / 2 : BLOCK_N / CG)) return -1;
+  auto kern = gemm_bf16_kernel<BLOCK_N, A_MN, B_MN, STAGES, CG, GLU>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)  // per (function, device)
     return fail("cudaFuncSetAttribute(MaxDynamicSharedMemorySize) failed");
   int dev = 0, sms = 0;
@@ -873,7 +938,16 @@ int gemm_bf16_launch(const GemmProblem& p, cudaStream_t stream) {
   const int vec = 16 / esz;
   ka.vec_ok = ((reinterpret_cast<uintptr_t>(p.c) & 15) == 0 && p.ldc % vec == 0 && p.c_group_stride % vec == 0) ? 1 : 0;
 
-  int bn = p.block_n;
+  if (p.glu) {
+    const auto rows16 = [](const void* c, long long ld) { return (reinterpret_cast<uintptr_t>(c) & 15) == 0 && ld % 8 == 0; };
+    if (p.mode == GEMM_GROUPED_CONTR || p.a.mn_major || p.b.mn_major || p.out_fp32 || p.accumulate || p.row_ptrs || p.n_dest > 0 || p.N % 16 != 0 ||
+        !rows16(p.c, p.ldc) || (p.gu && !rows16(p.gu, p.gu_ld)))
+      return fail("a gated product needs K-major operands, N % 16 == 0 and aligned bf16 outputs that are not added to");
+    ka.gu = p.gu;
+    ka.gu_ld = p.gu_ld;
+  }
+
+  int bn = p.glu ? 256 : p.block_n;
   const bool amn = p.a.mn_major, bmn = p.b.mn_major;
   if (bn == 0 && gemm_is_skinny(p)) return gemm_skinny_launch(p, nullptr, stream);
   if (bn == 0) {
@@ -915,6 +989,7 @@ int gemm_bf16_launch(const GemmProblem& p, cudaStream_t stream) {
   if ((bn == 32 || bn == 64) && (amn || bmn)) return fail("narrow tiles support K-major operands only");
   if (bn == 32) return launch<32, false, false>(p, ka, stream);
   if (bn == 64) return launch<64, false, false>(p, ka, stream);
+  if (p.glu) return pair ? launch<256, false, false, 2, true>(p, ka, stream) : launch<256, false, false, 1, true>(p, ka, stream);
   if (pair) {
     if (!amn && !bmn) return launch<256, false, false, 2>(p, ka, stream);
     if (!amn && bmn) return launch<256, false, true, 2>(p, ka, stream);

@@ -42,6 +42,9 @@ struct GemmProblem {
   int block_n;               // 0 = choose, else 128 or 256
   int pair;                  // tiles of two CTAs: 0 = choose, 1 = never, 2 = wherever they can be (dense, block_n 256)
   bool whole_k;              // block_n 0: every sum runs over K in one order, however few the rows
+  bool glu;                  // modes 0 and 1, K-major bf16: the rows of B are gate rows and, N / 2 further, up rows; C [M, N / 2] = silu(gate) * up
+  void* gu;                  // with glu, or null: gate | up themselves, [M, N] with row pitch gu_ld
+  long long gu_ld;
   int max_ctas;              // 0 = all SMs
   // Scattered output (bf16, no accumulate): row r of C is stored at byte address row_ptrs[r] (0 = drop the row)
   // instead of c + r*ldc. The addresses may lie in other GPUs' memory mapped into this process: the epilogue then

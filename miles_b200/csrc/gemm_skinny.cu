@@ -46,27 +46,10 @@ struct SkinnyArgs {
   int* status;
 };
 
-__device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-}
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
 __device__ __forceinline__ uint32_t cluster_size() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
   return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ float4 ld_cluster_f4(uint32_t local_addr, uint32_t rank) {
   uint32_t a;
@@ -93,7 +76,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   auto empty_bar = [&](int s) { return bar0 + 8u * (MAX_SK_STAGES + s); };
   const uint32_t done_bar = bar0 + 8u * (2 * MAX_SK_STAGES);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t rank = cluster_rank(), ranks = cluster_size();
+  const uint32_t rank = cluster_ctarank(), ranks = cluster_size();
   const int n0 = blockIdx.y * BM;
   const int kb0 = min(p.k_blocks, static_cast<int>(rank) * p.per_rank);
   const int k_iters = min(p.k_blocks, kb0 + p.per_rank) - kb0;

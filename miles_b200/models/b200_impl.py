@@ -210,6 +210,21 @@ class B200Qwen3:
         self.launches += 1
         return out
 
+    def _gated(self, x, w, keep: bool = False, serving: bool = False):
+        """``(gate | up if kept, silu(gate) * up)`` for a gate-up weight [2I, K]: one launch where tiles of 128 such columns fill
+        the device (csrc/gemm.cu), else the product and the activation. The same bits either way."""
+        T, I = x.shape[0], w.shape[0] // 2
+        mx = getattr(self, "mx", None)
+        if T > 128 and I % 8 == 0 and -(-T // 128) * -(-I // 128) >= 148 and x.is_contiguous() and not (mx and w.data_ptr() in mx):
+            gu = torch.empty(T, 2 * I, dtype=torch.bfloat16, device=x.device) if keep else None
+            act = torch.empty(T, I, dtype=torch.bfloat16, device=x.device)
+            self.C.gated_gemm(x, w, act, gu, None, None, self.status)
+            self.launches += 1
+            return gu, act
+        gu = self.linear(x, w, serving=serving)
+        self.launches += 1
+        return gu if keep else None, self.C.swiglu_fwd(gu)
+
     def linear_dgrad(self, dy, w):
         dx = torch.empty(dy.shape[0], w.shape[1], dtype=torch.bfloat16, device=dy.device)
         return self._gemm(dy, w, dx, False, True)
@@ -266,16 +281,24 @@ class B200Qwen3:
             yp = self._mx_linear(act, mx[w2.data_ptr()], plan.tile_group, plan.num_tiles, w2.shape[1])
             self.launches += 1
             return None, None, yp
-        gu = torch.empty(plan.max_rows, I2, dtype=torch.bfloat16, device=xp.device)
-        C.grouped_gemm_rows(xp, w1, gu, plan.tile_group, plan.num_tiles, False, False, 0, self.status)
-        act = C.swiglu_fwd(gu)
+        gated = plan.max_rows >= 48 * w1.shape[0]
+        gu = torch.empty(plan.max_rows, I2, dtype=torch.bfloat16, device=xp.device) if keep or not gated else None
+        if gated:
+            act = torch.empty(plan.max_rows, I2 // 2, dtype=torch.bfloat16, device=xp.device)
+            C.gated_gemm(xp, w1, act, gu, plan.tile_group, plan.num_tiles, self.status)
+        else:
+            # experts of few rows stream their weights, and the plain product does so faster, by more than the activation costs
+            # (us, 128 experts of 768 x 2048: 16 tokens 87.5 and 95.4 gated, 200 tokens 137 and 142, 1000 150 and 148, 4000 264 and 232)
+            C.grouped_gemm_rows(xp, w1, gu, plan.tile_group, plan.num_tiles, False, False, 0, self.status)
+            act = C.swiglu_fwd(gu)
+            self.launches += 1
         yp = torch.empty(plan.max_rows if scatter is None else 1, w2.shape[1], dtype=torch.bfloat16, device=xp.device)
         if scatter is None:
             C.grouped_gemm_rows(act, w2, yp, plan.tile_group, plan.num_tiles, False, False, 0, self.status)
         else:
             C.grouped_gemm_rows(act, w2, yp.expand(plan.max_rows, -1), plan.tile_group, plan.num_tiles, False, False, 0,
                                 self.status, scatter[0], scatter[1], scatter[2], scatter[3])
-        self.launches += 3
+        self.launches += 2
         return (gu, act, yp) if keep else (None, None, yp)
 
     def moe_forward(self, i, h2, replay_ids=None, record=None, keep=False, residual=None, serving=False):
@@ -479,14 +502,13 @@ class B200Qwen3:
                 return self.ep.moe_decode(self, i, x2, h2, record)
             y, _ = self.moe_forward(i, h2, replay_ids, record, keep=False, residual=x2, serving=serving)
             return y
-        gu = self.linear(h2, P[p + "mlp.gate_up.weight"], serving=serving)
-        self.launches += 1
+        _, act = self._gated(h2, P[p + "mlp.gate_up.weight"], serving=serving)
         if cfg.post_norms:
-            y = self.linear(C.swiglu_fwd(gu), P[p + "mlp.down.weight"], serving=serving)
+            y = self.linear(act, P[p + "mlp.down.weight"], serving=serving)
             yn, _ = C.rmsnorm_fwd(y, None, P[p + "post_mlp_ln.weight"], cfg.rms_eps)
             self.launches += 2
             return yn.add_(x2)
-        return self._row_parallel(C.swiglu_fwd(gu), P[p + "mlp.down.weight"], x2, serving)
+        return self._row_parallel(act, P[p + "mlp.down.weight"], x2, serving)
 
     def _full_kv(self, prefix, k, v, kc, vc):
         """``PrefixInfo.full_kv`` in one launch for caches of the activations' type."""
@@ -648,9 +670,7 @@ class B200Qwen3:
         if is_moe:
             y, saved = self.moe_forward(i, h2, replay_ids, None, keep=True, residual=x2 if output else None)
             return LayerActs(qkv, att, lse, ln2, post_attn, saved, None), y
-        gu = self.linear(h2, P[p + "mlp.gate_up.weight"])
-        act = C.swiglu_fwd(gu)
-        self.launches += 1
+        gu, act = self._gated(h2, P[p + "mlp.gate_up.weight"], keep=True)
         y = None
         if output and cfg.post_norms:
             y, _ = C.rmsnorm_fwd(self.linear(act, P[p + "mlp.down.weight"]), None, P[p + "post_mlp_ln.weight"], cfg.rms_eps)
