@@ -56,6 +56,44 @@ void grouped_gemm_rows(const at::Tensor& a, const at::Tensor& b, at::Tensor& c, 
   TORCH_CHECK(mb::gemm_bf16_launch(p, cur_stream()) == 0, "grouped_gemm_rows: ", mb::gemm_last_error());
 }
 
+// (log-probabilities of the targets, entropies, log-sum-exps, means) of softmax(h . w^T * inv_temp), all fp32 [T]; logits [T, V] fp32 or none.
+std::vector<at::Tensor> score_rows(const at::Tensor& h, const at::Tensor& w, const at::Tensor& targets, double inv_temp,
+                                   const c10::optional<at::Tensor>& logits, const c10::optional<at::Tensor>& status, int64_t pair) {
+  check_bf16_2d(h, "h");
+  check_bf16_2d(w, "w");
+  CHECK_I32(targets);
+  const int64_t T = h.size(0), V = w.size(0);
+  TORCH_CHECK(h.size(1) == w.size(1) && targets.numel() == T, "shapes differ");
+  const c10::cuda::CUDAGuard guard(h.device());
+  auto o = h.options().dtype(at::kFloat);
+  at::Tensor lp = at::empty({T}, o), ent = at::empty({T}, o), lse = at::empty({T}, o), px = at::empty({T}, o), tgt = at::empty({T}, o);
+  if (T == 0) return {lp, ent, lse, px};
+  at::Tensor part = at::empty({(V + 127) / 128, T, 4}, o);
+  mb::GemmProblem p{};
+  p.mode = mb::GEMM_DENSE;
+  p.M = T;
+  p.N = V;
+  p.K = h.size(1);
+  p.a = operand(h, false);
+  p.b = operand(w, false);
+  p.out_fp32 = true;
+  if (logits.has_value()) {
+    TORCH_CHECK(logits->scalar_type() == at::kFloat && logits->dim() == 2 && logits->size(0) == T && logits->size(1) == V, "logits must be fp32 [T, V]");
+    fill_out(p, *logits);
+    p.ldc = logits->stride(0);
+  }
+  p.score_part = part.data_ptr<float>();
+  p.targets = targets.data_ptr<int>();
+  p.score_target = tgt.data_ptr<float>();
+  p.inv_temp = inv_temp;
+  p.status = status_ptr(status);
+  p.pair = static_cast<int>(pair);
+  TORCH_CHECK(mb::gemm_bf16_launch(p, cur_stream()) == 0, "score_rows: ", mb::gemm_last_error());
+  mb::logprob_entropy_merge(part.data_ptr<float>(), tgt.data_ptr<float>(), targets.data_ptr<int>(), lp.data_ptr<float>(), ent.data_ptr<float>(),
+                            lse.data_ptr<float>(), px.data_ptr<float>(), T, V, cur_stream());
+  return {lp, ent, lse, px};
+}
+
 // act [rows, I] = silu(gate) * up for gate | up = a . b[g]^T, b [G, 2I, K] (or [2I, K] without tiles: one product over all rows);
 // gu [rows, 2I] or none: gate | up too.
 void gated_gemm(const at::Tensor& a, const at::Tensor& b, at::Tensor& act, const c10::optional<at::Tensor>& gu,
@@ -138,6 +176,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("b"), py::arg("c"), py::arg("tile_group"), py::arg("num_m_tiles"), py::arg("b_mn"), py::arg("accumulate"),
         py::arg("block_n"), py::arg("status"), py::arg("row_ptrs") = py::none(), py::arg("sig_ctrl") = py::none(),
         py::arg("sig_flags") = std::vector<int64_t>(), py::arg("sig_me") = 0);
+  m.def("score_rows", &score_rows, py::arg("h"), py::arg("w"), py::arg("targets"), py::arg("inv_temp"), py::arg("logits"), py::arg("status"),
+        py::arg("pair") = 0);
   m.def("gated_gemm", &gated_gemm, py::arg("a"), py::arg("b"), py::arg("act"), py::arg("gu"), py::arg("tile_group"), py::arg("num_m_tiles"),
         py::arg("status"), py::arg("pair") = 0);
   m.def("grouped_gemm_contr", &grouped_gemm_contr, "MoE weight-gradient GEMM (contraction over each group's rows)");

@@ -57,7 +57,13 @@ struct KArgs {
   int n_dest;
   void* gu;
   long long gu_ld;
+  float4* score_part;
+  const int* targets;
+  float* score_target;
+  float inv_temp;
 };
+
+enum Epilogue : int { EPI_PLAIN = 0, EPI_GLU = 1, EPI_SCORES = 2 };
 
 struct Tile {
   int a_mn0, b_mn0;  // M/N coordinates in the operand tensors
@@ -68,8 +74,8 @@ struct Tile {
   long long c_base;
 };
 
-// CG: CTAs that share a tile (BLOCK_M rows each). GLU: a tile is BLOCK_N / 2 gate columns and the up columns that go with them.
-template <int BLOCK_N, bool B_MN, int CG, bool GLU>
+// CG: CTAs that share a tile (BLOCK_M rows each). EPI_GLU: a tile is BLOCK_N / 2 gate columns and the up columns that go with them.
+template <int BLOCK_N, bool B_MN, int CG, int EPI>
 __device__ __forceinline__ int num_tiles_of(const KArgs& p) {
   const int n_tiles = (p.N + BLOCK_N - 1) / BLOCK_N;  // (of N / 2 by BLOCK_N / 2 as many)
   constexpr int TILE_M = BLOCK_M * CG;
@@ -84,11 +90,11 @@ __device__ __forceinline__ int num_tiles_of(const KArgs& p) {
 }
 
 // `rank`: of the CTA among those that share the tile; rows are its own, columns the whole tile's.
-template <int BLOCK_N, bool B_MN, int CG, bool GLU>
+template <int BLOCK_N, bool B_MN, int CG, int EPI>
 __device__ __forceinline__ Tile decode_tile(const KArgs& p, int t, int rank) {
   Tile r;
   constexpr int TILE_M = BLOCK_M * CG;
-  constexpr int TILE_N = GLU ? BLOCK_N / 2 : BLOCK_N;  // columns of the output
+  constexpr int TILE_N = EPI == EPI_GLU ? BLOCK_N / 2 : BLOCK_N;  // columns of the output
   const int n_tiles = (p.N + BLOCK_N - 1) / BLOCK_N;
   const int m_tiles = (p.M + TILE_M - 1) / TILE_M;
   if (p.mode == GEMM_DENSE) {
@@ -403,14 +409,20 @@ struct StagedEpilogue {
 // 1233, 9216 x 24576 x 4096 1202 -> 1288, its weight gradient 1116 -> 1209, 2048 x 151936 x 2048 to fp32 1044 -> 1159. Grouped
 // contractions gain nothing (131072 rows over 128 experts 872 and 893, 65536 rows 668 and 656) and stay with one CTA.
 //
-// GLU: the accumulator of a tile holds 128 gate columns and their 128 up columns, and silu(gate) * up leaves instead of them (or
+// EPI_GLU: the accumulator of a tile holds 128 gate columns and their 128 up columns, and silu(gate) * up leaves instead of them (or
 // beside them, for a backward): rounded to bf16 before the activation, as the separate kernel reads them, so the same bits. What it
 // saves is the activation's launch and its pass over gate and up. 131072 rows over 128 experts
 // of 768 x 2048: 931 -> 741 us (924 with gate and up kept), 65536 rows 492 -> 386 (429), 8000 rows 162 -> 144.
-template <int BLOCK_N, bool A_MN, bool B_MN, int STAGES, int CG, bool GLU>
+//
+// EPI_SCORES: the log-probabilities of an LM head need three numbers per row of its 150 thousand logits. Every thread of the
+// epilogue keeps maximum, sum of exponentials and their first moment about the maximum over 128 columns of its row, and
+// logprob.cu merges them: the logits need not be written, or not be read again. Scores of 12288
+// rows over 151936 x 2048 (in chunks of 2048 with their logits in fp32 through memory before): a pass of 16384 tokens 30.3 -> 28.8 ms.
+template <int BLOCK_N, bool A_MN, bool B_MN, int STAGES, int CG, int EPI>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                  const KArgs p) {
+  constexpr bool GLU = EPI == EPI_GLU, SCORES = EPI == EPI_SCORES;
   constexpr int B_ROWS = BLOCK_N / CG;  // of this CTA
   constexpr int B_STAGE_BYTES = B_ROWS * BLOCK_K * 2;
   constexpr uint32_t TMEM_COLS = 2 * BLOCK_N;  // 256 or 512: a power of two >= 32
@@ -469,7 +481,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   if constexpr (CG == 2) cluster_sync_all();  // both CTAs' barriers and TMEM are there before either uses the other's
   pdl_enter();
 
-  const int total_tiles = num_tiles_of<BLOCK_N, B_MN, CG, GLU>(p);
+  const int total_tiles = num_tiles_of<BLOCK_N, B_MN, CG, EPI>(p);
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -482,7 +494,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         else tma_load_2d(dst, map, bar, c0, c1);
       };
       for (int t = first_tile; ok && t < total_tiles; t += tile_step) {
-        const Tile tl = decode_tile<BLOCK_N, B_MN, CG, GLU>(p, t, rank);
+        const Tile tl = decode_tile<BLOCK_N, B_MN, CG, EPI>(p, t, rank);
         const int b_mn0 = tl.b_mn0 + rank * (GLU ? p.N / 2 : B_ROWS);  // (GLU, a pair: gate rows in the first CTA, up rows in the other)
         for (int kb = 0; kb < tl.k_iters; ++kb) {
           if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, p.status, ERR_WAIT_EMPTY)) {
@@ -542,7 +554,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     int iter = 0;  // counts only tiles that use an accumulator, so both roles stay in phase
     bool ok = true;
     for (int t = first_tile; ok && rank == 0 && t < total_tiles; t += tile_step) {
-      const Tile tl = decode_tile<BLOCK_N, B_MN, CG, GLU>(p, t, rank);
+      const Tile tl = decode_tile<BLOCK_N, B_MN, CG, EPI>(p, t, rank);
       if (tl.k_iters == 0) continue;  // epilogue writes zeros without touching TMEM
       const int acc = iter & 1;
       const uint32_t acc_phase = (iter >> 1) & 1u;
@@ -601,11 +613,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       const uint32_t stg = stage_buf + static_cast<uint32_t>(warp - 2) * 4096;
       int ready = -1;  // the tile whose first old values are on their way
       for (int t = first_tile; t < total_tiles; t += tile_step) {
-        const Tile tl = decode_tile<BLOCK_N, B_MN, CG, GLU>(p, t, rank);
+        const Tile tl = decode_tile<BLOCK_N, B_MN, CG, EPI>(p, t, rank);
         if (tl.k_iters == 0) continue;
         const int row0 = tl.c_row0 + quad * 32, acc = iter & 1, tn = t + tile_step;
         if (ready != t) e.begin(p, tl, row0, lane, half);
-        const Tile next = decode_tile<BLOCK_N, B_MN, CG, GLU>(p, tn < total_tiles ? tn : t, rank);
+        const Tile next = decode_tile<BLOCK_N, B_MN, CG, EPI>(p, tn < total_tiles ? tn : t, rank);
         const bool more = tn < total_tiles && next.k_iters > 0;
         if (!__all_sync(0xffffffffu, mbar_wait(tfull_bar(acc), (iter >> 1) & 1u, abort_flag, p.status, ERR_WAIT_TMEM_FULL))) break;
         tc_fence_after();
@@ -615,14 +627,16 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         ++iter;
       }
     };
-    const bool adds = !GLU && staged && p.accumulate;
-    if constexpr (BLOCK_N >= 64 && !GLU) {
+    const bool adds = EPI == EPI_PLAIN && staged && p.accumulate;
+    if constexpr (BLOCK_N >= 64 && EPI == EPI_PLAIN) {
       if (adds && p.out_fp32) add_tiles(StagedEpilogue<BLOCK_N, true, true>());
       else if (adds) add_tiles(StagedEpilogue<BLOCK_N, false, true>());
     }
     for (int t = first_tile; ok && !adds && t < total_tiles; t += tile_step) {
-      const Tile tl = decode_tile<BLOCK_N, B_MN, CG, GLU>(p, t, rank);
+      const Tile tl = decode_tile<BLOCK_N, B_MN, CG, EPI>(p, t, rank);
       const int row = tl.c_row0 + quad * 32 + lane;
+      int target = -1;
+      if (SCORES && row < tl.row_end) target = p.targets[row];
       uint32_t acc_regs[32];
       if (tl.k_iters == 0) {
         if (!p.accumulate) {
@@ -640,7 +654,62 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         break;
       }
       tc_fence_after();
-      if constexpr (GLU) {
+      if constexpr (SCORES) {
+        const uint32_t stg = stage_buf + static_cast<uint32_t>(warp - 2) * 4096;
+        const int row0 = tl.c_row0 + quad * 32, col0 = tl.c_col0 + half * (BLOCK_N / 2);
+        float m = -3.402823466e38f, s = 0.f, sy = 0.f;
+#pragma unroll 1
+        for (int c = 0; c < BLOCK_N / 64; ++c) {
+          const int col = col0 + c * 32;
+          if (col >= p.N) break;  // warp-uniform
+          tmem_ld_32x32(t_addr + half * (BLOCK_N / 2) + c * 32, acc_regs);
+          tmem_ld_wait();
+          if (p.c) {
+            if (p.vec_ok && col + 32 <= p.N) {  // rows of 128 bytes, through shared memory
+              const uint32_t mine = stg + lane * 128, x = lane & 7;
+#pragma unroll
+              for (int i = 0; i < 8; ++i) sts16(mine + ((i ^ x) << 4), acc_regs[4 * i], acc_regs[4 * i + 1], acc_regs[4 * i + 2], acc_regs[4 * i + 3]);
+              __syncwarp();
+              const int rows = tl.row_end - row0 - lane / 8;
+              float* at = static_cast<float*>(p.c) + (row0 + lane / 8) * p.ldc + col + (lane & 7) * 4;
+#pragma unroll
+              for (int it = 0; it < 8; ++it, at += 4 * p.ldc) {
+                const int r = it * 4 + lane / 8;
+                const uint4 v = lds16(stg + r * 128 + (((lane & 7) ^ (r & 7)) << 4));
+                if (it * 4 < rows) *reinterpret_cast<uint4*>(at) = v;
+              }
+              __syncwarp();
+            } else {
+              store_chunk(p, tl, row, col, acc_regs, false);
+            }
+          }
+          float v[32], mx = m;
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            v[i] = col + i < p.N ? __uint_as_float(acc_regs[i]) * p.inv_temp : -3.402823466e38f;
+            mx = fmaxf(mx, v[i]);
+          }
+          if (target >= col && target < col + 32) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (target == col + i) p.score_target[row] = v[i];
+          }
+          const float scale = __expf(m - mx);
+          sy = scale * (sy + s * (s > 0.f ? m - mx : 0.f));
+          s *= scale;
+          m = mx;
+          float ps[4] = {0.f, 0.f, 0.f, 0.f}, py[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            const float y = v[i] - m, e = __expf(y);
+            ps[i & 3] += e;
+            if (e > 0.f) py[i & 3] += e * y;  // (a masked column's y is -infinity)
+          }
+          s += (ps[0] + ps[1]) + (ps[2] + ps[3]);
+          sy += (py[0] + py[1]) + (py[2] + py[3]);
+        }
+        if (row < tl.row_end && col0 < p.N) p.score_part[static_cast<long long>(col0 / (BLOCK_N / 2)) * p.M + row] = make_float4(m, s, sy, 0.f);
+      } else if constexpr (GLU) {
         const uint32_t stg = stage_buf + static_cast<uint32_t>(warp - 2) * 4096;
         const int row0 = tl.c_row0 + quad * 32, col = tl.c_col0 + half * 64, width = p.N / 2;
         if (row0 >= tl.row_end) {  // (warp-uniform; the tiles of a few rows that decode steps have leave three of four quadrants empty)
@@ -851,7 +920,7 @@ int gemm_make_map(CUtensorMap* map, const GemmOperand& op, int box_rows) {
 
 namespace {
 
-template <int BLOCK_N, bool A_MN, bool B_MN, int CG = 1, bool GLU = false>
+template <int BLOCK_N, bool A_MN, bool B_MN, int CG = 1, int EPI = EPI_PLAIN>
 int launch(const GemmProblem& p, const KArgs& ka, cudaStream_t stream) {
   // (the 32 KB staging buffer takes a pipeline stage from the 128-wide variant)
   constexpr int STAGES = CG == 2 ? 6 : (BLOCK_N == 256 ? 4 : (BLOCK_N == 128 ? 5 : 8));
@@ -860,8 +929,8 @@ int launch(const GemmProblem& p, const KArgs& ka, cudaStream_t stream) {
                        8 * 4096 + 128;
   CUtensorMap ma, mb_;
   if (gemm_make_map(&ma, p.a, A_MN ? BLOCK_K : BLOCK_M)) return -1;
-  if (gemm_make_map(&mb_, p.b, B_MN ? BLOCK_K : GLU ? BLOCK_N / 2 : BLOCK_N / CG)) return -1;
-  auto kern = gemm_bf16_kernel<BLOCK_N, A_MN, B_MN, STAGES, CG, GLU>;
+  if (gemm_make_map(&mb_, p.b, B_MN ? BLOCK_K : EPI == EPI_GLU ? BLOCK_N / 2 : BLOCK_N / CG)) return -1;
+  auto kern = gemm_bf16_kernel<BLOCK_N, A_MN, B_MN, STAGES, CG, EPI>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)  // per (function, device)
     return fail("cudaFuncSetAttribute(MaxDynamicSharedMemorySize) failed");
   int dev = 0, sms = 0;
@@ -947,7 +1016,17 @@ int gemm_bf16_launch(const GemmProblem& p, cudaStream_t stream) {
     ka.gu_ld = p.gu_ld;
   }
 
-  int bn = p.glu ? 256 : p.block_n;
+  if (p.score_part) {
+    if (p.mode != GEMM_DENSE || p.a.mn_major || p.b.mn_major || (p.c && !p.out_fp32) || p.accumulate || p.row_ptrs || p.n_dest > 0 || p.glu ||
+        !p.targets || !p.score_target)
+      return fail("vocabulary scores need a dense K-major product, targets, and fp32 logits or none");
+    ka.score_part = reinterpret_cast<float4*>(p.score_part);
+    ka.targets = p.targets;
+    ka.score_target = p.score_target;
+    ka.inv_temp = p.inv_temp;
+  }
+
+  int bn = p.glu || p.score_part ? 256 : p.block_n;
   const bool amn = p.a.mn_major, bmn = p.b.mn_major;
   if (bn == 0 && gemm_is_skinny(p)) return gemm_skinny_launch(p, nullptr, stream);
   if (bn == 0) {
@@ -989,7 +1068,8 @@ int gemm_bf16_launch(const GemmProblem& p, cudaStream_t stream) {
   if ((bn == 32 || bn == 64) && (amn || bmn)) return fail("narrow tiles support K-major operands only");
   if (bn == 32) return launch<32, false, false>(p, ka, stream);
   if (bn == 64) return launch<64, false, false>(p, ka, stream);
-  if (p.glu) return pair ? launch<256, false, false, 2, true>(p, ka, stream) : launch<256, false, false, 1, true>(p, ka, stream);
+  if (p.glu) return pair ? launch<256, false, false, 2, EPI_GLU>(p, ka, stream) : launch<256, false, false, 1, EPI_GLU>(p, ka, stream);
+  if (p.score_part) return pair ? launch<256, false, false, 2, EPI_SCORES>(p, ka, stream) : launch<256, false, false, 1, EPI_SCORES>(p, ka, stream);
   if (pair) {
     if (!amn && !bmn) return launch<256, false, false, 2>(p, ka, stream);
     if (!amn && bmn) return launch<256, false, true, 2>(p, ka, stream);

@@ -45,6 +45,13 @@ struct GemmProblem {
   bool glu;                  // modes 0 and 1, K-major bf16: the rows of B are gate rows and, N / 2 further, up rows; C [M, N / 2] = silu(gate) * up
   void* gu;                  // with glu, or null: gate | up themselves, [M, N] with row pitch gu_ld
   long long gu_ld;
+  // Vocabulary scores (mode 0, K-major): instead of, or with c (fp32) beside, the products leave, for every row and 128 columns, the
+  // maximum m of x = product * inv_temp, sum exp(x - m) and sum exp(x - m) (x - m): score_part [ceil(N / 128)][M] of four
+  // floats; score_target[row] receives x at the row's target (untouched for targets outside [0, N)).
+  float* score_part;
+  const int* targets;
+  float* score_target;
+  float inv_temp;
   int max_ctas;              // 0 = all SMs
   // Scattered output (bf16, no accumulate): row r of C is stored at byte address row_ptrs[r] (0 = drop the row)
   // instead of c + r*ldc. The addresses may lie in other GPUs' memory mapped into this process: the epilogue then

@@ -109,6 +109,43 @@ __global__ void logprob_fwd_kernel(const T* __restrict__ logits, const int* __re
   }
 }
 
+// The end of it where the product already left (maximum, sum, moment about the maximum) for every 128 columns (EPI_SCORES of gemm.cu): part
+// [pieces][T], row_target[T] the targets' scaled logits. A lane per row, the pieces dealt to the warps in turn.
+constexpr int MERGE_WARPS = 16;
+__global__ void __launch_bounds__(32 * MERGE_WARPS)
+logprob_merge_kernel(const float4* __restrict__ part, const float* __restrict__ row_target, const int* __restrict__ targets,
+                     float* __restrict__ logprob, float* __restrict__ entropy, float* __restrict__ lse_out, float* __restrict__ psumx_out, int T,
+                     int V, int pieces) {
+  __shared__ Stat red[MERGE_WARPS][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int row = blockIdx.x * 32 + lane;
+  const auto merge = [](const Stat& a, const Stat& b) {
+    const float m = fmaxf(a.m, b.m), ca = __expf(a.m - m), cb = __expf(b.m - m);
+    Stat r{m, a.s * ca + b.s * cb, 0.f};
+    if (ca > 0.f) r.sx = ca * (a.sx + a.s * (a.m - m));
+    if (cb > 0.f) r.sx += cb * (b.sx + b.s * (b.m - m));
+    return r;
+  };
+  Stat st{-FLT_MAX, 0.f, 0.f};
+  if (row < T) {
+#pragma unroll 8
+    for (int i = warp; i < pieces; i += MERGE_WARPS) {
+      const float4 v = part[static_cast<long long>(i) * T + row];
+      st = merge(st, Stat{v.x, v.y, v.z});
+    }
+  }
+  red[warp][lane] = st;
+  __syncthreads();
+  if (warp > 0 || row >= T) return;
+  for (int w = 1; w < MERGE_WARPS; ++w) st = merge(st, red[w][lane]);
+  const float ls = logf(st.s), mean = st.sx / st.s, lse = st.m + ls;
+  lse_out[row] = lse;
+  psumx_out[row] = st.m + mean;
+  entropy[row] = ls - mean;  // (about the maximum: what the two have in common does not have to cancel)
+  const int t = targets[row];
+  logprob[row] = (t >= 0 && t < V) ? row_target[row] - lse : 0.f;
+}
+
 // VEC values per thread and step (16-byte loads of both types, 8- or 16-byte stores) where rows and pointers allow, else one.
 // In place over bf16 logits every value is read and written by the same thread. 2048 rows of 151936 fp32 logits: 622 us with
 // 4-byte loads and 2-byte stores, 277 us now (1.87 GB move).
@@ -183,6 +220,13 @@ void logprob_entropy_fwd(const void* logits, bool fp32, const int* targets, floa
   else
     logprob_fwd_kernel<bf16, 512><<<T, 512, 0, s>>>(static_cast<const bf16*>(logits), targets, logprob, entropy, lse,
                                                     psum_x, V, ld, inv_temp);
+}
+
+void logprob_entropy_merge(const float* part, const float* row_target, const int* targets, float* logprob, float* entropy, float* lse, float* psum_x,
+                           int T, int V, cudaStream_t s) {
+  if (T <= 0) return;
+  logprob_merge_kernel<<<(T + 31) / 32, 32 * MERGE_WARPS, 0, s>>>(reinterpret_cast<const float4*>(part), row_target, targets, logprob, entropy, lse,
+                                                                  psum_x, T, V, (V + 127) / 128);
 }
 
 void logprob_entropy_bwd(const void* logits, bool fp32, const int* targets, const float* lse, const float* psum_x,

@@ -699,7 +699,7 @@ class B200Qwen3:
         free, total = torch.cuda.mem_get_info(self.dev)
         return free + torch.cuda.memory_reserved(self.dev) - torch.cuda.memory_allocated(self.dev) - total // 7
 
-    def _plan_acts(self, T: int, head_rows: int) -> tuple[bool, int]:
+    def _plan_acts(self, T: int, head_rows: int, chunk: int = 0) -> tuple[bool, int]:
         """(whether the logits are kept, first layer whose activations are). Where a pass exchanges data with other ranks
         everything is recomputed: they have to take the same steps, and how much is free is each rank's own. So it is for a
         subclass with layers of its own."""
@@ -708,8 +708,14 @@ class B200Qwen3:
         if (self.ep is not None or self.tp is not None or self.cp_ctx is not None or getattr(self.store, "begin_pass", None) is not None
                 or any(getattr(cls, f) is not getattr(B200Qwen3, f) for f in ("layer_forward", "layer_backward", "forward_hidden", "layers_backward"))):
             return False, hi
-        return plan_kept(self._room_for_acts(), 4 * head_rows * self.store.lm_head().shape[0] if head_rows else 0,
+        # logits, and the chunk of their gradients
+        head = (4 * head_rows + 2 * min(head_rows, self.KEPT_CHUNK * chunk)) * self.store.lm_head().shape[0] if head_rows else 0
+        return plan_kept(self._room_for_acts(), head,
                          [self._layer_act_bytes(i, T) for i in range(lo, hi)], lo)
+
+    # Chunks of the LM head that go through the backward together where the logits are kept: each reads and writes the whole gradient of
+    # the head (151936 x 2048 in fp32: 12288 rows at the power cap 1014 TFLOP/s in chunks of 2048, 1240 in chunks of 8192).
+    KEPT_CHUNK = 4
 
     def layer_backward(self, i, x, dy, positions, cu, max_seqlen, replay_ids=None, acts: Optional[LayerActs] = None):
         """Back-propagate ``dy`` through layer i, from the activations its forward kept or else recomputed from its input
@@ -872,22 +878,29 @@ class B200Qwen3:
     def logprobs_entropy(self, hidden_rows, targets, inv_temp: float, chunk: int = 0, keep_stats: bool = False, keep_logits: Optional[list] = None):
         C = self.C
         chunk = chunk or self.lm_chunk
-        n = hidden_rows.shape[0]
-        lp = torch.empty(n, dtype=torch.float32, device=self.dev)
-        ent = torch.empty_like(lp)
-        lse = torch.empty_like(lp) if keep_stats else None
-        px = torch.empty_like(lp) if keep_stats else None
+        n, W = hidden_rows.shape[0], self.store.lm_head()
         tg = targets.to(torch.int32).contiguous()
+        # The scores leave with the product (csrc/gemm.cu) where its tiles fill the device: no logits at all for more rows at a time,
+        # unless the backward keeps them.
+        fused = -(-min(n, chunk) // 128) * -(-W.shape[0] // 256) >= 148 and type(self).logits is B200Qwen3.logits
+        if fused and keep_logits is None:
+            chunk = max(chunk, 16384)
+        out = []
         for a in range(0, n, chunk):
             b = min(a + chunk, n)
-            lg = self.logits(hidden_rows[a:b], serving=False)
-            l1, e1, s1, p1 = C.logprob_entropy_fwd(lg, tg[a:b], inv_temp)
-            self.launches += 1
-            lp[a:b], ent[a:b] = l1, e1
+            if fused:
+                lg = torch.empty(b - a, W.shape[0], dtype=torch.float32, device=self.dev) if keep_logits is not None else None
+                out.append(C.score_rows(hidden_rows[a:b].contiguous(), W, tg[a:b], inv_temp, lg, self.status))
+                self.launches += 2
+            else:
+                lg = self.logits(hidden_rows[a:b], serving=False)
+                out.append(C.logprob_entropy_fwd(lg, tg[a:b], inv_temp))
+                self.launches += 1
             if keep_logits is not None:
                 keep_logits.append(lg)
-            if keep_stats:
-                lse[a:b], px[a:b] = s1, p1
+        if not out:
+            out.append([torch.empty(0, dtype=torch.float32, device=self.dev)] * 4)
+        lp, ent, lse, px = out[0] if len(out) == 1 else (torch.cat(t) for t in zip(*out))
         return (lp, ent, lse, px) if keep_stats else (lp, ent)
 
     @torch.no_grad()
@@ -908,7 +921,7 @@ class B200Qwen3:
             max_seqlen = int((cu_seqlens[1:] - cu_seqlens[:-1]).max().item())
         inputs: list[torch.Tensor] = []
         acts: dict = {}
-        keep_head, keep_from = self._plan_acts(positions.shape[0], row_index.shape[0])
+        keep_head, keep_from = self._plan_acts(positions.shape[0], row_index.shape[0], chunk)
         keep = dict(save_acts=acts, keep_from=keep_from) if keep_from < self.store.layer_range[1] else {}
         h = self.forward_hidden(tokens, positions, cu_seqlens, replay=replay, max_seqlen=max_seqlen, save_inputs=inputs, x_in=x_in, **keep)
         x_last = inputs.pop()  # input of the final norm
@@ -916,6 +929,7 @@ class B200Qwen3:
         hr = h[rows].contiguous()
         tg = targets.to(torch.int32).contiguous()
         kept: Optional[list] = [] if keep_head else None
+        chunk *= self.KEPT_CHUNK if keep_head else 1
         with torch.no_grad():
             lp, ent, lse, px = self.logprobs_entropy(hr, tg, inv_temp, chunk, keep_stats=True, keep_logits=kept)
         lp_leaf, ent_leaf = lp.detach().requires_grad_(True), ent.detach().requires_grad_(True)

@@ -31,12 +31,12 @@ def test_kept_activations_change_nothing(name):
     tokens, pos, cu, rows, tg = _batch(cfg, [200, 333, 75], dev)
     coef = torch.randn(rows.numel(), device=dev)
     T = tokens.numel()
-    head = 4 * rows.numel() * cfg.vocab_size
+    head = 6 * rows.numel() * cfg.vocab_size
     layers = [model._layer_act_bytes(i, T) for i in range(cfg.num_layers)]
     out = []
     for room in (0, head + layers[-1], 1 << 40):
         model.act_room = room
-        assert model._plan_acts(T, rows.numel()) == ((False, cfg.num_layers), (True, cfg.num_layers - 1), (True, 0))[len(out)]
+        assert model._plan_acts(T, rows.numel(), model.lm_chunk) == ((False, cfg.num_layers), (True, cfg.num_layers - 1), (True, 0))[len(out)]
         store.zero_grads()
         record = []
         model.forward_logprobs(tokens, pos, cu, rows, tg, 1.0, record=record)
