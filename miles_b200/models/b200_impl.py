@@ -649,10 +649,14 @@ class B200Qwen3:
         return y
 
     def _decode_splits(self, B: int, meta: InferMeta) -> int:
-        # Two CTAs per SM at most: the splits of a sequence are a cluster that has to be placed as a whole. Clusters beyond the
-        # portable size of 8 fit only while they fill about two thirds of that (4 rows, 4 heads, us: 12 splits 19.5, 16 29.0).
+        # Two CTAs per SM, but the splits of a sequence are a cluster that has to be placed as a whole: pairs always fit, of
+        # larger ones some wait for a second round beyond 264 CTAs (us, 4 heads: 9 rows 7 splits 16.4, 8 24.2; 12 rows 5 16.2, 6 24.5; 18 rows 3 19.9, 4 26.9;
+        # 24 rows 2 25.6, 3 34.1; 8 heads: 5 rows 6 19.2, 7 29.0). Clusters beyond the portable size of 8 fit only while they fill
+        # about two thirds of the places (4 rows, 4 heads: 12 splits 19.5, 16 29.0).
         ctas = max(B * self.cfg.num_kv_heads, 1)
         splits = max(1, 296 // ctas)
+        if splits > 2:
+            splits = max(2, 264 // ctas)
         return splits if splits <= 8 else min(16, max(8, 192 // ctas))
 
     def _layer_acts(self, i, x, positions, cu, replay_ids=None, output: bool = False):
