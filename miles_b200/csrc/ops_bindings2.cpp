@@ -114,10 +114,11 @@ std::vector<at::Tensor> flash_attn_bwd(const at::Tensor& q, const at::Tensor& k,
   const c10::cuda::CUDAGuard guard(q.device());
   at::Tensor dq = at::empty({T, Hq, 128}, q.options());
   at::Tensor dk = at::empty({T, Hk, 128}, q.options()), dv = at::empty({T, Hk, 128}, q.options());
+  const at::Tensor o16 = reinterpret_cast<uintptr_t>(o.data_ptr()) % 16 ? o.clone() : o;  // read 16 bytes at a time
   at::Tensor scratch = at::empty({T * Hq * 128 + 2 * Hq * T}, q.options().dtype(at::kFloat));
   int* st = nullptr;
   if (status.has_value()) { CHECK_I32((*status)); st = status->data_ptr<int>(); }
-  const int rc = mb::flash_attn_bwd(q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), o.data_ptr(),
+  const int rc = mb::flash_attn_bwd(q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), o16.data_ptr(),
                                     d_o.data_ptr(), d_o.stride(0), lse.data_ptr<float>(), blocks.data_ptr<int>(), blocks.size(0),
                                     T, Hq, Hk, 128, scale, scratch.data_ptr<float>(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
                                     st, cur_stream());
