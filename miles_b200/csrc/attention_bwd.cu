@@ -57,6 +57,7 @@ constexpr int KTILE = 2 * ATOM_K;    // K or V block
 constexpr int QTILE = 2 * ATOM_Q;    // Q or dO tile
 constexpr int PTILE = ATOM_K;        // P^T or dS^T: 128 keys x 64 q
 constexpr int STAGES = 3;
+constexpr int SMS = 148;
 constexpr int BWD_THREADS = 15 * 32;
 constexpr int BWD_SMEM = 2 * KTILE + 4 * PTILE + STAGES * 2 * QTILE + STAGES * 2 * BQ * 4 + 256 + 1024;
 
@@ -70,11 +71,17 @@ struct FaBwdArgs {
   __nv_bfloat16* dv;
   long long T;
   float scale, scale_log2;
+  int split;           // CTAs, in a cluster, that share the query heads of a key block (a power of two that divides Hq / Hk)
   int* status;
 };
 
 __device__ __forceinline__ uint32_t swz_off(int row, int chunk16) {
   return static_cast<uint32_t>(row * 128 + ((chunk16 ^ (row & 7)) << 4));
+}
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
 }
 __device__ __forceinline__ float ex2(float x) {
   float y;
@@ -82,6 +89,10 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
+// SPLIT: p.split CTAs, a cluster, share a key block's query heads; each sums dV and dK of its own in TMEM, and at the end every CTA
+// adds up a part of the rows from all of them, in the order of their heads. One sequence of 4096, 32 query and 4 KV heads: 964 -> 519 us
+// (two CTAs), 389 + 388: 130 -> 62 (four); who gains from it is in bwd_split of ops/attention.py.
+template <bool SPLIT>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 fa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_do,
               const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
@@ -108,9 +119,12 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // Heads vary fastest: the list starts with the blocks that have the most queries after them, and all heads' long blocks have
   // to start before anyone's short ones (one head after another left SMs with 1.4 times the average work at the end).
-  const int4 blk = p.blocks[blockIdx.x / p.Hk];
-  const int hk = blockIdx.x % p.Hk;
-  const int G = p.Hq / p.Hk;
+  const int split = SPLIT ? p.split : 1;
+  const int job = blockIdx.x / split;
+  const int4 blk = p.blocks[job / p.Hk];
+  const int hk = job % p.Hk;
+  const int G = p.Hq / p.Hk / split;       // this CTA's query heads
+  const int hq0 = (hk * split + blockIdx.x % split) * G;
   const int kv_row0 = blk.x, kv_rows = blk.y, seq_end = blk.w;
   // query rows at or after the block's first key: global rows kv_row0 .. seq_end - 1
   const int q_total = seq_end - kv_row0;
@@ -170,7 +184,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     for (int it = 0; ok && it < n_it; ++it) {
       const int st = it % STAGES;
       const int g = it / n_qt, qt = it - g * n_qt;
-      const int hq = hk * G + g;
+      const int hq = hq0 + g;
       const int q_row0 = kv_row0 + qt * BQ;
       if (!mbar_wait(BAR(B_QE + st), ((it / STAGES) & 1) ^ 1, abort_flag, p.status, ERR_WAIT_EMPTY)) {
         ok = false;
@@ -339,7 +353,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     }
     // ---- epilogue: dV, dK (scaled) -> bf16
     if (ok) ok = mbar_wait(BAR(B_FIN), 0, abort_flag, p.status, ERR_WAIT_TMEM_FULL);
-    if (ok) {
+    if (!SPLIT && ok) {
       tc_fence_after();
       const long long orow = (static_cast<long long>(kv_row0 + row) * p.Hk + hk) * HD + half * 64;
       uint32_t o[32];
@@ -400,7 +414,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     for (int it = 0; it < n_it; ++it) {
       const int g = it / n_qt, qt = it - g * n_qt, buf = it & 1;
       if (!mbar_wait(BAR(B_ST + buf), (it >> 1) & 1, abort_flag, p.status, ERR_WAIT_FULL)) break;
-      tma_reduce_add_2d(&map_dq, pt_s + buf * 2 * PTILE, (hk * G + g) * HD, kv_row0 + qt * BQ);
+      tma_reduce_add_2d(&map_dq, pt_s + buf * 2 * PTILE, (hq0 + g) * HD, kv_row0 + qt * BQ);
       tma_store_commit();
       tma_store_wait_read<0>();
       mbar_arrive(BAR(B_PB + buf));
@@ -411,6 +425,48 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
 
   tc_fence_before();
   __syncthreads();
+  if constexpr (SPLIT) {
+    // ------------------------------------------------------------------ dV, dK of the cluster's heads added up, CTA by CTA
+    // (every thread of every CTA comes here, whatever happened before; a CTA that gave up has set the status, and its sums are void)
+    if (warp >= 2 && warp < 10) {
+      const int quad = warp & 3, half = (warp - 2) >> 2, row = quad * 32 + lane;
+      tc_fence_after();
+#pragma unroll 1
+      for (int c = 0; c < 4; ++c) {  // dV's two quarters of this half row, then dK's: over K, V, P^T and dS^T, which are done with
+        uint32_t o[32];
+        tmem_ld_32x32((c < 2 ? t_dV : t_dK) + (static_cast<uint32_t>(quad * 32) << 16) + half * 64 + (c & 1) * 32, o);
+        tmem_ld_wait();
+        const uint32_t dst = base + (c >> 1) * (BK * HD * 4) + row * (HD * 4);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + (((half * 16 + (c & 1) * 8 + i) ^ lane) << 4)), "r"(o[4 * i]),
+                       "r"(o[4 * i + 1]), "r"(o[4 * i + 2]), "r"(o[4 * i + 3])
+                       : "memory");
+      }
+      tc_fence_before();
+    }
+    cluster_sync_all();
+    const int rank = blockIdx.x % split, rows = BK / split;  // of the block, which this CTA adds up: eight values a thread and turn
+    for (int i = threadIdx.x; i < 2 * rows * (HD / 8); i += BWD_THREADS) {
+      const int which = i / (rows * (HD / 8)), row = rank * rows + i / (HD / 8) % rows, c = i % (HD / 8);
+      const uint32_t src = base + which * (BK * HD * 4) + row * (HD * 4);
+      const uint32_t src0 = src + (((2 * c) ^ (row & 31)) << 4), src1 = src + (((2 * c + 1) ^ (row & 31)) << 4);
+      float v[8] = {};
+      for (int r = 0; r < split; ++r) {
+        const float4 x = ld_cluster_f4(map_to_rank(src0, r)), y = ld_cluster_f4(map_to_rank(src1, r));
+        v[0] += x.x, v[1] += x.y, v[2] += x.z, v[3] += x.w;
+        v[4] += y.x, v[5] += y.y, v[6] += y.z, v[7] += y.w;
+      }
+      if (row < kv_rows) {
+        const float sc = which == 0 ? 1.f : p.scale;
+        __nv_bfloat16* dst = (which == 0 ? p.dv : p.dk) + (static_cast<long long>(kv_row0 + row) * p.Hk + hk) * HD + c * 8;
+        *reinterpret_cast<uint4*>(dst) = make_uint4(pack_bf16(v[0] * sc, v[1] * sc), pack_bf16(v[2] * sc, v[3] * sc),
+                                                    pack_bf16(v[4] * sc, v[5] * sc), pack_bf16(v[6] * sc, v[7] * sc));
+      }
+    }
+    __syncwarp();
+    cluster_sync_all();  // no CTA leaves while another still reads its shared memory
+  }
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);
@@ -528,10 +584,13 @@ const char* flash_attn_bwd_last_error() { return g_err.c_str(); }
 // pitches; lse [Hq, T]; blocks int32 [n, 4]; scratch fp32: dq_acc [T*Hq*128] (zeroed here) then dsum [Hq*T], lse2 [Hq*T].
 int flash_attn_bwd(const void* q, long long q_ld, const void* k, long long k_ld, const void* v, long long v_ld, const void* o,
                    const void* d_o, long long do_ld, const float* lse, const int* blocks, int num_blocks, long long T, int Hq,
-                   int Hk, int head_dim, float scale, float* scratch, void* dq, void* dk, void* dv, int* status,
+                   int Hk, int head_dim, float scale, int split, float* scratch, void* dq, void* dk, void* dv, int* status,
                    cudaStream_t stream) {
   if (head_dim != HD) return fail("flash_attn_bwd supports head_dim 128 only");
   if (Hq % Hk != 0) return fail("query heads must be a multiple of kv heads");
+  const int heads = Hq / Hk;
+  if ((split != 1 && split != 2 && split != 4) || heads % split != 0)
+    return fail("split must be 1, 2 or 4 and divide the query heads of a kv head");
   if (T <= 0 || num_blocks <= 0) return 0;
   float* dq_acc = scratch;
   float* dsum = scratch + T * Hq * HD;
@@ -549,7 +608,8 @@ int flash_attn_bwd(const void* q, long long q_ld, const void* k, long long k_ld,
   if (make_map(&mk, k, T, static_cast<long long>(Hk) * HD, k_ld, BK)) return -1;
   if (make_map(&mv, v, T, static_cast<long long>(Hk) * HD, v_ld, BK)) return -1;
   if (make_dq_map(&mdq, dq_acc, T, Hq)) return -1;
-  if (cudaFuncSetAttribute(fa_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_SMEM) != cudaSuccess)
+  auto kernel = split > 1 ? fa_bwd_kernel<true> : fa_bwd_kernel<false>;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_SMEM) != cudaSuccess)
     return fail("cudaFuncSetAttribute(MaxDynamicSharedMemorySize) failed for the attention backward");
   FaBwdArgs a;
   a.blocks = reinterpret_cast<const int4*>(blocks);
@@ -562,12 +622,24 @@ int flash_attn_bwd(const void* q, long long q_ld, const void* k, long long k_ld,
   a.T = T;
   a.scale = scale;
   a.scale_log2 = scale * 1.4426950408889634f;
+  a.split = split;
   a.status = status;
-  fa_bwd_kernel<<<num_blocks * Hk, BWD_THREADS, BWD_SMEM, stream>>>(mq, mdo, mk, mv, mdq, a);
-  if (cudaPeekAtLastError() != cudaSuccess) return fail("attention backward launch failed");
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(split);
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(num_blocks) * Hk * split);
+  cfg.blockDim = dim3(BWD_THREADS);
+  cfg.dynamicSmemBytes = BWD_SMEM;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, kernel, mq, mdo, mk, mv, mdq, a) != cudaSuccess) return fail("attention backward launch failed");
   const long long n4 = T * Hq * HD / 4;
   long long cb = (n4 + 255) / 256;
-  if (cb > 148 * 8) cb = 148 * 8;
+  if (cb > SMS * 8) cb = SMS * 8;
   f32_to_bf16_kernel<<<static_cast<unsigned>(cb), 256, 0, stream>>>(reinterpret_cast<const float4*>(dq_acc),
                                                                    reinterpret_cast<uint2*>(dq), n4);
   return 0;

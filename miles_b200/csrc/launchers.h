@@ -120,7 +120,7 @@ const char* flash_attn_last_error();
 // the sequence}; scratch fp32 [T*Hq*128 + 2*Hq*T]; dq [T, Hq, 128], dk / dv [T, Hk, 128] bf16 contiguous.
 int flash_attn_bwd(const void* q, long long q_ld, const void* k, long long k_ld, const void* v, long long v_ld, const void* o,
                    const void* d_o, long long do_ld, const float* lse, const int* blocks, int num_blocks, long long T, int Hq,
-                   int Hk, int head_dim, float scale, float* scratch, void* dq, void* dk, void* dv, int* status,
+                   int Hk, int head_dim, float scale, int split, float* scratch, void* dq, void* dk, void* dv, int* status,
                    cudaStream_t stream);
 const char* flash_attn_bwd_last_error();
 

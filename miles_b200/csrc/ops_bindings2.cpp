@@ -100,7 +100,7 @@ std::vector<at::Tensor> flash_attn_fwd(const at::Tensor& q, const at::Tensor& k,
 // Backward of the causal self-attention over packed sequences. Returns {dq, dk, dv}.
 std::vector<at::Tensor> flash_attn_bwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& o,
                                        const at::Tensor& d_o, const at::Tensor& lse, const at::Tensor& blocks, double scale,
-                                       const c10::optional<at::Tensor>& status) {
+                                       const c10::optional<at::Tensor>& status, int64_t split) {
   CHECK_I32(blocks);
   for (const at::Tensor* t : {&q, &k, &v, &o, &d_o})
     TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kBFloat16 && t->dim() == 3 && t->size(2) == 128 && t->stride(2) == 1 &&
@@ -120,7 +120,7 @@ std::vector<at::Tensor> flash_attn_bwd(const at::Tensor& q, const at::Tensor& k,
   if (status.has_value()) { CHECK_I32((*status)); st = status->data_ptr<int>(); }
   const int rc = mb::flash_attn_bwd(q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), o16.data_ptr(),
                                     d_o.data_ptr(), d_o.stride(0), lse.data_ptr<float>(), blocks.data_ptr<int>(), blocks.size(0),
-                                    T, Hq, Hk, 128, scale, scratch.data_ptr<float>(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
+                                    T, Hq, Hk, 128, scale, split, scratch.data_ptr<float>(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
                                     st, cur_stream());
   TORCH_CHECK(rc == 0, mb::flash_attn_bwd_last_error());
   return {dq, dk, dv};
@@ -302,7 +302,8 @@ void register_more(pybind11::module_& m) {
   m.def("moe_decode_up", &moe_decode_up);
   m.def("moe_decode_fits", &moe_decode_fits);
   m.def("moe_decode_plan_size", &moe_decode_plan_size);
-  m.def("flash_attn_bwd", &flash_attn_bwd);
+  m.def("flash_attn_bwd", &flash_attn_bwd, py::arg("q"), py::arg("k"), py::arg("v"), py::arg("o"), py::arg("d_o"), py::arg("lse"),
+        py::arg("blocks"), py::arg("scale"), py::arg("status"), py::arg("split") = 1);
   m.def("router_small", &router_small);
   m.def("gather_prefix_kv", &gather_prefix_kv);
   m.def("moe_small_up", &moe_small_up);

@@ -107,7 +107,8 @@ class B200Qwen3:
         if isinstance(lse, tuple):
             return self._attention_cp_backward(d_out, lse)
         dq, dk, dv = self.C.flash_attn_bwd(q, k, v, out, d_out.contiguous(), lse, self._tiles.get_bwd(cu),
-                                           self.cfg.head_dim ** -0.5, self.status)
+                                           self.cfg.head_dim ** -0.5, self.status,
+                                           self._tiles.get_bwd_split(cu, q.shape[1], k.shape[1]))
         self.launches += 3
         return dq, dk, dv
 
@@ -141,7 +142,7 @@ class B200Qwen3:
         lse_f, qf, kf, vf, out_f, cu = saved
         do_f = heads_to_sequence(d_out.contiguous(), lens, cp, rank, group, layout).contiguous()
         dqf, dkf, dvf = self.C.flash_attn_bwd(qf, kf, vf, out_f, do_f, lse_f, self._tiles.get_bwd(cu), self.cfg.head_dim ** -0.5,
-                                              self.status)
+                                              self.status, self._tiles.get_bwd_split(cu, qf.shape[1], kf.shape[1]))
         self.launches += 3
         return tuple(sequence_to_heads(t, lens, cp, rank, group, layout).contiguous() for t in (dqf, dkf, dvf))
 

@@ -56,6 +56,27 @@ def build_bwd_blocks(seq_lens: Sequence[int]) -> torch.Tensor:
     return torch.tensor(rows, dtype=torch.int32).view(-1, 4)
 
 
+def bwd_split(blocks: int, longest: int, total: int, q_heads: int, kv_heads: int) -> int:
+    """CTAs (1, 2 or 4) that share the query heads of a key block in the backward kernel: for ``blocks`` key blocks of which the
+    first of the longest sequence has ``longest`` tiles of 64 queries to go through for each head, and all together ``total``.
+
+    A CTA has an SM to itself and spends about as long on its start and end as on ten tiles. So a launch lasts as long as its longest
+    CTA or as the work laid over the SMs, whichever is longer, and the split with the least of it wins; clusters of four find
+    room on 132 of the 148 SMs. Measured, us for one / two / four CTAs: 389 + 388 tokens (32 query and 4 KV heads) 130 / 85 / 62,
+    one of 2048 470 / 267 / 177, one of 4096 964 / 519 / 556, one of 6000 1424 / 990 / 1107, nine of 200 97 / 73 / 99; but
+    24 of 200 138 / 159 / 214, eight of 1024 368 / 390 / 515, six of 2731 1355 / 1439 / 1875."""
+    group = q_heads // kv_heads
+    best, best_cost = 1, None
+    for split, sms in ((1, 148), (2, 148), (4, 132)):
+        if group % split:
+            break
+        ctas = blocks * kv_heads * split
+        cost = max(longest * group / split + 10, (total * q_heads + 10 * ctas) / sms)
+        if best_cost is None or cost < best_cost:
+            best, best_cost = split, cost
+    return best
+
+
 class TileCache:
     """Remembers the tile table of the last ``cu_seqlens`` tensor (identity, not value, is compared)."""
 
@@ -64,13 +85,21 @@ class TileCache:
         self._tiles = None
         self._bwd_cu = None
         self._bwd = None
+        self._bwd_work = (0, 0, 0)  # key blocks, query tiles of the longest, query tiles of all
 
     def get_bwd(self, cu: torch.Tensor) -> torch.Tensor:
         if self._bwd_cu is not cu:
             lens = (cu[1:] - cu[:-1]).tolist()
-            self._bwd = build_bwd_blocks(lens).to(cu.device, non_blocking=True)
+            blocks = build_bwd_blocks(lens)
+            tiles = (blocks[:, 3] - blocks[:, 0] + 63) // 64
+            self._bwd_work = (len(blocks), int(tiles[0]) if len(blocks) else 0, int(tiles.sum()))
+            self._bwd = blocks.to(cu.device, non_blocking=True)
             self._bwd_cu = cu
         return self._bwd
+
+    def get_bwd_split(self, cu: torch.Tensor, q_heads: int, kv_heads: int) -> int:
+        self.get_bwd(cu)
+        return bwd_split(*self._bwd_work, q_heads, kv_heads)
 
     def get(self, cu: torch.Tensor) -> torch.Tensor:
         if self._cu is not cu:

@@ -14,14 +14,14 @@ def _inputs(T, Hq, Hk):
     return [torch.randn(T, h, 128, device="cuda", generator=g).bfloat16() for h in (Hq, Hk, Hk, Hq)]
 
 
-def _run(q, k, v, do, lens):
+def _run(q, k, v, do, lens, split=1):
     from miles_b200.ops import _ext
     from miles_b200.ops.attention import build_bwd_blocks, build_tiles
 
     C = _ext.load(required=True)
     st = torch.zeros(1, dtype=torch.int32, device="cuda")
     o, lse = C.flash_attn_fwd(q, k, v, build_tiles(lens).cuda(), SCALE, st)
-    grads = C.flash_attn_bwd(q, k, v, o, do, lse, build_bwd_blocks(lens).cuda(), SCALE, st)
+    grads = C.flash_attn_bwd(q, k, v, o, do, lse, build_bwd_blocks(lens).cuda(), SCALE, st, split=split)
     assert int(st.item()) == 0
     return o, grads
 
@@ -79,3 +79,15 @@ def test_rows_that_start_off_a_16_byte_boundary():
     shifted.copy_(o)
     blocks = build_bwd_blocks([100]).cuda()
     _check(q, k, v, do, o, C.flash_attn_bwd(q, k, v, shifted, do, lse, blocks, SCALE, st), 0, 100)
+
+
+# a lone row, a block's edges, more blocks than the device has room for at once; every number of CTAs that divides the heads
+@pytest.mark.parametrize("lens", [[1], [127, 129], [200] * 12])
+@pytest.mark.parametrize("Hq,Hk,split", [(8, 4, 2), (16, 2, 1), (16, 2, 2), (16, 2, 4), (12, 1, 4)])
+def test_heads_shared_by_a_cluster(lens, Hq, Hk, split):
+    q, k, v, do = _inputs(sum(lens), Hq, Hk)
+    o, grads = _run(q, k, v, do, lens, split)
+    a = 0
+    for n in lens:
+        _check(q, k, v, do, o, grads, a, a + n)
+        a += n
