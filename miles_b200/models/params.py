@@ -338,7 +338,9 @@ class ParamStore:
     def zero_grads(self) -> None:
         for g in self.grad.values():
             if g is not None:
-                g.zero_()
+                # four bytes at a time where they divide: 1.6 GB of bf16 410 us, as float 215 (16-bit fills do half as much a thread)
+                words = g.element_size() == 2 and g.is_cuda and g.is_contiguous() and g.numel() % 2 == 0 and g.data_ptr() % 4 == 0
+                (g.view(-1).view(torch.float32) if words else g).zero_()
 
     def free_grads(self) -> None:
         self.grad = {"dense": None, "expert": None}
