@@ -63,7 +63,7 @@ struct KArgs {
   float inv_temp;
 };
 
-enum Epilogue : int { EPI_PLAIN = 0, EPI_GLU = 1, EPI_SCORES = 2 };
+enum Epilogue : int { EPI_PLAIN = 0, EPI_GLU = 1, EPI_SCORES = 2, EPI_ADD = 3 };
 
 struct Tile {
   int a_mn0, b_mn0;  // M/N coordinates in the operand tensors
@@ -246,9 +246,8 @@ __device__ __forceinline__ void store_chunk(const KArgs& p, const Tile& t, int r
 
 // ---- staged epilogue: a warp's 32 x (128 bytes) chunks pass through shared memory, so that every global access covers whole
 // 128-byte (accumulating bf16: 64-byte) row segments instead of 32 pieces of 16 bytes, each its own wavefront, and so that the
-// rows that are added to can be asked for several chunks ahead, the first ones while the tile is still being multiplied. A
-// weight gradient of few tokens is nothing but that read-modify-write: 128 experts of 1536 x 2048 in bf16 with 48 tokens each
-// 704 us before, 469 us now (1.6 GB); 151936 x 2048 in fp32 with 583 tokens 914 -> 594 us (2.5 GB). Without adding: 2048 x
+// rows that are added to can be asked for several chunks ahead, the first ones while the tile is still being multiplied (weight
+// gradients of few tokens, nothing but that read-modify-write, take the adding epilogue below). Without adding: 2048 x
 // 151936 x 2048 to fp32 1122 -> 1014 us, 131072 expert rows of 768 x 2048 427 -> 376 us.
 // `stg`: 4 KB of shared memory of this warp; 16-byte piece i of row r lies at piece i ^ (r & 7) (conflict-free both ways).
 __device__ __forceinline__ void sts16(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
@@ -400,6 +399,100 @@ struct StagedEpilogue {
   }
 };
 
+// ---- adding epilogue (EPI_ADD): the rows that are added to come by `cp.async` into the buffers in which they are added to and from
+// which they leave, a piece of 32 rows x 128 bytes each, one or two of them a warp; a piece that has left makes room for the next one
+// without a buffer, of this tile or the next. Bound by reading and writing C where the contraction is short. Old values in registers
+// (StagedEpilogue) are asked for as early, but a warp has to wait for all of its loads to have the first of them: 128 experts of
+// 1536 x 2048 in bf16, 777 tokens over them with eight experts each 463 -> 281 us (1.6 GB: 5.7 TB/s), 4096 tokens 428 -> 340, 8192 527 -> 465;
+// in fp32, by pairs, 151936 x 2048 with 776 tokens 652 -> 561 us (2.5 GB), 5120 x 2048 with 16384 333 -> 316, 24576 x 4096 with 9216 1256 -> 1201.
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+
+// Buffers of a warp: one beside the four stages of a 256-wide tile of one CTA, which take the room of the second.
+constexpr int add_buffers(int block_n, int stages, int cg) { return block_n == 256 && cg == 1 && stages == 4 ? 1 : 2; }
+
+template <int BLOCK_N, bool FP32, int BUFFERS>
+struct AddEpilogue {
+  static constexpr int ESZ = FP32 ? 4 : 2;
+  static constexpr int COLS = 128 / ESZ;                // of a piece
+  static constexpr int PIECES = BLOCK_N / 2 / COLS;     // of one warp: half a tile's
+  static constexpr int AHEAD = PIECES < BUFFERS ? PIECES : BUFFERS;
+  static_assert(PIECES % AHEAD == 0, "a piece's buffer is the same in every tile");
+
+  // Asks for piece c of the warp's half of a tile (rows past the end and pieces past column N, a multiple of COLS, read nothing) and closes the group.
+  static __device__ __forceinline__ void ask(const KArgs& p, const Tile& t, int row0, int c, int lane, int half, uint32_t stg) {
+    const int col = t.c_col0 + (half * PIECES + c) * COLS;
+    if (col < p.N) {
+      const int rows = t.row_end - row0 - lane / 8;
+      const uint8_t* at = static_cast<const uint8_t*>(p.c) + (t.c_base + (row0 + lane / 8) * p.ldc + col) * ESZ + (lane & 7) * 16;
+      const long long step = 4 * p.ldc * ESZ;
+#pragma unroll
+      for (int it = 0; it < 8; ++it, at += step) {
+        const int r = it * 4 + lane / 8;
+        if (it * 4 < rows) cp_async16(stg + r * 128 + (((lane & 7) ^ (r & 7)) << 4), at);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+
+  // The tile's first AHEAD pieces have been asked for; afterwards those of `next` have, if `more`.
+  static __device__ __forceinline__ void run(const KArgs& p, const Tile& t, const Tile& next, bool more, int row0, int next_row0, int lane,
+                                             int half, uint32_t t_addr, uint32_t stg0) {
+    t_addr += half * (BLOCK_N / 2);
+#pragma unroll 1
+    for (int c = 0; c < PIECES; ++c) {
+      const int col = t.c_col0 + (half * PIECES + c) * COLS;
+      const uint32_t stg = stg0 + (c % AHEAD) * 4096;
+      asm volatile("cp.async.wait_group %0;" ::"n"(AHEAD - 1) : "memory");
+      __syncwarp();
+      if (col < p.N) {  // warp-uniform
+        const uint32_t mine = stg + lane * 128, x = lane & 7;
+#pragma unroll
+        for (int h = 0; h < COLS / 32; ++h) {
+          uint32_t acc[32];
+          tmem_ld_32x32(t_addr + c * COLS + h * 32, acc);
+          tmem_ld_wait();
+          const float* f = reinterpret_cast<const float*>(acc);
+          if constexpr (FP32) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const uint4 o = lds16(mine + ((i ^ x) << 4));
+              sts16(mine + ((i ^ x) << 4), __float_as_uint(f[4 * i] + __uint_as_float(o.x)), __float_as_uint(f[4 * i + 1] + __uint_as_float(o.y)),
+                    __float_as_uint(f[4 * i + 2] + __uint_as_float(o.z)), __float_as_uint(f[4 * i + 3] + __uint_as_float(o.w)));
+            }
+          } else {  // added in fp32, rounded once
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const uint32_t at = mine + (((h * 4 + i) ^ x) << 4);
+              const uint4 o = lds16(at);
+              const __nv_bfloat162* ob = reinterpret_cast<const __nv_bfloat162*>(&o);
+              const float2 o0 = __bfloat1622float2(ob[0]), o1 = __bfloat1622float2(ob[1]), o2 = __bfloat1622float2(ob[2]), o3 = __bfloat1622float2(ob[3]);
+              sts16(at, pack_bf16(f[8 * i] + o0.x, f[8 * i + 1] + o0.y), pack_bf16(f[8 * i + 2] + o1.x, f[8 * i + 3] + o1.y),
+                    pack_bf16(f[8 * i + 4] + o2.x, f[8 * i + 5] + o2.y), pack_bf16(f[8 * i + 6] + o3.x, f[8 * i + 7] + o3.y));
+            }
+          }
+        }
+        __syncwarp();
+        const int rows = t.row_end - row0 - lane / 8;
+        uint8_t* at = static_cast<uint8_t*>(p.c) + (t.c_base + (row0 + lane / 8) * p.ldc + col) * ESZ + (lane & 7) * 16;
+        const long long step = 4 * p.ldc * ESZ;
+#pragma unroll
+        for (int it = 0; it < 8; ++it, at += step) {
+          const int r = it * 4 + lane / 8;
+          const uint4 v = lds16(stg + r * 128 + (((lane & 7) ^ (r & 7)) << 4));
+          if (it * 4 < rows) *reinterpret_cast<uint4*>(at) = v;
+        }
+        __syncwarp();
+      }
+      const bool own = c + AHEAD < PIECES;
+      if (own || more) ask(p, own ? t : next, own ? row0 : next_row0, own ? c + AHEAD : c + AHEAD - PIECES, lane, half, stg);
+      else asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+  }
+};
+
 // CG = 2: a pair of CTAs (a cluster) multiplies 256 x 256 tiles with `cta_group::2`: each holds its 128 rows of A and half of B's,
 // so that a tile's operands are read from shared memory, and from L2, two thirds as often for the same work. That is what bounds the
 // one-CTA tile: per 16 of K it reads 12 KB of shared memory and receives another 12 KB in the 128 clocks of its product (at 128 bytes
@@ -423,6 +516,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                  const KArgs p) {
   constexpr bool GLU = EPI == EPI_GLU, SCORES = EPI == EPI_SCORES;
+  constexpr int ADD_BUFFERS = add_buffers(BLOCK_N, STAGES, CG);
   constexpr int B_ROWS = BLOCK_N / CG;  // of this CTA
   constexpr int B_STAGE_BYTES = B_ROWS * BLOCK_K * 2;
   constexpr uint32_t TMEM_COLS = 2 * BLOCK_N;  // 256 or 512: a power of two >= 32
@@ -627,7 +721,32 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         ++iter;
       }
     };
-    const bool adds = EPI == EPI_PLAIN && staged && p.accumulate;
+    if constexpr (EPI == EPI_ADD) {
+      const uint32_t stg = stage_buf + static_cast<uint32_t>(warp - 2) * (ADD_BUFFERS * 4096);
+      auto add_pieces = [&](auto e) {
+        using E = decltype(e);
+        bool asked = false;  // the next tile's first pieces
+        for (int t = first_tile; t < total_tiles; t += tile_step) {
+          const Tile tl = decode_tile<BLOCK_N, B_MN, CG, EPI>(p, t, rank);
+          if (tl.k_iters == 0) continue;
+          const int row0 = tl.c_row0 + quad * 32, acc = iter & 1, tn = t + tile_step;
+          if (!asked)
+            for (int c = 0; c < E::AHEAD; ++c) E::ask(p, tl, row0, c, lane, half, stg + c * 4096);
+          const Tile next = decode_tile<BLOCK_N, B_MN, CG, EPI>(p, tn < total_tiles ? tn : t, rank);
+          asked = tn < total_tiles && next.k_iters > 0;
+          if (!__all_sync(0xffffffffu, mbar_wait(tfull_bar(acc), (iter >> 1) & 1u, abort_flag, p.status, ERR_WAIT_TMEM_FULL))) break;
+          tc_fence_after();
+          E::run(p, tl, next, asked, row0, next.c_row0 + quad * 32, lane, half,
+                 tmem_base + acc * BLOCK_N + (static_cast<uint32_t>(quad * 32) << 16), stg);
+          release(acc);
+          ++iter;
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+      };
+      if (p.out_fp32) add_pieces(AddEpilogue<BLOCK_N, true, ADD_BUFFERS>());
+      else add_pieces(AddEpilogue<BLOCK_N, false, ADD_BUFFERS>());
+    }
+    const bool adds = EPI == EPI_ADD || (EPI == EPI_PLAIN && staged && p.accumulate);
     if constexpr (BLOCK_N >= 64 && EPI == EPI_PLAIN) {
       if (adds && p.out_fp32) add_tiles(StagedEpilogue<BLOCK_N, true, true>());
       else if (adds) add_tiles(StagedEpilogue<BLOCK_N, false, true>());
@@ -920,13 +1039,13 @@ int gemm_make_map(CUtensorMap* map, const GemmOperand& op, int box_rows) {
 
 namespace {
 
-template <int BLOCK_N, bool A_MN, bool B_MN, int CG = 1, int EPI = EPI_PLAIN>
+template <int BLOCK_N, bool A_MN, bool B_MN, int CG = 1, int EPI = EPI_PLAIN, int FEWER = 0>
 int launch(const GemmProblem& p, const KArgs& ka, cudaStream_t stream) {
-  // (the 32 KB staging buffer takes a pipeline stage from the 128-wide variant)
-  constexpr int STAGES = CG == 2 ? 6 : (BLOCK_N == 256 ? 4 : (BLOCK_N == 128 ? 5 : 8));
+  // (the 32 KB staging buffer takes a pipeline stage from the 128-wide variant; FEWER more go to the adding epilogue's buffers)
+  constexpr int STAGES = (CG == 2 ? 6 : (BLOCK_N == 256 ? 4 : (BLOCK_N == 128 ? 5 : 8))) - FEWER;
   constexpr int B_STAGE_BYTES = BLOCK_N / CG * BLOCK_K * 2;
   constexpr int SMEM = STAGES * (A_STAGE_BYTES + B_STAGE_BYTES) + 8 * (2 * STAGES + 5) + 1024 +
-                       8 * 4096 + 128;
+                       8 * 4096 * (EPI == EPI_ADD ? add_buffers(BLOCK_N, STAGES, CG) : 1) + 128;
   CUtensorMap ma, mb_;
   if (gemm_make_map(&ma, p.a, A_MN ? BLOCK_K : BLOCK_M)) return -1;
   if (gemm_make_map(&mb_, p.b, B_MN ? BLOCK_K : EPI == EPI_GLU ? BLOCK_N / 2 : BLOCK_N / CG)) return -1;
@@ -1070,6 +1189,20 @@ int gemm_bf16_launch(const GemmProblem& p, cudaStream_t stream) {
   if (bn == 64) return launch<64, false, false>(p, ka, stream);
   if (p.glu) return pair ? launch<256, false, false, 2, EPI_GLU>(p, ka, stream) : launch<256, false, false, 1, EPI_GLU>(p, ka, stream);
   if (p.score_part) return pair ? launch<256, false, false, 2, EPI_SCORES>(p, ka, stream) : launch<256, false, false, 1, EPI_SCORES>(p, ka, stream);
+  // Weight gradients add to whole pieces of 128 bytes (what ends within one stays with the staged epilogue, whose ragged columns find
+  // their lines in L1: 1000 x 1048, K = 333, 9.5 and 12.4 us). One CTA's 256-wide tiles take the adding epilogue's second buffer from
+  // their stages, which long contractions miss; by rows per group, us staged / two buffers and three stages / one and four, 128 experts
+  // of 1536 x 2048: 112 rows 459 / 281 / 381, 319 428 / 340 / 391, 575 527 / 497 / 465, 813 630 / 641 / 622, 1087 757 / 811 / 767;
+  // dense in fp32: 8192 x 2048, K = 60, 23.0 / 21.1 / 25.5, 2048 x 4096, K = 333, 16.5 / 15.5 / 16.7, 2048 x 2048, K = 777, 12.5 / 12.5 / 13.3,
+  // 128 x 2048, K = 16384, 92 / 106 / 93.
+  if (p.accumulate && amn && bmn && ka.vec_ok && p.N % (p.out_fp32 ? 32 : 64) == 0) {
+    if (pair) return launch<256, true, true, 2, EPI_ADD, 1>(p, ka, stream);
+    if (bn == 128) return launch<128, true, true, 1, EPI_ADD>(p, ka, stream);
+    const bool grouped = p.mode == GEMM_GROUPED_CONTR;
+    const long long k = grouped ? p.a.rows / (p.num_groups > 0 ? p.num_groups : 1) : p.K;
+    if (k < (grouped ? 448 : 1024)) return launch<256, true, true, 1, EPI_ADD, 1>(p, ka, stream);
+    if (grouped && k < 800) return launch<256, true, true, 1, EPI_ADD>(p, ka, stream);
+  }
   if (pair) {
     if (!amn && !bmn) return launch<256, false, false, 2>(p, ka, stream);
     if (!amn && bmn) return launch<256, false, true, 2>(p, ka, stream);
