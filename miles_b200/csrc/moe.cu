@@ -451,7 +451,7 @@ __global__ void permute_kernel(const bf16* __restrict__ x, const int* __restrict
       for (int u = 0; u < 4; ++u) v[u] = (src >= 0 && c0 + 32 * u < vec_per_row) ? from[c0 + 32 * u] : make_uint4(0, 0, 0, 0);
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-        if (c0 + 32 * u < vec_per_row) to[c0 + 32 * u] = v[u];
+        if (c0 + 32 * u < vec_per_row) __stcs(to + c0 + 32 * u, v[u]);
     }
   }
 }
@@ -502,7 +502,7 @@ combine_kernel(const bf16* __restrict__ y_perm, const int* __restrict__ dest_row
       }
 #pragma unroll
       for (int k = 0; k < 8; ++k)
-        if (row[k] >= 0) v[k] = reinterpret_cast<const uint4*>(y_perm + static_cast<long long>(row[k]) * H)[c];
+        if (row[k] >= 0) v[k] = __ldcs(reinterpret_cast<const uint4*>(y_perm + static_cast<long long>(row[k]) * H) + c);
 #pragma unroll
       for (int k = 0; k < 8; ++k)
         if (row[k] >= 0) acc8(v[k], w[k], a);
@@ -538,7 +538,7 @@ __global__ void combine_bwd_kernel(const bf16* __restrict__ dout, const bf16* __
         gr[u] = yr[u] = make_uint4(0, 0, 0, 0);
         if (c0 + 32 * u < vec_per_row) {
           gr[u] = g[c0 + 32 * u];
-          if (dtopk_w) yr[u] = y[c0 + 32 * u];
+          if (dtopk_w) yr[u] = __ldcs(y + c0 + 32 * u);
         }
       }
 #pragma unroll
@@ -546,7 +546,7 @@ __global__ void combine_bwd_kernel(const bf16* __restrict__ dout, const bf16* __
         if (c0 + 32 * u >= vec_per_row) break;
         float a[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         acc8(gr[u], w, a);
-        dst[c0 + 32 * u] = pack8(a);
+        __stcs(dst + c0 + 32 * u, pack8(a));
         if (dtopk_w) {
           const __nv_bfloat162* gb = reinterpret_cast<const __nv_bfloat162*>(&gr[u]);
           const __nv_bfloat162* yb = reinterpret_cast<const __nv_bfloat162*>(&yr[u]);
