@@ -10,16 +10,19 @@
 //
 //   router_decode    the product of small_gemv.cuh over a cluster of a CTA per 16 experts, whose first one routes
 //   moe_decode_up    act[pair, I] = silu(gate) * up for the experts in use; a tile is eight gate rows and their eight up rows,
-//                    whose sums meet before either is rounded
+//                    whose sums, rounded to bf16, meet in the epilogue
 //   moe_decode_down  y[t] = residual[t] + sum over the token's experts of w * W2[e] act[pair]
 //
 // Plan (int32): [0] experts in use; from [4] on 20 values for each of them, in the order of their ids: id, three unused, the
 // pair (token * top_k + choice) of each of the eight tokens or -1, the tokens' weights as fp32 bits.
 //
+// Sums run in the order, and are rounded where, the kernels of decode_stream.cu and moe_combine have it: the values are theirs bit for bit,
+// and a row's do not depend on the other rows of the step.
+//
 // Measured, us in a captured chain over 128 experts of 768 x 2048, against six launches (product, routing, up, down with SwiGLU,
-// combination; one CTA per SM with items of 64 KB): 1 token 31.7 -> 25.4, 2 tokens 50.9 -> 37.0, 4 tokens 71.6 -> 53.7, 8 tokens
-// 107 -> 87.5. Alone, for 8 and 64 experts in use: up 15.2 -> 11.3 and 72.8 -> 62.6 (their bytes at 6.5 TB/s: 7.7 and 62), down
-// and combination 11.6 -> 8.7 and 44 -> 34.4 (3.9 and 31).
+// combination; one CTA per SM with items of 64 KB): 1 token 31.7 -> 26.4, 2 tokens 50.9 -> 37.6, 4 tokens 71.6 -> 57.7, 8 tokens
+// 107 -> 87.8. Alone, 1 and 8 tokens (8 and some 52 experts): up 12.0 and 54.2 (their bytes at 6.5 TB/s: 7.7 and 50), down and
+// combination 8.9 and 28.4 (3.9 and 25).
 //
 // Experts too many or too wide for this (`moe_decode_fits`) take decode_small.cu and decode_stream.cu.
 //
@@ -48,6 +51,7 @@ constexpr int THREADS = 32 * (1 + CWARPS);
 constexpr int RING = 100 * 1024;    // of one of two CTAs on an SM
 constexpr int RING_ALONE = 200 * 1024;
 constexpr int MAX_STAGES = 6;
+constexpr int MAX_REGS = 112;       // of a thread: two CTAs on an SM
 
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
@@ -62,6 +66,16 @@ __device__ __forceinline__ uint4 lds16(uint32_t addr) {
 __device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, %0;" ::"n"(32 * CWARPS) : "memory"); }
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The first CTA's counterpart of an address in this CTA's shared memory, and stores to it.
+__device__ __forceinline__ uint32_t of_first(const void* local) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(local)), "r"(0u));
+  return a;
+}
+__device__ __forceinline__ void st_cluster(uint32_t addr, float v) { asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
+__device__ __forceinline__ void st_cluster(uint32_t addr, bf16 v) {
+  asm volatile("st.shared::cluster.u16 [%0], %1;" ::"r"(addr), "h"(__bfloat16_as_ushort(v)) : "memory");
 }
 // Copies in flight get a bounded chance to land before shared memory is released.
 __device__ __forceinline__ void let_copies_land() {
@@ -187,11 +201,7 @@ router_decode_kernel(const bf16* __restrict__ x, int T, const bf16* __restrict__
                      int renorm, int* __restrict__ topk_ids, float* __restrict__ topk_w, int* __restrict__ plan) {
   __shared__ float lg[TOK * MAX_E];
   cluster_sync();  // (all CTAs run before one stores into another's shared memory; the predecessor is still busy)
-  gemv_tile<true>(x, T, g, eps, W, H, [&](int t, int n, float v) {  // to the first CTA's copy
-    uint32_t a;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(lg + t * E + n)), "r"(0u));
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
-  });
+  gemv_tile<true>(x, T, g, eps, W, H, [&](int t, int n, float v) { st_cluster(of_first(lg + t * E + n), v); });
   cluster_sync();
   if (blockIdx.x == 0) route(lg, T, E, K, renorm, topk_ids, topk_w, plan);
 }
@@ -208,14 +218,19 @@ struct UpArgs {
   int* status;
 };
 
-constexpr int UP_CHUNKS = 4;  // 32-wide k chunks of a warp in a stage
+constexpr int UP_STAGE = 4;  // 256-wide k slices in a stage
 
-// NCH: 32-wide chunks per warp, K = NCH * 256. Items are (expert, eight columns of I), in contiguous runs.
+// K = NCH * 256. Items are (expert, eight columns of I), in contiguous runs. A warp sums the slice of k that a warp of
+// decode_stream.cu sums (`SL` 32-wide chunks of every 2048), in its order, so the values are the same. A stage holds whole slices: of a
+// contraction of several stages the first four warps multiply one, the other four the next (and all wait for every stage: a warp that
+// left one out could take the phase before the last for the one that it waits for).
 template <int NCH>
-__global__ void __launch_bounds__(THREADS) moe_up_kernel(const UpArgs a) {
+__global__ void __maxnreg__(MAX_REGS) moe_up_kernel(const UpArgs a) {
   constexpr int K = NCH * 256;
-  constexpr int CS = NCH < UP_CHUNKS ? NCH : UP_CHUNKS;
+  constexpr int CS = NCH < UP_STAGE ? NCH : UP_STAGE;
   constexpr int PARTS = (NCH + CS - 1) / CS;
+  constexpr int LAST = NCH - (PARTS - 1) * CS;  // slices of the last stage
+  constexpr int SL = PARTS == 1 ? NCH : 8, BLOCKS = (NCH + 7) / 8;
   constexpr int PITCH = CS * 512 + 64;  // (skewed: a warp's sixteen-byte reads touch every bank once)
   constexpr int STAGE = ROWS * PITCH;
   extern __shared__ uint8_t smem_raw[];
@@ -267,7 +282,6 @@ __global__ void __launch_bounds__(THREADS) moe_up_kernel(const UpArgs a) {
       const bf16* src = a.W + row * K;
 #pragma unroll
       for (int p = 0; p < PARTS; ++p) {
-        constexpr int LAST = NCH - (PARTS - 1) * CS;
         const uint32_t bytes = (p == PARTS - 1 ? LAST : CS) * 512u;
         ok = __all_sync(0xffffffffu, ok && mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, a.status, ERR_WAIT_EMPTY));
         if (!ok) break;
@@ -286,15 +300,14 @@ __global__ void __launch_bounds__(THREADS) moe_up_kernel(const UpArgs a) {
     // ------------------------------------------------------------------ consumers
     const int cw = warp - 1, ct = threadIdx.x - 32;
     const int r = lane >> 2, c = lane & 3;
-    // this lane's share of its token's row, scaled by the norm's weights; in a stage of n chunks per warp, warp w has chunks
-    // w * n .. w * n + n - 1
-    uint4 xa[NCH];
+    // this lane's share of its token's row, scaled by the norm's weights
+    uint4 xa[BLOCKS * SL];
     float ss = 0.f;
 #pragma unroll
-    for (int u = 0; u < NCH; ++u) {
-      constexpr int LAST = NCH - (PARTS - 1) * CS;
-      const int p = u / CS, n = p == PARTS - 1 ? LAST : CS;
-      xa[u] = load_act<true>(a.x + static_cast<long long>(r) * K, a.norm_w, p * CS * 256 + (cw * n + u - p * CS) * 32 + c * 8, r < a.T, ss);
+    for (int u = 0; u < BLOCKS * SL; ++u) {
+      const int k = u / SL * 2048 + (cw * SL + u % SL) * 32;
+      xa[u] = make_uint4(0u, 0u, 0u, 0u);
+      if (k < K) xa[u] = load_act<true>(a.x + static_cast<long long>(r) * K, a.norm_w, k + c * 8, r < a.T, ss);  // (warp-uniform)
     }
     int begin, end;
     run(begin, end);
@@ -311,18 +324,18 @@ __global__ void __launch_bounds__(THREADS) moe_up_kernel(const UpArgs a) {
       float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int p = 0; p < PARTS; ++p) {
-        constexpr int LAST = NCH - (PARTS - 1) * CS;
-        const int n = p == PARTS - 1 ? LAST : CS;
+        const int slice = PARTS == 1 ? cw : cw & 3;
         ok = ok && mbar_wait(full_bar(stage), phase, abort_flag, a.status, ERR_WAIT_FULL);
         if (ok) {
-          const uint32_t sa = base + stage * STAGE + r * PITCH + (cw * n * 32 + c * 8) * 2, sb = sa + 8 * PITCH;
+          if (PARTS == 1 || ((p & 1) == cw >> 2 && slice < (p == PARTS - 1 ? LAST : CS))) {  // (this warp's)
+            const uint32_t sa = base + stage * STAGE + r * PITCH + (slice * SL * 32 + c * 8) * 2, sb = sa + 8 * PITCH;
 #pragma unroll
-          for (int u = 0; u < CS; ++u)
-            if (u < n) {
-              const uint4 w0 = lds16(sa + u * 64), w1 = lds16(sb + u * 64), xv = xa[p * CS + u < NCH ? p * CS + u : 0];
+            for (int u = 0; u < SL; ++u) {
+              const uint4 w0 = lds16(sa + u * 64), w1 = lds16(sb + u * 64), xv = xa[p / 2 * SL + u];
               mma16816(acc, w0.x, w1.x, w0.y, w1.y, xv.x, xv.y);
               mma16816(acc, w0.z, w1.z, w0.w, w1.w, xv.z, xv.w);
             }
+          }
           __syncwarp();
           if (lane == 0) mbar_arrive(empty_bar(stage));
         }
@@ -343,7 +356,7 @@ __global__ void __launch_bounds__(THREADS) moe_up_kernel(const UpArgs a) {
         float v = 0.f;
 #pragma unroll
         for (int w = 0; w < CWARPS; ++w) v += red[par][w][ei + 8 * eh][ej];
-        v *= rs;
+        v = __bfloat162float(__float2bfloat16(v * rs));  // gate and up are bf16 everywhere else, too
         const float up = __shfl_xor_sync(0xffffffffu, v, 8);
         if (ok && eh == 0 && pair >= 0) a.out[static_cast<long long>(pair) * a.I + t * 8 + ei] = __float2bfloat16(v / (1.f + __expf(-v)) * up);
       }
@@ -357,28 +370,31 @@ __global__ void __launch_bounds__(THREADS) moe_up_kernel(const UpArgs a) {
 }
 
 // ---------------------------------------------------------------------------------------------- down
-// A CTA owns 16 rows of the output, for all tokens, and walks over the experts in use (a cluster of two deals them out alternately
-// and adds its two sums in rank order); an expert's tile is one contiguous copy. Each expert's product is added to the running
-// sums with the tokens' weights in fp32, so the eight k slices of the warps meet once, at the end. A lane's activations of the
-// next expert are asked for while it multiplies this one.
+// A CTA owns 16 rows of the output, for all tokens, and walks over the experts in use (a cluster of two deals them out alternately);
+// an expert's tile is one contiguous copy. Its product, summed over the warps' k slices (those of decode_stream.cu) and rounded to bf16,
+// waits in the first CTA's shared memory for the end, where a token's pairs are added in the order of its choices: neither the other tokens'
+// experts nor the CTA that had an expert show in a sum, and the values are those of a product per pair and `moe_combine`. A lane's
+// activations of the next expert are asked for while it multiplies this one.
 struct DownArgs {
   const bf16* W;         // [E, H, I]
   const bf16* act;       // [pairs, I]
   const int* plan;
   const bf16* residual;  // [T, H]
   bf16* out;             // [T, H]
-  int T, E, H, I, stages;
+  int T, K, E, H, I, stages;
   int* status;
 };
 
-// CPW: 32-wide k chunks per warp (the last warps of a width that is not a multiple of 8 * 32 have fewer).
+constexpr int MAX_PAIRS = TOK * 32;
+
+// CPW: 32-wide k chunks of a warp: contiguous up to four, else eight of every 2048 (warps behind the end of k have fewer).
 template <int CPW>
-__global__ void __launch_bounds__(THREADS) moe_down_kernel(const DownArgs a) {
+__global__ void __maxnreg__(MAX_REGS) moe_down_kernel(const DownArgs a) {
+  constexpr int SL = CPW <= 4 ? CPW : 8;
   extern __shared__ uint8_t smem_raw[];
-  __shared__ float red[CWARPS][ROWS][TOK];
-  __shared__ float sum_s[TOK][ROWS];
-  __shared__ int pair_s[MAX_E][TOK];  // [expert of this CTA][token] -> pair, or -1
-  __shared__ float w_s[MAX_E][TOK];
+  __shared__ float red[2][CWARPS][ROWS][TOK];
+  __shared__ short pair_s[MAX_E][TOK];  // [expert of this CTA][token] -> pair, or -1
+  __shared__ float w_s[MAX_PAIRS];      // the pairs' weights (the first CTA's copy is used, as with their products)
   __shared__ __align__(8) unsigned long long bars[2 * MAX_STAGES];
   __shared__ int abort_s;
   volatile int* abort_flag = &abort_s;
@@ -386,7 +402,8 @@ __global__ void __launch_bounds__(THREADS) moe_down_kernel(const DownArgs a) {
   const uint32_t bar0 = smem_u32(bars);
   auto full_bar = [&](int s) { return bar0 + 8u * s; };
   auto empty_bar = [&](int s) { return bar0 + 8u * (MAX_STAGES + s); };
-  const int pitch = a.I * 2, stage_bytes = ROWS * pitch;
+  const int pitch = a.I * 2, stage_bytes = ROWS * pitch, pairs = a.T * a.K;
+  bf16* y_s = reinterpret_cast<bf16*>(smem_raw + (base - smem_u32(smem_raw)) + a.stages * stage_bytes);  // [pairs][ROWS]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     abort_s = 0;
@@ -396,7 +413,11 @@ __global__ void __launch_bounds__(THREADS) moe_down_kernel(const DownArgs a) {
     }
     fence_barrier_init();
   }
-  __syncthreads();
+  for (int i = threadIdx.x; i < pairs; i += THREADS) {  // (a choice without an expert adds nothing)
+    w_s[i] = 0.f;
+    reinterpret_cast<uint4*>(y_s)[2 * i] = reinterpret_cast<uint4*>(y_s)[2 * i + 1] = make_uint4(0u, 0u, 0u, 0u);
+  }
+  cluster_sync();  // (the other CTA runs before one stores into its shared memory; the predecessor is still busy)
   pdl_enter();
   const int rank = blockIdx.x, ranks = gridDim.x;  // (the cluster spans the grid's first dimension)
   const int row0 = blockIdx.y * ROWS;
@@ -433,37 +454,39 @@ __global__ void __launch_bounds__(THREADS) moe_down_kernel(const DownArgs a) {
     // ------------------------------------------------------------------ consumers
     const int cw = warp - 1, ct = threadIdx.x - 32;
     const int r = lane >> 2, c = lane & 3;
-    for (int i = ct; rank + i / TOK * ranks < a.E; i += 32 * CWARPS) {  // (records behind the last one are not used)
-      const int* rec = a.plan + PLAN_HEAD + (rank + i / TOK * ranks) * PLAN_REC;
-      pair_s[i / TOK][i % TOK] = rec[REC_PAIR + i % TOK];
-      w_s[i / TOK][i % TOK] = __int_as_float(rec[REC_W + i % TOK]);
-    }
     const int n = min(a.plan[0], a.E);
     const int mine = n > rank ? (n - rank + ranks - 1) / ranks : 0;
+    for (int i = ct; rank + i / TOK * ranks < a.E; i += 32 * CWARPS) {  // (records behind the last one are not used)
+      const int* rec = a.plan + PLAN_HEAD + (rank + i / TOK * ranks) * PLAN_REC;
+      const int pair = rec[REC_PAIR + i % TOK];
+      const float w = __int_as_float(rec[REC_W + i % TOK]);
+      const bool has = i / TOK < mine && pair >= 0 && pair < pairs;
+      pair_s[i / TOK][i % TOK] = static_cast<short>(has ? pair : -1);
+      if (has) st_cluster(of_first(w_s + pair), w);
+    }
     consumer_sync();
-    const int k0 = cw * CPW * 32 + c * 8;  // first k of this lane; chunks that lie beyond I are skipped (warp-uniform)
+    const auto k_of = [&](int u) { return u / SL * 2048 + (cw * SL + u % SL) * 32; };  // chunks that lie beyond I are skipped (warp-uniform)
     auto load = [&](int i, uint4 (&x)[CPW]) {
       const int pair = pair_s[i][r];
 #pragma unroll
       for (int u = 0; u < CPW; ++u) {
         x[u] = make_uint4(0u, 0u, 0u, 0u);
-        if (pair >= 0 && k0 + u * 32 < a.I) x[u] = ldg16(a.act + static_cast<long long>(pair) * a.I + k0 + u * 32);
+        if (pair >= 0 && k_of(u) < a.I) x[u] = ldg16(a.act + static_cast<long long>(pair) * a.I + k_of(u) + c * 8);
       }
     };
-    float y[4] = {0.f, 0.f, 0.f, 0.f};
     uint4 xa[CPW], xn[CPW];
     if (mine > 0) load(0, xa);
     bool ok = true;
-    for (int i = 0; ok && i < mine; ++i) {
+    for (int i = 0; i < mine; ++i) {
       if (i + 1 < mine) load(i + 1, xn);
       float acc[4] = {0.f, 0.f, 0.f, 0.f};
-      ok = mbar_wait(full_bar(stage), phase, abort_flag, a.status, ERR_WAIT_FULL);
+      ok = ok && mbar_wait(full_bar(stage), phase, abort_flag, a.status, ERR_WAIT_FULL);
       if (ok) {
-        const uint32_t sa = base + stage * stage_bytes + r * pitch + k0 * 2, sb = sa + 8 * pitch;
+        const uint32_t sa = base + stage * stage_bytes + r * pitch + c * 16, sb = sa + 8 * pitch;
 #pragma unroll
         for (int u = 0; u < CPW; ++u) {
-          if (k0 - c * 8 + u * 32 < a.I) {  // warp-uniform
-            const uint4 w0 = lds16(sa + u * 64), w1 = lds16(sb + u * 64);
+          if (k_of(u) < a.I) {
+            const uint4 w0 = lds16(sa + k_of(u) * 2), w1 = lds16(sb + k_of(u) * 2);
             mma16816(acc, w0.x, w1.x, w0.y, w1.y, xa[u].x, xa[u].y);
             mma16816(acc, w0.z, w1.z, w0.w, w1.w, xa[u].z, xa[u].w);
           }
@@ -471,46 +494,43 @@ __global__ void __launch_bounds__(THREADS) moe_down_kernel(const DownArgs a) {
         __syncwarp();
         if (lane == 0) mbar_arrive(empty_bar(stage));
       }
+      float(&part)[CWARPS][ROWS][TOK] = red[i & 1];
+      part[cw][r][2 * c] = acc[0];
+      part[cw][r][2 * c + 1] = acc[1];
+      part[cw][r + 8][2 * c] = acc[2];
+      part[cw][r + 8][2 * c + 1] = acc[3];
+      consumer_sync();
+      if (ct >> 7 == (i & 1)) {  // half of the threads sum an expert's slices, the other half the next one's (the buffers alternate, too)
+        const int row = (ct & 127) >> 3, t = ct & 7, pair = pair_s[i][t];
+        float v = 0.f;
 #pragma unroll
-      for (int h = 0; h < 2; ++h)
-        if (pair_s[i][2 * c + h] >= 0) {  // (a column of zeros against infinite weights is no number)
-          const float w = w_s[i][2 * c + h];
-          y[h] += w * acc[h];
-          y[2 + h] += w * acc[2 + h];
-        }
+        for (int w = 0; w < CWARPS; ++w) v += part[w][row][t];
+        if (ok && pair >= 0) st_cluster(of_first(y_s + pair * ROWS + row), __float2bfloat16(v));
+      }
 #pragma unroll
       for (int u = 0; u < CPW; ++u) xa[u] = xn[u];
       advance();
-    }
-    red[cw][r][2 * c] = y[0];
-    red[cw][r][2 * c + 1] = y[1];
-    red[cw][r + 8][2 * c] = y[2];
-    red[cw][r + 8][2 * c + 1] = y[3];
-    consumer_sync();
-    if (ct < ROWS * TOK) {
-      const int t = ct / ROWS, row = ct % ROWS;
-      float v = 0.f;
-#pragma unroll
-      for (int w = 0; w < CWARPS; ++w) v += red[w][row][t];
-      sum_s[t][row] = v;
     }
   }
   // every thread of every CTA of the cluster arrives, whatever happened before
   __syncthreads();
   cluster_sync();
   if (writes) {
-    float v = sum_s[ot][orow];
-    if (ranks > 1) {
-      uint32_t remote;
-      float o;
-      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(&sum_s[ot][orow])), "r"(1u));
-      asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(o) : "r"(remote) : "memory");
-      v += o;
+    float v = res + 0.f;
+    for (int k0 = 0; k0 < a.K; k0 += 8) {
+      float w[8], y[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int pair = ot * a.K + min(k0 + k, a.K - 1);
+        w[k] = w_s[pair];
+        y[k] = __bfloat162float(y_s[pair * ROWS + orow]);
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (k0 + k < a.K) v = fmaf(w[k], y[k], v);
     }
-    a.out[at] = __float2bfloat16(res + v);
+    a.out[at] = __float2bfloat16(v);
   }
-  __syncwarp();
-  cluster_sync();  // no CTA leaves while another still reads its shared memory
 }
 
 // ---------------------------------------------------------------------------------------------- host side
@@ -535,7 +555,7 @@ cudaError_t launch_cluster(void (*kernel)(P...), dim3 grid, int threads, size_t 
 
 template <int NCH>
 cudaError_t launch_up(UpArgs a, int max_active, cudaStream_t s) {
-  constexpr int CS = NCH < UP_CHUNKS ? NCH : UP_CHUNKS;
+  constexpr int CS = NCH < UP_STAGE ? NCH : UP_STAGE;
   constexpr int STAGE = ROWS * (CS * 512 + 64);
   a.stages = RING / STAGE < MAX_STAGES ? RING / STAGE : MAX_STAGES;
   const int smem = a.stages * STAGE + 128;
@@ -548,11 +568,11 @@ cudaError_t launch_up(UpArgs a, int max_active, cudaStream_t s) {
 
 template <int CPW>
 cudaError_t launch_down(DownArgs a, cudaStream_t s) {
-  const int stage = ROWS * a.I * 2;
-  const bool two = 3 * stage <= RING;  // CTAs on an SM
-  a.stages = (two ? RING : RING_ALONE) / stage;
+  const int stage = ROWS * a.I * 2, outs = a.T * a.K * ROWS * 2;
+  const bool two = 3 * stage + outs <= RING;  // CTAs on an SM
+  a.stages = ((two ? RING : RING_ALONE) - outs) / stage;
   if (a.stages > MAX_STAGES) a.stages = MAX_STAGES;
-  const int smem = a.stages * stage + 128;
+  const int smem = a.stages * stage + outs + 128;
   auto kern = moe_down_kernel<CPW>;
   const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
@@ -609,7 +629,7 @@ int moe_decode_up(const void* x, int T, const void* norm_w, float eps, const voi
   return gemm_fail("moe_decode_up: unsupported width");
 }
 
-int moe_decode_down(const void* act, const void* W2, const int* plan, const void* residual, int T, int E, int H, int I, void* y, int* status,
+int moe_decode_down(const void* act, const void* W2, const int* plan, const void* residual, int T, int K, int E, int H, int I, void* y, int* status,
                     cudaStream_t s) {
   DownArgs a = {};
   a.W = static_cast<const bf16*>(W2);
@@ -618,14 +638,16 @@ int moe_decode_down(const void* act, const void* W2, const int* plan, const void
   a.residual = static_cast<const bf16*>(residual);
   a.out = static_cast<bf16*>(y);
   a.T = T;
+  a.K = K;
   a.E = E;
   a.H = H;
   a.I = I;
   a.status = status;
 #define MB_DOWN(N) \
   case N: return launched(launch_down<N>(a, s), "moe_decode_down")
-  switch ((I / 32 + CWARPS - 1) / CWARPS) {
-    MB_DOWN(1); MB_DOWN(2); MB_DOWN(3); MB_DOWN(4); MB_DOWN(5); MB_DOWN(6); MB_DOWN(7); MB_DOWN(8); MB_DOWN(9);
+  // chunks of a warp as launch_stream of decode_stream.cu deals them
+  switch (I % 256 == 0 && I <= 1024 ? I / 256 : I <= 2048 ? 8 : 10) {
+    MB_DOWN(1); MB_DOWN(2); MB_DOWN(3); MB_DOWN(4); MB_DOWN(8); MB_DOWN(10);
   }
 #undef MB_DOWN
   return gemm_fail("moe_decode_down: unsupported width");

@@ -146,7 +146,7 @@ int router_decode(const void* x, int T, const void* norm_w, float eps, const voi
                   float* topk_w, int* plan, cudaStream_t s);
 int moe_decode_up(const void* x, int T, const void* norm_w, float eps, const void* W1, const int* plan, int max_active, int E, int H, int I,
                   void* act, int* status, cudaStream_t s);
-int moe_decode_down(const void* act, const void* W2, const int* plan, const void* residual, int T, int E, int H, int I, void* y, int* status,
+int moe_decode_down(const void* act, const void* W2, const int* plan, const void* residual, int T, int K, int E, int H, int I, void* y, int* status,
                     cudaStream_t s);
 
 // ---- rl.cu

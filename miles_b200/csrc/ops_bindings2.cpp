@@ -200,7 +200,7 @@ void moe_decode_down(const at::Tensor& act, const at::Tensor& W2, const at::Tens
   TORCH_CHECK(W2.dim() == 3 && T >= 1 && T <= 8 && pairs % T == 0 && W2.size(2) == I && y.size(1) == H && residual.numel() == y.numel() &&
                   plan.numel() >= mb::moe_decode_plan_size(E) && mb::moe_decode_fits(E, pairs / T, H, I), "moe_decode_down: unsupported shape");
   const c10::cuda::CUDAGuard guard(act.device());
-  const int rc = mb::moe_decode_down(act.data_ptr(), W2.data_ptr(), plan.data_ptr<int>(), residual.data_ptr(), T, E, H, I, y.data_ptr(),
+  const int rc = mb::moe_decode_down(act.data_ptr(), W2.data_ptr(), plan.data_ptr<int>(), residual.data_ptr(), T, pairs / T, E, H, I, y.data_ptr(),
                                      status.has_value() ? status->data_ptr<int>() : nullptr, cur_stream());
   TORCH_CHECK(rc == 0, mb::gemm_last_error());
 }

@@ -31,7 +31,7 @@ def _same_plan(a, b, T):
 # per tile, few and all experts, one expert per token, more choices than lanes in a half-warp
 @pytest.mark.parametrize("T, E, K, H, I", [(1, 128, 8, 2048, 768), (8, 128, 8, 2048, 768), (3, 16, 2, 512, 96), (8, 16, 16, 1024, 256),
                                            (5, 32, 4, 4096, 1024), (2, 16, 2, 2560, 2112), (7, 48, 1, 256, 32), (4, 128, 8, 1792, 1408),
-                                           (8, 112, 32, 768, 512)])
+                                           (8, 112, 32, 768, 512), (6, 32, 4, 1280, 800), (8, 16, 4, 2816, 2048), (8, 48, 32, 1024, 2112)])
 def test_fused_decode_experts(T, E, K, H, I):
     from miles_b200.ops import _ext
 
@@ -65,11 +65,26 @@ def test_fused_decode_experts(T, E, K, H, I):
     assert err <= 1.02 * err2 and err < 6e-3
     y = torch.empty(T, H, device=DEV).bfloat16()
     C.moe_decode_down(act, W2, plan, x, y, st)
-    assert st.item() == 0
     yp = torch.einsum("pi,phi->ph", act.double(), W2[ids.flatten().long()].double()).view(T, K, H)
     want = x.double() + (w.double()[..., None] * yp).sum(1)
-    # fp32 sums of I * K terms (2^-24 of their size each) and one rounding to bf16
-    assert ((y.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-4 * want.abs().mean()).all()
+    # fp32 sums of I * K terms (2^-24 of their size each), every pair rounded to bf16 and the sum once more: half a unit in the last of eight
+    # bits is at most 2^-8 of a value (and 2^-8 of the pairs' share of the sum)
+    pairs = (w.double()[..., None] * yp).abs().sum(1)
+    assert ((y.double() - want).abs() <= 2 ** -8 * (want.abs() + 1.01 * pairs) + 1e-4 * want.abs().mean()).all()
+    # the unfused kernels, bit for bit
+    yp2 = torch.empty(T * K, H, device=DEV).bfloat16()
+    C.moe_small_down(gu, W2, active, pc, pl, min(E, T * K), yp2, st)
+    y2 = C.moe_combine(yp2, torch.arange(T * K, **i32), w, T, K, x)
+    assert torch.equal(act, C.swiglu_fwd(gu)) and torch.equal(y, y2)
+    # and every row what it is alone: neither the others' experts nor its place among the rows shows
+    for t in range(T):
+        one, i1, w1 = torch.empty(1, H, device=DEV).bfloat16(), torch.empty(1, K, **i32), torch.empty(1, K, device=DEV)
+        a1 = torch.empty(K, I, device=DEV).bfloat16()
+        C.router_decode(x[t:t + 1], nw, 1e-6, Wr, True, i1, w1, plan)
+        C.moe_decode_up(x[t:t + 1], nw, 1e-6, W1, plan, a1, st)
+        C.moe_decode_down(a1, W2, plan, x[t:t + 1], one, st)
+        assert torch.equal(i1[0], ids[t]) and torch.equal(w1[0], w[t]) and torch.equal(one[0], y[t])
+    assert st.item() == 0
 
 
 def test_router_ties_and_values_that_cannot_be_chosen():
