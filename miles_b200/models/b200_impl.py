@@ -194,8 +194,9 @@ class B200Qwen3:
 
     def linear(self, x, w, out_dtype=torch.bfloat16, serving=False):
         """``x @ w^T``. In passes that train or score, every sum over K of 33 rows and more runs in one order, so that a sample's
-        log-probs and gradients do not depend on how much else is in its pack. Passes of the engine (``serving``) may split
-        the contraction of up to 128 rows over a cluster (csrc/gemm_skinny.cu)."""
+        log-probs do not depend on how much else is in its pack. (Gradients do, in their last bits: those of the weights add up the pack, dQ is
+        summed by atomics, and who adds up the heads of dK and dV is chosen by the pack's lengths, ops/attention.py.) Passes of the
+        engine (``serving``) may split the contraction of up to 128 rows over a cluster (csrc/gemm_skinny.cu)."""
         T, (N, K) = x.shape[0], w.shape
         mx = getattr(self, "mx", None)
         if mx and T > 32 and out_dtype == torch.bfloat16 and w.data_ptr() in mx:
@@ -879,15 +880,23 @@ class B200Qwen3:
     def logits(self, hidden_rows, out_dtype=torch.float32, serving=True):
         return self.linear(hidden_rows.contiguous(), self.store.lm_head(), out_dtype, serving)
 
+    # From this many rows of the head on the scores leave with its product (csrc/gemm.cu). The two ways add a row's exponentials in different
+    # orders, so the vocabulary alone decides: how many rows a pass has, scores at a time or keeps must not show in a row's score. us for
+    # logits and kernel / fused, 2048 columns: 32000 rows with 8 tokens 50 / 50, 33 52 / 46, 512 89 / 75, 8192 1125 / 751; 4096 rows
+    # with one token 26 / 40, 129 32 / 40, 512 38 / 38, 8192 241 / 144; 151936 rows with one token 254 / 216.
+    SCORE_VOCAB = 32000
+
+    def _fused_scores(self, vocab: int) -> bool:
+        return vocab >= self.SCORE_VOCAB and type(self).logits is B200Qwen3.logits
+
     @torch.no_grad()
     def logprobs_entropy(self, hidden_rows, targets, inv_temp: float, chunk: int = 0, keep_stats: bool = False, keep_logits: Optional[list] = None):
         C = self.C
         chunk = chunk or self.lm_chunk
         n, W = hidden_rows.shape[0], self.store.lm_head()
         tg = targets.to(torch.int32).contiguous()
-        # The scores leave with the product (csrc/gemm.cu) where its tiles fill the device: no logits at all for more rows at a time,
-        # unless the backward keeps them.
-        fused = -(-min(n, chunk) // 128) * -(-W.shape[0] // 256) >= 148 and type(self).logits is B200Qwen3.logits
+        # no logits at all for more rows at a time, unless the backward keeps them
+        fused = self._fused_scores(W.shape[0])
         if fused and keep_logits is None:
             chunk = max(chunk, 16384)
         out = []

@@ -54,3 +54,26 @@ def test_no_rows_and_wide_scores():
     assert lp[0] == 0 and lse[0] == big and ent[0] == 0 and lp[1] == -2 * big and lse[1] == big
     assert abs(lse[2].item() - torch.log(torch.tensor(512.0)).item()) < 1e-5 and abs(ent[2].item() - lse[2].item()) < 1e-5
     assert all(t.numel() == 0 for t in C.score_rows(h[:0], w, tg[:0], 1.0, None, None))
+
+
+@pytest.mark.parametrize("vocab", [4096, 31992, 32000])
+def test_a_row_scores_the_same_in_any_company(vocab):
+    """However many rows there are, are scored at a time, or keep their logits. (Up to 32 rows, heads below SCORE_VOCAB take the
+    engine's products, whose sums are split.)"""
+    from miles_b200.models import ParamStore, build_model, get_config
+
+    cfg = get_config("qwen3-smoke")
+    cfg.vocab_size = vocab
+    model = build_model(cfg, ParamStore(cfg, torch.device(DEV), torch.bfloat16, init_std=0.05, seed=3), "b200")
+    g = torch.Generator(device=DEV).manual_seed(vocab)
+    h = torch.randn(3000, cfg.hidden_size, device=DEV, generator=g).bfloat16()
+    tg = torch.randint(0, vocab, (3000,), device=DEV, generator=g)
+    want = model.logprobs_entropy(h, tg, 1.0, keep_stats=True)
+    assert model._fused_scores(vocab) == (vocab == 32000)
+    for n in (33, 128, 129, 2048, 2999) + ((1, 8, 32) if vocab == 32000 else ()):
+        for kw in (dict(), dict(keep_logits=[]), dict(chunk=128), dict(chunk=128, keep_logits=[])):
+            if n % kw.get("chunk", 2048) in range(1, 33) and vocab < 32000:
+                continue
+            got = model.logprobs_entropy(h[:n], tg[:n], 1.0, keep_stats=True, **kw)
+            assert all(torch.equal(a, b[:n]) for a, b in zip(got, want)), (n, kw)
+    model.check_status()
