@@ -292,10 +292,14 @@ std::vector<at::Tensor> logprob_entropy_fwd(const at::Tensor& logits, const at::
 
 // Returns dlogits as bf16 [T, V]; for bf16 logits the result overwrites the input buffer.
 at::Tensor logprob_entropy_bwd(at::Tensor& logits, const at::Tensor& targets, const at::Tensor& lse, const at::Tensor& px,
-                               const c10::optional<at::Tensor>& dlp, const c10::optional<at::Tensor>& dent, double inv_temp) {
+                               const c10::optional<at::Tensor>& dlp, const c10::optional<at::Tensor>& dent, double inv_temp,
+                               const c10::optional<at::Tensor>& into) {
   const c10::cuda::CUDAGuard guard(logits.device());
   const bool fp32 = logits.scalar_type() == at::kFloat;
-  at::Tensor out = fp32 ? at::empty(logits.sizes(), logits.options().dtype(at::kBFloat16)) : logits;
+  if (into.has_value())
+    TORCH_CHECK(into->is_cuda() && into->scalar_type() == at::kBFloat16 && into->sizes() == logits.sizes() && into->stride(1) == 1,
+                "out must be bf16 of the logits' shape with contiguous rows");
+  at::Tensor out = into.has_value() ? *into : fp32 ? at::empty(logits.sizes(), logits.options().dtype(at::kBFloat16)) : logits;
   mb::logprob_entropy_bwd(logits.data_ptr(), fp32, targets.data_ptr<int>(), lse.data_ptr<float>(), px.data_ptr<float>(),
                           opt_ptr<float>(dlp), opt_ptr<float>(dent), out.data_ptr(), logits.size(0), logits.size(1),
                           logits.stride(0), out.stride(0), inv_temp, cur_stream());
@@ -331,6 +335,7 @@ void register_elementwise(pybind11::module_& m) {
         pybind11::arg("K"), pybind11::arg("residual") = c10::optional<at::Tensor>());
   m.def("moe_combine_bwd", &moe_combine_bwd);
   m.def("logprob_entropy_fwd", &logprob_entropy_fwd);
-  m.def("logprob_entropy_bwd", &logprob_entropy_bwd);
+  m.def("logprob_entropy_bwd", &logprob_entropy_bwd, pybind11::arg("logits"), pybind11::arg("targets"), pybind11::arg("lse"), pybind11::arg("px"),
+        pybind11::arg("dlp"), pybind11::arg("dent"), pybind11::arg("inv_temp"), pybind11::arg("out") = pybind11::none());
   register_more(m);
 }

@@ -714,14 +714,15 @@ class B200Qwen3:
         if (self.ep is not None or self.tp is not None or self.cp_ctx is not None or getattr(self.store, "begin_pass", None) is not None
                 or any(getattr(cls, f) is not getattr(B200Qwen3, f) for f in ("layer_forward", "layer_backward", "forward_hidden", "layers_backward"))):
             return False, hi
-        # logits, and the chunk of their gradients
-        head = (4 * head_rows + 2 * min(head_rows, self.KEPT_CHUNK * chunk)) * self.store.lm_head().shape[0] if head_rows else 0
+        head = 4 * head_rows * self.store.lm_head().shape[0] if head_rows else 0
         return plan_kept(self._room_for_acts(), head,
                          [self._layer_act_bytes(i, T) for i in range(lo, hi)], lo)
 
-    # Chunks of the LM head that go through the backward together where the logits are kept: each reads and writes the whole gradient of
-    # the head (151936 x 2048 in fp32: 12288 rows at the power cap 1014 TFLOP/s in chunks of 2048, 1240 in chunks of 8192).
-    KEPT_CHUNK = 4
+    # ``chunk`` rows of fp32 logits are what --log-probs-chunk-size lets the head hold at a time. In the same bytes are
+    #  - the bf16 gradients of twice as many rows, which therefore go through the head's gradient together, whether their logits were kept or
+    #    are recomputed chunk by chunk (each pass over that gradient, 151936 x 2048 in fp32, reads and writes 2.5 GB);
+    #  - what the fused product leaves of 32 times as many (16 bytes for 128 columns); more than 16384 rows gain nothing.
+    GRAD_CHUNKS, SCORE_CHUNKS, SCORE_ROWS = 2, 32, 16384
 
     def layer_backward(self, i, x, dy, positions, cu, max_seqlen, replay_ids=None, acts: Optional[LayerActs] = None):
         """Back-propagate ``dy`` through layer i, from the activations its forward kept or else recomputed from its input
@@ -889,16 +890,24 @@ class B200Qwen3:
     def _fused_scores(self, vocab: int) -> bool:
         return vocab >= self.SCORE_VOCAB and type(self).logits is B200Qwen3.logits
 
+    def _logits_again(self, hidden_rows, w, whole_k: bool):
+        """Logits for a backward that did not keep them: the values of the forward, which fused scores sum over whole rows of the head."""
+        if not whole_k:
+            return self.logits(hidden_rows, serving=False)
+        out = torch.empty(hidden_rows.shape[0], w.shape[0], dtype=torch.float32, device=hidden_rows.device)
+        self.C.gemm(hidden_rows, w, out, False, False, False, 0, self.status, whole_k=True)
+        self.launches += 1
+        return out
+
     @torch.no_grad()
     def logprobs_entropy(self, hidden_rows, targets, inv_temp: float, chunk: int = 0, keep_stats: bool = False, keep_logits: Optional[list] = None):
         C = self.C
         chunk = chunk or self.lm_chunk
         n, W = hidden_rows.shape[0], self.store.lm_head()
         tg = targets.to(torch.int32).contiguous()
-        # no logits at all for more rows at a time, unless the backward keeps them
         fused = self._fused_scores(W.shape[0])
-        if fused and keep_logits is None:
-            chunk = max(chunk, 16384)
+        if fused and keep_logits is None:  # no logits at all
+            chunk = max(chunk, min(self.SCORE_CHUNKS * chunk, self.SCORE_ROWS))
         out = []
         for a in range(0, n, chunk):
             b = min(a + chunk, n)
@@ -943,7 +952,6 @@ class B200Qwen3:
         hr = h[rows].contiguous()
         tg = targets.to(torch.int32).contiguous()
         kept: Optional[list] = [] if keep_head else None
-        chunk *= self.KEPT_CHUNK if keep_head else 1
         with torch.no_grad():
             lp, ent, lse, px = self.logprobs_entropy(hr, tg, inv_temp, chunk, keep_stats=True, keep_logits=kept)
         lp_leaf, ent_leaf = lp.detach().requires_grad_(True), ent.detach().requires_grad_(True)
@@ -957,16 +965,22 @@ class B200Qwen3:
             W = self.store.lm_head()
             gW = G["embed.weight"] if cfg.tie_embeddings else G["lm_head.weight"]
             dhr = torch.empty_like(hr)
-            for j, a in enumerate(range(0, hr.shape[0], chunk)):
-                b = min(a + chunk, hr.shape[0])
-                lg = kept[j] if kept is not None else self.logits(hr[a:b], serving=False)
-                dl = C.logprob_entropy_bwd(lg, tg[a:b], lse[a:b].contiguous(), px[a:b].contiguous(), dlp[a:b].contiguous(),
-                                           dent[a:b].contiguous() if dent is not None else None, inv_temp)
-                del lg
-                if kept is not None:
-                    kept[j] = None
-                self._gemm(dl, W, dhr[a:b], False, True)
-                self.linear_wgrad(dl, hr[a:b], gW)
-                self.launches += 1
+            whole_k = self._fused_scores(W.shape[0])
+            n, step = hr.shape[0], self.GRAD_CHUNKS * chunk
+            for g0 in range(0, n, step):
+                g1 = min(g0 + step, n)
+                dl = torch.empty(g1 - g0, W.shape[0], dtype=torch.bfloat16, device=hr.device)
+                for a in range(g0, g1, chunk):
+                    b = min(a + chunk, g1)
+                    lg = kept[a // chunk] if kept is not None else self._logits_again(hr[a:b], W, whole_k)
+                    C.logprob_entropy_bwd(lg, tg[a:b], lse[a:b].contiguous(), px[a:b].contiguous(), dlp[a:b].contiguous(),
+                                          dent[a:b].contiguous() if dent is not None else None, inv_temp, dl[a - g0:b - g0])
+                    del lg
+                    if kept is not None:
+                        kept[a // chunk] = None
+                    self.launches += 1
+                self._gemm(dl, W, dhr[g0:g1], False, True)
+                self.linear_wgrad(dl, hr[g0:g1], gW)
+                del dl
             self._trunk_backward(inputs, x_last, h, rows, dhr, tokens, positions, cu_seqlens, max_seqlen, replay, acts)
         return loss.detach(), metrics, lp.detach(), ent.detach()

@@ -50,3 +50,73 @@ def test_kept_activations_change_nothing(name):
         for n, g in grads.items():  # (dQ and the head norms are summed with atomics, whose order differs from run to run)
             want = out[0][3][n]
             assert (g - want).norm() <= 1e-2 * want.norm() + 1e-12, n
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name, vocab", [("qwen3-smoke", 4096), ("qwen3-smoke", 32000), ("qwen3-smoke-moe", 32000)])
+def test_head_in_chunks_does_not_depend_on_what_is_kept(name, vocab):
+    """Several chunks, a short last one (of few rows, which the engine's products would split), logits by either way: scores, and all
+    gradients that no atomic sum touches, are the same bit for bit whatever there was room for."""
+    from miles_b200.models import ParamStore, build_model, get_config
+    from test_b200_model import _batch
+
+    dev = torch.device("cuda")
+    cfg = get_config(name)
+    cfg.vocab_size, cfg.tie_embeddings = vocab, False  # (an embedding's gradient is an atomic sum)
+    store = ParamStore(cfg, dev, torch.bfloat16, init_std=0.05, seed=7)
+    store.allocate_grads(torch.float32)
+    model = build_model(cfg, store, "b200")
+    tokens, pos, cu, rows, tg = _batch(cfg, [200, 333, 75], dev)
+    rows, tg = rows[:64 * 6 + (9 if vocab == 32000 else 40)], tg[:64 * 6 + (9 if vocab == 32000 else 40)]
+    coef = torch.randn(rows.numel(), device=dev)
+    model.lm_chunk = 64
+    record = []
+    want = model.forward_logprobs(tokens, pos, cu, rows, tg, 1.0, record=record)
+    replay = torch.stack(record, 1) if record else None
+    last = f"layers.{cfg.num_layers - 1}."
+    exact = ["lm_head.weight", "final_norm.weight"] + [n for n in store.grads if n.startswith(last) and ("mlp." in n or "moe.w" in n)]
+    assert len(exact) >= 4
+    out = []
+    for room in (0, 4 * rows.numel() * vocab, 1 << 40):
+        model.act_room = room
+        assert model._plan_acts(tokens.numel(), rows.numel(), 64)[0] == (room > 0)
+        store.zero_grads()
+        loss, _, lp, ent = model.forward_backward(tokens, pos, cu, rows, tg, 1.0, lambda lp, ent: ((lp * coef).sum() / 50 + 0.01 * ent.sum(), {}),
+                                                  replay=replay)
+        model.check_status()
+        assert torch.equal(lp, want[0]) and torch.equal(ent, want[1])
+        out.append({n: store.grads[n].clone() for n in exact})
+    for grads in out[1:]:
+        for n, g in grads.items():
+            assert g.abs().max() > 0 and torch.equal(g, out[0][n]), n
+
+
+@pytest.mark.gpu
+def test_scores_keep_to_the_chunks_bytes():
+    """Scoring and differentiating hold what ``lm_chunk`` rows of fp32 logits take, and as much again for the logits' gradients."""
+    from miles_b200.models import ParamStore, build_model, get_config
+
+    dev = torch.device("cuda")
+    cfg = get_config("qwen3-smoke")
+    cfg.vocab_size, cfg.num_layers = 64000, 1
+    store = ParamStore(cfg, dev, torch.bfloat16, init_std=0.05, seed=7)
+    store.allocate_grads(torch.float32)
+    model = build_model(cfg, store, "b200")
+    n, model.lm_chunk, model.act_room = 8192, 128, 0
+    h = torch.randn(n, cfg.hidden_size, device=dev).bfloat16()
+    tokens, pos = torch.randint(0, cfg.vocab_size, (n,), device=dev).int(), torch.arange(n, device=dev).int()
+    chunk = 4 * model.lm_chunk * cfg.vocab_size
+
+    def peak(f):
+        f()
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        f()
+        return torch.cuda.max_memory_allocated() - before
+
+    rows = 64 * n * 4 + 4 * n * 2 * cfg.hidden_size  # statistics, and the hidden rows with their gradients
+    assert peak(lambda: model.logprobs_entropy(h, tokens, 1.0)) <= chunk + rows
+    one = torch.tensor([0, 1], dtype=torch.int32, device=dev)  # (one token, whose row is scored again and again: the head is nearly all there is)
+    assert peak(lambda: model.forward_backward(tokens[:1], pos[:1], one, torch.zeros(n, dtype=torch.int64, device=dev), tokens, 1.0,
+                                               lambda lp, ent: (lp.sum(), {}))) <= 2 * chunk + rows + (1 << 20)
