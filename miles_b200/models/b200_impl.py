@@ -68,6 +68,11 @@ def plan_kept(room: int, head_bytes: int, layer_bytes: list, first: int) -> tupl
     return head, keep
 
 
+def _out_of_memory(e: RuntimeError) -> bool:
+    """What the allocator raises, be it called by PyTorch or by the extension."""
+    return isinstance(e, torch.OutOfMemoryError) or "out of memory" in str(e)
+
+
 class B200Qwen3:
     def __init__(self, cfg: ModelConfig, store: ParamStore, ep=None, tp=None):
         assert cfg.head_dim == 128, "the sm_100a attention/rope kernels are specialised for head_dim 128"
@@ -691,19 +696,32 @@ class B200Qwen3:
         """Bytes of one layer's ``LayerActs`` over T tokens (matrices; the per-row statistics are a hundredth of them)."""
         cfg = self.cfg
         H, D = cfg.hidden_size, cfg.head_dim
-        cols = 3 * H + (3 * cfg.num_q_heads + 3 * cfg.num_kv_heads) * D  # h1, h2, x2; qkv and q, k; att
+        cols = 3 * H + (3 * cfg.num_q_heads + 3 * cfg.num_kv_heads) * D + (H if cfg.post_norms else 0)  # h1, h2, x2; qkv and q, k; att; post_attn
         if not cfg.layer_is_moe(i):
             return 2 * T * (cols + 3 * cfg.ffn_hidden_size)
         rows = T * cfg.moe_top_k + cfg.num_experts * 63
         return 2 * T * cols + 2 * rows * (2 * H + 3 * cfg.moe_ffn_hidden_size) + 4 * T * cfg.num_experts
 
-    def _room_for_acts(self) -> int:
-        """Bytes a training pass may hold on to: what the device and the allocator's cache have free beyond a seventh of the
-        device, the share that every part of this package that sizes itself by free memory leaves to activations."""
+    def _pass_bytes(self, T: int, head_rows: int, chunk: int) -> int:
+        """Bytes that a training pass holds whatever it keeps: the layers' inputs, the rows that are scored and their gradients, and the larger of
+        a chunk of the head (logits, and the gradients of GRAD_CHUNKS) and a layer on its way back (its activations recomputed, their
+        gradients, dQ in fp32; the shared expert's, which nobody keeps)."""
+        cfg = self.cfg
+        lo, hi = self.store.layer_range
+        H = cfg.hidden_size
+        layer = max((self._layer_act_bytes(i, T) for i in range(lo, hi)), default=0)
+        work = 2 * layer + 4 * T * cfg.num_q_heads * cfg.head_dim + 12 * T * cfg.shared_expert_ffn
+        head = (4 + 2 * self.GRAD_CHUNKS) * min(head_rows, chunk) * self.store.lm_head().shape[0] if head_rows else 0
+        return 2 * T * H * (hi - lo + 4) + 4 * head_rows * H + max(work, head)
+
+    def _room_for_acts(self, needed: int = 0) -> int:
+        """Bytes a training pass that needs ``needed`` anyway may hold on to: what the device and the allocator's cache have free beyond a seventh
+        of the device, the share that every part of this package that sizes itself by free memory leaves to activations, or beyond
+        what the pass needs and a fourth of that share (for pieces that do not fit together), whichever is more."""
         if self.act_room is not None:
             return self.act_room
         free, total = torch.cuda.mem_get_info(self.dev)
-        return free + torch.cuda.memory_reserved(self.dev) - torch.cuda.memory_allocated(self.dev) - total // 7
+        return free + torch.cuda.memory_reserved(self.dev) - torch.cuda.memory_allocated(self.dev) - max(total // 7, needed + total // 28)
 
     def _plan_acts(self, T: int, head_rows: int, chunk: int = 0) -> tuple[bool, int]:
         """(whether the logits are kept, first layer whose activations are). Where a pass exchanges data with other ranks
@@ -715,8 +733,21 @@ class B200Qwen3:
                 or any(getattr(cls, f) is not getattr(B200Qwen3, f) for f in ("layer_forward", "layer_backward", "forward_hidden", "layers_backward"))):
             return False, hi
         head = 4 * head_rows * self.store.lm_head().shape[0] if head_rows else 0
-        return plan_kept(self._room_for_acts(), head,
+        return plan_kept(self._room_for_acts(self._pass_bytes(T, head_rows, chunk)), head,
                          [self._layer_act_bytes(i, T) for i in range(lo, hi)], lo)
+
+    def _forward_keeping(self, keep_from: int, inputs: list, acts: dict, *args, **kw):
+        """``forward_hidden`` that keeps the layers' inputs, and the activations of the layers from ``keep_from`` on. Where memory runs out for
+        those after all (whoever shares the device may have taken some), it starts again and keeps none."""
+        if keep_from < self.store.layer_range[1]:
+            try:
+                return self.forward_hidden(*args, save_inputs=inputs, save_acts=acts, keep_from=keep_from, **kw)
+            except RuntimeError as e:
+                if not _out_of_memory(e):
+                    raise
+            inputs.clear()
+            acts.clear()
+        return self.forward_hidden(*args, save_inputs=inputs, **kw)
 
     # ``chunk`` rows of fp32 logits are what --log-probs-chunk-size lets the head hold at a time. In the same bytes are
     #  - the bf16 gradients of twice as many rows, which therefore go through the head's gradient together, whether their logits were kept or
@@ -866,8 +897,7 @@ class B200Qwen3:
         inputs: list = []
         acts: dict = {}
         keep_from = self._plan_acts(positions.shape[0], 0)[1]
-        keep = dict(save_acts=acts, keep_from=keep_from) if keep_from < self.store.layer_range[1] else {}
-        h = self.forward_hidden(tokens, positions, cu_seqlens, replay=replay, max_seqlen=max_seqlen, save_inputs=inputs, x_in=x_in, **keep)
+        h = self._forward_keeping(keep_from, inputs, acts, tokens, positions, cu_seqlens, replay=replay, max_seqlen=max_seqlen, x_in=x_in)
         x_last = inputs.pop()
         rows = row_index.long()
         leaf = h[rows].float().detach().requires_grad_(True)
@@ -945,15 +975,24 @@ class B200Qwen3:
         inputs: list[torch.Tensor] = []
         acts: dict = {}
         keep_head, keep_from = self._plan_acts(positions.shape[0], row_index.shape[0], chunk)
-        keep = dict(save_acts=acts, keep_from=keep_from) if keep_from < self.store.layer_range[1] else {}
-        h = self.forward_hidden(tokens, positions, cu_seqlens, replay=replay, max_seqlen=max_seqlen, save_inputs=inputs, x_in=x_in, **keep)
+        h = self._forward_keeping(keep_from, inputs, acts, tokens, positions, cu_seqlens, replay=replay, max_seqlen=max_seqlen, x_in=x_in)
         x_last = inputs.pop()  # input of the final norm
         rows = row_index.long()
         hr = h[rows].contiguous()
         tg = targets.to(torch.int32).contiguous()
         kept: Optional[list] = [] if keep_head else None
-        with torch.no_grad():
-            lp, ent, lse, px = self.logprobs_entropy(hr, tg, inv_temp, chunk, keep_stats=True, keep_logits=kept)
+        stats = None
+        if keep_head:
+            try:
+                stats = self.logprobs_entropy(hr, tg, inv_temp, chunk, keep_stats=True, keep_logits=kept)
+            except RuntimeError as e:
+                if not _out_of_memory(e):
+                    raise
+                kept.clear()
+        if stats is None:
+            kept = None
+            stats = self.logprobs_entropy(hr, tg, inv_temp, chunk, keep_stats=True)
+        lp, ent, lse, px = stats
         lp_leaf, ent_leaf = lp.detach().requires_grad_(True), ent.detach().requires_grad_(True)
         with torch.enable_grad():
             loss, metrics = loss_fn(lp_leaf, ent_leaf)

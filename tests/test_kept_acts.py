@@ -17,6 +17,38 @@ def test_plan_kept_without_head():
     assert plan_kept(100, 0, [], 3) == (False, 3)
 
 
+@pytest.mark.parametrize("name, tokens, free_gb", [("qwen3-8B", 2048, 150), ("qwen3-8B", 16384, 60), ("qwen3-8B", 98304, 150), ("qwen3-8B", 131072, 165),
+                                                   ("qwen3-4B", 98304, 100), ("qwen3-30B-A3B", 16384, 30), ("qwen3-30B-A3B", 65536, 100)])
+def test_what_is_kept_leaves_room_for_the_pass(monkeypatch, name, tokens, free_gb):
+    """Activations are kept only beyond what the pass needs anyway: the inputs of all layers, a layer on its way back, a chunk of the head."""
+    import types
+
+    from miles_b200.models import get_config
+    from miles_b200.models.b200_impl import B200Qwen3
+
+    cfg = get_config(name)
+    model = B200Qwen3.__new__(B200Qwen3)
+    head = types.SimpleNamespace(shape=(cfg.vocab_size, cfg.hidden_size))
+    model.__dict__.update(cfg=cfg, store=types.SimpleNamespace(layer_range=(0, cfg.num_layers), lm_head=lambda: head), ep=None, tp=None, cp_ctx=None,
+                          act_room=None, dev="cuda")
+    free, total, cached = int(free_gb * 1e9), int(192e9), int(5e9)
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda dev: (free - cached, total))
+    monkeypatch.setattr(torch.cuda, "memory_reserved", lambda dev: total - free + cached)
+    monkeypatch.setattr(torch.cuda, "memory_allocated", lambda dev: total - free)
+    head_rows, chunk = tokens * 3 // 4, 2048
+    keep_head, keep_from = model._plan_acts(tokens, head_rows, chunk)
+    layer = model._layer_act_bytes(0, tokens)
+    # written out again: inputs, hidden rows and gradients around them; recomputed activations and their gradients, or logits and dlogits
+    need = 2 * tokens * cfg.hidden_size * (cfg.num_layers + 1) + 4 * head_rows * cfg.hidden_size
+    work = max(2 * layer + 4 * tokens * cfg.num_q_heads * cfg.head_dim, 8 * chunk * cfg.vocab_size)
+    kept = (4 * head_rows * cfg.vocab_size if keep_head else 0) + (cfg.num_layers - keep_from) * layer
+    assert kept == 0 or kept + need + work + total // 28 <= free
+    assert kept <= max(0, free - total // 7)
+    if tokens <= 16384 and name == "qwen3-8B":  # (and room that is there is used)
+        assert kept > 0
+        assert keep_from == 0 or kept + layer > free - total // 7
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("name", ["qwen3-smoke", "qwen3-smoke-moe", "glm4moe-smoke", "glm4-smoke", "qwen2moe-smoke"])
 def test_kept_activations_change_nothing(name):
@@ -120,3 +152,45 @@ def test_scores_keep_to_the_chunks_bytes():
     one = torch.tensor([0, 1], dtype=torch.int32, device=dev)  # (one token, whose row is scored again and again: the head is nearly all there is)
     assert peak(lambda: model.forward_backward(tokens[:1], pos[:1], one, torch.zeros(n, dtype=torch.int64, device=dev), tokens, 1.0,
                                                lambda lp, ent: (lp.sum(), {}))) <= 2 * chunk + rows + (1 << 20)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("where", ["layer", "head"])
+def test_a_pass_that_runs_out_of_memory_keeps_nothing(monkeypatch, where):
+    from miles_b200.models import ParamStore, build_model, get_config
+    from test_b200_model import _batch
+
+    dev = torch.device("cuda")
+    cfg = get_config("qwen3-smoke")
+    store = ParamStore(cfg, dev, torch.bfloat16, init_std=0.05, seed=7)
+    store.allocate_grads(torch.float32)
+    model = build_model(cfg, store, "b200")
+    tokens, pos, cu, rows, tg = _batch(cfg, [200, 75], dev)
+    run = lambda: model.forward_backward(tokens, pos, cu, rows, tg, 1.0, lambda lp, ent: (lp.sum(), {}))  # noqa: E731
+    model.act_room = 0
+    store.zero_grads()
+    want = run()
+    exact = ["final_norm.weight", "lm_head.weight", f"layers.{cfg.num_layers - 1}.mlp.down.weight"]
+    grads = {n: store.grads[n].clone() for n in exact}
+    model.act_room, calls = 1 << 40, []
+    layer_acts, scores = model._layer_acts, model.logprobs_entropy
+
+    def short_layer(i, *a, output=False, **kw):
+        calls.append((i, output))
+        if output and i == 1:
+            raise torch.OutOfMemoryError("CUDA out of memory. Tried to allocate 1 GiB")
+        return layer_acts(i, *a, output=output, **kw)
+
+    def short_head(*a, keep_logits=None, **kw):
+        calls.append(keep_logits is not None)
+        if keep_logits is not None:
+            keep_logits.append(None)
+            raise RuntimeError("CUDA out of memory. Tried to allocate 1 GiB")
+        return scores(*a, **kw)
+
+    monkeypatch.setattr(model, *(("_layer_acts", short_layer) if where == "layer" else ("logprobs_entropy", short_head)))
+    store.zero_grads()
+    got = run()
+    assert calls == ([(0, True), (1, True), (1, False), (0, False)] if where == "layer" else [True, False])
+    assert torch.equal(got[0], want[0]) and torch.equal(got[2], want[2])
+    assert all(torch.equal(store.grads[n], g) for n, g in grads.items())
