@@ -68,6 +68,20 @@ def plan_kept(room: int, head_bytes: int, layer_bytes: list, first: int) -> tupl
     return head, keep
 
 
+ALL_LAYERS = 1 << 30
+
+
+def recompute_policy(args) -> tuple[int, bool]:
+    """(how many of a stage's first layers are recomputed in the backward whatever there is room for, whether the logits are):
+    ``--recompute-granularity full`` asks for all layers, or for --recompute-num-layers of them with ``--recompute-method block``;
+    without it, and with ``none`` and ``selective``, those are recomputed whose activations do not fit. ``--recompute-loss-function`` asks
+    for the logits."""
+    layers = 0
+    if getattr(args, "recompute_granularity", None) == "full":
+        layers = int(args.recompute_num_layers or 0) if getattr(args, "recompute_method", None) == "block" else ALL_LAYERS
+    return layers, bool(getattr(args, "recompute_loss_function", None))
+
+
 def _out_of_memory(e: RuntimeError) -> bool:
     """What the allocator raises, be it called by PyTorch or by the extension."""
     return isinstance(e, torch.OutOfMemoryError) or "out of memory" in str(e)
@@ -91,6 +105,8 @@ class B200Qwen3:
         self._ident: Optional[torch.Tensor] = None
         self.small_decode = True  # weight-streaming kernels for decode steps of at most SMALL_T rows
         self.act_room: Optional[int] = None  # bytes of activations a training pass may keep (None: by what is free, see _room_for_acts)
+        self.recompute_layers = 0     # of the stage's first layers no activations are kept, whatever there is room for (recompute_policy)
+        self.recompute_logits = False
         self.lm_chunk = 2048      # rows of the LM head per pass (--log-probs-chunk-size)
 
     def attention(self, q, k, v, cu):
@@ -732,9 +748,11 @@ class B200Qwen3:
         if (self.ep is not None or self.tp is not None or self.cp_ctx is not None or getattr(self.store, "begin_pass", None) is not None
                 or any(getattr(cls, f) is not getattr(B200Qwen3, f) for f in ("layer_forward", "layer_backward", "forward_hidden", "layers_backward"))):
             return False, hi
-        head = 4 * head_rows * self.store.lm_head().shape[0] if head_rows else 0
-        return plan_kept(self._room_for_acts(self._pass_bytes(T, head_rows, chunk)), head,
-                         [self._layer_act_bytes(i, T) for i in range(lo, hi)], lo)
+        head = 4 * head_rows * self.store.lm_head().shape[0] if head_rows and not self.recompute_logits else 0
+        first = min(lo + self.recompute_layers, hi)
+        if first == hi and not head:
+            return False, hi
+        return plan_kept(self._room_for_acts(self._pass_bytes(T, head_rows, chunk)), head, [self._layer_act_bytes(i, T) for i in range(first, hi)], first)
 
     def _forward_keeping(self, keep_from: int, inputs: list, acts: dict, *args, **kw):
         """``forward_hidden`` that keeps the layers' inputs, and the activations of the layers from ``keep_from`` on. Where memory runs out for

@@ -185,6 +185,12 @@ class TrainActor:
         else:
             self.model = build_model(self.cfg, store, "b200" if want_b200 else "torch", ep=self.ep_dispatcher, tp=self.tp_exchange)
             self.is_torch = not want_b200
+        if hasattr(self.model, "recompute_layers"):
+            from ..models.b200_impl import recompute_policy
+
+            self.model.recompute_layers, self.model.recompute_logits = recompute_policy(args)
+            if (getattr(args, "log_probs_chunk_size", -1) or -1) > 0:
+                self.model.lm_chunk = int(args.log_probs_chunk_size)
         self.loss_cfg = LossConfig.from_args(args)
         self.loss_cfg.args = args  # plug-ins (custom TIS / reducer functions) read their own options from the command line
         if getattr(args, "custom_tis_function_path", None):

@@ -97,7 +97,7 @@ TRAINER_FLAGS = [
     ("--num-layers-at-start-in-bf16", "i", 0, {}), ("--num-layers-at-end-in-bf16", "i", 0, {}),
     ("--reuse-grad-buf-for-mxfp8-param-ag", "b", False, {}),
     # memory / recompute
-    ("--recompute-granularity", "s", "full", {"choices": ["full", "selective", "none"]}),
+    ("--recompute-granularity", "s", None, {"choices": ["full", "selective", "none"]}),
     ("--recompute-method", "s", "uniform", {}), ("--recompute-num-layers", "i", 1, {}),
     # checkpoint / misc
     ("--ckpt-format", "s", "torch_dist", {"choices": ["torch_dist", "torch"]}),

@@ -74,7 +74,7 @@ IGNORED = {
     "dashboard_flush_interval": "dashboard events are appended to their files as they happen: there is no buffer to flush",
     "mtp_num_layers": "the multi-token-prediction layer is not built: the model trains and serves without it (training it, --enable-mtp-training, is rejected)",
     # sharded backend: activations are recomputed per layer; checkpoints stage through host copies per unit
-    "gradient_checkpointing": "layers are recomputed from their inputs as far as their activations do not fit beside the rest",
+    "gradient_checkpointing": "layer inputs are the only activations that passes over a sharded store keep: every layer is recomputed in the backward",
     "fsdp_state_dict_cpu_offload": "checkpoint and export copies are always staged in host memory, unit by unit",
     # Megatron / TransformerEngine kernel and fusion switches: one fused sm_100a path exists here
     "attention_backend": "one attention implementation (tcgen05 flash attention)",
@@ -91,10 +91,6 @@ IGNORED = {
     "disable_bias_linear": "projections have no bias unless the model config says so",
     "group_query_attention": "derived from the head counts",
     "use_rotary_position_embeddings": "rotary embedding is the only position embedding",
-    "recompute_granularity": "layers are recomputed from their inputs as far as their activations do not fit beside the rest",
-    "recompute_method": "layers are recomputed from their inputs as far as their activations do not fit beside the rest",
-    "recompute_num_layers": "layers are recomputed from their inputs as far as their activations do not fit beside the rest",
-    "recompute_loss_function": "the LM head runs in row chunks and recomputes its logits in the backward unless they fit beside the rest",
     "overlap_grad_reduce": "the partitioned optimizer reduces inside its own kernels",
     "overlap_param_gather": "the partitioned optimizer pushes parameters inside its own kernels",
     "overlap_cpu_optimizer_d2h_h2d": "host-resident optimizer state is always streamed on side streams",

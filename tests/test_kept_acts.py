@@ -30,7 +30,7 @@ def test_what_is_kept_leaves_room_for_the_pass(monkeypatch, name, tokens, free_g
     model = B200Qwen3.__new__(B200Qwen3)
     head = types.SimpleNamespace(shape=(cfg.vocab_size, cfg.hidden_size))
     model.__dict__.update(cfg=cfg, store=types.SimpleNamespace(layer_range=(0, cfg.num_layers), lm_head=lambda: head), ep=None, tp=None, cp_ctx=None,
-                          act_room=None, dev="cuda")
+                          act_room=None, dev="cuda", recompute_layers=0, recompute_logits=False)
     free, total, cached = int(free_gb * 1e9), int(192e9), int(5e9)
     monkeypatch.setattr(torch.cuda, "mem_get_info", lambda dev: (free - cached, total))
     monkeypatch.setattr(torch.cuda, "memory_reserved", lambda dev: total - free + cached)
@@ -47,6 +47,31 @@ def test_what_is_kept_leaves_room_for_the_pass(monkeypatch, name, tokens, free_g
     if tokens <= 16384 and name == "qwen3-8B":  # (and room that is there is used)
         assert kept > 0
         assert keep_from == 0 or kept + layer > free - total // 7
+
+
+# layers 3 .. 9 of 24, logits and activations that all fit: what the command line asks to recompute is recomputed
+@pytest.mark.parametrize("flags, want", [([], (True, 3)), (["--recompute-granularity", "full"], (True, 10)),
+                                         (["--recompute-granularity", "full", "--recompute-loss-function"], (False, 10)),
+                                         (["--recompute-loss-function"], (False, 3)), (["--recompute-granularity", "selective"], (True, 3)),
+                                         (["--recompute-granularity", "none"], (True, 3)),
+                                         (["--recompute-granularity", "full", "--recompute-method", "uniform", "--recompute-num-layers", "2"], (True, 10)),
+                                         (["--recompute-granularity", "full", "--recompute-method", "block", "--recompute-num-layers", "4"], (True, 7)),
+                                         (["--recompute-granularity", "full", "--recompute-method", "block", "--recompute-num-layers", "40"], (True, 10))])
+def test_recomputation_that_is_asked_for(flags, want):
+    import types
+
+    from miles_b200.models import get_config
+    from miles_b200.models.b200_impl import B200Qwen3, recompute_policy
+    from miles_b200.utils.arguments import parse_args
+
+    args = parse_args(["--num-rollout", "1", "--rollout-batch-size", "2", "--n-samples-per-prompt", "2", "--model-preset", "qwen3-tiny"] + flags)
+    cfg = get_config("qwen3-0.6B")
+    model = B200Qwen3.__new__(B200Qwen3)
+    head = types.SimpleNamespace(shape=(cfg.vocab_size, cfg.hidden_size))
+    model.__dict__.update(cfg=cfg, store=types.SimpleNamespace(layer_range=(3, 10), lm_head=lambda: head), ep=None, tp=None, cp_ctx=None,
+                          act_room=1 << 50, dev="cuda")
+    model.recompute_layers, model.recompute_logits = recompute_policy(args)
+    assert model._plan_acts(1000, 500, 2048) == want
 
 
 @pytest.mark.gpu
