@@ -16,6 +16,9 @@ import contextlib
 import torch
 
 
+SLACK = 256 << 20  # for what else is mapped meanwhile
+
+
 class MemorySaver:
     _instance = None
 
@@ -58,7 +61,13 @@ class MemorySaver:
         return int(self.C.vmm_pause(tag, keep_contents)) if self.available else 0
 
     def resume(self, tag: str) -> int:
-        return int(self.C.vmm_resume(tag)) if self.available else 0
+        """Maps the tag's memory again; returns the number of bytes mapped. PyTorch's allocator gives back what it has cached where that much is
+        not free: a training pass in between holds on to activations as far as there is room, and what was paused counted as room."""
+        if not self.available:
+            return 0
+        if self.stats().get(tag, (0, 0))[1] + SLACK > torch.cuda.mem_get_info()[0]:
+            torch.cuda.empty_cache()
+        return int(self.C.vmm_resume(tag))
 
     def stats(self) -> dict:
         return dict(self.C.vmm_stats()) if self.available else {}
