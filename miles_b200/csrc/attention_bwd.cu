@@ -595,6 +595,14 @@ int flash_attn_bwd(const void* q, long long q_ld, const void* k, long long k_ld,
   float* dq_acc = scratch;
   float* dsum = scratch + T * Hq * HD;
   float* lse2 = dsum + T * Hq;
+  // the operands' alignment is checked here, before anything reads them
+  CUtensorMap mq, mdo, mk, mv, mdq;
+  if (make_map(&mq, q, T, static_cast<long long>(Hq) * HD, q_ld, BQ)) return -1;
+  if (make_map(&mdo, d_o, T, static_cast<long long>(Hq) * HD, do_ld, BQ)) return -1;
+  if (make_map(&mk, k, T, static_cast<long long>(Hk) * HD, k_ld, BK)) return -1;
+  if (make_map(&mv, v, T, static_cast<long long>(Hk) * HD, v_ld, BK)) return -1;
+  if (make_dq_map(&mdq, dq_acc, T, Hq)) return -1;
+  if ((reinterpret_cast<uintptr_t>(o) & 15) != 0) return fail("attention operand base must be 16-byte aligned");
   cudaError_t e = cudaMemsetAsync(dq_acc, 0, sizeof(float) * T * Hq * HD, stream);
   if (e != cudaSuccess) return fail("cudaMemsetAsync failed for the dQ accumulator");
   {
@@ -602,12 +610,6 @@ int flash_attn_bwd(const void* q, long long q_ld, const void* k, long long k_ld,
     fa_bwd_prep_kernel<<<static_cast<unsigned>(blocks_n), 256, 0, stream>>>(
         static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(d_o), lse, dsum, lse2, T, Hq);
   }
-  CUtensorMap mq, mdo, mk, mv, mdq;
-  if (make_map(&mq, q, T, static_cast<long long>(Hq) * HD, q_ld, BQ)) return -1;
-  if (make_map(&mdo, d_o, T, static_cast<long long>(Hq) * HD, do_ld, BQ)) return -1;
-  if (make_map(&mk, k, T, static_cast<long long>(Hk) * HD, k_ld, BK)) return -1;
-  if (make_map(&mv, v, T, static_cast<long long>(Hk) * HD, v_ld, BK)) return -1;
-  if (make_dq_map(&mdq, dq_acc, T, Hq)) return -1;
   auto kernel = split > 1 ? fa_bwd_kernel<true> : fa_bwd_kernel<false>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_SMEM) != cudaSuccess)
     return fail("cudaFuncSetAttribute(MaxDynamicSharedMemorySize) failed for the attention backward");

@@ -91,3 +91,20 @@ def test_heads_shared_by_a_cluster(lens, Hq, Hk, split):
     for n in lens:
         _check(q, k, v, do, o, grads, a, a + n)
         a += n
+
+
+@pytest.mark.parametrize("which", ["q", "k", "v", "d_o"])
+def test_misaligned_operands_are_refused_before_anything_reads_them(which):
+    """Nothing is launched: the refusal comes from the host, and what follows on the stream runs."""
+    from miles_b200.ops import _ext
+    from miles_b200.ops.attention import build_bwd_blocks, build_tiles
+
+    C = _ext.load(required=True)
+    t = dict(zip(("q", "k", "v", "d_o"), _inputs(100, 4, 2)))
+    o, lse = C.flash_attn_fwd(t["q"], t["k"], t["v"], build_tiles([100]).cuda(), SCALE, None)
+    off = torch.empty(t[which].numel() + 8, dtype=torch.bfloat16, device="cuda")[4:-4].view(t[which].shape)
+    assert off.data_ptr() % 16 == 8 and off.is_contiguous()
+    t[which] = off.copy_(t[which])
+    with pytest.raises(RuntimeError, match="16-byte aligned"):
+        C.flash_attn_bwd(t["q"], t["k"], t["v"], o, t["d_o"], lse, build_bwd_blocks([100]).cuda(), SCALE, None)
+    torch.cuda.synchronize()

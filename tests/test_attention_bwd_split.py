@@ -16,3 +16,14 @@ def test_split(lens, Hq, Hk, split):
     tiles = [-(-(n - c) // 64) for c, n in blocks]
     assert cache._bwd_work == (len(blocks), max(tiles), sum(tiles)) and cache.get_bwd(cu).shape[0] == len(blocks)
     assert cache.get_bwd_split(torch.zeros(1, dtype=torch.int32), Hq, Hk) in (1, 2, 4)  # (a pack without sequences)
+
+
+def test_operands_are_checked_before_the_first_launch():
+    """From the source: maps, which check the alignment, come before the memset and the kernel that reads 16 bytes at a time."""
+    from pathlib import Path
+
+    import miles_b200
+
+    text = (Path(miles_b200.__file__).resolve().parent / "csrc" / "attention_bwd.cu").read_text()
+    body = text[text.index("int flash_attn_bwd("):]
+    assert body.rindex("make_map(") < body.index("cudaMemsetAsync(") < body.index("<<<")
