@@ -638,7 +638,11 @@ int flash_attn_bwd(const void* q, long long q_ld, const void* k, long long k_ld,
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, kernel, mq, mdo, mk, mv, mdq, a) != cudaSuccess) return fail("attention backward launch failed");
+  e = cudaLaunchKernelEx(&cfg, kernel, mq, mdo, mk, mv, mdq, a);
+  if (e != cudaSuccess) {
+    cudaGetLastError();  // (reported here)
+    return fail(std::string("attention backward launch failed: ") + cudaGetErrorString(e));
+  }
   const long long n4 = T * Hq * HD / 4;
   long long cb = (n4 + 255) / 256;
   if (cb > SMS * 8) cb = SMS * 8;

@@ -753,7 +753,11 @@ int flash_attn_fwd(const void* q, long long q_ld, const void* k, long long k_ld,
     return fa_fail("cudaFuncSetAttribute(MaxDynamicSharedMemorySize) failed for attention");
   const long long blocks = paired ? static_cast<long long>(num_tiles) * (Hq / 2) : static_cast<long long>(num_tiles) * Hq;
   const int grid = static_cast<int>(paired && blocks > sms ? sms : blocks);
-  if (pdl_launch(kern, grid, paired ? FP_THREADS : FA_THREADS, smem, stream, mq, mk, mv, a) != cudaSuccess) return fa_fail("attention forward launch failed");
+  const cudaError_t e = pdl_launch(kern, grid, paired ? FP_THREADS : FA_THREADS, smem, stream, mq, mk, mv, a);
+  if (e != cudaSuccess) {
+    cudaGetLastError();  // (reported here)
+    return fa_fail(std::string("attention forward launch failed: ") + cudaGetErrorString(e));
+  }
   return 0;
 }
 
