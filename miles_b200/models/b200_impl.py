@@ -38,6 +38,16 @@ class MoeCtx:
     num_tiles: torch.Tensor
     max_rows: int
     align: int = 1
+    pairs: int = 0  # routed pairs to expect among max_rows (0: as many)
+
+    def gated(self) -> bool:
+        """Whether the gate-up product of these rows takes SwiGLU into its epilogue (csrc/gemm.cu). Experts of few rows stream their weights, which
+        the plain product does faster, by more than the activation costs; where every expert's rows are padded to whole tiles the activation
+        works through the padding, too, and nothing is lost. us, plain product and activation / gated, 128 experts of 768 x 2048: 16 tokens
+        111 / 118, 200 153 / 159, 777 (49 pairs an expert) 159 / 162, 1500 171 / 168, 4000 255 / 226; 128 of 1536 x 4096: 200 tokens 513 / 517, 400
+        (25 pairs) 525 / 523, 1000 548 / 534; padded to 64 rows, gate and up kept: 16 tokens 124 / 125, 200 171 / 170, 777 169 / 170, 1500
+        183 / 178, 4000 267 / 249."""
+        return self.align > 1 or (self.pairs or self.max_rows) >= 48 * (self.offsets.numel() - 1)
 
 
 class LayerActs(NamedTuple):
@@ -287,9 +297,7 @@ class B200Qwen3:
         max_rows = max(T * K + E_local * (align - 1), 1)
         counts, offsets, dest, src, tg, nt = self.C.moe_build_permutation(ids, E_local, max_rows, align)
         self.launches += self.C.moe_permutation_launches(T, K, max_rows, E_local)
-        ctx = MoeCtx(ids, None, None, offsets, dest, src, tg, nt, max_rows)
-        ctx.align = align
-        return ctx
+        return MoeCtx(ids, None, None, offsets, dest, src, tg, nt, max_rows, align, T * K)
 
     def _experts_fwd(self, xp, plan: MoeCtx, w1, w2, keep: bool, scatter=None):
         """``scatter = (row_ptrs, ctrl, flag_ptrs, rank)``: the second GEMM stores every output row at its own
@@ -304,14 +312,12 @@ class B200Qwen3:
             yp = self._mx_linear(act, mx[w2.data_ptr()], plan.tile_group, plan.num_tiles, w2.shape[1])
             self.launches += 1
             return None, None, yp
-        gated = plan.max_rows >= 48 * w1.shape[0]
+        gated = plan.gated()
         gu = torch.empty(plan.max_rows, I2, dtype=torch.bfloat16, device=xp.device) if keep or not gated else None
         if gated:
             act = torch.empty(plan.max_rows, I2 // 2, dtype=torch.bfloat16, device=xp.device)
             C.gated_gemm(xp, w1, act, gu, plan.tile_group, plan.num_tiles, self.status)
         else:
-            # experts of few rows stream their weights, and the plain product does so faster, by more than the activation costs
-            # (us, 128 experts of 768 x 2048: 16 tokens 87.5 and 95.4 gated, 200 tokens 137 and 142, 1000 150 and 148, 4000 264 and 232)
             C.grouped_gemm_rows(xp, w1, gu, plan.tile_group, plan.num_tiles, False, False, 0, self.status)
             act = C.swiglu_fwd(gu)
             self.launches += 1

@@ -99,7 +99,7 @@ class EpDecodeLL:
             self.region.base, self.layout, self.rank, self.E, self.rows, 1, self.ctrl, self.wait_ns, self.status)
         from ..models.b200_impl import MoeCtx
 
-        plan = MoeCtx(None, None, None, offsets, dest, row_src, tiles, totals, row_src.numel())
+        plan = MoeCtx(None, None, None, offsets, dest, row_src, tiles, totals, row_src.numel(), pairs=T * self.K)
         xp = C.moe_permute(self.xg, row_src, totals, self.K)
         _, _, yp = model._experts_fwd(xp, plan, P[p + "moe.w1"], P[p + "moe.w2"], keep=False)
         C.ep_ll_return(yp, dest, src_rows, self.bases, self.layout, self.rank, self.rows, self.ctrl)

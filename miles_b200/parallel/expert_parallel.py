@@ -116,6 +116,7 @@ class ExpertParallel:
         ids_flat = ids.reshape(-1)
         self._send(h2, ids_flat, route, K)
         plan = self._recv_plan(model, 64 if keep else 1)
+        plan.pairs = n_entries  # (as many come as go, on average; the plan has room for the worst case)
         xp = C.moe_permute(self.xrecv, plan.src, plan.num_tiles, 1)
         if self.fused_epilogue:
             gu, act, _ = model._experts_fwd(xp, plan, P[p + "w1"], P[p + "w2"], keep, scatter=self._scatter_args(plan))
