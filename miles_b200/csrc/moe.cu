@@ -431,9 +431,27 @@ assign_kernel(const int* __restrict__ ids, int n, int E, const int* __restrict__
   }
 }
 
+// Permuted rows are written by one kernel and read by the next. Up to half of L2 (126 MB) they are still there when they are read; beyond
+// that they only push out what is (weights, the rows of the tokens), and go first (PASSING). us with / without, 8 choices of 128 experts,
+// 2048 columns: 16384 tokens (537 MB) permute 164 / 169, combine 135 / 148; 8192 tokens (268 MB) 67 / 73 and 66 / 75; at 2048 and 777 tokens
+// (67 and 58 MB), alone or with the products behind, the two differ by less than their runs do. 24 decode steps of 16 rows (0.5 MB)
+// 85.2 / 84.1 ms, in another run 86.4 / 86.1.
+constexpr long long PASSING_BYTES = 64ll << 20;
+template <bool PASSING>
+__device__ __forceinline__ void put_row(uint4* p, const uint4& v) {
+  if constexpr (PASSING) __stcs(p, v);
+  else *p = v;
+}
+template <bool PASSING>
+__device__ __forceinline__ uint4 take_row(const uint4* p) {
+  if constexpr (PASSING) return __ldcs(p);
+  else return *p;
+}
+
 // x_perm[row] = x[row_src[row] / K] or zeros for padding rows. One warp per row, four 16-byte loads of it in flight per lane
 // (131072 rows of 2048: 158 us when every thread placed its own 16 bytes after a 64-bit division, 148 us now; the copy alone
 // is 604 MB).
+template <bool PASSING>
 __global__ void permute_kernel(const bf16* __restrict__ x, const int* __restrict__ row_src,
                                const int* __restrict__ num_m_tiles, bf16* __restrict__ x_perm, int max_rows, int H,
                                int K) {
@@ -451,7 +469,7 @@ __global__ void permute_kernel(const bf16* __restrict__ x, const int* __restrict
       for (int u = 0; u < 4; ++u) v[u] = (src >= 0 && c0 + 32 * u < vec_per_row) ? from[c0 + 32 * u] : make_uint4(0, 0, 0, 0);
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-        if (c0 + 32 * u < vec_per_row) __stcs(to + c0 + 32 * u, v[u]);
+        if (c0 + 32 * u < vec_per_row) put_row<PASSING>(to + c0 + 32 * u, v[u]);
     }
   }
 }
@@ -479,6 +497,7 @@ __device__ __forceinline__ uint4 pack8(const float (&a)[8]) {
 // 16-byte columns of one token after another; the rows of up to eight choices are asked for together and added in order
 // (16384 tokens, 8 choices, 2048 columns: 185 us with one load in flight per thread, 128 us with eight; 671 MB move).
 constexpr int COMBINE_THREADS = 128;
+template <bool PASSING>
 __global__ void __launch_bounds__(COMBINE_THREADS)
 combine_kernel(const bf16* __restrict__ y_perm, const int* __restrict__ dest_row, const float* __restrict__ topk_w,
                const bf16* __restrict__ residual, bf16* __restrict__ out, int T, int K, int H) {
@@ -502,7 +521,7 @@ combine_kernel(const bf16* __restrict__ y_perm, const int* __restrict__ dest_row
       }
 #pragma unroll
       for (int k = 0; k < 8; ++k)
-        if (row[k] >= 0) v[k] = __ldcs(reinterpret_cast<const uint4*>(y_perm + static_cast<long long>(row[k]) * H) + c);
+        if (row[k] >= 0) v[k] = take_row<PASSING>(reinterpret_cast<const uint4*>(y_perm + static_cast<long long>(row[k]) * H) + c);
 #pragma unroll
       for (int k = 0; k < 8; ++k)
         if (row[k] >= 0) acc8(v[k], w[k], a);
@@ -512,6 +531,7 @@ combine_kernel(const bf16* __restrict__ y_perm, const int* __restrict__ dest_row
 }
 
 // One warp per permuted row: dy_perm[row] = w * dout[token]; dw[entry] = <dout[token], y_perm[row]>.
+template <bool PASSING>
 __global__ void combine_bwd_kernel(const bf16* __restrict__ dout, const bf16* __restrict__ y_perm,
                                    const int* __restrict__ row_src, const int* __restrict__ num_m_tiles,
                                    const float* __restrict__ topk_w, bf16* __restrict__ dy_perm,
@@ -538,7 +558,7 @@ __global__ void combine_bwd_kernel(const bf16* __restrict__ dout, const bf16* __
         gr[u] = yr[u] = make_uint4(0, 0, 0, 0);
         if (c0 + 32 * u < vec_per_row) {
           gr[u] = g[c0 + 32 * u];
-          if (dtopk_w) yr[u] = __ldcs(y + c0 + 32 * u);
+          if (dtopk_w) yr[u] = take_row<PASSING>(y + c0 + 32 * u);
         }
       }
 #pragma unroll
@@ -546,7 +566,7 @@ __global__ void combine_bwd_kernel(const bf16* __restrict__ dout, const bf16* __
         if (c0 + 32 * u >= vec_per_row) break;
         float a[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         acc8(gr[u], w, a);
-        __stcs(dst + c0 + 32 * u, pack8(a));
+        put_row<PASSING>(dst + c0 + 32 * u, pack8(a));
         if (dtopk_w) {
           const __nv_bfloat162* gb = reinterpret_cast<const __nv_bfloat162*>(&gr[u]);
           const __nv_bfloat162* yb = reinterpret_cast<const __nv_bfloat162*>(&yr[u]);
@@ -564,6 +584,8 @@ __global__ void combine_bwd_kernel(const bf16* __restrict__ dout, const bf16* __
     }
   }
 }
+
+bool passing(long long rows, int H) { return rows * H * 2 > PASSING_BYTES; }
 
 int grid_for(long long items, int threads, int cap = 148 * 8) {
   long long b = (items + threads - 1) / threads;
@@ -644,7 +666,7 @@ cudaError_t moe_build_permutation(const int* topk_ids, int T, int K, int E, int 
 void moe_permute(const void* x, const int* row_src, const int* num_m_tiles, void* x_perm, int max_rows, int H, int K,
                  cudaStream_t s) {
   if (max_rows <= 0) return;
-  pdl_launch(permute_kernel, grid_for(max_rows, 8), 256, 0, s, static_cast<const bf16*>(x), row_src, num_m_tiles,
+  pdl_launch(passing(max_rows, H) ? permute_kernel<true> : permute_kernel<false>, grid_for(max_rows, 8), 256, 0, s, static_cast<const bf16*>(x), row_src, num_m_tiles,
                                                        static_cast<bf16*>(x_perm), max_rows, H, K);
 }
 
@@ -652,7 +674,7 @@ void moe_combine(const void* y_perm, const int* dest_row, const float* topk_w, c
                  int K, int H, cudaStream_t s) {
   if (T <= 0) return;
   const dim3 grid(T, (H / 8 + COMBINE_THREADS - 1) / COMBINE_THREADS);
-  pdl_launch(combine_kernel, grid, COMBINE_THREADS, 0, s, static_cast<const bf16*>(y_perm), dest_row, topk_w,
+  pdl_launch(passing(static_cast<long long>(T) * K, H) ? combine_kernel<true> : combine_kernel<false>, grid, COMBINE_THREADS, 0, s, static_cast<const bf16*>(y_perm), dest_row, topk_w,
                                                   static_cast<const bf16*>(residual), static_cast<bf16*>(out), T, K, H);
 }
 
@@ -664,7 +686,8 @@ void moe_combine_bwd(const void* dout, const void* y_perm, const int* row_src, c
                      const float* topk_w, void* dy_perm, float* dtopk_w, int max_rows, int K, int H, cudaStream_t s) {
   if (max_rows <= 0) return;
   const int wpb = 8;
-  combine_bwd_kernel<<<grid_for(max_rows, wpb), wpb * 32, 0, s>>>(
+  const auto kernel = passing(max_rows, H) ? combine_bwd_kernel<true> : combine_bwd_kernel<false>;
+  kernel<<<grid_for(max_rows, wpb), wpb * 32, 0, s>>>(
       static_cast<const bf16*>(dout), static_cast<const bf16*>(y_perm), row_src, num_m_tiles, topk_w,
       static_cast<bf16*>(dy_perm), dtopk_w, max_rows, K, H);
 }
