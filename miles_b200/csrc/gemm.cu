@@ -1191,16 +1191,20 @@ int gemm_bf16_launch(const GemmProblem& p, cudaStream_t stream) {
   if (p.score_part) return pair ? launch<256, false, false, 2, EPI_SCORES>(p, ka, stream) : launch<256, false, false, 1, EPI_SCORES>(p, ka, stream);
   // Weight gradients add to whole pieces of 128 bytes (what ends within one stays with the staged epilogue, whose ragged columns find
   // their lines in L1: 1000 x 1048, K = 333, 9.5 and 12.4 us). One CTA's 256-wide tiles take the adding epilogue's second buffer from
-  // their stages, which long contractions miss; by rows per group, us staged / two buffers and three stages / one and four, 128 experts
-  // of 1536 x 2048: 112 rows 459 / 281 / 381, 319 428 / 340 / 391, 575 527 / 497 / 465, 813 630 / 641 / 622, 1087 757 / 811 / 767;
-  // dense in fp32: 8192 x 2048, K = 60, 23.0 / 21.1 / 25.5, 2048 x 4096, K = 333, 16.5 / 15.5 / 16.7, 2048 x 2048, K = 777, 12.5 / 12.5 / 13.3,
-  // 128 x 2048, K = 16384, 92 / 106 / 93.
+  // their stages, which long contractions miss. us staged / two buffers and three stages / one and four, by rows per group:
+  //   128 of 1536 x 2048   128 455 / 293 / 387, 384 455 / 387 / 418, 448 486 / 450 / 445, 704 636 / 648 / 597, 1024 808 / 871 / 816
+  //   64 of 2048 x 1408    256 310 / 179 / 222, 448 282 / 218 / 226, 576 280 / 253 / 245, 832 323 / 339 / 317, 1536 665 / 706 / 675
+  //   16 of 8192 x 4096    256 605 / 433 / 551, 448 677 / 601 / 615, 704 951 / 945 / 878, 1024 1136 / 1222 / 1121, 1536 1508 / 1662 / 1555
+  // so the lines lie within 4 % of the best everywhere. Dense in fp32, by K:
+  //   8192 x 2048          64 41 / 33 / 41, 333 43 / 35 / 43, 777 47 / 45 / 47, 960 47 / 49 / 49, 2048 70 / 78 / 72
+  //   4096 x 12288         64 111 / 76 / 96, 333 113 / 80 / 102, 777 115 / 115 / 111, 960 117 / 127 / 113, 1536 150 / 170 / 150
+  //   2560 x 2560          64 25 / 20 / 25, 777 29 / 27 / 29, 1088 31 / 31 / 31, 2048 41 / 43 / 41
   if (p.accumulate && amn && bmn && ka.vec_ok && p.N % (p.out_fp32 ? 32 : 64) == 0) {
     if (pair) return launch<256, true, true, 2, EPI_ADD, 1>(p, ka, stream);
     if (bn == 128) return launch<128, true, true, 1, EPI_ADD>(p, ka, stream);
     const bool grouped = p.mode == GEMM_GROUPED_CONTR;
     const long long k = grouped ? p.a.rows / (p.num_groups > 0 ? p.num_groups : 1) : p.K;
-    if (k < (grouped ? 448 : 1024)) return launch<256, true, true, 1, EPI_ADD, 1>(p, ka, stream);
+    if (k < (grouped ? 448 : 800)) return launch<256, true, true, 1, EPI_ADD, 1>(p, ka, stream);
     if (grouped && k < 800) return launch<256, true, true, 1, EPI_ADD>(p, ka, stream);
   }
   if (pair) {

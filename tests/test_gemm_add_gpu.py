@@ -22,7 +22,7 @@ def _old(shape, dtype):
 # a lone row, rows that end inside a warp's, one piece of columns, several tiles a CTA; contractions that end inside a block of 64, of
 # one block, and too long for the small variants; pairs; columns that end inside a piece
 @pytest.mark.parametrize("M, N, K, bn, pair", [(8, 64, 8, 0, 0), (152, 192, 200, 128, 1), (1000, 128, 60, 128, 1), (4104, 4096, 72, 128, 1),
-                                               (72, 320, 64, 256, 1), (5000, 2048, 333, 256, 1), (3000, 2048, 1100, 256, 1),
+                                               (72, 320, 64, 256, 1), (5000, 2048, 333, 256, 1), (3000, 2048, 790, 256, 1), (3000, 2048, 810, 256, 1), (3000, 2048, 1100, 256, 1),
                                                (1000, 1088, 640, 256, 2), (6016, 2048, 100, 256, 2), (200, 200, 96, 0, 0)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_adds_to_what_is_there(M, N, K, bn, pair, dtype):
