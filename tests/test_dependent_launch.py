@@ -11,6 +11,7 @@ import miles_b200
 
 CSRC = Path(miles_b200.__file__).resolve().parent / "csrc"
 LET_IN = ("pdl_enter()", "pdl_let_dependents_in()")
+ALLOC = re.compile(r"\btmem_alloc\w*\(")  # by one CTA, or by a pair
 
 
 def _kernels(path):
@@ -32,13 +33,16 @@ def _kernels(path):
 def test_tensor_memory_is_allocated_before_dependents_are_let_in(path):
     for name, body in _kernels(path):
         lets = [body.index(w) for w in LET_IN if w in body]
-        if lets and "tmem_alloc(" in body:
-            assert body.rindex("tmem_alloc(") < min(lets), f"{path.name}: {name}"
+        allocs = [m.start() for m in ALLOC.finditer(body)]
+        if lets and allocs:
+            assert max(allocs) < min(lets), f"{path.name}: {name}"
 
 
 def test_the_search_sees_the_kernels_it_is_about():
-    both = {name for path in CSRC.glob("*.cu") for name, body in _kernels(path) if "tmem_alloc(" in body and any(w in body for w in LET_IN)}
-    assert {"fa_fwd_kernel", "gemm_bf16_kernel", "gemm_skinny_kernel"} <= both
+    both = {name: {body[m.start():m.end() - 1] for m in ALLOC.finditer(body)} for path in CSRC.glob("*.cu") for name, body in _kernels(path)
+            if any(w in body for w in LET_IN)}
+    assert {"fa_fwd_kernel", "fa_fwd_pair_kernel", "gemm_bf16_kernel", "gemm_skinny_kernel"} <= {name for name, allocs in both.items() if allocs}
+    assert both["gemm_bf16_kernel"] == {"tmem_alloc", "tmem_alloc_pair"}
 
 
 def _chain(ext, b, src, after):
