@@ -69,11 +69,11 @@ void moe_router_bwd(const float* probs, const int* topk_ids, const float* topk_w
 // logprob of `target`, entropy, and (kept for the backward) row max and log-sum-exp.
 void logprob_entropy_fwd(const void* logits, bool fp32, const int* targets, float* logprob, float* entropy, float* lse,
                          float* psum_x, int T, int V, long long ld, float inv_temp, cudaStream_t s);
-// dlogits = inv_temp * ( dlp * (onehot - p) - dH * p * (x - sum p x) ), written as bf16 with row pitch ld_out
-// (in place is allowed for bf16 logits).
 // part [ceil(V / 128)][T] of four floats and row_target [T]: what the scores epilogue of gemm.cu leaves
 void logprob_entropy_merge(const float* part, const float* row_target, const int* targets, float* logprob, float* entropy, float* lse, float* psum_x,
                            int T, int V, cudaStream_t s);
+// dlogits = inv_temp * ( dlp * (onehot - p) - dH * p * (x - sum p x) ), written as bf16 with row pitch ld_out
+// (in place is allowed for bf16 logits).
 void logprob_entropy_bwd(const void* logits, bool fp32, const int* targets, const float* lse, const float* psum_x,
                          const float* dlogprob, const float* dentropy, void* dlogits, int T, int V, long long ld,
                          long long ld_out, float inv_temp, cudaStream_t s);
