@@ -31,7 +31,7 @@
 //
 // Measured with the kernels around it, 32 heads, before (sums into dQ by `red.global.add.f32`, 64 instructions a thread and tile,
 // which the read-out warps could not issue faster than one in some 80 clocks; a warp issuing the products) -> now: 9216 tokens in one
-// sequence, 8 KV heads, 3.07 -> 2.10 ms (567 -> 828 TFLOP/s); 16384 in six sequences, 4 KV heads, 1.89 -> 1.38 (485 -> 664); with the
+// sequence, 8 KV heads, 3.07 -> 2.10 ms (567 -> 828 TFLOP/s); 16384 in six sequences, 4 KV heads, 1.89 -> 1.41 (485 -> 649); with the
 // read-out waiting for its own copies 2.28 and 1.48. A tile takes some 3300 clocks, its products 1664.
 //
 // Reference counterpart: the flash-attention backward behind `--attention-backend flash`
