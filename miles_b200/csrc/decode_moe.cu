@@ -417,6 +417,7 @@ __global__ void __maxnreg__(MAX_REGS) moe_down_kernel(const DownArgs a) {
     w_s[i] = 0.f;
     reinterpret_cast<uint4*>(y_s)[2 * i] = reinterpret_cast<uint4*>(y_s)[2 * i + 1] = make_uint4(0u, 0u, 0u, 0u);
   }
+  __syncwarp();
   cluster_sync();  // (the other CTA runs before one stores into its shared memory; the predecessor is still busy)
   pdl_enter();
   const int rank = blockIdx.x, ranks = gridDim.x;  // (the cluster spans the grid's first dimension)
